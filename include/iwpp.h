@@ -61,7 +61,7 @@ typedef enum iwpp_queue_variant {
  * (iwpp_autotune). */
 typedef struct iwpp_config {
     int tile_rows;             /* 32 or 64 rows per tile; 0 = default: 64, or 32 when the
-                                  job has fewer than 2.5 64-row tiles per resident warp
+                                  job has at most one 64-row tile per multiprocessor
                                   (mutex queue: always 64) */
     long long queue_capacity;  /* entries per queue buffer; 0 = default; < 0: that multiple
                                   of the job's tile count */
@@ -73,10 +73,10 @@ typedef struct iwpp_config {
     int clip_marker;           /* 1: marker = min(marker, mask) before reconstructing */
     int plain_loads;           /* 1: never use TMA box loads (else TMA whenever base and
                                   pitch are 16-byte aligned) */
-    int solver;                /* in-tile solver: 0 = automatic, 1 = row sweeps (fewest
-                                  instructions), 2 = vertical / horizontal passes
-                                  (shortest latency), 3 = revisits by a per-tile pixel
-                                  queue in shared memory (first visits by passes) */
+    int solver;                /* in-tile solver: 0 = default, the vertical / horizontal
+                                  passes (2, several warps per tile), 1 = row sweeps (one
+                                  warp per tile), 3 = revisits by a per-tile pixel queue in
+                                  shared memory (first visits by row sweeps) */
     int front_passes;          /* the front stage: the pixels at the mask's largest value
                                   raised by connected-component labelling, init_passes
                                   whole-image passes (default 2), and the tile engine started

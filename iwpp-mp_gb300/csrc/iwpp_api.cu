@@ -151,32 +151,15 @@ long long tiles_of(int w, int h, int dtype, int th) {
     return ((w + tw - 1) / tw) * (((long long)h + th - 1) / th);
 }
 
-// Warps the persistent grid keeps resident with 64-row tiles on a device
-// (queried once per device and variant; 0 when it cannot be queried).
-int resident_warps64(int variant, int device) {
-    static std::atomic<int> cache[64][4];
-    if (device < 0 || device >= 64 || variant < 0 || variant > 3) return 0;
-    int w = cache[device][variant].load(std::memory_order_relaxed);
-    if (w == 0) {
-        LaunchInfo li;
-        if (engine_prepare(variant, 64, device, &li) != cudaSuccess) return 0;
-        w = li.grid * kWarps;
-        cache[device][variant].store(w, std::memory_order_relaxed);
-    }
-    return w;
-}
-
 // Tile height for calls that leave it at its default: 64-row tiles (fewer
-// tile boundaries to cross, fewer revisits) for jobs with at least two and a
-// half of them per warp the grid keeps resident; below that the warps run
-// short of independent tiles whenever the front narrows, and 32-row tiles
-// (twice the tiles) finish sooner.  Measured on single h-dome images:
-// 2048^2-4096^2 uint8 and 4096^2 uint16 (0.3-2.2 tiles per warp) 5-25 %
-// faster with 32 rows; 6144^2 and 8192^2 uint8 (2.5-4.5 per warp), the
-// 64-image batch and 16384^2 images (18-20 per warp) faster with 64.
-// The mutex queue is bound by its one lock (every take and insert is a
-// critical section), so its cost grows with the tile count: 64 rows always
-// (4096^2 uint8: 26 ms with 2048 tiles, 45 ms with 4096).
+// tile boundaries to cross, fewer visits), or 32 for jobs with at most one
+// 64-row tile per SM, which would leave SMs without one.  Measured on h-dome
+// images, 32 rows by four warps / 64 rows by eight, us: 256^2 uint8 41 / 43
+// (8-connected 80 / 70), 512^2 8-connected 117 / 132, uint16 98 / 112, int32
+// 121 / 123, 1024^2 uint8 73 / 68 (120 / 122); above that 64 rows: 1536^2
+// uint8 77 / 66, 1024^2 uint16 124 / 106, 4096^2 uint8 191 / 144 (64 rows by
+// two warps).  The mutex queue is bound by its one lock (every take and insert
+// is a critical section), so its cost grows with the tile count: 64 rows always.
 int default_tile_rows(int variant, long long tiles64) {
     if (variant == IWPP_QUEUE_MUTEX) return 64;
     int device = -1;
@@ -184,8 +167,7 @@ int default_tile_rows(int variant, long long tiles64) {
         cudaGetLastError();
         return 64;
     }
-    const int resident = resident_warps64(variant, device);
-    return resident > 0 && 2ll * tiles64 < 5ll * resident ? 32 : 64;
+    return tiles64 <= engine_sm_count(device) ? 32 : 64;
 }
 
 long long job_tiles64(const iwpp_image* imgs, int n) {
@@ -613,6 +595,10 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     EngineArgs a{};
     a.imgs = reinterpret_cast<const ImgDesc*>(base + l.off_imgs);
     a.nimg = (int)job.descs.size();
+    if (a.nimg == 1) {
+        a.one = job.descs[0];
+        a.one.tmaps = job.has_tma[0] ? base + l.off_tmaps : nullptr;
+    }
     a.G = (unsigned)job.G;
     a.state = reinterpret_cast<unsigned*>(base + l.off_state);
     a.q0 = reinterpret_cast<unsigned*>(base + l.off_q0);
@@ -728,13 +714,12 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
         if (e != cudaSuccess) return cuda_status(e);
     }
     long long grid = 1;
+    LaunchInfo li{};
     if (job.G > 0) {
-        LaunchInfo li;
-        e = engine_prepare(job.variant, job.tile_rows, device, &li);
+        e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job.G, device, &li);
         if (e != cudaSuccess) return cuda_status(e);
         grid = li.grid;
-        const long long useful = (job.G + kWarps - 1) / kWarps;
-        if (grid > useful) grid = useful;
+        if (grid > job.G) grid = job.G;
         if (job.cfg.grid_ctas > 0 && job.cfg.grid_ctas < grid) grid = job.cfg.grid_ctas;
         if (grid < 1) grid = 1;
     }
@@ -743,7 +728,7 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     if (e != cudaSuccess) return cuda_status(e);
     ++nl;
     if (job.G > 0) {
-        e = engine_launch(a, job.variant, job.tile_rows, (int)grid, s);
+        e = engine_launch(a, job.variant, li, (int)grid, s);
         if (e != cudaSuccess) return cuda_status(e);
         ++nl;
     }
@@ -1066,7 +1051,7 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
         }
         // Warm the kernel attributes before capture.
         LaunchInfo li;
-        if (rc == IWPP_OK && job.G > 0) rc = cuda_status(engine_prepare(job.variant, job.tile_rows, h->device, &li));
+        if (rc == IWPP_OK && job.G > 0) rc = cuda_status(engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job.G, h->device, &li));
     }
     if (rc == IWPP_OK) {
         e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);

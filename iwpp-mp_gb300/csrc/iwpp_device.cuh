@@ -1,16 +1,15 @@
 // iwpp_device.cuh -- device building blocks of the GB300 reconstruction
-// engine: one-warp tile visits (TMA fetch with halo, raster / anti-raster
-// sweeps to local convergence, write-back, neighbour detection).
+// engine: tile visits by a CTA (TMA fetch with halo, vertical and horizontal
+// passes to local convergence, write-back, neighbour detection).
 //
 // Layout: a tile is TH rows x TW pixels with TW * sizeof(pixel) = 128 bytes
-// (TW = 128 uint8, 64 uint16, 32 int32).  One warp owns one tile at a time.
-// Shared memory holds the tile plus the halo rows above and below as dense
-// 128-byte rows (SMEM row r = image row y0 - 1 + r), so one TMA box load per
-// image plane fetches it.  Lane L owns the 32-bit word with pixels
-// [L*PPW, L*PPW + PPW) of every row (PPW = 4 / 2 / 1); during a row step it
-// unpacks them to one pixel per register so every min / max is a native
-// 32-bit instruction.  Vertical propagation runs row by row; horizontal
-// propagation is a warp scan over the max-min semiring.
+// (TW = 128 uint8, 64 uint16, 32 int32).  One CTA owns one tile at a time, a
+// warp each block of eight rows.  Shared memory holds the tile plus the halo
+// rows above and below as dense 128-byte rows (SMEM row r = image row
+// y0 - 1 + r), so one TMA box load per image plane fetches it.  A 32-bit word
+// holds PPW = 4 / 2 / 1 pixels.  Vertical propagation walks a block's rows
+// with a word column per lane; horizontal propagation is a lane's own chain
+// and a scan over eight lanes in the max-min semiring.
 //
 // Reference counterparts (IWPP MP/src/MorphologicalReconstruction.cu):
 //   tile fetch with a one-pixel halo        MR.cu:232-312
@@ -143,13 +142,25 @@ enum : unsigned {
 __device__ __constant__ static const int kNbDx[8] = {0, 0, -1, 1, -1, 1, -1, 1};
 __device__ __constant__ static const int kNbDy[8] = {-1, 1, 0, 0, -1, -1, 1, 1};
 
-// Per-warp shared memory (128-byte aligned; TMA writes tm / tk densely).
+// In-tile solvers of a visit (iwpp_config.solver): passes, row sweeps, or
+// revisits by the pixel queue.
+enum : int { SOLVE_PASSES = 0, SOLVE_SWEEPS = 1, SOLVE_PQ = 2 };
+
+// A CTA's counters.
+struct VisitCount {
+    unsigned visits, pushes;
+    unsigned sweeps;     // rounds of passes, or sweeps
+    unsigned row_steps;  // rows processed
+    long long cycles[5];  // queue read, fetch, processing, dump, queue write (the first warp's clock)
+};
+
+// A tile's shared memory (128-byte aligned; TMA writes tm / tk densely).
 // SMEM row r holds image row y0 - 1 + r: row 0 is the halo above the tile,
 // rows 1..TH the tile, row TH+1 the halo below.  hL* / hR* hold the left /
 // right halo column pixels of the same rows.
-constexpr int kPqCap = 448;  // pixel-queue solver: FIFO entries per warp
+constexpr int kPqCap = 448;  // pixel-queue solver: FIFO entries
 template <int TH>
-struct __align__(128) WarpSmem {
+struct __align__(128) TileSmem {
     uint32_t tm[(TH + 2) * 32];
     uint32_t tk[(TH + 2) * 32];
     uint32_t hLm[TH + 2];
@@ -157,7 +168,22 @@ struct __align__(128) WarpSmem {
     uint32_t hRm[TH + 2];
     uint32_t hRk[TH + 2];
     unsigned long long mbar;
-    unsigned short pq[kPqCap];  // pixel-queue solver: tile pixel indices r * TW + c
+    // the visit the CTA's warps work on together; kept here rather than in
+    // registers, which the passes need
+    ImgDesc d;        // its image
+    int tx, ty;       // its place
+    unsigned sides;   // NB_* bits: halo sides to look at
+    unsigned nb;      // NB_* bits found by the warps
+    unsigned go;      // 1 a tile, 0 the job is over
+    VisitCount count;  // the first warp's counters
+    // a row beside a warp's first / last block rose: by the parity of the
+    // round, the warp, from above / below
+    unsigned mark[2][TH / 8][2];
+};
+// with the pixel-queue solver's FIFO: tile pixel indices r * TW + c
+template <int TH>
+struct __align__(128) TileSmemAlt : TileSmem<TH> {
+    unsigned short pq[kPqCap];
 };
 
 // ------------------------------------------------------- async-copy helpers
@@ -199,12 +225,23 @@ __device__ __forceinline__ void tma_load_2d(void* smem_dst, const void* tmap, in
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 
+// One word, global to shared, by the calling thread (4-byte aligned).  Goes
+// through L1: an acquire before it (which drops what L1 holds) makes it see
+// other SMs' released stores like any load.
+__device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
 // Global-memory flag accesses with acquire / release ordering at GPU scope.
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
     unsigned v;
     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+// acquire / release fence at GPU scope (cheaper than __threadfence, which is
+// sequentially consistent)
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
     asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
 }
@@ -327,7 +364,7 @@ __device__ __forceinline__ void hscan(uint32_t (&m)[N], const uint32_t (&k)[N], 
 // or when its halo inputs are new (`force`, folded into `dil` by the caller).
 // `chg` receives the rows that rose (bit r-1 for SMEM row r).
 template <int DT, int CONN, int TH, bool DOWN>
-__device__ __forceinline__ void sweep(WarpSmem<TH>& sm, int lane, unsigned long long dil, unsigned long long& chg,
+__device__ __forceinline__ void sweep(TileSmem<TH>& sm, int lane, unsigned long long dil, unsigned long long& chg,
                                       bool& col_changed, uint32_t edge_mask, unsigned& row_steps) {
     using P = Px<DT>;
     constexpr int N = P::PPW;
@@ -394,17 +431,30 @@ __device__ __forceinline__ void sweep(WarpSmem<TH>& sm, int lane, unsigned long 
 }
 
 // ------------------------------------------------------- in-tile passes
-// The tile converges through three kinds of pass, the separable form of the
-// reference's XForward / XBackward / YDownward / YUpward propagation
-// (MR.cu:34-161):
-//   vertical down / up: each lane walks its own columns over the rows, one
-//     row per step, taking the row before it (8-connectivity: its three
-//     upper / lower neighbours, the outer two through one shuffle each);
-//     no vote or scan per row, so a row costs a few dependent operations;
-//   horizontal: rows are independent, each gets a forward and a backward
-//     max-min scan across the warp (hscan); four rows are scanned together
-//     so their shuffle latencies overlap.
-// Rows are numbered as in shared memory (1..TH); masks use bit r-1.
+// The tile converges through vertical and horizontal passes, the separable
+// form of the reference's XForward / XBackward / YDownward / YUpward
+// propagation (MR.cu:34-161), on blocks of eight rows in shared memory:
+//   vertical (vblock): a lane walks its own word column over the block's
+//     rows, down and up, entered by the rows beside the block
+//     (8-connectivity: then a step that adds the diagonals);
+//   horizontal (hblock): eight lanes hold a row, 16 bytes each, so most of a
+//     row's closure is in-lane work and the clamp maps cross three lane steps
+//     instead of five.
+// What bounds both is a warp's own instruction rate: min, max and byte
+// permutes issue every other cycle in one of the SM's four schedulers, so a
+// block costs a warp its instructions twice over in cycles whatever else the
+// SM does (measured alone and with 24 warps per SM: vertical 4-connected one
+// direction 371 / 436 cycles per block, horizontal 682-932 / 870-1200).  A
+// tile is therefore visited by as many warps as it has blocks (solve_tile),
+// one on each scheduler, instead of by one warp block after block.
+// The halo columns enter once, before the passes (halo_columns): they do not
+// change during a visit, so no pass looks at them again.
+// Rows are numbered as in shared memory (1..TH); block b has rows 8b+1..8b+8.
+
+// What rose in a block (votes): its first row, the six between, its last row,
+// a pixel of the tile's first or last column; RF_AGAIN: a diagonal raised
+// something in the vertical pass, which a walk may carry on.
+enum : unsigned { RF_FIRST = 1u, RF_INNER = 2u, RF_LAST = 4u, RF_COL = 8u, RF_AGAIN = 16u, RF_ROWS = 7u };
 
 // OR of a per-lane 64-bit mask over the warp.
 __device__ __forceinline__ unsigned long long warp_or64(unsigned long long v) {
@@ -413,204 +463,177 @@ __device__ __forceinline__ unsigned long long warp_or64(unsigned long long v) {
     return ((unsigned long long)hi << 32) | lo;
 }
 
-// Vertical pass, downward (rows in increasing order) or upward, from the
-// first row of `dirty` (rows whose constraint towards the row before them,
-// in pass order, may be violated) to the tile's far edge.  It does not stop
-// where the rows stop rising: a vote there costs more latency on long
-// fronts than the rows it would save.  Returns the rows that rose
-// (warp-uniform); `col_now` (per lane) records a rise in the tile's first /
-// last pixel column; `steps` counts the rows processed.
-template <int DT, int CONN, int TH, bool DOWN>
-__device__ __forceinline__ unsigned long long vpass(WarpSmem<TH>& sm, int lane, unsigned long long dirty,
-                                                    uint32_t edge_mask, bool& col_now, unsigned& steps) {
-    using P = Px<DT>;
-    constexpr int N = P::PPW;
-    const int first = DOWN ? __ffsll((long long)dirty) : 64 - __clzll((long long)dirty);
-    const int count = DOWN ? TH - first + 1 : first;
-    steps += (unsigned)count;
-    unsigned long long chg = 0ull;
-    uint32_t diff = 0u;
-    if (CONN == 4) {
-        // columns are independent: packed min / max per word and row; uint8
-        // words run as two u16x2 chains (even and odd bytes), whose min / max
-        // are single instructions, so the chain is two of them per row
-        const uint32_t first_prev = sm.tm[(DOWN ? first - 1 : first + 1) * 32 + lane];
-        uint32_t plo = first_prev & 0x00ff00ffu, phi = (first_prev >> 8) & 0x00ff00ffu, prevw = first_prev;
-#pragma unroll 4
-        for (int i = 0; i < count; ++i) {
-            const int r = DOWN ? first + i : first - i;
-            const uint32_t old = sm.tm[r * 32 + lane];
-            const uint32_t kw = sm.tk[r * 32 + lane];
-            uint32_t nw;
-            if (DT == DT_U8) {
-                plo = __vmaxu2(old & 0x00ff00ffu, __vminu2(plo, kw & 0x00ff00ffu));
-                phi = __vmaxu2((old >> 8) & 0x00ff00ffu, __vminu2(phi, (kw >> 8) & 0x00ff00ffu));
-                nw = plo | (phi << 8);
-            } else {
-                nw = word_max<DT>(old, word_min<DT>(prevw, kw));
-                prevw = nw;
-            }
-            sm.tm[r * 32 + lane] = nw;
-            const uint32_t x = nw ^ old;
-            diff |= x;
-            if (x != 0u) chg |= 1ull << (r - 1);
-        }
-        col_now |= (diff & edge_mask) != 0u;
-        __syncwarp();
-        return warp_or64(chg);
-    }
-    if (CONN == 8 && DT != DT_I32) {
-        // packed 8-connected rows: the previous row's three-pixel maximum
-        // from the word itself and the words 16 bits to either side, built
-        // by funnel shifts from the neighbour lanes' words (the tile's halo
-        // columns at lanes 0 / 31).  uint16 words are u16x2 as they are;
-        // uint8 words run as their even (lo) and odd (hi) bytes, where the
-        // even bytes' neighbours are the odd half and the odd half shifted
-        // in from the left, the odd bytes' the even half and the even half
-        // shifted in from the right.
-        constexpr uint32_t E = 0x00ff00ffu;
-        const uint32_t first_prev = sm.tm[(DOWN ? first - 1 : first + 1) * 32 + lane];
-        uint32_t plo = DT == DT_U8 ? first_prev & E : first_prev;
-        uint32_t phi = (first_prev >> 8) & E;
-#pragma unroll 4
-        for (int i = 0; i < count; ++i) {
-            const int r = DOWN ? first + i : first - i;
-            const int rp = DOWN ? r - 1 : r + 1;
-            const uint32_t old = sm.tm[r * 32 + lane];
-            const uint32_t kw = sm.tk[r * 32 + lane];
-            uint32_t nw;
-            if (DT == DT_U8) {
-                uint32_t left = __shfl_up_sync(FULL, phi, 1), right = __shfl_down_sync(FULL, plo, 1);
-                if (lane == 0) left = sm.hLm[rp] << 16;
-                if (lane == 31) right = sm.hRm[rp];
-                const uint32_t dlo = __vimax3_u16x2(plo, phi, __funnelshift_l(left, phi, 16));
-                const uint32_t dhi = __vimax3_u16x2(phi, plo, __funnelshift_r(plo, right, 16));
-                plo = __vmaxu2(old & E, __vminu2(dlo, kw & E));
-                phi = __vmaxu2((old >> 8) & E, __vminu2(dhi, (kw >> 8) & E));
-                nw = plo | (phi << 8);
-            } else {
-                uint32_t left = __shfl_up_sync(FULL, plo, 1), right = __shfl_down_sync(FULL, plo, 1);
-                if (lane == 0) left = sm.hLm[rp] << 16;
-                if (lane == 31) right = sm.hRm[rp];
-                const uint32_t dil =
-                    __vimax3_u16x2(plo, __funnelshift_l(left, plo, 16), __funnelshift_r(plo, right, 16));
-                nw = __vmaxu2(old, __vminu2(dil, kw));
-                plo = nw;
-            }
-            sm.tm[r * 32 + lane] = nw;
-            const uint32_t x = nw ^ old;
-            diff |= x;
-            if (x != 0u) chg |= 1ull << (r - 1);
-        }
-        col_now |= (diff & edge_mask) != 0u;
-        __syncwarp();
-        return warp_or64(chg);
-    }
-    uint32_t prev[N];
-    P::unpack(sm.tm[(DOWN ? first - 1 : first + 1) * 32 + lane], prev);
-#pragma unroll 4
-    for (int i = 0; i < count; ++i) {
-        const int r = DOWN ? first + i : first - i;
-        const int rp = DOWN ? r - 1 : r + 1;
-        const uint32_t old = sm.tm[r * 32 + lane];
-        uint32_t m[N], k[N];
-        P::unpack(old, m);
-        P::unpack(sm.tk[r * 32 + lane], k);
-        if (CONN == 8) {
-            uint32_t left = __shfl_up_sync(FULL, prev[N - 1], 1);
-            uint32_t right = __shfl_down_sync(FULL, prev[0], 1);
-            if (lane == 0) left = sm.hLm[rp];
-            if (lane == 31) right = sm.hRm[rp];
-            if (N == 1) {
-                m[0] = P::mx(m[0], P::mn(P::mx3(left, prev[0], right), k[0]));
-            } else {
-#pragma unroll
-                for (int j = 0; j < N; ++j) {
-                    const uint32_t a = j == 0 ? left : prev[j - 1];
-                    const uint32_t c = j == N - 1 ? right : prev[j + 1];
-                    m[j] = P::mx(m[j], P::mn(P::mx3(a, prev[j], c), k[j]));
-                }
-            }
+// A row's words in the form the vertical walk uses: uint8 the word's even and
+// odd bytes, each byte doubled to 16 bits (which keeps the order and costs
+// one byte permute); others the word itself.
+template <int DT>
+struct VRow {
+    static constexpr int N = DT == DT_U8 ? 2 : 1;
+    uint32_t v[N];
+    __device__ __forceinline__ void set(uint32_t w) {
+        if constexpr (DT == DT_U8) {
+            v[0] = __byte_perm(w, 0u, 0x2200);
+            v[1] = __byte_perm(w, 0u, 0x3311);
         } else {
-#pragma unroll
-            for (int j = 0; j < N; ++j) m[j] = P::mx(m[j], P::mn(prev[j], k[j]));
+            v[0] = w;
         }
-        const uint32_t nw = P::pack(m);
-        sm.tm[r * 32 + lane] = nw;
-        const uint32_t x = nw ^ old;
-        diff |= x;
-        if (x != 0u) chg |= 1ull << (r - 1);
-#pragma unroll
-        for (int j = 0; j < N; ++j) prev[j] = m[j];
     }
-    col_now |= (diff & edge_mask) != 0u;
-    __syncwarp();
-    return warp_or64(chg);
+    __device__ __forceinline__ uint32_t word() const {
+        if constexpr (DT == DT_U8)
+            return __byte_perm(v[0], v[1], 0x6240);
+        else
+            return v[0];
+    }
+    __device__ __forceinline__ bool differs(const VRow& o) const {
+        if constexpr (DT == DT_U8)
+            return ((v[0] ^ o.v[0]) | (v[1] ^ o.v[1])) != 0u;
+        else
+            return v[0] != o.v[0];
+    }
+};
+
+// Diagonals: byte selectors that put the word one pixel to the left / right
+// of a row's together from the lane's word and its neighbour lane's (uint8:
+// of the odd / even half).  In the first / last lane, where the tile ends,
+// they pick a pixel that the lane has already.
+struct EdgeSel {
+    unsigned left, right;
+    __device__ __forceinline__ explicit EdgeSel(int lane)
+        : left(lane == 0 ? 0x5454u : 0x5432u), right(lane == 31 ? 0x3232u : 0x5432u) {}
+};
+
+template <int DT>
+__device__ __forceinline__ uint32_t vmx(uint32_t a, uint32_t b) {
+    return DT == DT_I32 ? (uint32_t)max((int)a, (int)b) : __vmaxu2(a, b);
+}
+template <int DT>
+__device__ __forceinline__ uint32_t vmn(uint32_t a, uint32_t b) {
+    return DT == DT_I32 ? (uint32_t)min((int)a, (int)b) : __vminu2(a, b);
 }
 
-// R independent rows scanned together in one direction (see hscan).
-template <int DT, bool FWD, int R>
-__device__ __forceinline__ void hscan_rows(uint32_t (&m)[R][Px<DT>::PPW], const uint32_t (&k)[R][Px<DT>::PPW],
-                                           const uint32_t (&cin)[R], int lane) {
-    using P = Px<DT>;
-    constexpr int N = P::PPW;
-    const int first = FWD ? 0 : N - 1, last = FWD ? N - 1 : 0;
-    const int edge_lane = FWD ? 0 : 31;
-    bool need = false;
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-#pragma unroll
-        for (int s = 1; s < N; ++s) {
-            const int j = FWD ? s : N - 1 - s;
-            const int jp = FWD ? j - 1 : j + 1;
-            m[q][j] = P::mx(m[q][j], P::mn(m[q][jp], k[q][j]));
-        }
-        uint32_t in_px = FWD ? __shfl_up_sync(FULL, m[q][last], 1) : __shfl_down_sync(FULL, m[q][last], 1);
-        if (lane == edge_lane) in_px = cin[q];
-        need |= P::gt(P::mn(in_px, k[q][first]), m[q][first]);
-    }
-    // A carry that does not raise a word's entry pixel raises nothing after
-    // it; rows that need no scan come out of it unchanged.
-    if (!__any_sync(FULL, need)) return;
-    uint32_t A[R], B[R];
-#pragma unroll
-    for (int q = 0; q < R; ++q) {
-        A[q] = m[q][last];
-        B[q] = k[q][0];
-#pragma unroll
-        for (int j = 1; j < N; ++j) B[q] = P::mn(B[q], k[q][j]);
-        if (lane == edge_lane) {
-            A[q] = P::mx(A[q], P::mn(cin[q], B[q]));
-            B[q] = P::MINPX;  // the entry lane becomes a constant: nothing before it
-        }
-    }
-    if (DT == DT_I32) {
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1)
-#pragma unroll
-            for (int q = 0; q < R; ++q) map_step_i32<FWD>(A[q], B[q], d);
+// Each pixel the larger of its left and right neighbours in the row (a lane
+// without a neighbour lane reads its own word).
+template <int DT>
+__device__ __forceinline__ VRow<DT> beside(const VRow<DT>& p, const EdgeSel& sel) {
+    VRow<DT> h;
+    if constexpr (DT == DT_U8) {
+        // the even bytes' neighbours are the odd half and the odd half
+        // shifted in from the left, the odd bytes' the even half and the even
+        // half shifted in from the right
+        const uint32_t left = __shfl_up_sync(FULL, p.v[1], 1), right = __shfl_down_sync(FULL, p.v[0], 1);
+        h.v[0] = __vmaxu2(p.v[1], __byte_perm(left, p.v[1], sel.left));
+        h.v[1] = __vmaxu2(p.v[0], __byte_perm(p.v[0], right, sel.right));
     } else {
-        uint32_t cur[R];
-#pragma unroll
-        for (int q = 0; q < R; ++q) cur[q] = A[q] | (B[q] << 16);
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1)
-#pragma unroll
-            for (int q = 0; q < R; ++q) cur[q] = map_step_packed<FWD>(cur[q], d);
-#pragma unroll
-        for (int q = 0; q < R; ++q) A[q] = cur[q] & 0xffffu;
+        const uint32_t left = __shfl_up_sync(FULL, p.v[0], 1), right = __shfl_down_sync(FULL, p.v[0], 1);
+        if (DT == DT_U16)
+            h.v[0] = __vmaxu2(__byte_perm(left, p.v[0], sel.left), __byte_perm(p.v[0], right, sel.right));
+        else
+            h.v[0] = vmx<DT>(left, right);
     }
+    return h;
+}
+
+// m = max(m, min(p, k)).
+template <int DT>
+__device__ __forceinline__ void vstep(VRow<DT>& m, const VRow<DT>& k, const VRow<DT>& p) {
 #pragma unroll
-    for (int q = 0; q < R; ++q) {
-        uint32_t c = FWD ? __shfl_up_sync(FULL, A[q], 1) : __shfl_down_sync(FULL, A[q], 1);
-        if (lane == edge_lane) c = cin[q];
+    for (int j = 0; j < VRow<DT>::N; ++j) m.v[j] = vmx<DT>(m.v[j], vmn<DT>(p.v[j], k.v[j]));
+}
+
+// What a row offers the row above or below it.
+template <int DT, int CONN>
+__device__ __forceinline__ VRow<DT> offers(const VRow<DT>& p, const EdgeSel& sel) {
+    VRow<DT> q = p;
+    if (CONN == 8) {
+        const VRow<DT> h = beside<DT>(p, sel);
 #pragma unroll
-        for (int s = 0; s < N; ++s) {
-            const int j = FWD ? s : N - 1 - s;
-            c = P::mn(c, k[q][j]);
-            m[q][j] = P::mx(m[q][j], c);
+        for (int j = 0; j < VRow<DT>::N; ++j) q.v[j] = vmx<DT>(p.v[j], h.v[j]);
+    }
+    return q;
+}
+
+// Vertical pass over block b.  `due`: the walks that violated constraints in
+// the block may call for (VD_DOWN, VD_UP), and the rows beside the block that
+// rose (VD_ABOVE, VD_BELOW), which call for a walk only if they raise the
+// block's first / last row: looked at first, since many do not.  Returns RF_*
+// (warp-uniform).
+// 8-connectivity: the rows beside the block enter with their diagonals, the
+// walks go straight up and down, and one step over all rows at once then adds
+// the diagonals between the block's rows; a path that a diagonal opens goes
+// on in the next pass (RF_AGAIN).  Walks that take the diagonals along wait
+// 24 cycles for a shuffle in every row (852 cycles a block alone), take a
+// fifth more instructions, and must be repeated whenever they change
+// anything, where this must only when a diagonal did.
+enum : unsigned { VD_DOWN = 1u, VD_UP = 2u, VD_ABOVE = 4u, VD_BELOW = 8u };
+template <int DT, int CONN>
+__device__ __forceinline__ unsigned vblock(uint32_t* tm, const uint32_t* tk, int lane, int b, uint32_t edge_mask,
+                                           const EdgeSel& sel, unsigned due) {
+    constexpr int N = VRow<DT>::N;
+    uint32_t* rows = tm + (8 * b + 1) * 32 + lane;
+    const uint32_t* krows = tk + (8 * b + 1) * 32 + lane;
+    VRow<DT> above, below;
+    above.set(rows[-32]);
+    below.set(rows[8 * 32]);
+    VRow<DT> m[8], k[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        m[i].set(rows[i * 32]);
+        k[i].set(krows[i * 32]);
+    }
+    if (due & (VD_DOWN | VD_ABOVE)) {
+        const VRow<DT> was = m[0];
+        vstep<DT>(m[0], k[0], offers<DT, CONN>(above, sel));
+        if (!(due & VD_DOWN) && __any_sync(FULL, m[0].differs(was))) due |= VD_DOWN;
+    }
+    if (due & (VD_UP | VD_BELOW)) {
+        const VRow<DT> was = m[7];
+        vstep<DT>(m[7], k[7], offers<DT, CONN>(below, sel));
+        if (!(due & VD_UP) && __any_sync(FULL, m[7].differs(was))) due |= VD_UP;
+    }
+    if (!(due & (VD_DOWN | VD_UP))) return 0u;
+    // A pixel that rose from the pixel above it cannot raise that one again,
+    // so a walk leaves the other direction clean.
+    if (due & VD_DOWN) {
+#pragma unroll
+        for (int i = 1; i < 8; ++i) vstep<DT>(m[i], k[i], m[i - 1]);
+    }
+    if (due & VD_UP) {
+#pragma unroll
+        for (int i = 6; i >= 0; --i) vstep<DT>(m[i], k[i], m[i + 1]);
+    }
+    uint32_t diag = 0u;
+    if (CONN == 8) {
+        VRow<DT> before, here = beside<DT>(m[0], sel);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            VRow<DT> after, q;
+            if (i < 7) after = beside<DT>(m[i + 1], sel);
+#pragma unroll
+            for (int j = 0; j < N; ++j)
+                q.v[j] = i == 0 ? after.v[j] : i == 7 ? before.v[j] : vmx<DT>(before.v[j], after.v[j]);
+            const VRow<DT> was = m[i];
+            vstep<DT>(m[i], k[i], q);
+#pragma unroll
+            for (int j = 0; j < N; ++j) diag |= was.v[j] ^ m[i].v[j];
+            before = here;
+            here = after;
         }
     }
+    // (the rows as they were are read again: registers are short here)
+    uint32_t inner = 0u;
+#pragma unroll
+    for (int i = 1; i < 7; ++i) inner |= m[i].word() ^ rows[i * 32];
+    const uint32_t first = m[0].word() ^ rows[0], last = m[7].word() ^ rows[7 * 32];
+    const uint32_t all = first | inner | last;
+    if (!__any_sync(FULL, all != 0u)) return 0u;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) rows[i * 32] = m[i].word();
+    unsigned f = __any_sync(FULL, first != 0u) ? RF_FIRST : 0u;
+    if (__any_sync(FULL, inner != 0u)) f |= RF_INNER;
+    if (__any_sync(FULL, last != 0u)) f |= RF_LAST;
+    if (__any_sync(FULL, (all & edge_mask) != 0u)) f |= RF_COL;
+    if (CONN == 8 && __any_sync(FULL, diag != 0u)) f |= RF_AGAIN;
+    return f;
 }
 
 // Q pairs of rows scanned together in one direction, uint8 / uint16: pixel
@@ -699,97 +722,186 @@ __device__ __forceinline__ void pair_unpack(const uint32_t (&p)[Px<DT>::PPW], ui
     }
 }
 
-// Horizontal pass over the rows in `rows` (in blocks of eight as four row
-// pairs for uint8 / uint16, of four for int32): forward then backward scan,
-// which leaves each row at its one-dimensional fixed point.  `nrows` counts
-// the rows of the blocks processed.
-template <int DT, int TH>
-__device__ __forceinline__ unsigned long long hpass(WarpSmem<TH>& sm, int lane, unsigned long long rows,
-                                                    uint32_t edge_mask, bool& col_now, unsigned& nrows) {
+// Horizontal pass over block b: each row to its one-dimensional fixed point.
+// Lane L holds 16 bytes (part L % 8) of two rows (pair L / 8 of the block): a
+// row's closure is a forward and a backward chain in the lane (side by side,
+// each from the row as it was: what a pixel gets comes from one side, so
+// their maximum is the closure), then, if some lane's outermost pixel can
+// raise its neighbour lane's, the lanes' clamp maps in both directions at
+// once (three steps of two shuffles each) and one pass applying what enters
+// each lane from either side.  A row spread over the 32 lanes, a word each,
+// needs five scan steps and shares every shuffle among fewer pixels (about
+// twice the instructions).  uint8, cycles of a block alone / of the SM with
+// it busy: 738 / 148; chains one after the other 801 / 141; sixteen lanes of
+// eight pixels 782 / 162.
+// uint8 / uint16 hold pixel j of the two rows in one word as u16x2 (uint8
+// bytes doubled, as in VRow); int32 the two rows in words of their own.
+template <int DT>
+struct HLane {
+    static constexpr int N = 4 * Px<DT>::PPW;       // pixels of a row that a lane holds
+    static constexpr int S = DT == DT_I32 ? 2 : 1;  // words per pixel of the row pair
+    static constexpr uint32_t MINV = DT == DT_I32 ? 0x80000000u : 0u;
+    __device__ static __forceinline__ uint32_t mx(uint32_t a, uint32_t b) {
+        return DT == DT_I32 ? (uint32_t)max((int)a, (int)b) : __vmaxu2(a, b);
+    }
+    __device__ static __forceinline__ uint32_t mn(uint32_t a, uint32_t b) {
+        return DT == DT_I32 ? (uint32_t)min((int)a, (int)b) : __vminu2(a, b);
+    }
+    __device__ static __forceinline__ uint32_t mx3(uint32_t a, uint32_t b, uint32_t c) {
+        return DT == DT_I32 ? (uint32_t)__vimax3_s32((int)a, (int)b, (int)c) : __vimax3_u16x2(a, b, c);
+    }
+    __device__ static __forceinline__ uint32_t mn3(uint32_t a, uint32_t b, uint32_t c) {
+        return DT == DT_I32 ? (uint32_t)__vimin3_s32((int)a, (int)b, (int)c) : __vimin3_u16x2(a, b, c);
+    }
+    __device__ static __forceinline__ bool any_gt(uint32_t a, uint32_t b) {
+        return DT == DT_I32 ? (int)a > (int)b : __vmaxu2(a, b) != b;
+    }
+    __device__ static __forceinline__ void split(const uint4& ra, const uint4& rb, uint32_t (&v)[S][N]) {
+        const uint32_t a[4] = {ra.x, ra.y, ra.z, ra.w}, b[4] = {rb.x, rb.y, rb.z, rb.w};
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            if constexpr (DT == DT_U8) {
+                v[0][4 * w] = __byte_perm(a[w], b[w], 0x4400);
+                v[0][4 * w + 1] = __byte_perm(a[w], b[w], 0x5511);
+                v[0][4 * w + 2] = __byte_perm(a[w], b[w], 0x6622);
+                v[0][4 * w + 3] = __byte_perm(a[w], b[w], 0x7733);
+            } else if constexpr (DT == DT_U16) {
+                v[0][2 * w] = __byte_perm(a[w], b[w], 0x5410);
+                v[0][2 * w + 1] = __byte_perm(a[w], b[w], 0x7632);
+            } else {
+                v[0][w] = a[w];
+                v[1][w] = b[w];
+            }
+        }
+    }
+    __device__ static __forceinline__ void join(const uint32_t (&v)[S][N], uint4& ra, uint4& rb) {
+        uint32_t a[4], b[4];
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+            if constexpr (DT == DT_U8) {
+                const uint32_t t = __byte_perm(v[0][4 * w], v[0][4 * w + 1], 0x6240);
+                const uint32_t u = __byte_perm(v[0][4 * w + 2], v[0][4 * w + 3], 0x6240);
+                a[w] = __byte_perm(t, u, 0x5410);
+                b[w] = __byte_perm(t, u, 0x7632);
+            } else if constexpr (DT == DT_U16) {
+                a[w] = __byte_perm(v[0][2 * w], v[0][2 * w + 1], 0x5410);
+                b[w] = __byte_perm(v[0][2 * w], v[0][2 * w + 1], 0x7632);
+            } else {
+                a[w] = v[0][w];
+                b[w] = v[1][w];
+            }
+        }
+        ra = make_uint4(a[0], a[1], a[2], a[3]);
+        rb = make_uint4(b[0], b[1], b[2], b[3]);
+    }
+};
+
+template <int DT>
+__device__ __forceinline__ unsigned hblock(uint32_t* tm, const uint32_t* tk, int lane, int b) {
     using P = Px<DT>;
-    constexpr int N = P::PPW;
-    unsigned long long chg = 0ull;
-    uint32_t diff = 0u;
-    if constexpr (DT != DT_I32) {
-        constexpr int Q = 4, R = 2 * Q;
-        static_assert(TH % R == 0, "tile rows: a multiple of 8");
-#pragma unroll 1
-        for (int b = 0; b < TH; b += R) {
-            if (((rows >> b) & ((1ull << R) - 1ull)) == 0ull) continue;
-            nrows += R;
-            uint32_t m[Q][N], k[Q][N], olda[Q], oldb[Q], cin[Q];
+    using H = HLane<DT>;
+    constexpr int N = H::N, S = H::S;
+    const int part = lane & 7, pair = lane >> 3;
+    const int at = (8 * b + 2 * pair + 1) * 32 + part * 4;
+    const uint4 oa = *reinterpret_cast<const uint4*>(&tm[at]);
+    const uint4 ob = *reinterpret_cast<const uint4*>(&tm[at + 32]);
+    uint32_t m[S][N], k[S][N];
+    H::split(oa, ob, m);
+    H::split(*reinterpret_cast<const uint4*>(&tk[at]), *reinterpret_cast<const uint4*>(&tk[at + 32]), k);
+    // the lane's own closure, then whether an outermost pixel can raise the
+    // pixel beside it in the next lane
+    bool need = false;
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int r = b + 2 * q + 1;
-                olda[q] = sm.tm[r * 32 + lane];
-                oldb[q] = sm.tm[(r + 1) * 32 + lane];
-                pair_pack<DT>(olda[q], oldb[q], m[q]);
-                pair_pack<DT>(sm.tk[r * 32 + lane], sm.tk[(r + 1) * 32 + lane], k[q]);
-                cin[q] = sm.hLm[r] | (sm.hLm[r + 1] << 16);
-            }
-            hscan_pairs<true, Q, N>(m, k, cin, lane);
+    for (int s = 0; s < S; ++s) {
+        uint32_t bw[N];
+        bw[N - 1] = m[s][N - 1];
 #pragma unroll
-            for (int q = 0; q < Q; ++q) cin[q] = sm.hRm[b + 2 * q + 1] | (sm.hRm[b + 2 * q + 2] << 16);
-            hscan_pairs<false, Q, N>(m, k, cin, lane);
+        for (int j = N - 2; j >= 0; --j) bw[j] = H::mx(m[s][j], H::mn(bw[j + 1], k[s][j]));
 #pragma unroll
-            for (int q = 0; q < Q; ++q) {
-                const int r = b + 2 * q + 1;
-                uint32_t na, nb;
-                pair_unpack<DT>(m[q], na, nb);
-                sm.tm[r * 32 + lane] = na;
-                sm.tm[(r + 1) * 32 + lane] = nb;
-                const uint32_t xa = na ^ olda[q], xb = nb ^ oldb[q];
-                diff |= xa | xb;
-                if (xa != 0u) chg |= 1ull << (b + 2 * q);
-                if (xb != 0u) chg |= 1ull << (b + 2 * q + 1);
-            }
-        }
-        col_now |= (diff & edge_mask) != 0u;
-        __syncwarp();
-        return warp_or64(chg);
+        for (int j = 1; j < N; ++j) m[s][j] = H::mx(m[s][j], H::mn(m[s][j - 1], k[s][j]));
+#pragma unroll
+        for (int j = 0; j + 1 < N; ++j) m[s][j] = H::mx(m[s][j], bw[j]);
+        uint32_t l = __shfl_up_sync(FULL, m[s][N - 1], 1, 8), r = __shfl_down_sync(FULL, m[s][0], 1, 8);
+        if (part == 0) l = H::MINV;
+        if (part == 7) r = H::MINV;
+        need |= H::any_gt(H::mn(l, k[s][0]), m[s][0]) || H::any_gt(H::mn(r, k[s][N - 1]), m[s][N - 1]);
     }
-    constexpr int R = 4;
-#pragma unroll 1
-    for (int b = 0; b < TH; b += R) {
-        if (((rows >> b) & ((1ull << R) - 1ull)) == 0ull) continue;
-        nrows += R;
-        uint32_t m[R][N], k[R][N], old[R], cin[R];
+    if (__any_sync(FULL, need)) {
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int r = b + q + 1;
-            old[q] = sm.tm[r * 32 + lane];
-            P::unpack(old[q], m[q]);
-            P::unpack(sm.tk[r * 32 + lane], k[q]);
-            cin[q] = sm.hLm[r];
-        }
-        hscan_rows<DT, true, R>(m, k, cin, lane);
+        for (int s = 0; s < S; ++s) {
+            // clamp maps (A, B) of the lane in either direction (see
+            // map_step_packed): the closure's exit pixel, the least mask
+            uint32_t Bf = k[s][0];
 #pragma unroll
-        for (int q = 0; q < R; ++q) cin[q] = sm.hRm[b + q + 1];
-        hscan_rows<DT, false, R>(m, k, cin, lane);
+            for (int j = 1; j + 1 < N; j += 2) Bf = H::mn3(Bf, k[s][j], k[s][j + 1]);
+            Bf = H::mn(Bf, k[s][N - 1]);
+            uint32_t Af = m[s][N - 1], Ab = m[s][0], Bb = Bf;
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const uint32_t nw = P::pack(m[q]);
-            sm.tm[(b + q + 1) * 32 + lane] = nw;
-            const uint32_t x = nw ^ old[q];
-            diff |= x;
-            if (x != 0u) chg |= 1ull << (b + q);
+            for (int d = 1; d < 8; d <<= 1) {
+                const uint32_t af = __shfl_up_sync(FULL, Af, d, 8), bf = __shfl_up_sync(FULL, Bf, d, 8);
+                const uint32_t ab = __shfl_down_sync(FULL, Ab, d, 8), bb = __shfl_down_sync(FULL, Bb, d, 8);
+                Af = H::mx(H::mn(af, Bf), Af);
+                Bf = H::mn(bf, Bf);
+                Ab = H::mx(H::mn(ab, Bb), Ab);
+                Bb = H::mn(bb, Bb);
+            }
+            uint32_t cf = __shfl_up_sync(FULL, Af, 1, 8), cb = __shfl_down_sync(FULL, Ab, 1, 8);
+            if (part == 0) cf = H::MINV;
+            if (part == 7) cb = H::MINV;
+            // what enters from the left reaches pixel j through the masks up
+            // to j, what enters from the right through those from j on
+            uint32_t f[N];
+#pragma unroll
+            for (int j = 0; j < N; ++j) f[j] = cf = H::mn(cf, k[s][j]);
+#pragma unroll
+            for (int j = N - 1; j >= 0; --j) {
+                cb = H::mn(cb, k[s][j]);
+                m[s][j] = H::mx3(m[s][j], f[j], cb);
+            }
         }
     }
-    col_now |= (diff & edge_mask) != 0u;
+    uint4 na, nb;
+    H::join(m, na, nb);
+    const uint32_t xa = (na.x ^ oa.x) | (na.y ^ oa.y) | (na.z ^ oa.z) | (na.w ^ oa.w);
+    const uint32_t xb = (nb.x ^ ob.x) | (nb.y ^ ob.y) | (nb.z ^ ob.z) | (nb.w ^ ob.w);
+    if (!__any_sync(FULL, (xa | xb) != 0u)) return 0u;
+    *reinterpret_cast<uint4*>(&tm[at]) = na;
+    *reinterpret_cast<uint4*>(&tm[at + 32]) = nb;
+    const uint32_t xc = part == 0   ? ((na.x ^ oa.x) | (nb.x ^ ob.x)) & P::FIRST_MASK
+                        : part == 7 ? ((na.w ^ oa.w) | (nb.w ^ ob.w)) & P::LAST_MASK
+                                    : 0u;
+    const unsigned va = __ballot_sync(FULL, xa != 0u), vb = __ballot_sync(FULL, xb != 0u);
+    unsigned f = (va & 0xffu) ? RF_FIRST : 0u;
+    if ((va & 0xffffff00u) | (vb & 0x00ffffffu)) f |= RF_INNER;
+    if (vb & 0xff000000u) f |= RF_LAST;
+    if (__any_sync(FULL, xc != 0u)) f |= RF_COL;
+    return f;
+}
+
+// Raises the first and last pixel column of block b from the halo columns
+// (for 8-connectivity their three neighbours there, corners included); lanes
+// 0-7 the rows of the first column, lanes 8-15 of the last.  Returns RF_*.
+template <int DT, int CONN, int TH>
+__device__ __forceinline__ unsigned halo_columns(TileSmem<TH>& sm, int lane, int b) {
+    using P = Px<DT>;
+    const int r = 8 * b + 1 + (lane & 7);
+    const bool right = (lane & 8) != 0;
+    const uint32_t* h = right ? sm.hRm : sm.hLm;
+    uint32_t v = h[r];
+    if (CONN == 8) v = P::mx3(v, h[r - 1], h[r + 1]);
+    const int off = right ? 128 - P::BPP : 0;
+    unsigned char* px = reinterpret_cast<unsigned char*>(&sm.tm[r * 32]) + off;
+    v = P::mn(v, P::ld_px(reinterpret_cast<const unsigned char*>(&sm.tk[r * 32]) + off));
+    const bool rose = lane < 16 && P::gt(v, P::ld_px(px));
     __syncwarp();
-    return warp_or64(chg);
+    if (rose) P::st_px(px, v);
+    const unsigned bal = __ballot_sync(FULL, rose);
+    const unsigned rows = (bal | (bal >> 8)) & 0xffu;
+    if (rows == 0u) return 0u;
+    return ((rows & 1u) ? RF_FIRST : 0u) | ((rows & 0x7eu) ? RF_INNER : 0u) | ((rows & 0x80u) ? RF_LAST : 0u) | RF_COL;
 }
 
 // --------------------------------------------------------------- tile visit
-struct VisitResult {
-    unsigned nb;         // NB_* bits: neighbours to notify
-    unsigned sweeps;     // sweeps run
-    unsigned row_steps;  // rows processed by the sweeps
-    bool ok;             // false: a bounded wait ran out (job error)
-    bool stored;         // rows of the tile were stored at the end of the visit
-    long long t_fetch, t_proc, t_dump;  // clock64 cycles per phase
-};
-
 template <int DT>
 __device__ __forceinline__ uint32_t load_word_plain(const unsigned char* row, int npx, bool coherent) {
     using P = Px<DT>;
@@ -803,121 +915,105 @@ __device__ __forceinline__ uint32_t load_word_plain(const unsigned char* row, in
     return P::pack(p);
 }
 
-// Stores the rows of `rows` (bit r for tile row r) from shared memory to the
-// tile's own pixels (MR.cu:335-364; here plain stores: the visiting warp owns
-// the tile).
+// Stores block b's rows from shared memory to the tile's own pixels
+// (MR.cu:335-364; here plain stores: the visiting CTA owns the tile).  Where
+// the rows lie on 16-byte boundaries and the tile inside the image's width,
+// eight lanes store a row, four rows per instruction.
 template <int DT, int TH>
-__device__ __forceinline__ void write_back_rows(const ImgDesc& d, const WarpSmem<TH>& sm, int lane, int y0, int rows,
-                                                int npx, size_t col_off, unsigned long long mask) {
+__device__ __forceinline__ void write_back_block(const ImgDesc& d, const TileSmem<TH>& sm, int lane, int b, int x0,
+                                                 int y0) {
     using P = Px<DT>;
-    if (npx <= 0) return;
-    for (int r = 0; r < rows; ++r) {
-        if ((mask >> r) & 1ull) {
-            unsigned char* mrow = d.marker + (size_t)(y0 + r) * d.pitch_m + col_off;
-            const uint32_t w = sm.tm[(r + 1) * 32 + lane];
-            if (npx >= P::PPW) {
-                __stcg(reinterpret_cast<unsigned int*>(mrow), w);
-            } else {
-                uint32_t p[P::PPW];
-                P::unpack(w, p);
+    const bool wide = x0 + 32 * P::PPW <= d.W && ((reinterpret_cast<size_t>(d.marker) | (size_t)d.pitch_m) & 15u) == 0u;
+    if (wide) {
 #pragma unroll
-                for (int i = 0; i < P::PPW; ++i)
-                    if (i < npx) P::st_px(mrow + i * P::BPP, p[i]);
-            }
+        for (int h = 0; h < 2; ++h) {
+            const int r = 8 * b + 4 * h + (lane >> 3);
+            if (y0 + r < d.H)
+                __stcg(reinterpret_cast<uint4*>(d.marker + (size_t)(y0 + r) * d.pitch_m + (size_t)x0 * P::BPP +
+                                                (lane & 7) * 16),
+                       *reinterpret_cast<const uint4*>(&sm.tm[(r + 1) * 32 + (lane & 7) * 4]));
+        }
+        return;
+    }
+    const int px0 = x0 + lane * P::PPW, npx = d.W - px0;
+    if (npx <= 0) return;
+#pragma unroll 1
+    for (int r = 8 * b; r < 8 * b + 8 && y0 + r < d.H; ++r) {
+        unsigned char* mrow = d.marker + (size_t)(y0 + r) * d.pitch_m + (size_t)px0 * P::BPP;
+        const uint32_t w = sm.tm[(r + 1) * 32 + lane];
+        if (npx >= P::PPW) {
+            __stcg(reinterpret_cast<unsigned int*>(mrow), w);
+        } else {
+            uint32_t p[P::PPW];
+            P::unpack(w, p);
+#pragma unroll
+            for (int i = 0; i < P::PPW; ++i)
+                if (i < npx) P::st_px(mrow + i * P::BPP, p[i]);
         }
     }
 }
 
-// Neighbour detection (MR.cu:366-512, pull form): the NB_* bits of the
-// neighbour tiles holding a pixel q next to a pixel p of this tile with
-// marker[q] < min(marker[p], mask[q]), looking only at the sides that rose.
-// The halo values in shared memory are the neighbours' pixels as fetched;
-// they can only have risen since, so a stale halo gives at most an extra
-// notification, never a missed one.
+// Neighbour detection (MR.cu:366-512, pull form) for block b: the NB_* bits
+// of the neighbour tiles holding a pixel q next to a pixel p of this block
+// with marker[q] < min(marker[p], mask[q]), looking only at the sides that
+// rose (f, RF_*).  The halo values in shared memory are the neighbours'
+// pixels as fetched; they can only have risen since, so a stale halo gives at
+// most an extra notification, never a missed one.
 template <int DT, int CONN, int TH>
-__device__ __forceinline__ unsigned detect_neighbours(const WarpSmem<TH>& sm, int lane, bool top_rose, bool bot_rose,
-                                                      bool side_rose) {
+__device__ __forceinline__ unsigned detect_neighbours(const TileSmem<TH>& sm, int lane, int b, unsigned f) {
+    const EdgeSel sel(lane);
     using P = Px<DT>;
+    constexpr int NB = TH / 8;
     unsigned nb = 0u;
-    uint32_t r0[P::PPW], r1[P::PPW], t_m[P::PPW], t_k[P::PPW], b_m[P::PPW], b_k[P::PPW];
-    P::unpack(sm.tm[32 + lane], r0);
-    P::unpack(sm.tm[TH * 32 + lane], r1);
-    P::unpack(sm.tm[lane], t_m);
-    P::unpack(sm.tk[lane], t_k);
-    P::unpack(sm.tm[(TH + 1) * 32 + lane], b_m);
-    P::unpack(sm.tk[(TH + 1) * 32 + lane], b_k);
-    uint32_t l0 = __shfl_up_sync(FULL, r0[P::PPW - 1], 1), n0 = __shfl_down_sync(FULL, r0[0], 1);
-    uint32_t l1 = __shfl_up_sync(FULL, r1[P::PPW - 1], 1), n1 = __shfl_down_sync(FULL, r1[0], 1);
-    if (lane == 0) l0 = l1 = P::MINPX;  // pixels of other tiles are not sources here
-    if (lane == 31) n0 = n1 = P::MINPX;
-    bool need_n = false, need_s = false;
-#pragma unroll
-    for (int j = 0; j < P::PPW; ++j) {
-        uint32_t v0 = r0[j], v1 = r1[j];
-        if (CONN == 8) {
-            v0 = P::mx3(j == 0 ? l0 : r0[j - 1], v0, j == P::PPW - 1 ? n0 : r0[j + 1]);
-            v1 = P::mx3(j == 0 ? l1 : r1[j - 1], v1, j == P::PPW - 1 ? n1 : r1[j + 1]);
-        }
-        need_n |= P::gt(P::mn(v0, t_k[j]), t_m[j]);
-        need_s |= P::gt(P::mn(v1, b_k[j]), b_m[j]);
+    const bool n = b == 0 && (f & RF_FIRST), s = b == NB - 1 && (f & RF_LAST);
+    if (n || s) {
+        // a step of the vertical walk over the halo row (one of the two: a
+        // tile has at least two blocks)
+        const int row = n ? 1 : TH, halo = n ? 0 : TH + 1;
+        VRow<DT> p, m, k;
+        p.set(sm.tm[row * 32 + lane]);
+        const uint32_t w = sm.tm[halo * 32 + lane];
+        m.set(w);
+        k.set(sm.tk[halo * 32 + lane]);
+        vstep<DT>(m, k, offers<DT, CONN>(p, sel));
+        if (__any_sync(FULL, m.word() != w)) nb |= n ? NB_N : NB_S;
     }
-    if (top_rose && __any_sync(FULL, need_n)) nb |= NB_N;
-    if (bot_rose && __any_sync(FULL, need_s)) nb |= NB_S;
-
-    if (side_rose) {
-        // W / E: lanes walk the tile's first / last pixel column
-        bool need_w = false, need_e = false;
-        for (int r = 1 + lane; r <= TH; r += 32) {
-            uint32_t f[P::PPW], l[P::PPW];
-            P::unpack(sm.tm[r * 32], f);
-            P::unpack(sm.tm[r * 32 + 31], l);
-            uint32_t fv = f[0], lv = l[P::PPW - 1];
+    if (f & RF_COL) {
+        // lanes 0-9 / 16-25: the rows from the one before the block to the
+        // one after it in the left / right halo column
+        const int i = lane & 15, r = 8 * b + i;
+        const bool right = (lane & 16) != 0;
+        bool up = false;
+        if (CONN == 8 ? i < 10 : i >= 1 && i < 9) {
+            const unsigned char* col = reinterpret_cast<const unsigned char*>(sm.tm) + (right ? 128 - P::BPP : 0);
+            uint32_t v = P::MINPX;
             if (CONN == 8) {
-                uint32_t fa[P::PPW], la[P::PPW];
-                if (r > 1) {
-                    P::unpack(sm.tm[(r - 1) * 32], fa);
-                    P::unpack(sm.tm[(r - 1) * 32 + 31], la);
-                    fv = P::mx(fv, fa[0]);
-                    lv = P::mx(lv, la[P::PPW - 1]);
-                }
-                if (r < TH) {
-                    P::unpack(sm.tm[(r + 1) * 32], fa);
-                    P::unpack(sm.tm[(r + 1) * 32 + 31], la);
-                    fv = P::mx(fv, fa[0]);
-                    lv = P::mx(lv, la[P::PPW - 1]);
-                }
+                if (r > 1) v = P::mx(v, P::ld_px(col + (r - 1) * 128));
+                if (r < TH) v = P::mx(v, P::ld_px(col + (r + 1) * 128));
             }
-            need_w |= P::gt(P::mn(fv, sm.hLk[r]), sm.hLm[r]);
-            need_e |= P::gt(P::mn(lv, sm.hRk[r]), sm.hRm[r]);
+            if (r >= 1 && r <= TH) v = P::mx(v, P::ld_px(col + r * 128));
+            v = P::mn(v, right ? sm.hRk[r] : sm.hLk[r]);
+            up = P::gt(v, right ? sm.hRm[r] : sm.hLm[r]);
         }
-        if (__any_sync(FULL, need_w)) nb |= NB_W;
-        if (__any_sync(FULL, need_e)) nb |= NB_E;
-    }
-    if (CONN == 8) {
-        uint32_t a[P::PPW], b[P::PPW], c[P::PPW], e[P::PPW];
-        P::unpack(sm.tm[32], a);
-        P::unpack(sm.tm[32 + 31], b);
-        P::unpack(sm.tm[TH * 32], c);
-        P::unpack(sm.tm[TH * 32 + 31], e);
-        if (top_rose && P::gt(P::mn(a[0], sm.hLk[0]), sm.hLm[0])) nb |= NB_NW;
-        if (top_rose && P::gt(P::mn(b[P::PPW - 1], sm.hRk[0]), sm.hRm[0])) nb |= NB_NE;
-        if (bot_rose && P::gt(P::mn(c[0], sm.hLk[TH + 1]), sm.hLm[TH + 1])) nb |= NB_SW;
-        if (bot_rose && P::gt(P::mn(e[P::PPW - 1], sm.hRk[TH + 1]), sm.hRm[TH + 1])) nb |= NB_SE;
+        const unsigned bal = __ballot_sync(FULL, up);
+        unsigned l = bal & 0xffffu, e = bal >> 16;
+        if (b == 0) {  // the corner rows
+            if (l & 1u) nb |= NB_NW;
+            if (e & 1u) nb |= NB_NE;
+            l &= ~1u;
+            e &= ~1u;
+        }
+        if (b == NB - 1) {
+            if (l & 0x200u) nb |= NB_SW;
+            if (e & 0x200u) nb |= NB_SE;
+            l &= ~0x200u;
+            e &= ~0x200u;
+        }
+        if (l) nb |= NB_W;
+        if (e) nb |= NB_E;
     }
     return nb;
 }
-
-// Early flush that does nothing: the tile's neighbours are notified once,
-// after the visit.
-struct NoEarlyFlush {
-    static constexpr bool kEnabled = false;
-    bool use_passes;
-    bool use_pq;  // revisits by the pixel queue (pq_solve)
-    __device__ bool passes(int) { return use_passes; }
-    __device__ bool pq() { return use_pq; }
-    __device__ bool want(int) { return false; }
-    __device__ void flush(unsigned, int) {}
-};
 
 // ------------------------------------------------------- pixel queue
 // Third in-tile solver, for revisits: a FIFO of tile pixels in shared memory
@@ -967,7 +1063,7 @@ __device__ __forceinline__ bool pq_raise(uint32_t* words, int r, int c, uint32_t
 }
 
 template <int DT, int CONN, int TH>
-__device__ bool pq_solve(WarpSmem<TH>& sm, int lane, unsigned long long& rows_chg, bool& col_now, unsigned& rounds) {
+__device__ bool pq_solve(TileSmemAlt<TH>& sm, int lane, unsigned long long& rows_chg, bool& col_now, unsigned& rounds) {
     using P = Px<DT>;
     constexpr int TW = 32 * P::PPW;
     int head = 0, tail = 0;  // warp-uniform
@@ -1060,176 +1156,354 @@ __device__ bool pq_solve(WarpSmem<TH>& sm, int lane, unsigned long long& rows_ch
     return true;
 }
 
-// One warp: fetch tile (tx, ty) of image d with its one-pixel halo, run
-// raster / anti-raster sweeps until a sweep after the first changes nothing,
-// store the rows that rose, and report the neighbour tiles to notify: those
-// holding a pixel q next to a pixel p of this tile with
-// marker[q] < min(marker[p], mask[q]) where p's side of the tile rose.
-// `sides` (NB_* bits) names the halo sides whose pixels are new since the
-// tile last converged (all sides on a first visit).
-//
-// `early` can publish intermediate results: after a sweep that raised a
-// boundary row or column, if early.want() says so (the engine asks for it
-// when the work queue runs dry, i.e. when the job is bound by its
-// propagation front), the rows risen so far are stored and the neighbours
-// they raise are handed to early.flush() while the sweeps go on.  The
-// returned `nb` then covers only what rose after the last flush.
-//
-// Inlined into the worker: as a called function its result, its
-// descriptor and its shared-memory tile reached it through generic
-// pointers, and its row loops re-read counters from the stack (two to four
-// local loads per row step); inlined, the kernel has no stack frame and
-// the tile is addressed as shared memory (15 % faster on 4096^2 h-domes).
-template <int DT, int CONN, int TH, class Early>
-__device__ __forceinline__ VisitResult visit_tile(const ImgDesc& d, int tx, int ty, WarpSmem<TH>& sm, int lane,
-                                               unsigned& phase, long long timeout_ns, unsigned sides, Early& early) {
-    using P = Px<DT>;
-    constexpr int TW = 32 * P::PPW;
-    VisitResult res{0u, 0u, 0u, true, false, 0, 0, 0};
-    const long long c0 = clock64();
-    const int x0 = tx * TW, y0 = ty * TH;
-    const int W = d.W, H = d.H;
-    const int px0 = x0 + lane * P::PPW;  // first pixel of this lane's word
-    const int npx = W - px0;             // >= PPW: full word, (0, PPW): partial, <= 0: outside
-    const size_t col_off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
-    const int rows = min(TH, H - y0);
+template <int W>
+__device__ __forceinline__ void cta_sync() {
+    if (W == 1)
+        __syncwarp();
+    else
+        __syncthreads();
+}
 
-    // ---- fetch (MR.cu:232-312)
+// Fetches tile (tx, ty) of image d with its one-pixel halo (MR.cu:232-312);
+// called by all W warps of the CTA.  Where the image has tensor maps, the
+// first thread issues one box of TH+2 rows x 128 bytes per plane (rows /
+// columns outside the image arrive as zeros), else the warps copy the words
+// asynchronously (all in flight at once, no registers; through registers in
+// batches of eight rows the fetch took four times as long).  The halo columns
+// are single pixels, a load per lane and block.  Returns false when the
+// bounded wait for the boxes ran out.
+template <int DT, int TH, int W>
+__device__ __forceinline__ bool fetch_tile(const ImgDesc& d, int tx, int ty, TileSmem<TH>& sm, int warp, int lane,
+                                           unsigned& phase, long long timeout_ns) {
+    using P = Px<DT>;
+    constexpr int TW = 32 * P::PPW, BPW = TH / 8 / W;  // blocks per warp
+    const int x0 = tx * TW, y0 = ty * TH;
+    const int W_ = d.W, H = d.H;
+    const int px0 = x0 + lane * P::PPW;  // first pixel of this lane's word
+    const int npx = W_ - px0;            // >= PPW: full word, (0, PPW): partial, <= 0: outside
+    const int r0 = warp == 0 ? 0 : 8 * BPW * warp + 1, r1 = warp == W - 1 ? TH + 1 : 8 * BPW * (warp + 1);
     const bool tma = d.tmaps != nullptr;
     if (tma) {
-        // one box of TH+2 rows x 128 bytes per plane, halo rows included;
-        // rows / columns outside the image arrive as zeros
-        fence_proxy_async_smem();  // earlier generic reads of tm / tk before the async writes
-        __syncwarp();
-        if (lane == 0) {
+        if (warp == 0 && lane == 0) {
+            fence_proxy_async_smem();  // earlier generic accesses of tm / tk before the async writes
             fence_proxy_async_global();
             mbar_arrive_expect_tx(&sm.mbar, 2u * 128u * (TH + 2));
             const unsigned char* maps = static_cast<const unsigned char*>(d.tmaps);
             tma_load_2d(sm.tm, maps, x0 * P::BPP, y0 - 1, &sm.mbar);
             tma_load_2d(sm.tk, maps + 128, x0 * P::BPP, y0 - 1, &sm.mbar);
         }
+        __syncwarp();
     } else {
-#pragma unroll 8
-        for (int r = 0; r < TH + 2; ++r) {
+        const size_t off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
+#pragma unroll 4
+        for (int r = r0; r <= r1; ++r) {
             const int y = y0 - 1 + r;
-            uint32_t mw = P::MINW, kw = P::MINW;
-            if (y >= 0 && y < H && npx > 0) {
-                mw = load_word_plain<DT>(d.marker + (size_t)y * d.pitch_m + col_off, npx, true);
-                kw = load_word_plain<DT>(d.mask + (size_t)y * d.pitch_k + col_off, npx, false);
+            const bool in_y = y >= 0 && y < H;
+            const unsigned char* mrow = d.marker + (size_t)y * d.pitch_m + off;
+            const unsigned char* krow = d.mask + (size_t)y * d.pitch_k + off;
+            if (in_y && npx >= P::PPW) {
+                cp_async_4(&sm.tm[r * 32 + lane], mrow);
+                cp_async_4(&sm.tk[r * 32 + lane], krow);
+            } else {
+                uint32_t mw = P::MINW, kw = P::MINW;
+                if (in_y && npx > 0) {
+                    mw = load_word_plain<DT>(mrow, npx, true);
+                    kw = load_word_plain<DT>(krow, npx, false);
+                }
+                sm.tm[r * 32 + lane] = mw;
+                sm.tk[r * 32 + lane] = kw;
             }
-            sm.tm[r * 32 + lane] = mw;
-            sm.tk[r * 32 + lane] = kw;
         }
     }
-    // halo columns (single pixels), in flight together with the box loads
-    for (int i = lane; i < TH + 2; i += 32) {
-        const int y = y0 - 1 + i;
-        uint32_t lm = P::MINPX, lk = P::MINPX, rm = P::MINPX, rk = P::MINPX;
-        if (y >= 0 && y < H) {
-            const unsigned char* mrow = d.marker + (size_t)y * d.pitch_m;
-            const unsigned char* krow = d.mask + (size_t)y * d.pitch_k;
-            if (x0 > 0) {
-                lm = P::ld_px_cg(mrow + (size_t)(x0 - 1) * P::BPP);
-                lk = P::ld_px(krow + (size_t)(x0 - 1) * P::BPP);
-            }
-            if (x0 + TW < W) {
-                rm = P::ld_px_cg(mrow + (size_t)(x0 + TW) * P::BPP);
-                rk = P::ld_px(krow + (size_t)(x0 + TW) * P::BPP);
-            }
+    {
+        // halo columns, in flight together with the rows: lanes 0-7 the left
+        // marker pixels of a block, then the left mask, right marker, right
+        // mask; the corner rows with the first and the last block
+        const int j = lane & 7, which = lane >> 3;
+        uint32_t* h = which == 0 ? sm.hLm : which == 1 ? sm.hLk : which == 2 ? sm.hRm : sm.hRk;
+        const int x = which < 2 ? x0 - 1 : x0 + TW;
+        const bool in_x = x >= 0 && x < W_;
+        const unsigned char* plane = (which & 1) ? d.mask : d.marker;
+        const long long pitch = (which & 1) ? d.pitch_k : d.pitch_m;
+        auto halo = [&](int r) -> uint32_t {
+            const int y = y0 - 1 + r;
+            if (!in_x || y < 0 || y >= H) return P::MINPX;
+            return P::ld_px_cg(plane + (size_t)y * pitch + (size_t)x * P::BPP);
+        };
+        uint32_t v[BPW], vc = 0u;
+#pragma unroll
+        for (int i = 0; i < BPW; ++i) v[i] = halo(8 * (BPW * warp + i) + 1 + j);
+        const int corner = warp == 0 && j == 0 ? 0 : warp == W - 1 && j == 7 ? TH + 1 : -1;
+        int corner2 = -1;
+        uint32_t vc2 = 0u;
+        if (corner >= 0) vc = halo(corner);
+        if (W == 1 && j == 7) {
+            corner2 = TH + 1;
+            vc2 = halo(corner2);
         }
-        sm.hLm[i] = lm;
-        sm.hLk[i] = lk;
-        sm.hRm[i] = rm;
-        sm.hRk[i] = rk;
+#pragma unroll
+        for (int i = 0; i < BPW; ++i) h[8 * (BPW * warp + i) + 1 + j] = v[i];
+        if (corner >= 0) h[corner] = vc;
+        if (corner2 >= 0) h[corner2] = vc2;
     }
     if (tma) {
         // bounded wait for the box loads
         const long long t0 = globaltimer_ns();
         unsigned spins = 0;
+        bool ok = true;
         while (!mbar_try_wait(&sm.mbar, phase)) {
             if ((++spins & 1023u) == 0u && globaltimer_ns() - t0 > timeout_ns) {
-                res.ok = false;
+                ok = false;
                 break;
             }
         }
         phase ^= 1u;
-        if (!res.ok) return res;
+        if (!__all_sync(FULL, ok)) return false;
         if (DT == DT_I32) {
             // zero fill is not the int32 minimum: rewrite what lies outside
-            if (y0 == 0) sm.tm[lane] = sm.tk[lane] = P::MINW;
-            for (int r = rows + 1; r < TH + 2; ++r) {
-                if (y0 - 1 + r >= H) sm.tm[r * 32 + lane] = sm.tk[r * 32 + lane] = P::MINW;
+            for (int r = r0; r <= r1; ++r) {
+                const int y = y0 - 1 + r;
+                if (npx <= 0 || y < 0 || y >= H) sm.tm[r * 32 + lane] = sm.tk[r * 32 + lane] = P::MINW;
             }
-            if (npx <= 0)
-                for (int r = 0; r < TH + 2; ++r) sm.tm[r * 32 + lane] = sm.tk[r * 32 + lane] = P::MINW;
+        }
+    } else {
+        cp_async_wait_all();
+    }
+    return true;
+}
+
+// What rose in a warp's blocks: masks by block, and the tile's first / last
+// row.
+struct Rose {
+    unsigned rows = 0u, col = 0u;
+    bool top = false, bottom = false;
+};
+
+// Local convergence (MR.cu:320-325) by the W warps of a CTA, each with the
+// blocks next to one another.  Every round a warp goes over its blocks
+// (downward, then upward, in turn), runs the vertical pass where a constraint
+// may be violated and, if that raised something (or the side columns did),
+// the horizontal pass; a block that rose is looked at again, as is the block
+// beside a first or last row that rose.  The warps read the rows beside their
+// blocks while their owners may be raising them: pixels only rise, so an old
+// value is a valid one, and the owner marks the reader's block after the row,
+// for the next round.  Rounds end when nothing is left to look at, at the
+// tile's fixed point; the result does not depend on the order of updates.
+// `sides` (NB_* bits) names the halo sides whose pixels are new since the
+// tile last converged (all sides on a first visit).  Returns false when the
+// rounds do not end (a defect, reported instead of a hang).
+template <int DT, int CONN, int TH, int W>
+__device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane, unsigned& row_steps, Rose& rose) {
+    using P = Px<DT>;
+    constexpr int BPW = TH / 8 / W;
+    constexpr unsigned LASTB = 1u << (BPW - 1);
+    const uint32_t edge_mask = lane == 0 ? P::FIRST_MASK : lane == 31 ? P::LAST_MASK : 0u;
+    const EdgeSel sel(lane);
+    const int b0 = BPW * warp;
+    // by block: due for the downward / upward walk, the row above / below
+    // rose, due for the horizontal pass
+    unsigned dd = 0u, du = 0u, da = 0u, db = 0u, dh = 0u;
+    unsigned marks = 0u;  // 1 the warp above, 2 the warp below is to look again
+    const unsigned sides = sm.sides;
+    // takes over what a pass raised (f, RF_*) in the warp's block i
+    auto took = [&](unsigned f, int i) {
+        if (!(f & RF_ROWS)) return;
+        rose.rows |= 1u << i;
+        if (f & RF_COL) rose.col |= 1u << i;
+        if (f & RF_FIRST) {
+            if (i > 0)
+                db |= 1u << (i - 1);
+            else if (warp > 0)
+                marks |= 1u;
+            else
+                rose.top = true;
+        }
+        if (f & RF_LAST) {
+            if (i < BPW - 1)
+                da |= 2u << i;
+            else if (warp < W - 1)
+                marks |= 2u;
+            else
+                rose.bottom = true;
+        }
+    };
+    if (sides == 0xffu) {
+        dd = du = dh = 2u * LASTB - 1u;
+    } else {
+        if (warp == 0 && (sides & (NB_N | NB_NW | NB_NE))) da |= 1u;
+        if (warp == W - 1 && (sides & (NB_S | NB_SW | NB_SE))) db |= LASTB;
+    }
+    if (sides & ~(NB_N | NB_S)) {
+#pragma unroll 1
+        for (int i = 0; i < BPW; ++i) {
+            const unsigned f = halo_columns<DT, CONN, TH>(sm, lane, b0 + i);
+            if (f & RF_ROWS) {
+                dd |= 1u << i;
+                du |= 1u << i;
+                dh |= 1u << i;
+                took(f, i);
+            }
+        }
+        __syncwarp();
+    }
+    bool up = false;
+#pragma unroll 1
+    for (unsigned round = 0;; ++round, up = !up) {
+        if (W > 1 && round != 0u) {
+            volatile unsigned* mine = sm.mark[round & 1u][warp];
+            const unsigned above = mine[0], below = mine[1];
+            __syncwarp();
+            if (above) da |= 1u;
+            if (below) db |= LASTB;
+            if (lane == 0 && above) mine[0] = 0u;
+            if (lane == 0 && below) mine[1] = 0u;
+        }
+#pragma unroll 1
+        for (int n = 0; n < BPW; ++n) {
+            const int i = up ? BPW - 1 - n : n;
+            const unsigned bit = 1u << i;
+            if ((dd | du | da | db) & bit) {
+                const unsigned due = ((dd & bit) ? VD_DOWN : 0u) | ((du & bit) ? VD_UP : 0u) |
+                                     ((da & bit) ? VD_ABOVE : 0u) | ((db & bit) ? VD_BELOW : 0u);
+                dd &= ~bit;
+                du &= ~bit;
+                da &= ~bit;
+                db &= ~bit;
+                const unsigned f = vblock<DT, CONN>(sm.tm, sm.tk, lane, b0 + i, edge_mask, sel, due);
+                __syncwarp();
+                row_steps += 8u;
+                took(f, i);
+                if (f & RF_ROWS) dh |= bit;
+                if (f & RF_AGAIN) {
+                    dd |= bit;
+                    du |= bit;
+                }
+            }
+            if (dh & bit) {
+                dh &= ~bit;
+                const unsigned f = hblock<DT>(sm.tm, sm.tk, lane, b0 + i);
+                __syncwarp();
+                row_steps += 8u;
+                took(f, i);
+                if (f & RF_ROWS) {
+                    dd |= bit;
+                    du |= bit;
+                }
+            }
+        }
+        bool more = (dd | du | da | db) != 0u;
+        if (W > 1) {
+            if (lane == 0 && marks != 0u) {
+                __threadfence_block();  // the rows before the marks
+                if (marks & 1u) *(volatile unsigned*)&sm.mark[(round & 1u) ^ 1u][warp - 1][1] = 1u;
+                if (marks & 2u) *(volatile unsigned*)&sm.mark[(round & 1u) ^ 1u][warp + 1][0] = 1u;
+            }
+            more = __syncthreads_or(more || marks != 0u) != 0;
+            marks = 0u;
+        }
+        if (!more || round > (1u << 20)) {
+            if (warp == 0 && lane == 0) sm.count.sweeps += round + 1u;
+            return !more;
         }
     }
-    __syncwarp();
-    const long long c1 = clock64();
-    res.t_fetch = c1 - c0;
+}
 
-    // ---- local convergence (MR.cu:320-325), by one of two solvers:
-    //   row sweeps (early.passes() false): raster / anti-raster sweeps, each
-    //     row a vertical update and a warp scan, until a sweep after the
-    //     first two changes nothing; fewest instructions per converged tile,
-    //     for when the GPU is full of work;
-    //   passes (early.passes() true): vertical and horizontal passes (see
-    //     vpass / hpass) until no rows are left whose constraints may be
-    //     violated; the shortest latency from a raised halo to a raised far
-    //     edge, for when the job is bound by its propagation front.
-    // Both are sequences of valid monotone updates that stop at the tile's
-    // fixed point, so they give the same bytes.
+// One visit of tile (tx, ty) by a CTA of W warps: fetch, local convergence,
+// store of the blocks that rose, and the neighbour tiles to notify in sm.nb.
+// Called by all warps; after it the stores are visible to the GPU and the
+// first warp may go on to the next tile.  Returns false when a bounded wait
+// ran out.
+template <int DT, int CONN, int TH, int W>
+__device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane, unsigned& phase, long long timeout_ns,
+                                           unsigned& row_steps) {
+    constexpr int BPW = TH / 8 / W;
+    const bool clerk = warp == 0 && lane == 0;  // keeps the visit's clock
+    if (clerk) sm.count.cycles[1] -= clock64();
+    bool ok = fetch_tile<DT, TH, W>(sm.d, sm.tx, sm.ty, sm, warp, lane, phase, timeout_ns);
+    if (W > 1) {
+        if (__syncthreads_or(!ok)) return false;
+    } else {
+        __syncwarp();
+        if (!ok) return false;
+    }
+    if (clerk) {
+        const long long t = clock64();
+        sm.count.cycles[1] += t;
+        sm.count.cycles[2] -= t;
+    }
+    Rose rose;
+    ok = solve_tile<DT, CONN, TH, W>(sm, warp, lane, row_steps, rose);
+    if (clerk) {
+        const long long t = clock64();
+        sm.count.cycles[2] += t;
+        sm.count.cycles[3] -= t;
+    }
+    if (rose.rows != 0u) {
+        unsigned nb = 0u;
+#pragma unroll 1
+        for (int i = 0; i < BPW; ++i) {
+            if (!((rose.rows >> i) & 1u)) continue;
+            write_back_block<DT, TH>(sm.d, sm, lane, BPW * warp + i, sm.tx * 32 * Px<DT>::PPW, sm.ty * TH);
+        }
+#pragma unroll 1
+        for (int i = 0; i < BPW; ++i) {
+            unsigned f = (rose.col >> i) & 1u ? RF_COL : 0u;
+            if (i == 0 && rose.top) f |= RF_FIRST;
+            if (i == BPW - 1 && rose.bottom) f |= RF_LAST;
+            if (f != 0u) nb |= detect_neighbours<DT, CONN, TH>(sm, lane, BPW * warp + i, f);
+        }
+        if (nb != 0u && lane == 0) atomicOr(&sm.nb, nb);
+        // release: the stores before the neighbours' DIRTY and before the
+        // tile's ACTIVE bit clears (its next owner reads them)
+        fence_gpu();
+    }
+    fence_proxy_async_smem();
+    cta_sync<W>();
+    if (clerk) sm.count.cycles[3] += clock64();
+    return ok;
+}
+
+// The visit with the alternative solvers, for callers that ask for them
+// (iwpp_config.solver 1 and 3), by a CTA of one warp.  All solvers are
+// sequences of valid monotone updates that stop at the tile's fixed point, so
+// they give the same bytes.
+template <int DT, int CONN, int TH>
+__device__ __forceinline__ bool visit_tile_alt(TileSmemAlt<TH>& sm, int lane, unsigned& phase, long long timeout_ns,
+                                               int solver, unsigned& row_steps) {
+    using P = Px<DT>;
+    constexpr int NB = TH / 8;
     constexpr unsigned long long ALL = TH == 64 ? ~0ull : ((1ull << TH) - 1ull);
     constexpr unsigned long long TOP = 1ull, BOT = 1ull << (TH - 1);
+    const long long c0 = clock64();
+    unsigned sides = sm.sides, sweeps = 0u;
+    const bool ok = fetch_tile<DT, TH, 1>(sm.d, sm.tx, sm.ty, sm, 0, lane, phase, timeout_ns);
+    __syncwarp();
+    if (!ok) return false;
+    const long long c1 = clock64();
     const uint32_t edge_mask = lane == 0 ? P::FIRST_MASK : lane == 31 ? P::LAST_MASK : 0u;
-    unsigned long long pend_rows = 0ull;  // rows risen since the last flush
-    bool col_changed = false;             // a side column rose since the last flush (per lane)
-    unsigned sweeps = 0;
-    long long t_flush = 0;
-    // After a pass that raised a boundary, with more passes to come: publish
-    // early if the engine asks for it.
-    auto maybe_flush = [&](unsigned long long chg, bool col_now) {
-        if (!Early::kEnabled) return;
-        const bool boundary = (chg & (TOP | BOT)) != 0ull || __any_sync(FULL, col_now);
-        if (!boundary || !early.want(lane)) return;
-        const long long f0 = clock64();
-        write_back_rows<DT, TH>(d, sm, lane, y0, rows, npx, col_off, pend_rows);
-        const unsigned nb = detect_neighbours<DT, CONN, TH>(sm, lane, (pend_rows & TOP) != 0ull,
-                                                            (pend_rows & BOT) != 0ull, __any_sync(FULL, col_changed));
-        __syncwarp();
-        if (nb != 0u) early.flush(nb, lane);
-        pend_rows = 0ull;
-        col_changed = false;
-        t_flush += clock64() - f0;
-    };
-    // A revisit by the pixel queue when asked for; if it cannot finish, the
-    // passes take the tile with every row dirty.
+    unsigned long long rose = 0ull;  // rows that rose
+    bool col = false;                // a side column rose (per lane)
     bool solved = false;
-    bool run_passes = early.passes(lane);
-    if (early.pq() && sides != 0xffu) {
-        unsigned long long rows_chg = 0ull;
-        bool col_now = false;
+    if (solver == SOLVE_PQ && sides != 0xffu) {
+        // a revisit by the pixel queue; if it cannot finish, the sweeps take
+        // the tile with every row dirty
         unsigned rounds = 0u;
-        solved = pq_solve<DT, CONN, TH>(sm, lane, rows_chg, col_now, rounds);
+        unsigned long long mine = 0ull;
+        solved = pq_solve<DT, CONN, TH>(sm, lane, mine, col, rounds);
         __syncwarp();
-        const unsigned long long chg = warp_or64(rows_chg);
-        pend_rows |= chg;
-        col_changed |= col_now;
-        res.row_steps += rounds;
-        ++sweeps;
-        if (!solved) {
-            run_passes = true;
-            sides = 0xffu;
-        }
+        rose = warp_or64(mine);
+        row_steps += rounds;
+        sweeps += 1u;
+        if (!solved) sides = 0xffu;
     }
-    if (solved) {
-    } else if (!run_passes) {
-        // Rows whose halo inputs are new are processed by the first two
-        // sweeps: the top row by the raster sweep (N, NW, NE), the bottom row
-        // by the anti-raster sweep (S, SW, SE), every row when a side column
-        // that feeds the sweep changed (W, and E through the up-right /
-        // down-right diagonals for 8-connectivity; the reverse for the
-        // anti-raster sweep).  Other rows are skipped while nothing they
+    if (!solved) {
+        // Row sweeps, raster and anti-raster, until one after the first two
+        // changes nothing.  Rows whose halo inputs are new are processed by
+        // the first two sweeps: the top row by the raster sweep (N, NW, NE),
+        // the bottom row by the anti-raster sweep (S, SW, SE), every row when
+        // a side column that feeds the sweep changed (W, and E through the
+        // up-right / down-right diagonals for 8-connectivity; the reverse for
+        // the anti-raster sweep).  Other rows are skipped while nothing they
         // depend on has changed.
         const unsigned side_down = CONN == 8 ? (NB_W | NB_E) : NB_W;
         const unsigned side_up = CONN == 8 ? (NB_W | NB_E) : NB_E;
@@ -1237,83 +1511,45 @@ __device__ __forceinline__ VisitResult visit_tile(const ImgDesc& d, int tx, int 
             (sides & side_down) ? ALL : (sides & (NB_N | NB_NW | NB_NE)) ? TOP : 0ull;
         const unsigned long long force_up = (sides & side_up) ? ALL : (sides & (NB_S | NB_SW | NB_SE)) ? BOT : 0ull;
         unsigned long long chg_prev = 0ull;
-        for (;;) {
+        for (unsigned n = 0;; ++n) {
             unsigned long long dil = chg_prev | (chg_prev << 1) | (chg_prev >> 1);
-            if (sweeps == 0) dil |= force_down;
-            if (sweeps == 1) dil |= force_up;
+            if (n == 0) dil |= force_down;
+            if (n == 1) dil |= force_up;
             dil &= ALL;
             unsigned long long chg = 0ull;
-            bool col_now = false;
             if (dil != 0ull) {
-                if ((sweeps & 1u) == 0u)
-                    sweep<DT, CONN, TH, true>(sm, lane, dil, chg, col_now, edge_mask, res.row_steps);
+                if ((n & 1u) == 0u)
+                    sweep<DT, CONN, TH, true>(sm, lane, dil, chg, col, edge_mask, row_steps);
                 else
-                    sweep<DT, CONN, TH, false>(sm, lane, dil, chg, col_now, edge_mask, res.row_steps);
+                    sweep<DT, CONN, TH, false>(sm, lane, dil, chg, col, edge_mask, row_steps);
             }
-            ++sweeps;
-            pend_rows |= chg;
-            col_changed |= col_now;
+            sweeps += 1u;
+            rose |= chg;
             chg_prev = chg;
-            if (chg == 0ull && sweeps >= 2) break;
-            if (chg != 0ull) maybe_flush(chg, col_now);
-        }
-    } else {
-        // dVd / dVu: rows whose constraint towards the row above / below may
-        // be violated; dH: rows whose horizontal constraints may be violated.
-        // A first visit has every row dirty; a revisit only the rows fed by
-        // the halo sides that rose: N (and the N corners) the top row for the
-        // downward pass, S the bottom row for the upward pass, W / E every
-        // row for the horizontal pass and, with 8-connectivity, for both
-        // vertical passes (their diagonals read the side columns).
-        const bool fresh = sides == 0xffu;
-        const bool side_we = (sides & (NB_W | NB_E)) != 0u;
-        unsigned long long dVd = (sides & (NB_N | NB_NW | NB_NE)) ? TOP : 0ull;
-        unsigned long long dVu = (sides & (NB_S | NB_SW | NB_SE)) ? BOT : 0ull;
-        unsigned long long dH = side_we ? ALL : 0ull;
-        if (fresh || (CONN == 8 && side_we)) dVd = dVu = ALL;
-        for (int it = 0; (dVd | dVu | dH) != 0ull; it = (it + 1) & 3) {
-            unsigned long long chg;
-            bool col_now = false;
-            if (it == 0) {
-                if (dVd == 0ull) continue;
-                chg = vpass<DT, CONN, TH, true>(sm, lane, dVd, edge_mask, col_now, res.row_steps);
-                dVd = 0ull;
-                dVu |= chg >> 1;
-                dH |= chg;
-            } else if (it == 2) {
-                if (dVu == 0ull) continue;
-                chg = vpass<DT, CONN, TH, false>(sm, lane, dVu, edge_mask, col_now, res.row_steps);
-                dVu = 0ull;
-                dVd |= (chg << 1) & ALL;
-                dH |= chg;
-            } else {
-                if (dH == 0ull) continue;
-                chg = hpass<DT, TH>(sm, lane, dH, edge_mask, col_now, res.row_steps);
-                dH = 0ull;
-                dVd |= (chg << 1) & ALL;
-                dVu |= chg >> 1;
-            }
-            ++sweeps;
-            pend_rows |= chg;
-            col_changed |= col_now;
-            if (chg != 0ull && (dVd | dVu | dH) != 0ull) maybe_flush(chg, col_now);
+            if (chg == 0ull && n >= 1u) break;
         }
     }
-    res.sweeps = sweeps;
     const long long c2 = clock64();
-    res.t_proc = c2 - c1 - t_flush;
-    res.t_dump = t_flush;
-    if (pend_rows == 0ull) return res;  // nothing rose since the last flush: nothing to store or notify
-
-    // ---- write back the rows that rose, then neighbour detection
-    write_back_rows<DT, TH>(d, sm, lane, y0, rows, npx, col_off, pend_rows);
-    res.stored = true;
-    const unsigned nb = detect_neighbours<DT, CONN, TH>(sm, lane, (pend_rows & TOP) != 0ull,
-                                                        (pend_rows & BOT) != 0ull, __any_sync(FULL, col_changed));
+    const unsigned f_col = __any_sync(FULL, col) ? RF_COL : 0u;
+    unsigned nb = 0u;
+    for (int b = 0; b < NB; ++b) {
+        const unsigned rb = (unsigned)(rose >> (8 * b)) & 0xffu;
+        if (rb != 0u) write_back_block<DT, TH>(sm.d, sm, lane, b, sm.tx * 32 * P::PPW, sm.ty * TH);
+        if (rose != 0ull)
+            nb |= detect_neighbours<DT, CONN, TH>(sm, lane, b,
+                                                  ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col);
+    }
+    if (lane == 0) sm.nb = nb;
+    if (rose != 0ull) fence_gpu();
+    fence_proxy_async_smem();
     __syncwarp();
-    res.nb = nb;
-    res.t_dump += clock64() - c2;
-    return res;
+    if (lane == 0) {
+        sm.count.sweeps += sweeps;
+        sm.count.cycles[1] += c1 - c0;
+        sm.count.cycles[2] += c2 - c1;
+        sm.count.cycles[3] += clock64() - c2;
+    }
+    return true;
 }
 
 }  // namespace iwpp

@@ -1,5 +1,6 @@
 // iwpp_engine.cu -- device side of the persistent tile engine (see
 // iwpp_engine.cuh for the design and the reference citations).
+#include <atomic>
 #include <cstdio>
 
 #include "iwpp_engine.cuh"
@@ -20,6 +21,7 @@ __device__ __forceinline__ unsigned ring_base(const EngineArgs& a) {
 // Image of global tile g: the last image whose tile_base <= g.
 __device__ __forceinline__ int find_image(const EngineArgs& a, unsigned g) {
     int lo = 0, hi = a.nimg - 1;
+#pragma unroll 1
     while (lo < hi) {
         const int mid = (lo + hi + 1) >> 1;
         if ((unsigned)__ldg(&a.imgs[mid].tile_base) <= g)
@@ -30,28 +32,42 @@ __device__ __forceinline__ int find_image(const EngineArgs& a, unsigned g) {
     return lo;
 }
 
-template <int TH, class Early>
-__device__ __forceinline__ VisitResult dispatch_visit(const ImgDesc& d, int tx, int ty, WarpSmem<TH>& sm, int lane,
-                                                     unsigned& phase, long long timeout_ns, unsigned sides,
-                                                     Early& early) {
-    const int mode = d.dtype * 2 + (d.conn == 8 ? 1 : 0);
-    switch (mode) {
-        case 0: return visit_tile<DT_U8, 4, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
-        case 1: return visit_tile<DT_U8, 8, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
-        case 2: return visit_tile<DT_U16, 4, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
-        case 3: return visit_tile<DT_U16, 8, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
-        case 4: return visit_tile<DT_I32, 4, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
-        default: return visit_tile<DT_I32, 8, TH>(d, tx, ty, sm, lane, phase, timeout_ns, sides, early);
+// A tile's shared memory in a kernel, and its visit for one pixel type and
+// connectivity.
+template <int TH, bool ALT>
+struct SmemOf {
+    using T = TileSmem<TH>;
+};
+template <int TH>
+struct SmemOf<TH, true> {
+    using T = TileSmemAlt<TH>;
+};
+
+template <int TH, int W, bool ALT, int DT, int CONN, class SM>
+__device__ __forceinline__ bool visit_as(const EngineArgs& a, SM& sm, int warp, int lane, unsigned& phase,
+                                         unsigned& row_steps) {
+    if constexpr (ALT)
+        return visit_tile_alt<DT, CONN, TH>(sm, lane, phase, a.timeout_ns, a.solver == 3 ? SOLVE_PQ : SOLVE_SWEEPS,
+                                            row_steps);
+    else
+        return visit_tile<DT, CONN, TH, W>(sm, warp, lane, phase, a.timeout_ns, row_steps);
+}
+
+template <int TH, int W, bool ALT, class SM>
+__device__ __forceinline__ bool dispatch_visit(const EngineArgs& a, SM& sm, int warp, int lane, unsigned& phase,
+                                               unsigned& row_steps) {
+    switch (sm.d.dtype * 2 + (sm.d.conn == 8 ? 1 : 0)) {
+        case 0: return visit_as<TH, W, ALT, DT_U8, 4>(a, sm, warp, lane, phase, row_steps);
+        case 1: return visit_as<TH, W, ALT, DT_U8, 8>(a, sm, warp, lane, phase, row_steps);
+        case 2: return visit_as<TH, W, ALT, DT_U16, 4>(a, sm, warp, lane, phase, row_steps);
+        case 3: return visit_as<TH, W, ALT, DT_U16, 8>(a, sm, warp, lane, phase, row_steps);
+        case 4: return visit_as<TH, W, ALT, DT_I32, 4>(a, sm, warp, lane, phase, row_steps);
+        default: return visit_as<TH, W, ALT, DT_I32, 8>(a, sm, warp, lane, phase, row_steps);
     }
 }
 
 // The side of a neighbour tile that faces direction `dir` of this tile.
 __device__ __constant__ static const int kNbOpposite[8] = {1, 0, 3, 2, 7, 6, 5, 4};
-
-struct WarpCounters {
-    unsigned long long visits = 0, sweeps = 0, pushes = 0, row_steps = 0;
-    long long phase[5] = {0, 0, 0, 0, 0};  // queue read, fetch, processing, dump, queue write
-};
 
 // ---------------------------------------------------------------- mutex
 
@@ -115,7 +131,7 @@ __device__ __forceinline__ void mutex_unlock(const EngineArgs& a, unsigned ticke
 // write queue with one atomicAdd reservation per warp
 // (IWPP MP DQ/src/globalQueue.cu:14-47).  A short insertion sets the
 // overflow flag (the reference's memLeak, MR.cu:524-526); the tiles stay
-// DIRTY and are recovered by the restart.
+// DIRTY and are recovered by the restart.  push_entries returns their number.
 // The mutex stack's insertion: one lock acquisition for the warp's entries.
 // `counted`: `pending` already holds them (entries moving from a CTA
 // buffer); else they are added to it before the release can publish them.
@@ -150,10 +166,9 @@ __device__ void mutex_push_global(const EngineArgs& a, bool want, unsigned gn, i
 }
 
 template <int VAR>
-__device__ void push_entries(const EngineArgs& a, bool want, unsigned gn, int lane, unsigned* wq,
-                             WarpCounters& cnt) {
+__device__ int push_entries(const EngineArgs& a, bool want, unsigned gn, int lane, unsigned* wq) {
     const unsigned ballot = __ballot_sync(FULL, want);
-    if (ballot == 0u) return;
+    if (ballot == 0u) return 0;
     const int n = __popc(ballot);
     const int rank = __popc(ballot & ((1u << lane) - 1u));
     if (VAR == VAR_MUTEX) {
@@ -192,118 +207,110 @@ __device__ void push_entries(const EngineArgs& a, bool want, unsigned gn, int la
                 atomicExch(&a.ctrl->overflow, 1u);
         }
     }
-    cnt.pushes += (unsigned)n;
+    return n;
 }
 
 // ------------------------------------------------- mutex: CTA buffers
 // The MP discipline keeps one LIFO stack under one lock, and what
 // serialises it is one acquisition per insertion and per take.  Each CTA
-// therefore keeps the entries its warps insert in a shared-memory buffer and
-// takes from it first; the global stack sees a batch take when the buffer
-// runs dry, a spill when it fills, and a share when the global stack is empty
-// while warps elsewhere wait.  Buffered entries count in `pending`, so the
-// termination rule (nothing pending, nothing stacked) is unchanged.
+// therefore keeps the entries it inserts in a shared-memory buffer and takes
+// from it first; the global stack sees a batch take when the buffer runs dry,
+// a spill when it fills, and a share when the global stack is empty while
+// CTAs elsewhere wait.  Buffered entries count in `pending`, so the
+// termination rule (nothing pending, nothing stacked) is unchanged.  The
+// CTA's first warp alone works the queue, so the buffer needs no lock.
 constexpr int kCtaBuf = 64;    // entries a CTA buffers
 constexpr int kCtaSpill = 48;  // above this a push spills the buffer down to kCtaKeep
 constexpr int kCtaKeep = 16;
 
 struct MutexCtaBuf {
-    int lock;
     int n;
-    int taker;    // 1 while one of this CTA's warps works the global stack
-    int waiting;  // this CTA's warps waiting for work
     unsigned e[kCtaBuf];
 };
 __shared__ MutexCtaBuf s_cq;
-
-// The buffer's lock, held by one of this CTA's warps for a few shared-memory
-// accesses at a time; the bound is never reached in a working job.
-__device__ __forceinline__ bool cq_lock(const EngineArgs& a) {
-    unsigned spins = 0;
-    while (atomicCAS(&s_cq.lock, 0, 1) != 0) {
-        __nanosleep(32);
-        if (++spins > (1u << 22)) {
-            set_error(a.ctrl, DEV_ERR_TIMEOUT);
-            return false;
-        }
-    }
-    __threadfence_block();
-    return true;
-}
-__device__ __forceinline__ void cq_unlock() {
-    __threadfence_block();
-    atomicExch(&s_cq.lock, 0);
-}
 
 __device__ __forceinline__ int cq_count() { return *(volatile int*)&s_cq.n; }
 
 // Moves up to 32 of the buffer's newest entries beyond `keep` to the global
 // stack (one acquisition).
 __device__ void cta_spill(const EngineArgs& a, int lane, int keep) {
-    int m = 0, base = 0;
-    if (lane == 0 && cq_lock(a)) {
-        m = min(max(s_cq.n - keep, 0), 32);
-        s_cq.n -= m;
-        base = s_cq.n;
-        if (m == 0) cq_unlock();
-    }
-    m = __shfl_sync(FULL, m, 0);
-    base = __shfl_sync(FULL, base, 0);
+    const int n = cq_count();
+    const int m = min(max(n - keep, 0), 32);
     if (m == 0) return;
-    const unsigned mine = lane < m ? *(volatile unsigned*)&s_cq.e[base + lane] : 0u;
+    const unsigned mine = lane < m ? *(volatile unsigned*)&s_cq.e[n - m + lane] : 0u;
     __syncwarp();
-    if (lane == 0) cq_unlock();
+    if (lane == 0) s_cq.n = n - m;
+    __syncwarp();
     mutex_push_global(a, lane < m, mine, lane, true);
 }
 
 // Inserts the entries of the lanes with `want` set into this CTA's buffer
 // (what does not fit goes to the global stack), spilling a full buffer.
-// `counted`: `pending` already holds them.
-__device__ void cta_push(const EngineArgs& a, bool want, unsigned gn, int lane, WarpCounters& cnt,
-                         bool counted = false) {
+// `counted`: `pending` already holds them.  Returns their number.
+__device__ int cta_push(const EngineArgs& a, bool want, unsigned gn, int lane, bool counted = false) {
     const unsigned ballot = __ballot_sync(FULL, want);
-    if (ballot == 0u) return;
+    if (ballot == 0u) return 0;
     const int n = __popc(ballot);
     const int rank = __popc(ballot & ((1u << lane) - 1u));
-    int base = 0, k = 0;
-    bool locked = false;
-    if (lane == 0) {
-        if (!counted) atomicAdd(&a.ctrl->pending, n);  // before any of them can be taken
-        locked = cq_lock(a);
-        if (locked) {
-            k = min(n, kCtaBuf - s_cq.n);
-            base = s_cq.n;
-            s_cq.n += k;
-        }
-    }
-    k = __shfl_sync(FULL, k, 0);
-    base = __shfl_sync(FULL, base, 0);
+    if (lane == 0 && !counted) atomicAdd(&a.ctrl->pending, n);  // before any of them can be taken
+    const int base = cq_count();
+    const int k = min(n, kCtaBuf - base);
     if (want && rank < k) *(volatile unsigned*)&s_cq.e[base + rank] = gn;
     __syncwarp();
-    if (locked) cq_unlock();
-    if (!counted) cnt.pushes += (unsigned)n;
+    if (lane == 0) s_cq.n = base + k;
+    __syncwarp();
     if (n > k) mutex_push_global(a, want && rank >= k, gn, lane, true);
-    if (__shfl_sync(FULL, cq_count(), 0) > kCtaSpill) cta_spill(a, lane, kCtaKeep);
+    if (cq_count() > kCtaSpill) cta_spill(a, lane, kCtaKeep);
+    return n;
 }
 
 // The buffer's newest entry, or ~0u.
-__device__ unsigned cta_take(const EngineArgs& a, int lane) {
-    unsigned g = ~0u;
-    if (lane == 0 && cq_count() > 0 && cq_lock(a)) {
-        if (s_cq.n > 0) g = *(volatile unsigned*)&s_cq.e[--s_cq.n];
-        cq_unlock();
-    }
-    return __shfl_sync(FULL, g, 0);
+__device__ unsigned cta_take(int lane) {
+    const int n = cq_count();
+    if (n == 0) return ~0u;
+    const unsigned g = *(volatile unsigned*)&s_cq.e[n - 1];
+    __syncwarp();
+    if (lane == 0) s_cq.n = n - 1;
+    __syncwarp();
+    return g;
 }
 
-// Marks the neighbour tiles in `nb` DIRTY and inserts them (VAR_UNIQUE /
-// VAR_ASYNC: only those that were neither pending nor being visited).  With
-// the async queue one of the newly dirty tiles is not inserted but returned:
-// the warp visits it next itself, following the propagation front without a
-// trip through the queue.  Returns ~0u when there is none.
+// ------------------------------------------------------------ one entry
+// Takes tile g.  False: another CTA owns it (that owner sees DIRTY when it
+// releases).  *sides: the halo sides to look at, 0 for a tile that is not
+// DIRTY.  One exchange sets ACTIVE and takes DIRTY and the sides over; where
+// the tile was ACTIVE already (a duplicate entry), what the exchange took
+// goes back to the owner, and an owner that released the tile in between
+// leaves it to this CTA.
+__device__ __forceinline__ bool take_tile(const EngineArgs& a, unsigned g, int lane, unsigned* sides) {
+    unsigned old = 0u;
+    if (lane == 0) {
+        for (;;) {
+            old = atomicExch(&a.state[g], ST_ACTIVE);
+            const unsigned rest = old & (ST_DIRTY | ST_SIDES);
+            if (!(old & ST_ACTIVE) || rest == 0u) break;
+            if (atomicOr(&a.state[g], rest) & (ST_ACTIVE | ST_DIRTY)) break;
+        }
+        fence_gpu();  // acquire: neighbours' stores before their DIRTY
+    }
+    old = __shfl_sync(FULL, old, 0);
+    if (old & ST_ACTIVE) return false;
+    *sides = (old & ST_DIRTY) == 0u ? 0u : (old & ST_SIDES) != 0u ? (old & ST_SIDES) >> ST_SIDE_SHIFT : 0xffu;
+    return true;
+}
+
+// After a visit of tile (tx, ty) = g: marks the neighbour tiles in `nb`
+// DIRTY and inserts them (VAR_UNIQUE / VAR_ASYNC: only those that were
+// neither pending nor being visited), and releases g, inserting it again if
+// it was marked DIRTY meanwhile (next round for the double / unique queues;
+// not revisited at once with half-updated neighbours).  The atomics of all of
+// them are in flight together.  With the async queue and the mutex stack one
+// of the newly dirty neighbours is not inserted but returned: the CTA visits
+// it next itself, following the propagation front without a trip through the
+// queue.  Returns ~0u when there is none.
 template <int VAR>
-__device__ unsigned notify(const EngineArgs& a, const ImgDesc& d, int tx, int ty, unsigned nb, int lane, unsigned* wq,
-                           WarpCounters& cnt, bool keep_one = true) {
+__device__ __forceinline__ unsigned leave_tile(const EngineArgs& a, const ImgDesc& d, int tx, int ty, unsigned g,
+                                               unsigned nb, int lane, unsigned* wq, int* pushed) {
     bool want = false, fresh = false;
     unsigned gn = 0u;
     if (lane < 8 && ((nb >> lane) & 1u)) {
@@ -315,11 +322,12 @@ __device__ unsigned notify(const EngineArgs& a, const ImgDesc& d, int tx, int ty
             fresh = (old & (ST_DIRTY | ST_ACTIVE)) == 0u;
             want = (VAR == VAR_UNIQUE || VAR == VAR_ASYNC) ? fresh : true;
         }
+    } else if (lane == 8) {
+        gn = g;
+        want = (atomicAnd(&a.state[g], ~ST_ACTIVE) & ST_DIRTY) != 0u;
     }
     unsigned cont = ~0u;
-    if ((VAR == VAR_ASYNC || VAR == VAR_MUTEX) && keep_one) {
-        // one newly dirty neighbour is kept by this warp (its next visit)
-        // instead of going through the queue
+    if (VAR == VAR_ASYNC || VAR == VAR_MUTEX) {
         const unsigned ballot = __ballot_sync(FULL, want && fresh);
         if (ballot != 0u) {
             const int leader = __ffs(ballot) - 1;
@@ -327,123 +335,8 @@ __device__ unsigned notify(const EngineArgs& a, const ImgDesc& d, int tx, int ty
             if (lane == leader) want = false;
         }
     }
-    if (VAR == VAR_MUTEX)
-        cta_push(a, want, gn, lane, cnt);
-    else
-        push_entries<VAR>(a, want, gn, lane, wq, cnt);
+    *pushed = VAR == VAR_MUTEX ? cta_push(a, want, gn, lane) : push_entries<VAR>(a, want, gn, lane, wq);
     return cont;
-}
-
-// Early publication for the async queue: while many warps wait for work
-// (the job is bound by its propagation front), a visit that raised a
-// boundary of its tile stores what it has and notifies those neighbours at
-// once instead of after its last sweep, so they can start while this tile is
-// still converging.  While the warps are busy it would only add revisits.
-template <int VAR>
-struct EarlyFlush {
-    static constexpr bool kEnabled = VAR == VAR_ASYNC;
-    const EngineArgs* a;
-    const ImgDesc* d;
-    int tx, ty;
-    WarpCounters* cnt;
-    bool use_passes;  // in-tile solver of this visit
-    bool use_pq;      // revisits by the pixel queue
-    // Front-bound: more than half of the grid's warps have claimed a ring
-    // position that no producer has filled yet (they wait for work).  A
-    // quarter or an eighth switches too early on h-dome images, three
-    // quarters too late on long corridors.
-    __device__ static bool sample(const EngineArgs& a, int lane) {
-        unsigned v = 0u;
-        if (lane == 0) {
-            const unsigned head = ld_volatile(&a.ctrl->ahead), tail = ld_volatile(&a.ctrl->atail);
-            v = (int)(head - tail) > (int)(gridDim.x * (unsigned)kWarps / 2u) ? 1u : 0u;
-        }
-        return __shfl_sync(FULL, v, 0) != 0u;
-    }
-    __device__ bool passes(int) { return use_passes; }
-    __device__ bool pq() { return use_pq; }
-    __device__ bool want(int lane) { return sample(*a, lane); }
-    __device__ void flush(unsigned nb, int lane) {
-        __threadfence();  // release: the rows just stored before the neighbours' DIRTY
-        __syncwarp();
-        notify<VAR>(*a, *d, tx, ty, nb, lane, nullptr, *cnt, false);
-    }
-};
-
-// ------------------------------------------------------------ one entry
-// Takes tile g unless another warp owns it (that owner sees DIRTY when it
-// releases), visits it once if it is DIRTY, notifies the neighbours it
-// raised, and releases it; if it was marked DIRTY meanwhile it is queued
-// again (next round for the double / unique queues) instead of being
-// revisited at once with half-updated neighbours.
-template <int VAR, int TH>
-__device__ bool process_entry(const EngineArgs& a, unsigned g, WarpSmem<TH>& sm, int lane, unsigned* wq,
-                              WarpCounters& cnt, unsigned& phase, unsigned* next = nullptr) {
-    if (next) *next = ~0u;
-    unsigned old = 0u;
-    if (lane == 0) old = atomicOr(&a.state[g], ST_ACTIVE);
-    old = __shfl_sync(FULL, old, 0);
-    if (old & ST_ACTIVE) return true;
-    if (lane == 0) old = atomicAnd(&a.state[g], ~(ST_DIRTY | ST_SIDES));
-    old = __shfl_sync(FULL, old, 0);
-    if (old & ST_DIRTY) {
-        unsigned sides = (old & ST_SIDES) >> ST_SIDE_SHIFT;
-        if (sides == 0u) sides = 0xffu;
-        __threadfence();  // acquire: neighbours' stores before their DIRTY
-        __syncwarp();
-        const int ii = find_image(a, g);
-        const ImgDesc d = a.imgs[ii];
-        const int t = (int)(g - (unsigned)d.tile_base);
-        const int ty = t / d.tiles_x, tx = t - ty * d.tiles_x;
-        // In-tile solver: row sweeps (fewest instructions) while the warps
-        // are busy, passes (shortest latency) while many wait for work (async
-        // queue; the round-based queues use the sweeps unless told otherwise).
-        // Solver 3: revisits by the pixel queue, first visits by passes.
-        bool use_passes = a.solver == 2 || a.solver == 3;
-        if (a.solver == 0 && VAR == VAR_ASYNC) use_passes = EarlyFlush<VAR_ASYNC>::sample(a, lane);
-        const bool use_pq = a.solver == 3;
-        VisitResult r;
-        if (VAR == VAR_ASYNC) {
-            EarlyFlush<VAR> early{&a, &d, tx, ty, &cnt, use_passes, use_pq};
-            r = dispatch_visit<TH>(d, tx, ty, sm, lane, phase, a.timeout_ns, sides, early);
-        } else {
-            NoEarlyFlush early{use_passes, use_pq};
-            r = dispatch_visit<TH>(d, tx, ty, sm, lane, phase, a.timeout_ns, sides, early);
-        }
-        if (!r.ok) {
-            if (lane == 0) set_error(a.ctrl, DEV_ERR_TIMEOUT);
-            return false;
-        }
-        cnt.visits += 1;
-        cnt.sweeps += r.sweeps;
-        cnt.row_steps += r.row_steps;
-        cnt.phase[1] += r.t_fetch;
-        cnt.phase[2] += r.t_proc;
-        cnt.phase[3] += r.t_dump;
-        const long long q0 = clock64();
-        if (r.nb != 0u || r.stored) {
-            // release: this tile's stores before the neighbours' DIRTY and
-            // before the tile's ACTIVE bit clears (its next owner reads them)
-            __threadfence();
-            __syncwarp();
-        }
-        if (r.nb != 0u) {
-            const unsigned cont = notify<VAR>(a, d, tx, ty, r.nb, lane, wq, cnt);
-            if (next) *next = cont;
-        }
-        cnt.phase[4] += clock64() - q0;
-    }
-    const long long q1 = clock64();
-    if (lane == 0) old = atomicAnd(&a.state[g], ~ST_ACTIVE);
-    old = __shfl_sync(FULL, old, 0);
-    if (old & ST_DIRTY) {
-        if (VAR == VAR_MUTEX)
-            cta_push(a, lane == 0, g, lane, cnt);
-        else
-            push_entries<VAR>(a, lane == 0, g, lane, wq, cnt);
-    }
-    cnt.phase[4] += clock64() - q1;
-    return true;
 }
 
 // ------------------------------------------------------- mutex worker
@@ -455,7 +348,7 @@ __device__ bool process_entry(const EngineArgs& a, unsigned g, WarpSmem<TH>& sm,
 // entry, 1 when the job is over for this warp (finished or an error), 2 when
 // there is nothing to take now.  On overflow the quiescent stack is refilled
 // with every tile (MR.cu:785-806).
-__device__ int mutex_global_take(const EngineArgs& a, int lane, WarpCounters& cnt, unsigned* g) {
+__device__ int mutex_global_take(const EngineArgs& a, int lane, unsigned* g) {
     // Look before queueing for the lock: a ticket only while the stack holds
     // more entries than there are warps in line (a ticket lock serves in
     // arrival order, so warps queued for an empty stack would delay every
@@ -483,9 +376,7 @@ __device__ int mutex_global_take(const EngineArgs& a, int lane, WarpCounters& cn
             outcome = 1;
         } else {
             if (top > 0) {
-                const int want = *(volatile int*)&s_cq.waiting + 1;
-                n = top / (int)gridDim.x;
-                n = n < want ? want : n;
+                n = max(top / (int)gridDim.x, 1);
                 n = n > kMutexBatch ? kMutexBatch : n;
                 n = n > top ? top : n;
                 base = top - n;
@@ -531,80 +422,53 @@ __device__ int mutex_global_take(const EngineArgs& a, int lane, WarpCounters& cn
     __ballot_sync(FULL, mine == ~0u);
     if (lane == 0) mutex_unlock(a, ticket, base);
     *g = __shfl_sync(FULL, mine, 0);
-    cta_push(a, lane >= 1 && lane < n, mine, lane, cnt, true);
+    cta_push(a, lane >= 1 && lane < n, mine, lane, true);
     return 0;
 }
 
-// One persistent launch.  A warp takes its next entry from its CTA's buffer;
-// when that is empty, one warp of the CTA at a time takes a batch from the
-// global LIFO stack for the CTA (mutex_global_take) while the others wait
-// for it.  Termination: nothing is stacked and no inserted entry is
-// unfinished (`pending` == 0, buffered entries included), which replaces
+// The queues, as the CTA's first warp works them: get() finds the next entry
+// (false when the job is over or failed), done() counts it finished after its
+// visit and those of the neighbours that the CTA went on to.
+
+// One persistent launch.  The next entry comes from the CTA's buffer; when
+// that is empty, a batch is taken from the global LIFO stack
+// (mutex_global_take).  Termination: nothing is stacked and no inserted entry
+// is unfinished (`pending` == 0, buffered entries included), which replaces
 // activeBlocksCount (IWPP MP/src/globalQueue.cu:134-145).
-template <int TH>
-__device__ void mutex_worker(const EngineArgs& a, WarpSmem<TH>& sm, int lane, WarpCounters& cnt, unsigned& phase) {
-    if (threadIdx.x == 0) {
-        s_cq.lock = 0;
-        s_cq.n = 0;
-        s_cq.taker = 0;
-        s_cq.waiting = 0;
-    }
-    __syncthreads();
+struct MutexQueue {
+    static constexpr int VAR = VAR_MUTEX;
+    unsigned* wq = nullptr;
+    unsigned ns = 64;
+
     // this CTA's slice of the initial stack, without the lock (it lies above
     // the stack's top, and `pending` counts it already); the lowest position
     // ends on the buffer's top, so it is taken first, as from the stack
-    {
+    __device__ void start(const EngineArgs& a, int lane) {
         const unsigned pf = ld_volatile(&a.ctrl->prefill);
         const unsigned base = ld_volatile(&a.ctrl->prefill_base) + blockIdx.x * pf;
-        for (unsigned j = threadIdx.x; j < pf; j += blockDim.x)
-            s_cq.e[j] = __ldcg(&a.q0[base + pf - 1u - j]);
-        if (threadIdx.x == 0) s_cq.n = (int)pf;
-        __syncthreads();
+        for (unsigned j = (unsigned)lane; j < pf; j += 32u) s_cq.e[j] = __ldcg(&a.q0[base + pf - 1u - j]);
+        if (lane == 0) s_cq.n = (int)pf;
+        __syncwarp();
     }
-    long long idle_since = 0;
-    unsigned idle_progress = 0u;
-    unsigned ns = 64;
-    bool idle = false;  // counted in ctrl->idle and s_cq.waiting
-    auto leave_idle = [&]() {
-        if (idle && lane == 0) {
-            atomicSub(&a.ctrl->idle, 1u);
-            atomicSub(&s_cq.waiting, 1);
-        }
-        idle = false;
-    };
-    for (;;) {
-        if (ld_volatile(&a.ctrl->error) != 0u) break;
-        const long long qr0 = clock64();
-        unsigned g = cta_take(a, lane);
-        int outcome = 0;  // 0 an entry, 1 exit, 2 nothing now
-        if (g == ~0u) {
-            int taker = 0;
-            if (lane == 0) taker = atomicCAS(&s_cq.taker, 0, 1) == 0 ? 1 : 0;
-            taker = __shfl_sync(FULL, taker, 0);
-            if (taker) {
-                outcome = mutex_global_take(a, lane, cnt, &g);
-                __syncwarp();
-                if (lane == 0) atomicExch(&s_cq.taker, 0);
-            } else {
-                // another warp of this CTA is at the global stack: wait for
-                // its batch, leaving when the job is over
-                int over = 0;
-                if (lane == 0)
-                    over = ld_volatile(&a.ctrl->pending) == 0 && stack_top(a.ctrl) == 0 &&
-                           ld_volatile(&a.ctrl->overflow) == 0u;
-                outcome = __shfl_sync(FULL, over, 0) ? 1 : 2;
+    __device__ bool get(const EngineArgs& a, int lane, unsigned* out) {
+        long long idle_since = 0;
+        unsigned idle_progress = 0u;
+        bool idle = false, got = false;  // idle: counted in ctrl->idle
+        ns = 64;
+        for (;;) {
+            if (ld_volatile(&a.ctrl->error) != 0u) break;
+            unsigned g = cta_take(lane);
+            const int outcome = g != ~0u ? 0 : mutex_global_take(a, lane, &g);
+            if (outcome == 1) break;
+            if (outcome == 0) {
+                got = g < a.G;
+                if (!got && lane == 0) set_error(a.ctrl, DEV_ERR_INTERNAL);  // an entry that names no tile
+                *out = g;
+                break;
             }
-        }
-        if (outcome == 1) break;
-        if (outcome == 2) {
             // nothing to take but work in flight: back off, bounded by progress
-            if (!idle) {
-                if (lane == 0) {
-                    atomicAdd(&a.ctrl->idle, 1u);
-                    atomicAdd(&s_cq.waiting, 1);
-                }
-                idle = true;
-            }
+            if (!idle && lane == 0) atomicAdd(&a.ctrl->idle, 1u);
+            idle = true;
             const unsigned prog = ld_volatile(&a.ctrl->progress);
             const long long now = globaltimer_ns();
             if (idle_since == 0 || prog != idle_progress) {
@@ -616,126 +480,117 @@ __device__ void mutex_worker(const EngineArgs& a, WarpSmem<TH>& sm, int lane, Wa
             }
             __nanosleep(ns);
             if (ns < 2048) ns <<= 1;
-            cnt.phase[0] += clock64() - qr0;
-            continue;
         }
-        leave_idle();
-        idle_since = 0;
-        ns = 64;
-        cnt.phase[0] += clock64() - qr0;
-        if (g >= a.G) {  // a consistency check: an entry names no tile
-            if (lane == 0) set_error(a.ctrl, DEV_ERR_INTERNAL);
-            break;
-        }
-        bool ok = true;
-        for (;;) {  // the entry, then the newly dirty neighbours it leaves behind
-            unsigned nxt = ~0u;
-            ok = process_entry<VAR_MUTEX, TH>(a, g, sm, lane, nullptr, cnt, phase, &nxt);
-            if (!ok || nxt == ~0u) break;
-            g = nxt;
-        }
-        if (!ok) break;
+        if (idle && lane == 0) atomicSub(&a.ctrl->idle, 1u);
+        return __shfl_sync(FULL, got ? 1 : 0, 0) != 0;
+    }
+    __device__ void done(const EngineArgs& a, int lane) {
         if (lane == 0) {
-            __threadfence();
             atomicAdd(&a.ctrl->progress, 1u);
             atomicSub(&a.ctrl->pending, 1);  // after this entry's insertions
         }
-        // share: the global stack is empty while warps elsewhere wait
+        // share: the global stack is empty while CTAs elsewhere wait
         int share = 0;
-        if (lane == 0 && cq_count() >= 2 && stack_top(a.ctrl) == 0 &&
-            ld_volatile(&a.ctrl->idle) > (unsigned)*(volatile int*)&s_cq.waiting)
-            share = 1;
-        if (__shfl_sync(FULL, share, 0)) cta_spill(a, lane, __shfl_sync(FULL, cq_count(), 0) / 2);
+        if (lane == 0 && cq_count() >= 2 && stack_top(a.ctrl) == 0 && ld_volatile(&a.ctrl->idle) > 0u) share = 1;
+        if (__shfl_sync(FULL, share, 0)) cta_spill(a, lane, cq_count() / 2);
     }
-    leave_idle();
-}
+};
 
-// ------------------------------------------------------- async worker
 // Ring positions 0..n0-1 are the initial tiles (no storage: every tile in
 // id order, or the seed list after the front stage); position p >= n0 lives in
-// slot (p - n0) % cap.  A warp claims the next position with one
-// atomicAdd and waits for a producer to fill it.  Every filled position is
-// claimed by exactly one warp, and when `pending` (filled, unfinished
-// entries) reaches zero no producer is left, so waiting warps leave.
-template <int TH>
-__device__ void async_worker(const EngineArgs& a, WarpSmem<TH>& sm, int lane, WarpCounters& cnt, unsigned& phase) {
-    const unsigned n0 = ring_base(a);
-    for (;;) {
-        const long long qr0 = clock64();
+// slot (p - n0) % cap.  A CTA claims the next position with one atomicAdd and
+// waits for a producer to fill it.  Every filled position is claimed by
+// exactly one CTA, and when `pending` (filled, unfinished entries) reaches
+// zero no producer is left: the CTA that finishes the last entry sets `done`
+// and fills the slots that CTAs wait at with kRingEnd, so a waiting CTA
+// watches its own slot and hardly ever the job's counters.
+constexpr unsigned kRingEnd = 0xffffffffu;
+
+struct AsyncQueue {
+    static constexpr int VAR = VAR_ASYNC;
+    unsigned* wq = nullptr;
+    unsigned n0 = 0;
+
+    __device__ void start(const EngineArgs& a, int) { n0 = ring_base(a); }
+    __device__ bool get(const EngineArgs& a, int lane, unsigned* out) {
         unsigned p = 0u;
         if (lane == 0) p = atomicAdd(&a.ctrl->ahead, 1u);
         p = __shfl_sync(FULL, p, 0);
-        unsigned g = a.init_list && p < n0 ? __ldcg(&a.init_list[p]) : p;
-        if (p >= n0) {
-            int outcome = 0;  // 0 got an entry, 1 exit
-            unsigned v = 0u;
-            if (lane == 0) {
-                const unsigned slot = (p - n0) % a.cap;
-                long long idle_since = globaltimer_ns();
-                unsigned idle_progress = ld_volatile(&a.ctrl->progress);
-                unsigned ns = 32, spins = 0;
-                for (;;) {
-                    // The slot is this warp's alone: watch it with plain loads
-                    // (a waiting warp issues no atomics) and take it once set.
-                    if (ld_volatile(&a.q0[slot]) != 0u) {
-                        v = atomicExch(&a.q0[slot], 0u);
+        if (p < n0) {
+            *out = a.init_list ? __ldcg(&a.init_list[p]) : p;
+            return true;
+        }
+        unsigned v = 0u;
+        if (lane == 0) {
+            const unsigned slot = (p - n0) % a.cap;
+            long long idle_since = globaltimer_ns();
+            unsigned idle_progress = 0u;
+            unsigned ns = 32, spins = 0;
+            for (;;) {
+                // The slot is this CTA's alone: watch it with plain loads (a
+                // waiting CTA issues no atomics) and take it once set.
+                if (ld_volatile(&a.q0[slot]) != 0u) {
+                    v = atomicExch(&a.q0[slot], 0u);
+                    break;
+                }
+                // the end of the job at the first look and now and then,
+                // progress (for the bound on the wait) rarely
+                if ((spins & 15u) == 0u && (ld_volatile(&a.ctrl->done) != 0u || ld_volatile(&a.ctrl->error) != 0u)) {
+                    v = kRingEnd;
+                    break;
+                }
+                if ((++spins & 63u) == 0u) {
+                    const unsigned prog = ld_volatile(&a.ctrl->progress);
+                    const long long now = globaltimer_ns();
+                    if (prog != idle_progress) {
+                        idle_progress = prog;
+                        idle_since = now;
+                    } else if (now - idle_since > a.timeout_ns) {
+                        set_error(a.ctrl, DEV_ERR_TIMEOUT);
+                        v = kRingEnd;
                         break;
                     }
-                    // the job's counters every eighth look
-                    if ((++spins & 7u) == 0u) {
-                        if (ld_volatile(&a.ctrl->pending) == 0 || ld_volatile(&a.ctrl->error) != 0u) {
-                            outcome = 1;
-                            break;
-                        }
-                        const unsigned prog = ld_volatile(&a.ctrl->progress);
-                        const long long now = globaltimer_ns();
-                        if (prog != idle_progress) {
-                            idle_progress = prog;
-                            idle_since = now;
-                        } else if (now - idle_since > a.timeout_ns) {
-                            set_error(a.ctrl, DEV_ERR_TIMEOUT);
-                            outcome = 1;
-                            break;
-                        }
-                    }
-                    __nanosleep(ns);
-                    if (ns < 256) ns <<= 1;
                 }
+                __nanosleep(ns);
+                if (ns < 256) ns <<= 1;
             }
-            outcome = __shfl_sync(FULL, outcome, 0);
-            cnt.phase[0] += clock64() - qr0;
-            if (outcome) return;
-            g = __shfl_sync(FULL, v, 0) - 1u;
-        } else {
-            cnt.phase[0] += clock64() - qr0;
         }
-        // visit the entry, then keep following the front while the visits
-        // leave a newly dirty neighbour behind
-        bool ok = true;
-        for (;;) {
-            unsigned nxt = ~0u;
-            ok = process_entry<VAR_ASYNC, TH>(a, g, sm, lane, nullptr, cnt, phase, &nxt);
-            if (!ok || nxt == ~0u) break;
-            g = nxt;
-        }
-        if (lane == 0) {
-            __threadfence();
-            atomicAdd(&a.ctrl->progress, 1u);
-            atomicSub(&a.ctrl->pending, 1);  // after this entry's insertions
-        }
-        if (!ok) return;
+        v = __shfl_sync(FULL, v, 0);
+        *out = v - 1u;
+        return v != kRingEnd;
     }
-}
+    __device__ void done(const EngineArgs& a, int lane) {
+        unsigned last = 0u, from = 0u, to = 0u;
+        if (lane == 0) {
+            atomicAdd(&a.ctrl->progress, 1u);
+            // after this entry's insertions, which counted themselves first
+            last = atomicSub(&a.ctrl->pending, 1) == 1 ? 1u : 0u;
+            if (last) {
+                // `done` first: a CTA that claims a position after `ahead` is
+                // read here sees it at its first look
+                atomicExch(&a.ctrl->done, 1u);
+                __threadfence();
+                from = ld_volatile(&a.ctrl->atail);
+                to = ld_volatile(&a.ctrl->ahead);
+            }
+        }
+        if (!__shfl_sync(FULL, last, 0)) return;
+        from = __shfl_sync(FULL, from, 0);
+        to = __shfl_sync(FULL, to, 0);
+        // at most one claimed position per CTA of the grid, fewer than `cap`
+        for (unsigned p = from + (unsigned)lane; (int)(to - p) > 0; p += 32u)
+            *(volatile unsigned*)&a.q0[(p - n0) % a.cap] = kRingEnd;
+    }
+};
 
 // --------------------------------------------------------- grid barrier
 // All CTAs of the (cooperative) launch.  The last CTA to arrive performs the
 // round transition.  Waits are bounded; returns false when the job failed.
 __device__ bool grid_barrier_round(const EngineArgs& a) {
-    __shared__ int s_ok;
-    __syncthreads();
+    int ok = 1;
+    __syncwarp();
     if (threadIdx.x == 0) {
         Ctrl* c = a.ctrl;
-        int ok = 1;
         const unsigned gen = ld_volatile(&c->bar_gen);
         __threadfence();
         const unsigned arrived = atomicAdd(&c->bar_count, 1u);
@@ -789,69 +644,163 @@ __device__ bool grid_barrier_round(const EngineArgs& a) {
             }
             __threadfence();
         }
-        s_ok = ok;
     }
-    __syncthreads();
-    return s_ok != 0;
+    return __shfl_sync(FULL, ok, 0) != 0;
 }
 
-// ------------------------------------------------------- round worker
-template <int VAR, int TH>
-__device__ void round_worker(const EngineArgs& a, WarpSmem<TH>& sm, int lane, WarpCounters& cnt, unsigned& phase) {
-    for (;;) {
-        const unsigned rn = ld_volatile(&a.ctrl->rn);
-        const unsigned vfull = ld_volatile(&a.ctrl->vfull);
-        const unsigned qsel = ld_volatile(&a.ctrl->qsel);
-        const unsigned* rq = qsel ? a.q1 : a.q0;
-        unsigned* wq = qsel ? a.q0 : a.q1;
+// ------------------------------------------------------- round queues
+template <int V>
+struct RoundQueue {
+    static constexpr int VAR = V;
+    unsigned* wq = nullptr;
+    unsigned rn = 0, vfull = 0;
+
+    __device__ void start(const EngineArgs& a, int) {
+        rn = ld_volatile(&a.ctrl->rn);
+        vfull = ld_volatile(&a.ctrl->vfull);
+        wq = ld_volatile(&a.ctrl->qsel) ? a.q0 : a.q1;
+    }
+    __device__ bool get(const EngineArgs& a, int lane, unsigned* out) {
         for (;;) {
-            const long long qr0 = clock64();
             unsigned idx = 0u;
             if (lane == 0) idx = atomicAdd(&a.ctrl->rcur, 1u);
             idx = __shfl_sync(FULL, idx, 0);
-            cnt.phase[0] += clock64() - qr0;
-            if (idx >= rn) break;
-            if (ld_volatile(&a.ctrl->error) != 0u) break;
-            const unsigned g = vfull ? idx : __ldcg(&rq[idx]);
-            if (!process_entry<VAR, TH>(a, g, sm, lane, wq, cnt, phase)) break;
+            if (idx < rn) {
+                *out = vfull ? idx : __ldcg(&(wq == a.q0 ? a.q1 : a.q0)[idx]);
+                return true;
+            }
+            if (!grid_barrier_round(a)) return false;
+            if (ld_volatile(&a.ctrl->done) != 0u) return false;
+            start(a, lane);
         }
-        const long long qb0 = clock64();
-        const bool ok_barrier = grid_barrier_round(a);
-        cnt.phase[0] += clock64() - qb0;
-        if (!ok_barrier) return;
-        if (ld_volatile(&a.ctrl->done) != 0u) return;
     }
-}
+    __device__ void done(const EngineArgs&, int) {}
+};
+
+template <int VAR>
+struct QueueOf {
+    using T = RoundQueue<VAR>;
+};
+template <>
+struct QueueOf<VAR_MUTEX> {
+    using T = MutexQueue;
+};
+template <>
+struct QueueOf<VAR_ASYNC> {
+    using T = AsyncQueue;
+};
 
 // --------------------------------------------------------------- kernels
-template <int VAR, int TH>
-__global__ void __launch_bounds__(kWarps * 32) engine_kernel(EngineArgs a) {
+// A CTA of W warps works on one tile at a time.  Its first warp runs the
+// queue and hands the tile to the CTA's warps through shared memory.  ALT:
+// the kernels with the alternative in-tile solvers, apart so that their
+// registers and code cost the passes nothing.  Registers: 24 warps per SM (80
+// registers) with four and eight warps per tile, 20 (96) with two, whose loop
+// over a warp's blocks needs them; 16 and 32 warps measured the same or
+// slower (32: a fifth slower, spills).
+template <int VAR, int TH, int W, bool ALT>
+__global__ void __launch_bounds__(32 * W, ALT ? 8 : W == 2 ? 10 : 24 / W) engine_kernel(EngineArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // 128-byte align the per-warp areas (the launch adds 128 bytes of slack)
+    // 128-byte align the tile (the launch adds 128 bytes of slack)
     const uint32_t base = smem_u32(smem_raw);
-    unsigned char* aligned = smem_raw + ((128u - (base & 127u)) & 127u);
-    WarpSmem<TH>& sm = reinterpret_cast<WarpSmem<TH>*>(aligned)[warp];
-    if (lane == 0) {
+    using Smem = typename SmemOf<TH, ALT>::T;
+    Smem& sm = *reinterpret_cast<Smem*>(smem_raw + ((128u - (base & 127u)) & 127u));
+    if (threadIdx.x == 0) {
         mbar_init(&sm.mbar, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        sm.nb = 0u;
+        sm.count = VisitCount{};
+        if (a.nimg == 1) sm.d = a.one;
+        else sm.d = a.imgs[0];
     }
-    __syncthreads();
-    unsigned phase = 0u;
-    WarpCounters cnt;
-    if (VAR == VAR_MUTEX)
-        mutex_worker<TH>(a, sm, lane, cnt, phase);
-    else if (VAR == VAR_ASYNC)
-        async_worker<TH>(a, sm, lane, cnt, phase);
-    else
-        round_worker<VAR, TH>(a, sm, lane, cnt, phase);
+    if (lane == 0) sm.mark[0][warp][0] = sm.mark[0][warp][1] = sm.mark[1][warp][0] = sm.mark[1][warp][1] = 0u;
+    cta_sync<W>();
+    unsigned phase = 0u, row_steps = 0u;
+    typename QueueOf<VAR>::T queue;
+    if (warp == 0) queue.start(a, lane);
+    bool visited = false;  // first warp: tile g was visited
+    unsigned g = 0u;
+    for (;;) {
+        if (warp == 0) {
+            bool have = false, found = false;  // an entry in hand (g); a tile to visit (g)
+            unsigned sides = 0u;
+            if (visited) {
+                const long long q0 = clock64();
+                const unsigned nb = sm.nb;
+                __syncwarp();
+                if (lane == 0) sm.nb = 0u;
+                int pushed = 0;
+                const unsigned cont = leave_tile<VAR>(a, sm.d, sm.tx, sm.ty, g, nb, lane, queue.wq, &pushed);
+                if (lane == 0) {
+                    sm.count.cycles[4] += clock64() - q0;
+                    sm.count.visits += 1u;
+                    sm.count.pushes += (unsigned)pushed;
+                }
+                if (cont != ~0u) {
+                    g = cont;
+                    have = true;
+                } else {
+                    queue.done(a, lane);
+                }
+            }
+            const long long q0 = clock64();
+            while (have || queue.get(a, lane, &g)) {
+                have = false;
+                if (take_tile(a, g, lane, &sides)) {
+                    if (sides != 0u) {
+                        found = true;
+                        break;
+                    }
+                    // not DIRTY: released at once, unless it became so
+                    bool again = false;
+                    if (lane == 0) again = (atomicAnd(&a.state[g], ~ST_ACTIVE) & ST_DIRTY) != 0u;
+                    const int pushed =
+                        VAR == VAR_MUTEX ? cta_push(a, again, g, lane) : push_entries<VAR>(a, again, g, lane, queue.wq);
+                    if (lane == 0) sm.count.pushes += (unsigned)pushed;
+                }
+                queue.done(a, lane);
+            }
+            if (found && a.nimg != 1 &&
+                !(g - (unsigned)sm.d.tile_base < (unsigned)(sm.d.tiles_x * sm.d.tiles_y))) {
+                // another image of the batch
+                const int ii = find_image(a, g);
+                __syncwarp();
+                const unsigned* src = reinterpret_cast<const unsigned*>(&a.imgs[ii]);
+                if (lane < (int)(sizeof(ImgDesc) / 4)) reinterpret_cast<unsigned*>(&sm.d)[lane] = __ldg(&src[lane]);
+                __syncwarp();
+            }
+            if (found) {
+                const int t = (int)(g - (unsigned)sm.d.tile_base), ty = t / sm.d.tiles_x;
+                if (lane == 0) {
+                    sm.ty = ty;
+                    sm.tx = t - ty * sm.d.tiles_x;
+                    sm.sides = sides;
+                }
+            }
+            if (lane == 0) {
+                sm.go = found ? 1u : 0u;
+                sm.count.cycles[0] += clock64() - q0;
+            }
+            visited = found;
+        }
+        cta_sync<W>();
+        if (sm.go == 0u) break;
+        if (!dispatch_visit<TH, W, ALT>(a, sm, warp, lane, phase, row_steps)) {
+            if (threadIdx.x == 0) set_error(a.ctrl, DEV_ERR_TIMEOUT);
+            break;
+        }
+    }
     if (lane == 0) {
-        if (cnt.visits) atomicAdd(&a.ctrl->visits, cnt.visits);
-        if (cnt.sweeps) atomicAdd(&a.ctrl->sweeps, cnt.sweeps);
-        if (cnt.pushes) atomicAdd(&a.ctrl->pushes, cnt.pushes);
-        if (cnt.row_steps) atomicAdd(&a.ctrl->row_steps, cnt.row_steps);
-        for (int i = 0; i < 5; ++i)
-            if (cnt.phase[i] > 0) atomicAdd(&a.ctrl->phase[i], (unsigned long long)cnt.phase[i]);
+        if (row_steps) atomicAdd(&a.ctrl->row_steps, (unsigned long long)row_steps);
+        if (warp == 0) {
+            const VisitCount& c = sm.count;
+            if (c.visits) atomicAdd(&a.ctrl->visits, (unsigned long long)c.visits);
+            if (c.sweeps) atomicAdd(&a.ctrl->sweeps, (unsigned long long)c.sweeps);
+            if (c.pushes) atomicAdd(&a.ctrl->pushes, (unsigned long long)c.pushes);
+            for (int i = 0; i < 5; ++i)
+                if (c.cycles[i] > 0) atomicAdd(&a.ctrl->phase[i], (unsigned long long)c.cycles[i]);
+        }
     }
 }
 
@@ -881,7 +830,7 @@ __global__ void engine_init_kernel(EngineArgs a, int variant) {
         c->rcur = 0u;
         c->qsel = 0u;
         c->vfull = seeded ? 0u : 1u;
-        c->done = n0 == 0u ? 1u : 0u;
+        c->done = n0 == 0u && !a.phantom ? 1u : 0u;
         c->overflow = n0 > a.cap && variant == VAR_MUTEX ? 1u : 0u;
         c->restarts = 0u;
         c->rounds = 0u;
@@ -964,13 +913,12 @@ __global__ void queue_test_insert_kernel(EngineArgs a, int copies) {
     const unsigned warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
     const unsigned total = a.G * (unsigned)copies;
-    WarpCounters cnt;
     for (unsigned base = warp * 32u; base < total; base += nwarps * 32u) {
         const unsigned idx = base + (unsigned)lane;
         bool want = idx < total;
         const unsigned g = want ? idx % a.G : 0u;
         if (VAR == VAR_UNIQUE && want) want = (atomicOr(&a.state[g], ST_DIRTY) & ST_DIRTY) == 0u;
-        push_entries<VAR>(a, want, g, lane, a.q1, cnt);
+        push_entries<VAR>(a, want, g, lane, a.q1);
         if (ld_volatile(&a.ctrl->error) != 0u) return;
     }
 }
@@ -1020,41 +968,86 @@ cudaError_t queue_selftest(const EngineArgs& a, int variant, int copies, unsigne
 }
 
 // ------------------------------------------------------------ host side
-template <int VAR, int TH>
-static void* kernel_ptr() {
-    return reinterpret_cast<void*>(&engine_kernel<VAR, TH>);
+template <int TH, int W, bool ALT>
+static void* select_variant(int variant) {
+    if (variant == VAR_MUTEX) return reinterpret_cast<void*>(&engine_kernel<VAR_MUTEX, TH, W, ALT>);
+    if (variant == VAR_DOUBLE) return reinterpret_cast<void*>(&engine_kernel<VAR_DOUBLE, TH, W, ALT>);
+    if (variant == VAR_ASYNC) return reinterpret_cast<void*>(&engine_kernel<VAR_ASYNC, TH, W, ALT>);
+    return reinterpret_cast<void*>(&engine_kernel<VAR_UNIQUE, TH, W, ALT>);
 }
 
-static void* select_kernel(int variant, int tile_rows) {
-    if (tile_rows == 32) {
-        if (variant == VAR_MUTEX) return kernel_ptr<VAR_MUTEX, 32>();
-        if (variant == VAR_DOUBLE) return kernel_ptr<VAR_DOUBLE, 32>();
-        if (variant == VAR_ASYNC) return kernel_ptr<VAR_ASYNC, 32>();
-        return kernel_ptr<VAR_UNIQUE, 32>();
+// The engine's kernel shapes: tile height, warps per tile, and whether it has
+// the alternative in-tile solvers.
+enum Shape : int { T32_W4, T64_W8, T64_W4, T64_W2, T32_ALT, T64_ALT, SHAPES };
+
+// Shape of a job's kernel.  solver: iwpp_config.solver (0 and 2 are the
+// passes, 1 and 3 the kernels with the alternative solvers).  Warps per tile:
+// the fewer tiles an SM has, the more warps work on one, since only a part
+// of a job's tiles can be visited at any time and a visit's length then sets
+// the pace; with many tiles the warps that wait for others of their tile cost
+// more.  Measured on h-dome images, 8 / 4 / 2 warps per 64-row tile, us:
+//   tiles per SM   0.8 (1024^2 u8)  68 / 76 / 86
+//                  3.4 (2048^2 u8)  88 / 90 / 99
+//                  7.6 (3072^2 u8)  126 / 113 / 116
+//                 13.5 (4096^2 u8)  195 / 152 / 144, 8-connected 366 / 331 / 322
+//                 30   (6144^2 u8)  400 / 298 / 256
+//                 54   (8192^2 u8)  791 / 561 / 453
+static Shape select_shape(int tile_rows, int solver, long long tiles, int sms) {
+    const bool alt = solver == 1 || solver == 3;
+    if (tile_rows == 32) return alt ? T32_ALT : T32_W4;
+    if (alt) return T64_ALT;
+    return 4 * tiles <= 27ll * sms ? T64_W8 : 2 * tiles <= 25ll * sms ? T64_W4 : T64_W2;
+}
+
+struct Kernel {
+    void* fn;
+    int threads;
+    size_t smem;
+};
+static Kernel kernel_of(int variant, Shape shape) {
+    constexpr size_t slack = 128;
+    switch (shape) {
+        case T32_W4: return {select_variant<32, 4, false>(variant), 128, slack + sizeof(TileSmem<32>)};
+        case T64_W8: return {select_variant<64, 8, false>(variant), 256, slack + sizeof(TileSmem<64>)};
+        case T64_W4: return {select_variant<64, 4, false>(variant), 128, slack + sizeof(TileSmem<64>)};
+        case T64_W2: return {select_variant<64, 2, false>(variant), 64, slack + sizeof(TileSmem<64>)};
+        case T32_ALT: return {select_variant<32, 1, true>(variant), 32, slack + sizeof(TileSmemAlt<32>)};
+        default: return {select_variant<64, 1, true>(variant), 32, slack + sizeof(TileSmemAlt<64>)};
     }
-    if (variant == VAR_MUTEX) return kernel_ptr<VAR_MUTEX, 64>();
-    if (variant == VAR_DOUBLE) return kernel_ptr<VAR_DOUBLE, 64>();
-    if (variant == VAR_ASYNC) return kernel_ptr<VAR_ASYNC, 64>();
-    return kernel_ptr<VAR_UNIQUE, 64>();
+}
+// below the size from which a kernel has to ask for its shared memory
+static_assert(128 + sizeof(TileSmemAlt<64>) <= 48 * 1024, "dynamic shared memory");
+
+// Multiprocessors of a device (asked once), 0 when it cannot be asked.
+int engine_sm_count(int device) {
+    static std::atomic<int> cache[64];
+    if (device < 0 || device >= 64) return 0;
+    int n = cache[device].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        cache[device].store(n, std::memory_order_relaxed);
+    }
+    return n;
 }
 
-static size_t smem_bytes(int tile_rows) {
-    return 128 + (tile_rows == 32 ? kWarps * sizeof(WarpSmem<32>) : kWarps * sizeof(WarpSmem<64>));
-}
-
-cudaError_t engine_prepare(int variant, int tile_rows, int device, LaunchInfo* li) {
-    void* k = select_kernel(variant, tile_rows);
-    const size_t smem = smem_bytes(tile_rows);
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    int per_sm = 0, sms = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kWarps * 32, smem);
-    if (e != cudaSuccess) return e;
-    e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    if (e != cudaSuccess) return e;
+cudaError_t engine_prepare(int variant, int tile_rows, int solver, long long tiles, int device, LaunchInfo* li) {
+    static std::atomic<int> per_sm_cache[64][4][SHAPES];  // resident CTAs, asked once
+    const int sms = engine_sm_count(device);
+    if (sms <= 0 || variant < 0 || variant > 3) return cudaErrorInvalidValue;
+    const Shape shape = select_shape(tile_rows, solver, tiles, sms);
+    std::atomic<int>& cached = per_sm_cache[device][variant][shape];
+    int per_sm = cached.load(std::memory_order_relaxed);
+    if (per_sm == 0) {
+        const Kernel k = kernel_of(variant, shape);
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.threads, k.smem);
+        if (e != cudaSuccess) return e;
+        cached.store(per_sm, std::memory_order_relaxed);
+    }
     li->grid = per_sm * sms;
-    li->block = kWarps * 32;
-    li->smem = smem;
+    li->shape = shape;
     return li->grid > 0 ? cudaSuccess : cudaErrorInvalidConfiguration;
 }
 
@@ -1066,12 +1059,12 @@ cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s)
     return cudaGetLastError();
 }
 
-cudaError_t engine_launch(const EngineArgs& a, int variant, int tile_rows, int grid, cudaStream_t s) {
-    void* k = select_kernel(variant, tile_rows);
+cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li, int grid, cudaStream_t s) {
+    const Kernel k = kernel_of(variant, static_cast<Shape>(li.shape));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
-    cfg.blockDim = dim3(kWarps * 32);
-    cfg.dynamicSmemBytes = smem_bytes(tile_rows);
+    cfg.blockDim = dim3((unsigned)k.threads);
+    cfg.dynamicSmemBytes = k.smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
@@ -1080,7 +1073,7 @@ cudaError_t engine_launch(const EngineArgs& a, int variant, int tile_rows, int g
     cfg.numAttrs = 1;
     EngineArgs args = a;
     void* params[] = {&args};
-    return cudaLaunchKernelExC(&cfg, k, params);
+    return cudaLaunchKernelExC(&cfg, k.fn, params);
 }
 
 }  // namespace iwpp

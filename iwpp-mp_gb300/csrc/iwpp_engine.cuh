@@ -18,12 +18,14 @@
 // of a host round trip, the unique queue de-duplicates when a tile is
 // inserted, and all insertions are warp-aggregated (one atomic per warp).
 //
+// A CTA works on one tile at a time; its first warp runs the queue.
+//
 // Tile ownership.  Each tile has a state word: DIRTY (needs a visit) and
-// ACTIVE (a warp is visiting it).  A warp that takes a tile sets ACTIVE; if
-// it was already set the entry is dropped (the owner will see DIRTY and
-// revisit).  The owner clears DIRTY before it reads the tile and releases
-// with CAS(ACTIVE -> 0), revisiting while DIRTY reappears.  So at most one
-// warp writes a tile's pixels, with plain stores, and every write that can
+// ACTIVE (a CTA is visiting it).  A CTA takes a tile by one exchange that sets
+// ACTIVE and takes DIRTY over, before it reads the tile; if ACTIVE was
+// already set what it took goes back and the entry is dropped (the owner will
+// see DIRTY and insert the tile again when it releases it).  So at most one
+// CTA writes a tile's pixels, with plain stores, and every write that can
 // raise a neighbour is followed by DIRTY on that neighbour after a fence.
 #pragma once
 
@@ -37,47 +39,54 @@ enum : unsigned { ST_DIRTY = 1u, ST_ACTIVE = 2u, ST_SIDE_SHIFT = 8u, ST_SIDES = 
 enum : int { VAR_MUTEX = 0, VAR_DOUBLE = 1, VAR_UNIQUE = 2, VAR_ASYNC = 3 };
 enum : unsigned { DEV_OK = 0u, DEV_ERR_TIMEOUT = 3u, DEV_ERR_OVERFLOW = 5u, DEV_ERR_INTERNAL = 9u };
 
-constexpr int kWarps = 4;       // warps (independent tile workers) per CTA
 constexpr int kMutexBatch = 8;  // entries taken per mutex acquisition
 constexpr int kMutexPrefill = 32;  // initial stack entries a CTA takes without the lock
 
+// Job counters.  What every warp hits with atomics and what waiting warps
+// watch lies in 128-byte lines of its own: one line's accesses go through one
+// L2 slice one after another, and with all of it in one line the waiting
+// warps' polls held up every insertion and release (4096^2 uint8 h-domes, one
+// warp per tile: 245 us with one line, 203 us with these and the waiting
+// warps watching their own slots; 517 and 375 us 8-connected, h = 100).
 struct Ctrl {
     unsigned rn;        // entries in the read queue (this round)
-    unsigned wn;        // insertions into the write queue (may exceed cap)
-    unsigned rcur;      // read cursor
     unsigned qsel;      // read queue = qsel ? q1 : q0
     unsigned vfull;     // the read queue is every tile 0..G-1
-    unsigned done;
-    unsigned overflow;  // an insertion did not fit since the last restart
     unsigned restarts;
     unsigned rounds;
-    unsigned bar_count;
-    unsigned bar_gen;
-    unsigned error;
-    unsigned lock_next;  // mutex stack: the ticket lock's next ticket
-    // mutex stack: the ticket being served (low half) and the number of
-    // stacked entries (high half) in one word, so a hand-over publishes the
-    // stack's top with the lock and the next holder reads both in one load
-    unsigned long long lock_word;
-    int pending;        // mutex: entries in the stack or taken and unfinished
-    unsigned progress;  // finished entries (for the no-progress timeout)
-    unsigned ahead;     // async ring: next position to claim
-    unsigned atail;     // async ring: next position to fill
+    unsigned ninit;     // initial entries (every tile, or the seed list after the front stage)
+    unsigned front_gate;  // front stage decided on the device: 1 run it, 0 leave the job to the engine
+    unsigned prefill;     // mutex: initial entries each CTA takes without the lock
+    unsigned prefill_base;  // mutex: stack position of CTA 0's slice (the stack's top below it)
     unsigned long long visits;
     unsigned long long sweeps;
     unsigned long long pushes;
     unsigned long long row_steps;
     unsigned long long phase[5];  // cycles: queue read, fetch, processing, dump, queue write
     unsigned long long top_pixels;    // pixels the top-level stage labelled
-    unsigned ninit;     // initial entries (every tile, or the seed list after the front stage)
-    unsigned front_gate;  // front stage decided on the device: 1 run it, 0 leave the job to the engine
-    unsigned idle;        // mutex: warps waiting for work
-    unsigned prefill;     // mutex: initial entries each CTA takes without the lock
-    unsigned prefill_base;  // mutex: stack position of CTA 0's slice (the stack's top below it)
+    // written when something ends; what waiting warps look at
+    alignas(128) unsigned done;
+    unsigned error;
+    unsigned overflow;  // an insertion did not fit since the last restart
+    alignas(128) unsigned wn;    // insertions into the write queue (may exceed cap)
+    alignas(128) unsigned rcur;  // read cursor
+    alignas(128) unsigned bar_count;
+    alignas(128) unsigned bar_gen;
+    alignas(128) unsigned lock_next;  // mutex stack: the ticket lock's next ticket
+    // mutex stack: the ticket being served (low half) and the number of
+    // stacked entries (high half) in one word, so a hand-over publishes the
+    // stack's top with the lock and the next holder reads both in one load
+    alignas(128) unsigned long long lock_word;
+    alignas(128) int pending;        // mutex, async: entries inserted and unfinished
+    alignas(128) unsigned progress;  // finished entries (for the no-progress timeout)
+    alignas(128) unsigned ahead;     // async ring: next position to claim
+    alignas(128) unsigned atail;     // async ring: next position to fill
+    alignas(128) unsigned idle;      // mutex: warps waiting for work
 };
 
 struct EngineArgs {
     const ImgDesc* imgs;
+    ImgDesc one;        // the image of a one-image job (nimg 1): read from the launch's parameters
     int nimg;
     unsigned G;         // tiles in the job
     unsigned* state;    // G tile state words
@@ -87,7 +96,7 @@ struct EngineArgs {
     Ctrl* ctrl;
     long long timeout_ns;
     int max_restarts;
-    int solver;  // 0 automatic, 1 row sweeps, 2 passes
+    int solver;  // 0 or 2 passes, 1 row sweeps, 3 pixel queue
     int phantom;  // test hook: one unit of work that never arrives (every wait runs out)
     int grid;     // CTAs of the engine launch (the mutex stack's first entries are split among them)
     int front;    // a seed check ran: the job's error word and top-pixel count stand
@@ -107,13 +116,14 @@ struct EngineArgs {
 // Host-side entry points implemented in iwpp_engine.cu.
 namespace iwpp {
 struct LaunchInfo {
-    int grid;
-    int block;
-    size_t smem;
+    int grid;   // CTAs that the device keeps resident
+    int shape;  // the kernel's shape (iwpp_engine.cu)
 };
-cudaError_t engine_prepare(int variant, int tile_rows, int device, LaunchInfo* li);
+int engine_sm_count(int device);
+// The kernel for a job of `tiles` tiles and its resident grid.
+cudaError_t engine_prepare(int variant, int tile_rows, int solver, long long tiles, int device, LaunchInfo* li);
 cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s);
-cudaError_t engine_launch(const EngineArgs& a, int variant, int tile_rows, int grid, cudaStream_t s);
+cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li, int grid, cudaStream_t s);
 cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s);
 // Adds to *count the pixels of d.marker that a neighbour could still raise.
 cudaError_t launch_fixed_point_check(const ImgDesc& d, unsigned long long* count, cudaStream_t s);

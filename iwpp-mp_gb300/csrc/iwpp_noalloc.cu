@@ -27,25 +27,22 @@
 namespace iwpp {
 namespace {
 
-static __device__ __align__(256) unsigned char g_noalloc_scratch[IWPP_NOALLOC_SCRATCH_BYTES];
-
-// The counters and the one image descriptor each take one 256-byte slot at
-// the start of the scratch (the size bound below counts on it).
-static_assert(sizeof(Ctrl) <= 256 && sizeof(ImgDesc) <= 256, "scratch header slots");
+// the documented scratch (tile states and ring behind two unused slots, which
+// keep the size bound where it was) and after it the job's counters
+constexpr size_t kCtrlAt = IWPP_NOALLOC_SCRATCH_BYTES;
+static __device__ __align__(256) unsigned char g_noalloc_scratch[kCtrlAt + sizeof(Ctrl)];
 
 constexpr int kMaxDevices = 64;
 constexpr int kNoallocTileRows = 64;
 
 std::mutex g_setup_mu;
 unsigned char* g_scratch_ptr[kMaxDevices] = {};
-LaunchInfo g_launch[kMaxDevices] = {};
 
-// Per-device set-up, done by the first call on a device with that device
-// current: the device address of the scratch array and the engine's launch
-// shape (kernel attributes, occupancy, SM count), both kept for the life of
-// the process so that later calls do no host-side queries.  A
-// cudaDeviceReset between calls would leave both stale; it is not supported.
-int device_setup(int device, unsigned char** out, LaunchInfo* li) {
+// The scratch array's device address, looked up by the first call on a device
+// with that device current and kept for the life of the process so that later
+// calls do no host-side queries.  A cudaDeviceReset between calls would leave
+// it stale; it is not supported.
+int device_setup(int device, unsigned char** out) {
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_scratch_ptr[device]) {
         void* p = nullptr;
@@ -54,23 +51,11 @@ int device_setup(int device, unsigned char** out, LaunchInfo* li) {
             cudaGetLastError();
             return IWPP_ERR_CUDA;
         }
-        LaunchInfo l{};
-        e = engine_prepare(VAR_ASYNC, kNoallocTileRows, device, &l);
-        if (e != cudaSuccess) {
-            cudaGetLastError();
-            return IWPP_ERR_CUDA;
-        }
-        g_launch[device] = l;
         g_scratch_ptr[device] = static_cast<unsigned char*>(p);
     }
     *out = g_scratch_ptr[device];
-    *li = g_launch[device];
     return IWPP_OK;
 }
-
-// Writes the single image descriptor into the scratch (a kernel parameter,
-// so no host-to-device copy is needed).
-__global__ void noalloc_store_desc(ImgDesc* dst, ImgDesc d) { *dst = d; }
 
 size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
@@ -100,8 +85,7 @@ extern "C" int iwpp_reconstruct_noalloc(void* marker, const void* mask, size_t p
     const long long tiles_y = ((long long)height + kNoallocTileRows - 1) / kNoallocTileRows;
     const long long G = tiles_x * tiles_y;
     const long long cap = G * 2 > 1024 ? G * 2 : 1024;  // async ring
-    const size_t off_img = align_up(sizeof(Ctrl), 256);
-    const size_t off_state = align_up(off_img + sizeof(ImgDesc), 256);
+    const size_t off_state = 512;
     const size_t off_ring = align_up(off_state + (size_t)G * 4u, 256);
     const size_t need = off_ring + (size_t)cap * 4u;
     if (G > 0x7fffffffll || need > (size_t)IWPP_NOALLOC_SCRATCH_BYTES) return IWPP_ERR_TOO_LARGE;
@@ -112,9 +96,13 @@ extern "C" int iwpp_reconstruct_noalloc(void* marker, const void* mask, size_t p
         return IWPP_ERR_NO_DEVICE;
     }
     unsigned char* base = nullptr;
-    LaunchInfo li;
-    int rc = device_setup(device, &base, &li);
+    int rc = device_setup(device, &base);
     if (rc != IWPP_OK) return rc;
+    LaunchInfo li;
+    if (engine_prepare(VAR_ASYNC, kNoallocTileRows, 0, G, device, &li) != cudaSuccess) {
+        cudaGetLastError();
+        return IWPP_ERR_CUDA;
+    }
 
     ImgDesc d{};
     d.marker = static_cast<unsigned char*>(marker);
@@ -132,33 +120,30 @@ extern "C" int iwpp_reconstruct_noalloc(void* marker, const void* mask, size_t p
     d.tile_rows = kNoallocTileRows;
 
     EngineArgs a{};
-    a.imgs = reinterpret_cast<const ImgDesc*>(base + off_img);
     a.nimg = 1;
     a.G = (unsigned)G;
     a.state = reinterpret_cast<unsigned*>(base + off_state);
     a.q0 = reinterpret_cast<unsigned*>(base + off_ring);
     a.q1 = a.q0;
     a.cap = (unsigned)cap;
-    a.ctrl = reinterpret_cast<Ctrl*>(base);
+    a.one = d;
+    a.ctrl = reinterpret_cast<Ctrl*>(base + kCtrlAt);
     a.timeout_ns = 10000ll * 1000000ll;
     a.max_restarts = 64;
     a.solver = 0;
 
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    noalloc_store_desc<<<1, 1, 0, s>>>(reinterpret_cast<ImgDesc*>(base + off_img), d);
-    cudaError_t e = cudaGetLastError();
     // the init kernel clears the state words, the ring and the counters that
     // the previous call left in the scratch
-    if (e == cudaSuccess) e = engine_launch_init(a, VAR_ASYNC, s);
+    cudaError_t e = engine_launch_init(a, VAR_ASYNC, s);
     if (e == cudaSuccess) {
         long long grid = li.grid;
-        const long long useful = (G + kWarps - 1) / kWarps;
-        if (grid > useful) grid = useful;
+        if (grid > G) grid = G;
         if (grid < 1) grid = 1;
-        e = engine_launch(a, VAR_ASYNC, kNoallocTileRows, (int)grid, s);
+        e = engine_launch(a, VAR_ASYNC, li, (int)grid, s);
     }
     Ctrl c;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&c, base, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&c, base + kCtrlAt, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         cudaGetLastError();
