@@ -260,6 +260,41 @@ struct Staged {
     size_t pitch;
     int w, h, dtype;
     bool owned;   // allocated for a plan: copied and freed by the plan
+    StageCopy in_m() const { return {user_marker, buf_m, (long long)user_pm, (long long)pitch, row(), h}; }
+    StageCopy in_k() const { return {user_mask, buf_k, (long long)user_pk, (long long)pitch, row(), h}; }
+    StageCopy out_m() const { return {buf_m, user_marker, (long long)pitch, (long long)user_pm, row(), h}; }
+    long long row() const { return (long long)w * bpp_of(dtype); }
+};
+
+// Where a handle's direct calls get their staging buffers from: a memory pool
+// that keeps up to kStagePoolKeep bytes between calls (the default pool gives
+// everything back at each synchronisation, and getting it again cost such a
+// call about 300 us, more than the reconstruction of a 6-megapixel image).
+// It goes with the handle.
+constexpr unsigned long long kStagePoolKeep = 256ull << 20;
+struct StagePool {
+    cudaMemPool_t pool = nullptr;
+    int device = 0;
+    cudaError_t alloc(void** out, size_t bytes, cudaStream_t s) {
+        if (!pool) {
+            cudaMemPoolProps props{};
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = device;
+            unsigned long long keep = kStagePoolKeep;
+            if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+                cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+                cudaGetLastError();
+                release();
+                return cudaMallocAsync(out, bytes, s);
+            }
+        }
+        return cudaMallocFromPoolAsync(out, bytes, pool, s);
+    }
+    void release() {
+        if (pool) cudaMemPoolDestroy(pool);
+        pool = nullptr;
+    }
 };
 
 struct Job {
@@ -267,6 +302,8 @@ struct Job {
     std::vector<Staged> staged;
     std::vector<CUtensorMap> tmaps;  // two per descriptor (marker, mask)
     std::vector<char> has_tma;
+    bool staged_in = false;  // the staging buffers hold the images
+    int stage_launches = 0;
     long long G = 0;
     int tile_rows = 64;
     int variant = IWPP_QUEUE_UNIQUE;
@@ -301,11 +338,11 @@ Layout job_layout(const Job& job) {
 // How images whose rows are not 4-byte aligned are handled.
 enum StageMode { STAGE_REJECT = 0, STAGE_ASYNC = 1, STAGE_OWNED = 2 };
 
-// STAGE_ASYNC: stream-ordered staging buffers, copied in now and back by
-// finish_staging.  STAGE_OWNED: plain allocations owned by the caller (a
+// STAGE_ASYNC: stream-ordered staging buffers (from `pool`, or the device's
+// default pool), copied in now and back by finish_staging.  STAGE_OWNED: plain allocations owned by the caller (a
 // plan), copies left to the caller.
 int build_job(Job& job, const iwpp_image* imgs, int n, int variant, const iwpp_config* cfgp, cudaStream_t s,
-              int staging, bool use_table = true) {
+              int staging, StagePool* pool, bool use_table = true) {
     job.cfg = resolve_config(cfgp);
     job.variant = resolve_variant(variant);
     if (use_table && n > 0 &&
@@ -407,17 +444,15 @@ int build_job(Job& job, const iwpp_image* imgs, int n, int variant, const iwpp_c
                 job.descs.push_back(d);
                 continue;
             }
-            e = cudaMallocAsync(&st.buf_m, pitch * im.height, s);
-            if (e == cudaSuccess) e = cudaMallocAsync(&st.buf_k, pitch * im.height, s);
-            if (e == cudaSuccess)
-                e = cudaMemcpy2DAsync(st.buf_m, pitch, im.marker, im.pitch_marker, row, im.height,
-                                      cudaMemcpyDeviceToDevice, s);
-            if (e == cudaSuccess)
-                e = cudaMemcpy2DAsync(st.buf_k, pitch, im.mask, im.pitch_mask, row, im.height,
-                                      cudaMemcpyDeviceToDevice, s);
+            auto alloc = [&](void** out) {
+                return pool ? pool->alloc(out, pitch * im.height, s) : cudaMallocAsync(out, pitch * im.height, s);
+            };
+            e = alloc(&st.buf_m);
+            if (e == cudaSuccess) e = alloc(&st.buf_k);
             if (e != cudaSuccess) {
                 if (st.buf_m) cudaFreeAsync(st.buf_m, s);
                 if (st.buf_k) cudaFreeAsync(st.buf_k, s);
+                cudaGetLastError();
                 return cuda_status(e);
             }
             st.pitch = pitch;
@@ -440,22 +475,33 @@ int build_job(Job& job, const iwpp_image* imgs, int n, int variant, const iwpp_c
         job.staged.push_back(st);
     }
     job.G = G;
+    if (staging == STAGE_ASYNC) {
+        std::vector<StageCopy> copies;
+        for (const auto& st : job.staged)
+            if (st.buf_m) {
+                copies.push_back(st.in_m());
+                copies.push_back(st.in_k());
+            }
+        const int rc = cuda_status(launch_stage_copies(copies, s, &job.stage_launches));
+        if (rc != IWPP_OK) return rc;
+        job.staged_in = true;
+    }
     return IWPP_OK;
 }
 
 int finish_staging(Job& job, cudaStream_t s) {
-    cudaError_t first = cudaSuccess;
+    std::vector<StageCopy> copies;
+    if (job.staged_in)
+        for (const auto& st : job.staged)
+            if (st.buf_m && !st.owned) copies.push_back(st.out_m());
+    const cudaError_t e = launch_stage_copies(copies, s, &job.stage_launches);
     for (auto& st : job.staged) {
         if (!st.buf_m || st.owned) continue;
-        const size_t row = (size_t)st.w * bpp_of(st.dtype);
-        cudaError_t e = cudaMemcpy2DAsync(st.user_marker, st.user_pm, st.buf_m, st.pitch, row, st.h,
-                                          cudaMemcpyDeviceToDevice, s);
-        if (first == cudaSuccess) first = e;
         cudaFreeAsync(st.buf_m, s);
         cudaFreeAsync(st.buf_k, s);
         st.buf_m = st.buf_k = nullptr;
     }
-    return cuda_status(first);
+    return cuda_status(e);
 }
 
 // Pinned host slots for the descriptor uploads of asynchronous calls: a
@@ -520,6 +566,7 @@ struct iwpp_handle_s {
     Ctrl* host_ctrl = nullptr;  // pinned
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     HostStaging staging;
+    StagePool stage_pool;
     cudaStream_t last_stream = nullptr;
     long long last_tiles = 0;
     int last_variant = IWPP_QUEUE_UNIQUE;
@@ -814,7 +861,7 @@ int run_job_sync(iwpp_handle h, const iwpp_image* imgs, int n, int variant, cons
     if (prev_dev != h->device) cudaSetDevice(h->device);
     Job job;
     int nl = 0;
-    rc = build_job(job, imgs, n, variant, cfg, s, STAGE_ASYNC);
+    rc = build_job(job, imgs, n, variant, cfg, s, STAGE_ASYNC, &h->stage_pool);
     if (rc == IWPP_OK) rc = enqueue_job(job, h->ws, s, h->device, true, h->ev0, h->ev1, true, &h->staging, &nl);
     const int rc_stage = finish_staging(job, s);
     if (rc == IWPP_OK) {
@@ -824,7 +871,7 @@ int run_job_sync(iwpp_handle h, const iwpp_image* imgs, int n, int variant, cons
             rc = cuda_status(e);
         else {
             cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-            rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, stats, ms, nl);
+            rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, stats, ms, nl + job.stage_launches);
         }
     } else {
         cudaStreamSynchronize(s);
@@ -883,7 +930,7 @@ int iwpp_handle_create(iwpp_handle* out, int device) {
     cudaSetDevice(device);
     iwpp_handle h = new (std::nothrow) iwpp_handle_s();
     if (!h) return IWPP_ERR_OOM;
-    h->device = device;
+    h->device = h->stage_pool.device = device;
     cudaError_t e = cudaMallocHost(&h->host_ctrl, sizeof(Ctrl));
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev0);
     if (e == cudaSuccess) e = cudaEventCreate(&h->ev1);
@@ -903,6 +950,7 @@ int iwpp_handle_destroy(iwpp_handle h) {
     cudaSetDevice(h->device);
     cudaDeviceSynchronize();
     h->staging.release();
+    h->stage_pool.release();
     if (h->ws.base) cudaFree(h->ws.base);
     if (h->host_ctrl) cudaFreeHost(h->host_ctrl);
     if (h->ev0) cudaEventDestroy(h->ev0);
@@ -949,7 +997,7 @@ int iwpp_reconstruct_batch_async(iwpp_handle h, const iwpp_image* images, int n,
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     Job job;
     int nl = 0;
-    int rc = build_job(job, images, n, variant, cfg, s, STAGE_ASYNC);
+    int rc = build_job(job, images, n, variant, cfg, s, STAGE_ASYNC, &h->stage_pool);
     if (rc == IWPP_OK) rc = enqueue_job(job, h->ws, s, h->device, true, h->ev0, h->ev1, true, &h->staging, &nl);
     const int rc2 = finish_staging(job, s);
     if (rc == IWPP_OK) rc = rc2;
@@ -1022,7 +1070,7 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
     p->h = h;
     Job job;
     cudaStream_t cs = nullptr;
-    int rc = build_job(job, images, n, variant, cfg, nullptr, STAGE_OWNED);
+    int rc = build_job(job, images, n, variant, cfg, nullptr, STAGE_OWNED, nullptr);
     for (const auto& st : job.staged)
         if (st.owned && st.buf_m) p->staged.push_back(st);
     cudaError_t e = cudaSuccess;
@@ -1058,24 +1106,19 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
         rc = cuda_status(e);
         if (rc == IWPP_OK) {
             // unaligned images: copy into the plan's staging buffers, run, copy back
+            std::vector<StageCopy> in, back;
+            int copies = 0;
             for (const auto& st : p->staged) {
-                const size_t row = (size_t)st.w * bpp_of(st.dtype);
-                if (e == cudaSuccess)
-                    e = cudaMemcpy2DAsync(st.buf_m, st.pitch, st.user_marker, st.user_pm, row, st.h,
-                                          cudaMemcpyDeviceToDevice, cs);
-                if (e == cudaSuccess)
-                    e = cudaMemcpy2DAsync(st.buf_k, st.pitch, st.user_mask, st.user_pk, row, st.h,
-                                          cudaMemcpyDeviceToDevice, cs);
+                in.push_back(st.in_m());
+                in.push_back(st.in_k());
+                back.push_back(st.out_m());
             }
+            e = launch_stage_copies(in, cs, &copies);
             rc = cuda_status(e);
             if (rc == IWPP_OK)
                 rc = enqueue_job(job, p->ws, cs, h->device, false, nullptr, nullptr, false, nullptr, &p->launches);
-            for (const auto& st : p->staged) {
-                const size_t row = (size_t)st.w * bpp_of(st.dtype);
-                if (rc == IWPP_OK)
-                    rc = cuda_status(cudaMemcpy2DAsync(st.user_marker, st.user_pm, st.buf_m, st.pitch, row, st.h,
-                                                       cudaMemcpyDeviceToDevice, cs));
-            }
+            if (rc == IWPP_OK) rc = cuda_status(launch_stage_copies(back, cs, &copies));
+            p->launches += copies;
             cudaError_t e2 = cudaStreamEndCapture(cs, &p->graph);
             if (rc == IWPP_OK) rc = cuda_status(e2);
         }
@@ -1247,7 +1290,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
         for (int r = 0; r < repeats; ++r) {
             if (restore() != IWPP_OK) return -1.0;
             Job job;
-            int jrc = build_job(job, images, n, v, &c, s, STAGE_ASYNC, false);
+            int jrc = build_job(job, images, n, v, &c, s, STAGE_ASYNC, &h->stage_pool, false);
             if (jrc == IWPP_OK) jrc = enqueue_job(job, h->ws, s, h->device, true, h->ev0, h->ev1, true, &h->staging);
             const int src = finish_staging(job, s);
             if (jrc == IWPP_OK) jrc = src;
@@ -1368,7 +1411,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
         rc = restore();
         if (rc == IWPP_OK) {
             Job job;
-            rc = build_job(job, images, n, v, &best, s, STAGE_ASYNC, false);
+            rc = build_job(job, images, n, v, &best, s, STAGE_ASYNC, &h->stage_pool, false);
             if (rc == IWPP_OK) rc = enqueue_job(job, h->ws, s, h->device, false, h->ev0, h->ev1, true, &h->staging);
             const int src = finish_staging(job, s);
             if (rc == IWPP_OK) rc = src;
@@ -1412,7 +1455,7 @@ int iwpp_clip(void* marker, const void* mask, size_t pitch_marker, size_t pitch_
         Job job;
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         iwpp_config c{};
-        rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC);
+        rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC, nullptr);
         if (rc == IWPP_OK && !job.descs.empty()) rc = cuda_status(launch_clip(job.descs[0], s));
         const int rc2 = finish_staging(job, s);
         return set_last(rc == IWPP_OK ? rc2 : rc);
@@ -1458,7 +1501,7 @@ int iwpp_sweep(void* marker, const void* mask, size_t pitch_marker, size_t pitch
     Job job;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     iwpp_config c{};
-    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC);
+    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC, nullptr);
     if (rc == IWPP_OK && !job.descs.empty()) {
         void* scratch = nullptr;
         const size_t sb = sweep_scratch_bytes(job.descs[0]);
@@ -1486,7 +1529,7 @@ int iwpp_sweep_timing(void* marker, const void* mask, size_t pitch_marker, size_
     Job job;
     cudaStream_t s = nullptr;
     iwpp_config c{};
-    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC);
+    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC, nullptr);
     void* scratch = nullptr;
     cudaEvent_t ev[5] = {};
     if (rc == IWPP_OK && !job.descs.empty()) {

@@ -29,6 +29,8 @@
 // raise a neighbour is followed by DIRTY on that neighbour after a fence.
 #pragma once
 
+#include <vector>
+
 #include "iwpp_device.cuh"
 
 namespace iwpp {
@@ -125,6 +127,16 @@ cudaError_t engine_prepare(int variant, int tile_rows, int solver, long long til
 cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s);
 cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li, int grid, cudaStream_t s);
 cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s);
+// Rows copied between a caller's image (any byte alignment) and an aligned
+// staging buffer, either way; all copies of a job in one launch (per 64).
+struct StageCopy {
+    const void* src;
+    void* dst;
+    long long src_pitch, dst_pitch;
+    long long row_bytes;
+    long long rows;
+};
+cudaError_t launch_stage_copies(const std::vector<StageCopy>& copies, cudaStream_t s, int* launches);
 // Adds to *count the pixels of d.marker that a neighbour could still raise.
 cudaError_t launch_fixed_point_check(const ImgDesc& d, unsigned long long* count, cudaStream_t s);
 // Queue self-test on workspace `a` (state G words, q0 / q1 cap entries each):

@@ -62,6 +62,73 @@ __global__ void clip_kernel(ImgDesc d) {
     }
 }
 
+// ---------------------------------------------------------------- staging
+// Copies the rows of up to 64 images at once (grid.y), a warp per row in
+// turn.  The row is written as the aligned words inside it, each put together
+// from the two aligned source words around it, and single bytes at the ends
+// (at most three each), so that a row of any alignment costs what an aligned
+// one does.  Bound by DRAM / L2 traffic: read and write each byte once.
+struct StageList {
+    StageCopy c[64];
+};
+
+__global__ void __launch_bounds__(256) stage_copy_kernel(const __grid_constant__ StageList list) {
+    const StageCopy& c = list.c[blockIdx.y];
+    const int lane = threadIdx.x & 31;
+    const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long y = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); y < c.rows; y += nwarps) {
+        const unsigned char* src = static_cast<const unsigned char*>(c.src) + y * c.src_pitch;
+        unsigned char* dst = static_cast<unsigned char*>(c.dst) + y * c.dst_pitch;
+        const long long n = c.row_bytes;
+        const long long lead = min((long long)((0u - (unsigned)reinterpret_cast<size_t>(dst)) & 3u), n);
+        const long long words = (n - lead) >> 2, tail = lead + 4 * words;
+        const unsigned char* from = src + lead;  // source of the first aligned word of dst
+        const unsigned sh = (unsigned)reinterpret_cast<size_t>(from) & 3u;
+        const unsigned* ws = reinterpret_cast<const unsigned*>(from - sh);
+        unsigned* wd = reinterpret_cast<unsigned*>(dst + lead);
+        if (sh == 0u) {
+#pragma unroll 4
+            for (long long i = lane; i < words; i += 32) wd[i] = ws[i];
+        } else {
+            // the source words around the row's first and last bytes hold
+            // bytes of other rows or of nothing: those words byte by byte
+#pragma unroll 4
+            for (long long i = lane; i < words; i += 32) {
+                unsigned w;
+                if (i > 0 && i + 1 < words) {
+                    w = __funnelshift_r(ws[i], ws[i + 1], 8 * sh);
+                } else {
+                    const unsigned char* b = from + 4 * i;
+                    w = (unsigned)b[0] | (unsigned)b[1] << 8 | (unsigned)b[2] << 16 | (unsigned)b[3] << 24;
+                }
+                wd[i] = w;
+            }
+        }
+        if (lane < 3 && lane < lead) dst[lane] = src[lane];
+        if (lane >= 4 && tail + lane - 4 < n) dst[tail + lane - 4] = src[tail + lane - 4];
+    }
+}
+
+cudaError_t launch_stage_copies(const std::vector<StageCopy>& copies, cudaStream_t s, int* launches) {
+    for (size_t i = 0; i < copies.size(); i += 64) {
+        StageList list{};
+        const size_t n = copies.size() - i < 64 ? copies.size() - i : 64;
+        long long rows = 1;
+        for (size_t j = 0; j < n; ++j) {
+            list.c[j] = copies[i + j];
+            rows = rows < copies[i + j].rows ? copies[i + j].rows : rows;
+        }
+        // eight rows per block at most in flight; four waves of blocks share
+        // the longest image
+        const long long want = (rows + 7) / 8, most = 152 * 32 / (long long)n + 1;
+        stage_copy_kernel<<<dim3((unsigned)(want < most ? want : most), (unsigned)n), 256, 0, s>>>(list);
+        const cudaError_t e = cudaGetLastError();
+        if (e != cudaSuccess) return e;
+        if (launches) ++*launches;
+    }
+    return cudaSuccess;
+}
+
 // ------------------------------------------------------ fixed-point check
 // Counts the pixels c that a neighbour p could still raise:
 // min(m[p], mask[c]) > m[c].  Zero on every reconstruction (it is a fixed

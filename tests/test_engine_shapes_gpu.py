@@ -61,3 +61,37 @@ def test_mixed_batch_many_tiles(conn):
     iwpp.reconstruct_batch(pairs, config=iwpp.Config.make(tile_rows=64))
     for (m, _, _), ref in zip(pairs, refs):
         assert np.array_equal(m.cpu().numpy().view(ref.dtype), ref)
+
+
+@pytest.mark.parametrize("dt", [0, 1])
+@pytest.mark.parametrize("conn", [4, 8])
+@pytest.mark.parametrize("off_m,off_k", [(1, 0), (0, 1), (3, 2), (2, 2)])
+def test_rows_off_the_word_boundary(dt, conn, off_m, off_k):
+    # views at an odd pixel of a larger buffer and of odd pitches: rows start
+    # at every byte of a word, one word, part of a word and several tiles wide;
+    # nothing around the view changes
+    import torch
+    rng = np.random.default_rng(off_m * 10 + off_k + conn)
+    for w, h, pad_m, pad_k in ((1, 3, 0, 2), (3, 40, 2, 0), (TW[dt] - 1, 33, 0, 0), (2 * TW[dt] + 5, 130, 3, 1),
+                               (3 * TW[dt] + 2, 67, 1, 4)):
+        mask = synth.noise_mask(w, h, dt, 5 + w, 1.5, 3)
+        marker = synth.hdome_marker(mask, 60)
+        ref = oracle.reconstruct(marker, mask, conn)
+        t = torch.uint8 if dt == 0 else torch.int16
+
+        def view(a, off, pad):
+            buf = torch.from_numpy(rng.integers(0, 120, (w + pad) * h + off, dtype=np.int64)).to(t).cuda()
+            v = torch.as_strided(buf, (h, w), (w + pad, 1), off)
+            v.copy_(torch.from_numpy(a.view(np.int16) if dt == 1 else a))
+            return buf, v
+
+        (bm, m), (bk, k) = view(marker, off_m, pad_m), view(mask, off_k, pad_k)
+        before = bm.clone()
+        for variant in ("async", "unique"):
+            for solver in (0, 1):
+                bm.copy_(before)
+                iwpp.reconstruct(m, k, connectivity=conn, variant=variant, config=iwpp.Config.make(solver=solver))
+                assert np.array_equal(m.cpu().numpy().view(ref.dtype), ref), (w, h, variant, solver)
+                around = torch.ones_like(bm, dtype=torch.bool)
+                torch.as_strided(around, (h, w), (w + pad_m, 1), off_m).fill_(False)
+                assert torch.equal(bm[around], before[around]), (w, h, variant, solver)
