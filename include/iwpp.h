@@ -66,7 +66,7 @@ typedef struct iwpp_config {
     long long queue_capacity;  /* entries per queue buffer; 0 = default; < 0: that multiple
                                   of the job's tile count */
     int init_passes;           /* whole-image passes first (+X, +Y, -X, -Y each); -1 = default
-                                  (0; 2 inside the front stage) */
+                                  (0; 2 with front_passes 1) */
     int grid_ctas;             /* persistent grid size; 0 = one full wave */
     int max_restarts;          /* queue-overflow restarts allowed; 0 = default (64) */
     int timeout_ms;            /* bound on every device-side wait; 0 = default (10000) */
@@ -79,7 +79,7 @@ typedef struct iwpp_config {
                                   shared memory (first visits by row sweeps) */
     int front_passes;          /* the front stage: the pixels at the mask's largest value
                                   raised by connected-component labelling, init_passes
-                                  whole-image passes (default 2), and the tile engine started
+                                  whole-image passes, and the tile engine started
                                   from the tiles still holding a pixel a neighbour can raise:
                                   0 = default (the tuning table's choice, else 3 when the job's
                                   largest image has 2^26 pixels or more and 2 below that),
@@ -201,7 +201,7 @@ IWPP_API int iwpp_queue_selftest(int device, int variant, int grid_side, int cop
  * MorphologicalReconstruction.cuh:6-7, and commented-out sweeps, MR.cu:792-795).
  * Times candidate configurations on the caller's own batch -- the untuned
  * default for large images, tile rows 64 / 32 x in-tile solver, the best of
- * those started from a seed check, the front stage with 1 / 2 / 3 / 4 / 8
+ * those started from a seed check, the front stage with 0 / 1 / 2 / 3 / 4 / 8
  * whole-image passes, then (if it lost) 1, 2, 4, ... 64 initial raster +
  * anti-raster passes while each doubling is faster, then (mutex / double
  * queues) queue capacity 1x / 16x the tiles --
@@ -214,7 +214,7 @@ typedef struct iwpp_tune_result {
     iwpp_config best;  /* fastest configuration */
     double best_ms;    /* its median device time */
     double default_ms; /* median device time of the untuned default (default tile height, automatic
-                          solver; front_passes 3 with 2 passes for images of 2^26 pixels or more) */
+                          solver; front_passes 3 for images of 2^26 pixels or more) */
     int candidates;    /* configurations timed */
     int reserved;
 } iwpp_tune_result;

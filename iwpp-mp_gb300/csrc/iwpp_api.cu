@@ -206,10 +206,14 @@ Layout layout_for(long long n_imgs, long long G, long long cap, bool two_queues,
     return l;
 }
 
-// Whole-image passes after the top-level stage when the caller leaves
-// init_passes at its default: measured on the 16384^2 spirals (uint8 /
-// uint16 / int32, ms), 1: 4.02 / 7.30 / 12.31, 2: 3.62 / 6.73 / 10.18,
-// 3: 3.67 / 7.17 / 10.46, 4: 4.13 / 8.10 / 11.74.
+// Whole-image passes after the top-level stage when the caller asks for the
+// stage (front_passes 1) and leaves init_passes at its default.  Jobs decided
+// on the device run none: what the passes cover the engine now does sooner
+// (16384^2 spirals with 0 / 1 / 2 / 3 passes, ms: uint8 2.57 / 2.85 / 3.03 /
+// 3.49, uint16 4.12 / 5.15 / 5.62 / 6.45, 16384 x 12000 int32 5.35 / 6.45 /
+// 6.45 / 7.24; 9001 x 9999 uint8 1.11 / 3.37 / 5.56 / 7.86), and without them
+// the labelling itself can add the tiles that it raises pixels in to the first
+// check's list, which spares the second check over both planes.
 constexpr int kFrontFullPasses = 2;
 // Untuned jobs whose largest image has at least this many pixels decide on
 // the device whether to take the front stage (front_passes 3): the seed
@@ -231,7 +235,7 @@ bool job_seeded(const Config& c) { return job_front(c) || c.front_passes == 4; }
 
 // Whole-image raster / anti-raster passes a job runs before the engine.
 int job_full_passes(const Config& c) {
-    if (job_front(c) && c.dflt_init) return kFrontFullPasses;
+    if (c.front_passes == 1 && c.dflt_init) return kFrontFullPasses;
     return c.init_passes;
 }
 
@@ -707,6 +711,9 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
             ++nl;
         }
     // the front stage's view of the images: gated by the device's decision
+    const int full_passes = job_full_passes(job.cfg);
+    // a gated job without passes checks once: the labelling marks what it raises
+    const bool marks = gated && full_passes == 0;
     std::vector<ImgDesc> fdescs = job.descs;
     if (gated)
         for (auto& d : fdescs) d.gate = &a.ctrl->front_gate;
@@ -724,13 +731,13 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
             if (e == cudaSuccess) e = cudaMemsetAsync(seed_count, 0, sizeof(unsigned), s);
             if (e == cudaSuccess)
                 e = launch_seed_batch(a.imgs, job.descs, nullptr, a.state, seed_list, seed_count, s, &nl);
-            if (e == cudaSuccess) e = launch_front_decide(&c->front_gate, seed_count, (unsigned)job.G, s, &nl);
+            if (e == cudaSuccess) e = launch_front_decide(&c->front_gate, seed_count, (unsigned)job.G, !marks, s, &nl);
         }
         for (size_t i = 0; i < fdescs.size() && e == cudaSuccess; ++i)
-            e = launch_top(fdescs[i], base + l.off_sweep, &c->top_pixels, device, s, &nl);
+            e = launch_top(fdescs[i], base + l.off_sweep, &c->top_pixels,
+                           marks ? SeedMarks{a.state, seed_list, seed_count} : SeedMarks{}, device, s, &nl);
         if (e != cudaSuccess) return cuda_status(e);
     }
-    const int full_passes = job_full_passes(job.cfg);
     for (int p = 0; p < full_passes; ++p)
         for (const auto& d : fdescs)
             for (int dir = 0; dir < 4; ++dir) {
@@ -746,16 +753,16 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
             }
     if (seeded) {
         // the tile engine starts from the tiles still holding a pixel that a
-        // neighbour can raise (a gated job that left the stage out keeps the
-        // list of its first check: the decision emptied it otherwise); the
-        // error word and top-pixel count of a job without the stage are
+        // neighbour can raise (a gated job keeps the list of its first check
+        // when it left the stage out, or with what the labelling added to it);
+        // the error word and top-pixel count of a job without the stage are
         // zeroed here (the engine's initialisation keeps them)
         if (!front) {
             e = cudaMemsetAsync(&a.ctrl->error, 0, sizeof(a.ctrl->error), s);
             if (e == cudaSuccess) e = cudaMemsetAsync(&a.ctrl->top_pixels, 0, sizeof(a.ctrl->top_pixels), s);
         }
         if (!gated && e == cudaSuccess) e = cudaMemsetAsync(seed_count, 0, sizeof(unsigned), s);
-        if (e == cudaSuccess)
+        if (e == cudaSuccess && !marks)
             e = launch_seed_batch(a.imgs, job.descs, gated ? &a.ctrl->front_gate : nullptr, a.state, seed_list,
                                   seed_count, s, &nl);
         if (e != cudaSuccess) return cuda_status(e);
@@ -1335,7 +1342,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
             // (the front stage as the device decides, with its default passes)
             iwpp_config c{};
             c.tile_rows = dflt_th;
-            c.init_passes = kFrontFullPasses;
+            c.init_passes = 0;
             c.front_passes = 3;
             consider(c, true);
         }
@@ -1355,12 +1362,12 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
             c.front_passes = 4;
             consider(c, false);
         }
-        // stage 2: the front stage (top-level labelling, then 1 / 2 / 3 / 4 / 8
+        // stage 2: the front stage (top-level labelling, then 0 / 1 / 2 / 3 / 4 / 8
         // whole-image passes, then the engine from the seed check) with the
         // best tile height and solver; long propagation paths want it
         if (best_ms >= 0.0) {
             const iwpp_config base = best;
-            for (int ip : {1, 2, 3, 4, 8}) {
+            for (int ip : {0, 1, 2, 3, 4, 8}) {
                 iwpp_config c = base;
                 c.front_passes = 1;
                 c.init_passes = ip;

@@ -72,7 +72,28 @@ struct TopArgs {
     unsigned* relabel;       // the tiles with more top-level pixels than a list holds
     int aligned16;           // mask rows start on 16-byte boundaries
     unsigned long long* top_pixels;  // the job's count of pixels labelled
+    SeedMarks marks;         // nullable pointers: where raised pixels mark engine tiles
 };
+
+// Marks the engine tiles that a raised pixel (y, x) can make due: its own,
+// and across a tile edge or corner its neighbours.  A tile enters the list
+// once, with all sides, as from the seed check.
+template <int DT>
+__device__ __forceinline__ void mark_raised(const TopArgs& a, int y, int x) {
+    if (a.marks.state == nullptr) return;
+    constexpr int TW = 32 * Px<DT>::PPW;
+    const ImgDesc& d = a.d;
+    const int ty = y / d.tile_rows, tx = x / TW, r = y - ty * d.tile_rows, c = x - tx * TW;
+    const int y0 = r == 0 && ty > 0 ? ty - 1 : ty, y1 = r == d.tile_rows - 1 && ty + 1 < d.tiles_y ? ty + 1 : ty;
+    const int x0 = c == 0 && tx > 0 ? tx - 1 : tx, x1 = c == TW - 1 && tx + 1 < d.tiles_x ? tx + 1 : tx;
+    for (int yy = y0; yy <= y1; ++yy)
+        for (int xx = x0; xx <= x1; ++xx) {
+            const unsigned g = (unsigned)d.tile_base + (unsigned)(yy * d.tiles_x + xx);
+            if (*(volatile unsigned*)&a.marks.state[g] & ST_DIRTY) continue;
+            if (!(atomicOr(&a.marks.state[g], ST_DIRTY | ST_SIDES) & ST_DIRTY))
+                a.marks.list[atomicAdd(a.marks.count, 1u)] = g;
+        }
+}
 
 __device__ __forceinline__ int g_find(int* parent, int x) {
     for (;;) {
@@ -535,7 +556,10 @@ __global__ void top_apply_list_kernel(TopArgs a) {
             const int p = (int)(u & 0xffffu), r = p / TW, c = p - r * TW;
             const uint32_t v = top_key<DT>(__ldcg(&a.gmax[__ldcg(&a.gparent[t * kTopSlots + s])]));
             unsigned char* px = d.marker + (size_t)(ty * kTopRows + r) * d.pitch_m + (size_t)(tx * TW + c) * P::BPP;
-            if (P::gt(v, P::ld_px(px))) P::st_px(px, v);
+            if (P::gt(v, P::ld_px(px))) {
+                P::st_px(px, v);
+                mark_raised<DT>(a, ty * kTopRows + r, tx * TW + c);
+            }
         }
     }
 }
@@ -593,6 +617,7 @@ __global__ void __launch_bounds__(kTopThreads, 4) top_apply_label_kernel(TopArgs
                 if (P::gt(v, m[j])) {
                     m[j] = v;
                     chg = true;
+                    mark_raised<DT>(a, ty * kTopRows + (w >> 5), tx * TW + (w & 31) * P::PPW + j);
                 }
             }
             if (!chg) continue;
@@ -627,14 +652,13 @@ __device__ __forceinline__ uint32_t seed_px(const ImgDesc& d, int y, int x) {
     return P::ld_px(d.marker + (size_t)y * d.pitch_m + (size_t)x * P::BPP);
 }
 
-// The check with wide lanes: a lane holds WPL words (8 or 16 bytes) of
-// a row, so a warp covers WPL engine tiles side by side (32 / WPL lanes
-// each); the words are updated with byte / half-word SIMD, the side
-// neighbours of a word's pixels come from funnel shifts of the adjacent
-// words, and rows are loaded kSeedAhead ahead into a register ring (one
-// vector load per lane where the address allows it, else word by word;
-// rows start on 4-byte boundaries).  Eight-byte lanes keep the registers
-// per thread low enough for eight CTAs per SM.
+// The check with wide lanes: a lane holds WPL words (8 bytes) of a row, so a
+// warp covers WPL engine tiles side by side (32 / WPL lanes each); the words
+// are taken apart as in the engine's vertical pass (VRow: byte SIMD is not in
+// hardware, 16-bit pairs are), the side neighbours of a word's pixels come
+// from permutes with the adjacent words, and rows are loaded kSeedAhead ahead
+// into a register ring (one vector load per lane where the address allows
+// it, else word by word; rows start on 4-byte boundaries).
 constexpr int kSeedAhead = 2;
 constexpr int kSeedThreads = 128;
 constexpr int kSeedWords = 2;  // words per lane
@@ -677,7 +701,7 @@ template <int DT, int WPL>
 __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsigned* state, unsigned* list,
                                           unsigned* nlist) {
     using P = Px<DT>;
-    constexpr int BITS = 8 * P::BPP;  // bits per pixel
+    constexpr int N = VRow<DT>::N;
     constexpr int TW = 32 * P::PPW;   // pixels per engine tile row
     constexpr int LPT = 32 / WPL;     // lanes per tile
     const int lane = threadIdx.x & 31;
@@ -692,10 +716,15 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
         if (lane == 31) return seed_px<DT>(d, y, xr);
         return P::MINPX;
     };
-    // window: marker rows r - 1, r, mask row r, halo pixels
-    uint32_t mu[WPL], mc[WPL], kc[WPL];
-    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0 - 1, b0, row_bytes, mu);
-    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0, b0, row_bytes, mc);
+    // window: marker rows r - 1, r (taken apart), mask row r, halo pixels
+    uint32_t w0[WPL], kc[WPL];
+    VRow<DT> mu[WPL], mc[WPL];
+    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0 - 1, b0, row_bytes, w0);
+#pragma unroll
+    for (int w = 0; w < WPL; ++w) mu[w].set(w0[w]);
+    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0, b0, row_bytes, w0);
+#pragma unroll
+    for (int w = 0; w < WPL; ++w) mc[w].set(w0[w]);
     seed_load<DT, WPL>(d, d.mask, d.pitch_k, y0, b0, row_bytes, kc);
     uint32_t hu = halo(y0 - 1), hc = halo(y0);
     // ring slot i holds marker / mask / halo of row r + 1 + i
@@ -713,16 +742,17 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
         }
         rh[i] = halo(y);
     }
-    bool mine = false;
+    uint32_t rose = 0u;
     for (int r0 = 0; r0 < rows; r0 += kSeedAhead) {
 #pragma unroll
         for (int i = 0; i < kSeedAhead; ++i) {
             const int r = r0 + i;
             if (r >= rows) break;  // warp-uniform
-            uint32_t md[WPL], kn[WPL];
+            uint32_t kn[WPL];
+            VRow<DT> md[WPL];
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
-                md[w] = rm[i][w];
+                md[w].set(rm[i][w]);
                 kn[w] = rk[i][w];
             }
             const uint32_t hd = rh[i];
@@ -739,24 +769,41 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
             }
             // what a column offers its side neighbours: itself, or with
             // 8-connectivity the largest of its three rows
-            uint32_t V[WPL], S[WPL];
+            VRow<DT> V[WPL], S[WPL];
 #pragma unroll
-            for (int w = 0; w < WPL; ++w) {
-                V[w] = word_max<DT>(mu[w], md[w]);
-                S[w] = d.conn == 8 ? word_max<DT>(V[w], mc[w]) : mc[w];
-            }
+            for (int w = 0; w < WPL; ++w)
+#pragma unroll
+                for (int j = 0; j < N; ++j) {
+                    V[w].v[j] = vmx<DT>(mu[w].v[j], md[w].v[j]);
+                    S[w].v[j] = d.conn == 8 ? vmx<DT>(V[w].v[j], mc[w].v[j]) : mc[w].v[j];
+                }
             const uint32_t hs = d.conn == 8 ? P::mx(P::mx(hu, hc), hd) : hc;
-            uint32_t left = __shfl_up_sync(FULL, S[WPL - 1], 1), right = __shfl_down_sync(FULL, S[0], 1);
-            if (lane == 0) left = BITS == 32 ? hs : hs << (32 - BITS);
-            if (lane == 31) right = hs;
+            // the pixel in every place of a word
+            const uint32_t hw = DT == DT_U8 ? __byte_perm(hs, 0u, 0x0000) : DT == DT_U16 ? hs * 0x10001u : hs;
+            uint32_t left = __shfl_up_sync(FULL, S[WPL - 1].v[N - 1], 1), right = __shfl_down_sync(FULL, S[0].v[0], 1);
+            if (lane == 0) left = hw;
+            if (lane == 31) right = hw;
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
-                // clamped funnel shifts: a shift of 32 (int32) yields the
-                // adjacent word itself
-                const uint32_t lw = __funnelshift_lc(w == 0 ? left : S[w - 1], S[w], BITS);
-                const uint32_t rw = __funnelshift_rc(S[w], w == WPL - 1 ? right : S[w + 1], BITS);
-                const uint32_t best = word_max<DT>(V[w], word_max<DT>(lw, rw));
-                mine |= word_any_gt<DT>(word_min<DT>(best, kc[w]), mc[w]);
+                const uint32_t lw = w == 0 ? left : S[w - 1].v[N - 1], rw = w == WPL - 1 ? right : S[w + 1].v[0];
+                VRow<DT> k, best;
+                k.set(kc[w]);
+                if constexpr (DT == DT_U8) {
+                    // even bytes: the odd half, and it shifted in from the
+                    // left; odd bytes: the even half, and it shifted in from
+                    // the right
+                    best.v[0] = __vimax3_u16x2(V[w].v[0], S[w].v[1], __byte_perm(lw, S[w].v[1], 0x5432));
+                    best.v[1] = __vimax3_u16x2(V[w].v[1], S[w].v[0], __byte_perm(S[w].v[0], rw, 0x5432));
+                } else if constexpr (DT == DT_U16) {
+                    best.v[0] = __vimax3_u16x2(V[w].v[0], __byte_perm(lw, S[w].v[0], 0x5432),
+                                               __byte_perm(S[w].v[0], rw, 0x5432));
+                } else {
+                    best.v[0] = (uint32_t)__vimax3_s32((int)V[w].v[0], (int)lw, (int)rw);
+                }
+                VRow<DT> m = mc[w];
+                vstep<DT>(m, k, best);
+#pragma unroll
+                for (int j = 0; j < N; ++j) rose |= m.v[j] ^ mc[w].v[j];
             }
 #pragma unroll
             for (int w = 0; w < WPL; ++w) {
@@ -768,6 +815,7 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
             hc = hd;
         }
     }
+    const bool mine = rose != 0u;
     // a tile is bad when one of its lanes saw a pixel to raise
     const unsigned bad = __ballot_sync(FULL, mine);
     const int tx = gx * WPL + q;
@@ -870,16 +918,17 @@ __global__ void __launch_bounds__(kSeedThreads, 6)
 // sparse seeds) propagates over long paths, one dependent tile visit per tile for
 // the engine alone, which the labelling and the whole-image passes cover
 // in a fixed number of sweeps; a large front (h-dome markers, dense seeds)
-// is short-range work the engine does faster alone.  With the stage the
-// seed list is emptied for the check after the passes; without it the list
-// of this check seeds the engine.
+// is short-range work the engine does faster alone.  Without the stage the
+// list of this check seeds the engine; with it the labelling adds the tiles
+// that it raises pixels in, or (`recheck`: whole-image passes follow) the
+// list is emptied for the check after the passes.
 constexpr unsigned kFrontDecideRatio = 64;
 
-__global__ void front_decide_kernel(unsigned* gate, unsigned* count, unsigned G) {
+__global__ void front_decide_kernel(unsigned* gate, unsigned* count, unsigned G, int recheck) {
     const unsigned n = *(volatile unsigned*)count;
     const unsigned front = n > 0u && (unsigned long long)n * kFrontDecideRatio < (unsigned long long)G ? 1u : 0u;
     *gate = front;
-    if (front) *count = 0u;
+    if (front && recheck) *count = 0u;
 }
 
 // ------------------------------------------------------------------ host
@@ -925,8 +974,8 @@ static cudaError_t launch_top_t(const TopArgs& a, int sms, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-cudaError_t launch_top(const ImgDesc& d, void* scratch, unsigned long long* top_pixels, int device, cudaStream_t s,
-                       int* launches) {
+cudaError_t launch_top(const ImgDesc& d, void* scratch, unsigned long long* top_pixels, const SeedMarks& marks,
+                       int device, cudaStream_t s, int* launches) {
     if (d.W == 0 || d.H == 0) return cudaSuccess;
     TopArgs a{};
     a.d = d;
@@ -960,6 +1009,7 @@ cudaError_t launch_top(const ImgDesc& d, void* scratch, unsigned long long* top_
     a.relabel = reinterpret_cast<unsigned*>(p);
     a.aligned16 = (reinterpret_cast<uintptr_t>(d.mask) & 15u) == 0u && (d.pitch_k & 15) == 0;
     a.top_pixels = top_pixels;
+    a.marks = marks;
     int sms = 0;
     cudaError_t e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (e == cudaSuccess) e = cudaMemsetAsync(a.thr_key, 0, sizeof(unsigned), s);
@@ -997,8 +1047,9 @@ cudaError_t launch_seed_batch(const ImgDesc* dev_descs, const std::vector<ImgDes
     return cudaGetLastError();
 }
 
-cudaError_t launch_front_decide(unsigned* gate, unsigned* count, unsigned G, cudaStream_t s, int* launches) {
-    front_decide_kernel<<<1, 1, 0, s>>>(gate, count, G);
+cudaError_t launch_front_decide(unsigned* gate, unsigned* count, unsigned G, bool recheck, cudaStream_t s,
+                                int* launches) {
+    front_decide_kernel<<<1, 1, 0, s>>>(gate, count, G, recheck ? 1 : 0);
     if (launches) ++*launches;
     return cudaGetLastError();
 }
