@@ -8,11 +8,14 @@
 //         rule m = max(m, min(prev, mask)) along one axis.
 //   +X / -X: one warp per row, the whole row as one max-min scan (128-byte
 //            chunks, carry from chunk to chunk), exact and coalesced.
-//   +Y / -Y: one warp per 128-byte column strip walking the full height,
+//   +Y / -Y: 4-connected, one warp per column strip (or segment of one),
 //            rows streamed through shared memory with cp.async far ahead;
 //            8-connectivity also takes the two diagonal pixels of the
-//            previous row inside the strip.  Every pixel is written by one
-//            thread, so the result is deterministic.
+//            previous row inside a 128-byte strip, segments of rows first on
+//            their own, then their entries.  The result is the walk's, row
+//            by row, whatever the order.
+#include <type_traits>
+
 #include "iwpp_engine.cuh"
 
 namespace iwpp {
@@ -421,11 +424,8 @@ __global__ void sweep_x16p_kernel(ImgDesc d) {
 }
 
 // --------------------------------------------------------------- Y sweeps
-// 4-byte asynchronous global -> shared copy (cp.async, LDGSTS) and its
-// group bookkeeping.
-__device__ __forceinline__ void cp_async4(void* smem_dst, const void* gmem_src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
-}
+// 16-byte asynchronous global -> shared copy (cp.async, LDGSTS) and its group
+// bookkeeping.
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gmem_src) : "memory");
 }
@@ -435,101 +435,202 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
-// One warp per 128-byte column strip, walking the full height.  The chain
-// through the rows is a few operations per row; memory latency is hidden by
-// a ring of kRing rows per plane in shared memory, filled with cp.async
-// kRing rows ahead (groups of kGroup rows).  Each lane reads and writes its
-// own word of every row only, so no row is read after this thread wrote it.
+// The 4-connected sweeps stream rows through a ring in shared memory, kRing
+// rows of a plane ahead, in cp.async groups of kGroup rows.
 constexpr int kRing = 64, kGroup = 8;
 
-template <int DT, int CONN, bool DOWN>
-__global__ void __launch_bounds__(32) sweep_y_kernel(ImgDesc d) {
-    if (gated_off(d)) return;
+// 8-connected vertical sweeps.  A 128-byte column strip is closed: its rows
+// take the three pixels of the row before them inside the strip (a lane holds
+// a word).  Row by row that is a chain of about 50 cycles a row (a shuffle and
+// five dependent operations), and with the diagonals a run of rows is no
+// per-column map that could be composed; one warp walking a strip's whole
+// height took 500 us for 4096 rows whatever the width.  But the sweep is the
+// least solution of "each row at least what the row before it offers", so the
+// rows can be taken in any order that ends with no row left to raise:
+//   sweep_y8_local_kernel: segments of kSeg8 rows, a warp each, as if nothing
+//     entered them;
+//   sweep_y8_enter_kernel, kY8Enter times: a warp per segment, what the row
+//     before the segment offers, on from there while the rows rise; the row
+//     before it may itself be rising meanwhile;
+//   sweep_y8_settle_kernel: a warp per strip, the segments in order, any entry
+//     that still raises something, on from there while the rows rise.
+// Same bytes as the walk.  Measured on 4096^2 uint8 h-domes (+Y / -Y, us): the
+// walk 496 / 516; segments of 64 rows with 1 / 2 / 4 / 8 enter steps 144 / 81 /
+// 70 / 87, of 128 rows 70 / 60 / 66 / 83, of 32 rows 304 / 203 / 111 / 105.
+// Bound by the chain: a row is about 100 cycles of one warp.
+constexpr int kSeg8 = 128;
+constexpr int kY8Enter = 2;
+constexpr int kY8Threads = 128;
+
+// A lane's word column of a strip, rows by their index in sweep order.
+template <int DT, bool DOWN>
+struct Strip8 {
     using P = Px<DT>;
-    constexpr int TW = 32 * P::PPW;
-    constexpr int N = P::PPW;
-    constexpr int NG = kRing / kGroup;
-    __shared__ uint32_t ring_m[kRing][32];
-    __shared__ uint32_t ring_k[kRing][32];
-    const int lane = threadIdx.x & 31;
-    const int strip = (int)blockIdx.x;
-    const int strips = (d.W + TW - 1) / TW;
-    if (strip >= strips) return;
-    const int px0 = strip * TW + lane * P::PPW, npx = d.W - px0;
-    const size_t off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
-    const int H = d.H;
-    auto row_of = [&](int i) { return DOWN ? i : H - 1 - i; };
-    // row i (in sweep order) into slot i % kRing: a full word asynchronously,
-    // a partial word (right edge) or a word past the image by plain loads
-    auto issue = [&](int i) {
-        const int slot = i % kRing;
-        if (i >= H) return;
-        const int y = row_of(i);
-        const unsigned char* mrow = d.marker + (size_t)y * d.pitch_m + off;
-        const unsigned char* krow = d.mask + (size_t)y * d.pitch_k + off;
-        if (npx >= P::PPW) {
-            cp_async4(&ring_m[slot][lane], mrow);
-            cp_async4(&ring_k[slot][lane], krow);
-        } else {
-            uint32_t mw = P::MINW, kw = P::MINW;
-            if (npx > 0) load_pair<DT>(mrow, krow, npx, mw, kw);
-            ring_m[slot][lane] = mw;
-            ring_k[slot][lane] = kw;
-        }
-    };
-    for (int g = 0; g < NG; ++g) {
-        for (int q = 0; q < kGroup; ++q) issue(g * kGroup + q);
-        cp_async_commit();
+    unsigned char* m;
+    const unsigned char* k;
+    long long pitch_m, pitch_k;
+    int npx, H;
+    __device__ __forceinline__ Strip8(const ImgDesc& d, int strip, int lane) : H(d.H) {
+        const int px0 = strip * 32 * P::PPW + lane * P::PPW;
+        npx = d.W - px0;
+        const size_t off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
+        const int first = DOWN ? 0 : d.H - 1;
+        pitch_m = DOWN ? d.pitch_m : -d.pitch_m;
+        pitch_k = DOWN ? d.pitch_k : -d.pitch_k;
+        m = d.marker + (size_t)first * d.pitch_m + off;
+        k = d.mask + (size_t)first * d.pitch_k + off;
     }
-    uint32_t prev[N];
+    __device__ __forceinline__ uint32_t marker(int i) const {
+        return i < H && npx > 0 ? load_word_plain<DT>(m + i * pitch_m, npx, true) : P::MINW;
+    }
+    __device__ __forceinline__ uint32_t mask(int i) const {
+        return i < H && npx > 0 ? load_word_plain<DT>(k + i * pitch_k, npx, false) : P::MINW;
+    }
+    __device__ __forceinline__ void store(int i, uint32_t w) const {
+        if (npx > 0) store_word_plain<DT>(m + i * pitch_m, npx, w);
+    }
+    // Walks rows from `i` below row i - 1 (in `prev`), the next eight rows'
+    // loads ahead of the chain; with STOP until a group of eight ends with a
+    // row that does not rise, else to row `end`.  Strips inside the image's
+    // width (all but the last) run on bare words: with the checks for a
+    // partial word in every row a row took 300 cycles.
+    template <bool STOP>
+    __device__ __forceinline__ void walk(const VRow<DT>& prev, int i, int end, const EdgeSel& sel) const {
+        if (__all_sync(FULL, npx >= P::PPW))
+            walk_rows<STOP, true>(prev, i, end, sel);
+        else
+            walk_rows<STOP, false>(prev, i, end, sel);
+    }
+    template <bool STOP, bool WORDS>
+    __device__ __forceinline__ void walk_rows(VRow<DT> prev, int i, int end, const EdgeSel& sel) const {
+        const unsigned char *pm = m + i * pitch_m, *pk = k + i * pitch_k;
+        auto load = [&](const unsigned char* p, long long pitch, uint32_t (&w)[8]) {
 #pragma unroll
-    for (int j = 0; j < N; ++j) prev[j] = P::MINPX;
-    for (int base = 0; base < H; base += kGroup) {
-        cp_async_wait<NG - 1>();  // the group holding rows base .. base + kGroup - 1
-        __syncwarp();
-        // Straight-line code for the group: all ring reads first, then the
-        // chain through the rows (two operations per pixel), then the
-        // stores; rows past the image are computed on stale slots and not
-        // stored.
-        const int sb = base % kRing;
-        uint32_t mw[kGroup], kw[kGroup], out[kGroup];
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q) {
-            mw[q] = ring_m[sb + q][lane];
-            kw[q] = ring_k[sb + q][lane];
+            for (int q = 0; q < 8; ++q)
+                w[q] = WORDS     ? __ldcg(reinterpret_cast<const unsigned int*>(p + q * pitch))
+                       : npx > 0 ? load_word_plain<DT>(p + q * pitch, npx, true)
+                                 : P::MINW;
+        };
+        uint32_t old[8], kw[8];
+        if (i + 8 <= end) {
+            load(pm, pitch_m, old);
+            load(pk, pitch_k, kw);
         }
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q) {
-            uint32_t m[N], k[N];
-            P::unpack(mw[q], m);
-            P::unpack(kw[q], k);
-            if (CONN == 8) {
-                uint32_t left = __shfl_up_sync(FULL, prev[N - 1], 1), right = __shfl_down_sync(FULL, prev[0], 1);
-                if (lane == 0) left = P::MINPX;
-                if (lane == 31) right = P::MINPX;
-#pragma unroll
-                for (int j = 0; j < N; ++j) {
-                    const uint32_t a = j == 0 ? left : prev[j - 1];
-                    const uint32_t b = j == N - 1 ? right : prev[j + 1];
-                    m[j] = P::mx(m[j], P::mn(P::mx3(a, prev[j], b), k[j]));
-                }
-            } else {
-#pragma unroll
-                for (int j = 0; j < N; ++j) m[j] = P::mx(m[j], P::mn(prev[j], k[j]));
+#pragma unroll 1
+        for (; i + 8 <= end; i += 8) {
+            uint32_t nm[8], nk[8];
+            const unsigned char *qm = pm + 8 * pitch_m, *qk = pk + 8 * pitch_k;
+            if (i + 16 <= end) {
+                load(qm, pitch_m, nm);
+                load(qk, pitch_k, nk);
             }
-            out[q] = P::pack(m);
+            uint32_t x = 0u;
 #pragma unroll
-            for (int j = 0; j < N; ++j) prev[j] = m[j];
+            for (int q = 0; q < 8; ++q) {
+                VRow<DT> v, kv;
+                v.set(old[q]);
+                kv.set(kw[q]);
+                vstep<DT>(v, kv, offers<DT, 8>(prev, sel));
+                const uint32_t w = v.word();
+                x = w ^ old[q];
+                if (WORDS) {
+                    if (x != 0u)
+                        *reinterpret_cast<unsigned int*>(const_cast<unsigned char*>(pm) + q * pitch_m) = w;
+                } else if (x != 0u) {
+                    store(i + q, w);
+                }
+                prev = v;
+            }
+            if (STOP && !__any_sync(FULL, x != 0u)) return;
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                old[q] = nm[q];
+                kw[q] = nk[q];
+            }
+            pm = qm;
+            pk = qk;
         }
-#pragma unroll
-        for (int q = 0; q < kGroup; ++q)
-            if (base + q < H && npx > 0 && out[q] != mw[q])
-                store_word_plain<DT>(d.marker + (size_t)row_of(base + q) * d.pitch_m + off, npx, out[q]);
-        __syncwarp();  // the slots just read are refilled next
-        for (int q = 0; q < kGroup; ++q) issue(base + kRing + q);
-        cp_async_commit();
+#pragma unroll 1
+        for (; i < end; ++i) {
+            const uint32_t was = marker(i);
+            VRow<DT> v, kv;
+            v.set(was);
+            kv.set(mask(i));
+            vstep<DT>(v, kv, offers<DT, 8>(prev, sel));
+            const uint32_t w = v.word();
+            if (w != was) store(i, w);
+            if (STOP && !__any_sync(FULL, w != was)) return;
+            prev = v;
+        }
     }
-    cp_async_wait<0>();
+};
+
+template <int DT, bool DOWN>
+__global__ void __launch_bounds__(kY8Threads) sweep_y8_local_kernel(ImgDesc d, int strips, int segs) {
+    if (gated_off(d)) return;
+    const int lane = threadIdx.x & 31;
+    const long long wid = (long long)blockIdx.x * (kY8Threads / 32) + (threadIdx.x >> 5);
+    if (wid >= (long long)strips * segs) return;
+    const int seg = (int)(wid / strips), strip = (int)(wid - (long long)seg * strips);
+    const Strip8<DT, DOWN> st(d, strip, lane);
+    const EdgeSel sel(lane);
+    const int i0 = seg * kSeg8, end = min(i0 + kSeg8, d.H);
+    VRow<DT> prev;
+    prev.set(Px<DT>::MINW);
+    st.template walk<false>(prev, i0, end, sel);
+}
+
+template <int DT, bool DOWN>
+__global__ void __launch_bounds__(kY8Threads) sweep_y8_enter_kernel(ImgDesc d, int strips, int segs) {
+    if (gated_off(d)) return;
+    const int lane = threadIdx.x & 31;
+    const long long wid = (long long)blockIdx.x * (kY8Threads / 32) + (threadIdx.x >> 5);
+    if (wid >= (long long)strips * (segs - 1)) return;
+    const int seg = 1 + (int)(wid / strips), strip = (int)(wid % strips);
+    const Strip8<DT, DOWN> st(d, strip, lane);
+    const int i0 = seg * kSeg8;
+    VRow<DT> prev;
+    prev.set(st.marker(i0 - 1));
+    st.template walk<true>(prev, i0, min(i0 + kSeg8, d.H), EdgeSel(lane));
+}
+
+template <int DT, bool DOWN>
+__global__ void __launch_bounds__(32) sweep_y8_settle_kernel(ImgDesc d, int segs) {
+    if (gated_off(d)) return;
+    const int lane = threadIdx.x;
+    const Strip8<DT, DOWN> st(d, (int)blockIdx.x, lane);
+    const EdgeSel sel(lane);
+#pragma unroll 1
+    for (int s0 = 1; s0 < segs; s0 += 8) {
+        // eight entries' rows in flight together; a walk that goes past an
+        // entry below has satisfied it, and one that does not reach it leaves
+        // the row above it as read
+        uint32_t above[8], first[8], kw[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int i = (s0 + q) * kSeg8;
+            above[q] = i < d.H ? st.marker(i - 1) : Px<DT>::MINW;
+            first[q] = st.marker(i);
+            kw[q] = st.mask(i);
+        }
+        unsigned due = 0u;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            VRow<DT> p, v, kv;
+            p.set(above[q]);
+            v.set(first[q]);
+            kv.set(kw[q]);
+            vstep<DT>(v, kv, offers<DT, 8>(p, sel));
+            if (__any_sync(FULL, v.word() != first[q])) due |= 1u << q;
+        }
+        while (due != 0u) {
+            const int i = (s0 + __ffs((int)due) - 1) * kSeg8;
+            due &= due - 1u;
+            VRow<DT> prev;
+            prev.set(st.marker(i - 1));
+            st.template walk<true>(prev, i, d.H, sel);
+        }
+    }
 }
 
 // Vertical sweep for 4-connectivity, int32 (the whole-image init passes use
@@ -870,10 +971,20 @@ static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void*
         const unsigned blocks = (unsigned)strips;
         const bool down = direction == 1;
         if (d.conn == 8) {
-            if (down)
-                sweep_y_kernel<DT, 8, true><<<blocks, 32, 0, s>>>(d);
-            else
-                sweep_y_kernel<DT, 8, false><<<blocks, 32, 0, s>>>(d);
+            const int segs = (d.H + kSeg8 - 1) / kSeg8;
+            auto run = [&](auto dir) {
+                constexpr bool D = decltype(dir)::value;
+                auto grid = [&](long long n) {
+                    return (unsigned)((n * strips + kY8Threads / 32 - 1) / (kY8Threads / 32));
+                };
+                sweep_y8_local_kernel<DT, D><<<grid(segs), kY8Threads, 0, s>>>(d, strips, segs);
+                if (segs == 1) return 1;
+                for (int r = 0; r < kY8Enter; ++r)
+                    sweep_y8_enter_kernel<DT, D><<<grid(segs - 1), kY8Threads, 0, s>>>(d, strips, segs);
+                sweep_y8_settle_kernel<DT, D><<<blocks, 32, 0, s>>>(d, segs);
+                return 2 + kY8Enter;
+            };
+            return down ? run(std::true_type{}) : run(std::false_type{});
         } else if (DT == DT_I32) {
             const unsigned nblocks = (unsigned)((d.W + 31) / 32);
             if (scratch && sweep_scratch_bytes(d) > 0) {

@@ -644,14 +644,6 @@ __global__ void __launch_bounds__(kTopThreads, 4) top_apply_label_kernel(TopArgs
 // pixel DIRTY on all sides and appends it to the seed list; other tiles get
 // state 0.
 
-// A marker pixel, the least value outside the image.
-template <int DT>
-__device__ __forceinline__ uint32_t seed_px(const ImgDesc& d, int y, int x) {
-    using P = Px<DT>;
-    if (y < 0 || y >= d.H || x < 0 || x >= d.W) return P::MINPX;
-    return P::ld_px(d.marker + (size_t)y * d.pitch_m + (size_t)x * P::BPP);
-}
-
 // The check with wide lanes: a lane holds WPL words (8 bytes) of a row, so a
 // warp covers WPL engine tiles side by side (32 / WPL lanes each); the words
 // are taken apart as in the engine's vertical pass (VRow: byte SIMD is not in
@@ -659,41 +651,9 @@ __device__ __forceinline__ uint32_t seed_px(const ImgDesc& d, int y, int x) {
 // from permutes with the adjacent words, and rows are loaded kSeedAhead ahead
 // into a register ring (one vector load per lane where the address allows
 // it, else word by word; rows start on 4-byte boundaries).
-constexpr int kSeedAhead = 2;
+constexpr int kSeedAhead = 3;
 constexpr int kSeedThreads = 128;
 constexpr int kSeedWords = 2;  // words per lane
-
-// WPL words of row y from byte b0 (pixels past the row or outside the image:
-// the least value).
-template <int DT, int WPL>
-__device__ __forceinline__ void seed_load(const ImgDesc& d, const unsigned char* base, long long pitch, int y,
-                                          long long b0, long long row_bytes, uint32_t (&w)[WPL]) {
-    using P = Px<DT>;
-#pragma unroll
-    for (int i = 0; i < WPL; ++i) w[i] = P::MINW;
-    if (y < 0 || y >= d.H || b0 >= row_bytes) return;
-    const unsigned char* p = base + (size_t)y * pitch + b0;
-    if (b0 + 4 * WPL <= row_bytes && (reinterpret_cast<uintptr_t>(p) & (4 * WPL - 1)) == 0) {
-        if constexpr (WPL == 4) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(p));
-            w[0] = v.x;
-            w[1] = v.y;
-            w[2] = v.z;
-            w[3] = v.w;
-        } else {
-            const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
-            w[0] = v.x;
-            w[1] = v.y;
-        }
-        return;
-    }
-    // rows only 4-byte aligned, or the row's last lane: word by word
-#pragma unroll
-    for (int i = 0; i < WPL; ++i) {
-        const long long b = b0 + 4 * i;
-        if (b < row_bytes) w[i] = load_word_plain<DT>(p + 4 * i, (int)((row_bytes - b) / P::BPP), false);
-    }
-}
 
 // One unit of the check: the WPL engine tiles of tile row ty, group gx of
 // image d.  All lanes of the warp.
@@ -710,37 +670,70 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
     const long long row_bytes = (long long)d.W * P::BPP;
     const int y0 = ty * TH, rows = min(TH, d.H - y0);
     const long long b0 = (long long)gx * (128 * WPL) + lane * (4 * WPL);
-    const int xl = gx * WPL * TW - 1, xr = (gx + 1) * WPL * TW;  // halo columns
-    auto halo = [&](int y) -> uint32_t {
-        if (lane == 0) return seed_px<DT>(d, y, xl);
-        if (lane == 31) return seed_px<DT>(d, y, xr);
-        return P::MINPX;
+    // Rows are read through running pointers, the halo columns (lane 0 the
+    // pixel left of the group, lane 31 the one right of it) too: with the
+    // addresses worked out per row, and a branch for either halo pixel, that
+    // was most of the check's instructions.
+    const unsigned char* pm = d.marker + (long long)(y0 - 1) * d.pitch_m + b0;
+    const unsigned char* pk = d.mask + (long long)y0 * d.pitch_k + b0;
+    const int hx = lane == 0 ? gx * WPL * TW - 1 : (gx + 1) * WPL * TW;
+    const bool halo_lane = (lane == 0 && hx >= 0) || (lane == 31 && hx < d.W);
+    const unsigned char* ph = d.marker + (long long)(y0 - 1) * d.pitch_m + (long long)hx * P::BPP;
+    const bool inside = b0 < row_bytes;
+    const bool vec = b0 + 4 * WPL <= row_bytes &&
+                     ((reinterpret_cast<uintptr_t>(pm) | reinterpret_cast<uintptr_t>(pk) | (uintptr_t)d.pitch_m |
+                       (uintptr_t)d.pitch_k) & (4 * WPL - 1)) == 0;
+    const bool fast = __all_sync(FULL, vec || !inside);
+    int ym = y0 - 1, yk = y0;  // the rows the pointers are at
+    auto load = [&](const unsigned char* q, bool in, uint32_t (&w)[WPL]) {
+#pragma unroll
+        for (int i = 0; i < WPL; ++i) w[i] = P::MINW;
+        if (!in || !inside) return;
+        if (fast) {
+            const uint2 v = __ldg(reinterpret_cast<const uint2*>(q));
+            w[0] = v.x;
+            w[1] = v.y;
+        } else {
+            // rows only 4-byte aligned, or the row's last lane: word by word
+#pragma unroll
+            for (int i = 0; i < WPL; ++i) {
+                const long long b = b0 + 4 * i;
+                if (b < row_bytes) w[i] = load_word_plain<DT>(q + 4 * i, (int)((row_bytes - b) / P::BPP), false);
+            }
+        }
+    };
+    auto next_marker = [&](uint32_t (&w)[WPL], uint32_t& h) {
+        const bool in = (unsigned)ym < (unsigned)d.H;
+        load(pm, in, w);
+        h = P::MINPX;
+        if (halo_lane && in) h = P::ld_px(ph);
+        pm += d.pitch_m;
+        ph += d.pitch_m;
+        ++ym;
+    };
+    auto next_mask = [&](uint32_t (&w)[WPL]) {  // past the tile's rows: nothing can rise
+        load(pk, yk < y0 + rows, w);
+        pk += d.pitch_k;
+        ++yk;
     };
     // window: marker rows r - 1, r (taken apart), mask row r, halo pixels
     uint32_t w0[WPL], kc[WPL];
+    uint32_t hu, hc;
     VRow<DT> mu[WPL], mc[WPL];
-    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0 - 1, b0, row_bytes, w0);
+    next_marker(w0, hu);
 #pragma unroll
     for (int w = 0; w < WPL; ++w) mu[w].set(w0[w]);
-    seed_load<DT, WPL>(d, d.marker, d.pitch_m, y0, b0, row_bytes, w0);
+    next_marker(w0, hc);
 #pragma unroll
     for (int w = 0; w < WPL; ++w) mc[w].set(w0[w]);
-    seed_load<DT, WPL>(d, d.mask, d.pitch_k, y0, b0, row_bytes, kc);
-    uint32_t hu = halo(y0 - 1), hc = halo(y0);
+    next_mask(kc);
     // ring slot i holds marker / mask / halo of row r + 1 + i
     uint32_t rm[kSeedAhead][WPL], rk[kSeedAhead][WPL];
     uint32_t rh[kSeedAhead];
 #pragma unroll
     for (int i = 0; i < kSeedAhead; ++i) {
-        const int y = y0 + 1 + i;
-        seed_load<DT, WPL>(d, d.marker, d.pitch_m, y, b0, row_bytes, rm[i]);
-        if (i + 1 < rows) {
-            seed_load<DT, WPL>(d, d.mask, d.pitch_k, y, b0, row_bytes, rk[i]);
-        } else {
-#pragma unroll
-            for (int w = 0; w < WPL; ++w) rk[i][w] = P::MINW;
-        }
-        rh[i] = halo(y);
+        next_marker(rm[i], rh[i]);
+        next_mask(rk[i]);
     }
     uint32_t rose = 0u;
     for (int r0 = 0; r0 < rows; r0 += kSeedAhead) {
@@ -756,17 +749,8 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
                 kn[w] = rk[i][w];
             }
             const uint32_t hd = rh[i];
-            {
-                const int y = y0 + r + 1 + kSeedAhead;
-                seed_load<DT, WPL>(d, d.marker, d.pitch_m, y, b0, row_bytes, rm[i]);
-                if (r + 1 + kSeedAhead < rows) {
-                    seed_load<DT, WPL>(d, d.mask, d.pitch_k, y, b0, row_bytes, rk[i]);
-                } else {
-#pragma unroll
-                    for (int w = 0; w < WPL; ++w) rk[i][w] = P::MINW;
-                }
-                rh[i] = halo(y);
-            }
+            next_marker(rm[i], rh[i]);
+            next_mask(rk[i]);
             // what a column offers its side neighbours: itself, or with
             // 8-connectivity the largest of its three rows
             VRow<DT> V[WPL], S[WPL];
@@ -830,7 +814,7 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
 template <int DT, int WPL>
 __global__ void __launch_bounds__(kSeedThreads, 8)
     seed_wide_kernel(const ImgDesc d, unsigned* state, unsigned* list, unsigned* nlist) {
-    static_assert(WPL == 2 || WPL == 4, "8- or 16-byte lanes");
+    static_assert(WPL == 2, "8-byte lanes");
     if (gated_off(d)) return;
     const int gx_n = (d.tiles_x + WPL - 1) / WPL;
     const long long units = (long long)gx_n * d.tiles_y;
