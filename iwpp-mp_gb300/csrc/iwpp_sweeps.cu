@@ -14,8 +14,6 @@
 //            previous row inside a 128-byte strip, segments of rows first on
 //            their own, then their entries.  The result is the walk's, row
 //            by row, whatever the order.
-#include <type_traits>
-
 #include "iwpp_engine.cuh"
 
 namespace iwpp {
@@ -439,38 +437,42 @@ __device__ __forceinline__ void cp_async_wait() {
 // rows of a plane ahead, in cp.async groups of kGroup rows.
 constexpr int kRing = 64, kGroup = 8;
 
-// 8-connected vertical sweeps.  A 128-byte column strip is closed: its rows
-// take the three pixels of the row before them inside the strip (a lane holds
-// a word).  Row by row that is a chain of about 50 cycles a row (a shuffle and
-// five dependent operations), and with the diagonals a run of rows is no
+// Vertical sweeps by strips (8-connected ones, and 4-connected ones of rows
+// that the ring kernels below do not stream).  A 128-byte column strip is
+// closed: its rows take the three pixels (4-connected: one) of the row before
+// them inside the strip (a lane holds a word).  Row by row that is a chain of
+// 50 cycles a row and more, and with the diagonals a run of rows is no
 // per-column map that could be composed; one warp walking a strip's whole
 // height took 500 us for 4096 rows whatever the width.  But the sweep is the
 // least solution of "each row at least what the row before it offers", so the
 // rows can be taken in any order that ends with no row left to raise:
-//   sweep_y8_local_kernel: segments of kSeg8 rows, a warp each, as if nothing
-//     entered them;
-//   sweep_y8_enter_kernel, kY8Enter times: a warp per segment, what the row
-//     before the segment offers, on from there while the rows rise; the row
-//     before it may itself be rising meanwhile;
-//   sweep_y8_settle_kernel: a warp per strip, the segments in order, any entry
+//   sweep_strip_local_kernel: segments of kStripRows rows, a warp each, as if
+//     nothing entered them;
+//   sweep_strip_enter_kernel, kStripEnter times: a warp per segment, what the
+//     row before the segment offers, on from there while the rows rise; the
+//     row before it may itself be rising meanwhile;
+//   sweep_strip_settle_kernel: a warp per strip, the segments in order, any entry
 //     that still raises something, on from there while the rows rise.
 // Same bytes as the walk.  Measured on 4096^2 uint8 h-domes (+Y / -Y, us): the
 // walk 496 / 516; segments of 64 rows with 1 / 2 / 4 / 8 enter steps 144 / 81 /
 // 70 / 87, of 128 rows 70 / 60 / 66 / 83, of 32 rows 304 / 203 / 111 / 105.
 // Bound by the chain: a row is about 100 cycles of one warp.
-constexpr int kSeg8 = 128;
-constexpr int kY8Enter = 2;
-constexpr int kY8Threads = 128;
+constexpr int kStripRows = 128;
+constexpr int kStripEnter = 2;
+// images up to this height: one walk, whose launch is all it costs (1024 x 182
+// uint16 12 us; in segments 29 and three more launches)
+constexpr int kStripWhole = 384;
+constexpr int kStripThreads = 128;
 
 // A lane's word column of a strip, rows by their index in sweep order.
-template <int DT, bool DOWN>
-struct Strip8 {
+template <int DT, int CONN, bool DOWN>
+struct Strip {
     using P = Px<DT>;
     unsigned char* m;
     const unsigned char* k;
     long long pitch_m, pitch_k;
     int npx, H;
-    __device__ __forceinline__ Strip8(const ImgDesc& d, int strip, int lane) : H(d.H) {
+    __device__ __forceinline__ Strip(const ImgDesc& d, int strip, int lane) : H(d.H) {
         const int px0 = strip * 32 * P::PPW + lane * P::PPW;
         npx = d.W - px0;
         const size_t off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
@@ -530,7 +532,7 @@ struct Strip8 {
                 VRow<DT> v, kv;
                 v.set(old[q]);
                 kv.set(kw[q]);
-                vstep<DT>(v, kv, offers<DT, 8>(prev, sel));
+                vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
                 const uint32_t w = v.word();
                 x = w ^ old[q];
                 if (WORDS) {
@@ -556,7 +558,7 @@ struct Strip8 {
             VRow<DT> v, kv;
             v.set(was);
             kv.set(mask(i));
-            vstep<DT>(v, kv, offers<DT, 8>(prev, sel));
+            vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
             const uint32_t w = v.word();
             if (w != was) store(i, w);
             if (STOP && !__any_sync(FULL, w != was)) return;
@@ -565,40 +567,41 @@ struct Strip8 {
     }
 };
 
-template <int DT, bool DOWN>
-__global__ void __launch_bounds__(kY8Threads) sweep_y8_local_kernel(ImgDesc d, int strips, int segs) {
+template <int DT, int CONN, bool DOWN>
+__global__ void __launch_bounds__(kStripThreads) sweep_strip_local_kernel(ImgDesc d, int strips, int segs,
+                                                                    int seg_rows) {
     if (gated_off(d)) return;
     const int lane = threadIdx.x & 31;
-    const long long wid = (long long)blockIdx.x * (kY8Threads / 32) + (threadIdx.x >> 5);
+    const long long wid = (long long)blockIdx.x * (kStripThreads / 32) + (threadIdx.x >> 5);
     if (wid >= (long long)strips * segs) return;
     const int seg = (int)(wid / strips), strip = (int)(wid - (long long)seg * strips);
-    const Strip8<DT, DOWN> st(d, strip, lane);
+    const Strip<DT, CONN, DOWN> st(d, strip, lane);
     const EdgeSel sel(lane);
-    const int i0 = seg * kSeg8, end = min(i0 + kSeg8, d.H);
+    const int i0 = seg * seg_rows, end = min(i0 + seg_rows, d.H);
     VRow<DT> prev;
     prev.set(Px<DT>::MINW);
     st.template walk<false>(prev, i0, end, sel);
 }
 
-template <int DT, bool DOWN>
-__global__ void __launch_bounds__(kY8Threads) sweep_y8_enter_kernel(ImgDesc d, int strips, int segs) {
+template <int DT, int CONN, bool DOWN>
+__global__ void __launch_bounds__(kStripThreads) sweep_strip_enter_kernel(ImgDesc d, int strips, int segs) {
     if (gated_off(d)) return;
     const int lane = threadIdx.x & 31;
-    const long long wid = (long long)blockIdx.x * (kY8Threads / 32) + (threadIdx.x >> 5);
+    const long long wid = (long long)blockIdx.x * (kStripThreads / 32) + (threadIdx.x >> 5);
     if (wid >= (long long)strips * (segs - 1)) return;
     const int seg = 1 + (int)(wid / strips), strip = (int)(wid % strips);
-    const Strip8<DT, DOWN> st(d, strip, lane);
-    const int i0 = seg * kSeg8;
+    const Strip<DT, CONN, DOWN> st(d, strip, lane);
+    const int i0 = seg * kStripRows;
     VRow<DT> prev;
     prev.set(st.marker(i0 - 1));
-    st.template walk<true>(prev, i0, min(i0 + kSeg8, d.H), EdgeSel(lane));
+    st.template walk<true>(prev, i0, min(i0 + kStripRows, d.H), EdgeSel(lane));
 }
 
-template <int DT, bool DOWN>
-__global__ void __launch_bounds__(32) sweep_y8_settle_kernel(ImgDesc d, int segs) {
+template <int DT, int CONN, bool DOWN>
+__global__ void __launch_bounds__(32) sweep_strip_settle_kernel(ImgDesc d, int segs) {
     if (gated_off(d)) return;
     const int lane = threadIdx.x;
-    const Strip8<DT, DOWN> st(d, (int)blockIdx.x, lane);
+    const Strip<DT, CONN, DOWN> st(d, (int)blockIdx.x, lane);
     const EdgeSel sel(lane);
 #pragma unroll 1
     for (int s0 = 1; s0 < segs; s0 += 8) {
@@ -608,7 +611,7 @@ __global__ void __launch_bounds__(32) sweep_y8_settle_kernel(ImgDesc d, int segs
         uint32_t above[8], first[8], kw[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
-            const int i = (s0 + q) * kSeg8;
+            const int i = (s0 + q) * kStripRows;
             above[q] = i < d.H ? st.marker(i - 1) : Px<DT>::MINW;
             first[q] = st.marker(i);
             kw[q] = st.mask(i);
@@ -620,11 +623,11 @@ __global__ void __launch_bounds__(32) sweep_y8_settle_kernel(ImgDesc d, int segs
             p.set(above[q]);
             v.set(first[q]);
             kv.set(kw[q]);
-            vstep<DT>(v, kv, offers<DT, 8>(p, sel));
+            vstep<DT>(v, kv, offers<DT, CONN>(p, sel));
             if (__any_sync(FULL, v.word() != first[q])) due |= 1u << q;
         }
         while (due != 0u) {
-            const int i = (s0 + __ffs((int)due) - 1) * kSeg8;
+            const int i = (s0 + __ffs((int)due) - 1) * kStripRows;
             due &= due - 1u;
             VRow<DT> prev;
             prev.set(st.marker(i - 1));
@@ -938,15 +941,29 @@ cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s) {
     return cudaGetLastError();
 }
 
+// A vertical sweep by 128-byte strips; returns the launches.
+template <int DT, int CONN, bool DOWN>
+static int launch_strips(const ImgDesc& d, int strips, cudaStream_t s) {
+    const bool whole = d.H <= kStripWhole;
+    const int seg_rows = whole ? d.H : kStripRows, segs = whole ? 1 : (d.H + kStripRows - 1) / kStripRows;
+    auto grid = [&](long long n) { return (unsigned)((n * strips + kStripThreads / 32 - 1) / (kStripThreads / 32)); };
+    sweep_strip_local_kernel<DT, CONN, DOWN><<<grid(segs), kStripThreads, 0, s>>>(d, strips, segs, seg_rows);
+    if (whole) return 1;
+    for (int r = 0; r < kStripEnter; ++r)
+        sweep_strip_enter_kernel<DT, CONN, DOWN><<<grid(segs - 1), kStripThreads, 0, s>>>(d, strips, segs);
+    sweep_strip_settle_kernel<DT, CONN, DOWN><<<(unsigned)strips, 32, 0, s>>>(d, segs);
+    return 2 + kStripEnter;
+}
+
 template <int DT>
 static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void* scratch) {
     using P = Px<DT>;
     constexpr int TW = 32 * P::PPW;
+    const bool aligned16 =
+        ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
+        ((d.pitch_m | d.pitch_k) & 15) == 0;
     if (direction == 0 || direction == 2) {
         const unsigned blocks = blocks_for((long long)d.H * 32, 128);
-        const bool aligned16 =
-            ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
-            ((d.pitch_m | d.pitch_k) & 15) == 0;
         if (aligned16 && DT == DT_U8) {
             // two rows per warp (uint16 measured no faster: its lanes hold
             // half as many pixels, so the scan is a smaller share)
@@ -968,24 +985,19 @@ static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void*
         return 1;
     } else {
         const int strips = (d.W + TW - 1) / TW;
-        const unsigned blocks = (unsigned)strips;
         const bool down = direction == 1;
-        if (d.conn == 8) {
-            const int segs = (d.H + kSeg8 - 1) / kSeg8;
-            auto run = [&](auto dir) {
-                constexpr bool D = decltype(dir)::value;
-                auto grid = [&](long long n) {
-                    return (unsigned)((n * strips + kY8Threads / 32 - 1) / (kY8Threads / 32));
-                };
-                sweep_y8_local_kernel<DT, D><<<grid(segs), kY8Threads, 0, s>>>(d, strips, segs);
-                if (segs == 1) return 1;
-                for (int r = 0; r < kY8Enter; ++r)
-                    sweep_y8_enter_kernel<DT, D><<<grid(segs - 1), kY8Threads, 0, s>>>(d, strips, segs);
-                sweep_y8_settle_kernel<DT, D><<<blocks, 32, 0, s>>>(d, segs);
-                return 2 + kY8Enter;
-            };
-            return down ? run(std::true_type{}) : run(std::false_type{});
-        } else if (DT == DT_I32) {
+        if (d.conn == 8)
+            return down ? launch_strips<DT, 8, true>(d, strips, s) : launch_strips<DT, 8, false>(d, strips, s);
+        // 4-connected rows off the 16-byte boundary, or not a whole number of
+        // the ring kernels' strips wide: those kernels load what is not 16
+        // bytes element by element (2000 x 768 uint8 240 us, by strips 42;
+        // 1416 x 5514 uint8 574 and 54, uint16 487 and 54; 708 x 5514 int32
+        // 1640 and 33).  The others stay with them: their segments' maps
+        // compose, so a long vertical path costs nothing (16384^2 spiral 250
+        // us, by strips 1614; without one 250 and 222).
+        if (!aligned16 || (long long)d.W * P::BPP % (DT == DT_I32 ? 128 : 64) != 0)
+            return down ? launch_strips<DT, 4, true>(d, strips, s) : launch_strips<DT, 4, false>(d, strips, s);
+        if (DT == DT_I32) {
             const unsigned nblocks = (unsigned)((d.W + 31) / 32);
             if (scratch && sweep_scratch_bytes(d) > 0) {
                 const int nseg = (d.H + kSegRows - 1) / kSegRows;

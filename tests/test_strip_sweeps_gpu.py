@@ -1,5 +1,6 @@
-"""8-connected vertical whole-image sweeps, which run in segments of 128 rows:
-heights at and around the segment edges, paths that cross many of them
+"""Vertical whole-image sweeps by strips (8-connected, and 4-connected of rows off
+the 16-byte boundary), which run in one walk up to 384 rows and above that in
+segments of 128: heights at and around those, paths that cross many of them
 (straight, diagonal, along a strip's edge), against the restatement."""
 import numpy as np
 import pytest
@@ -18,12 +19,12 @@ def _dev(a):
 
 
 @pytest.mark.parametrize("dt", [0, 1, 2])
-@pytest.mark.parametrize("h", [1, 7, 64, 127, 128, 129, 136, 257, 641, 1100])
-def test_tall_8_connected_sweeps(dt, h):
+@pytest.mark.parametrize("h", [1, 7, 64, 383, 384, 385, 392, 512, 513, 641, 1100])
+def test_strip_sweeps(dt, h):
     rng = np.random.default_rng(h * 10 + dt)
     info = np.iinfo(NP[dt])
     levels = np.linspace(info.min, info.max, 9).astype(np.int64)
-    for w in (1, 5, TW[dt], 2 * TW[dt] + 3):
+    for w in (1, 5, TW[dt], 2 * TW[dt] + 3, TW[dt] + 4):
         mask = levels[rng.integers(0, 8, (h, w))].astype(NP[dt])
         y = np.arange(h)
         mask[:, w // 2] = info.max                      # a straight path
@@ -34,7 +35,8 @@ def test_tall_8_connected_sweeps(dt, h):
         marker[at] = mask[at]
         marker[0], marker[-1] = mask[0], mask[-1]
         for d in (1, 3):
-            tm, tk = _dev(marker), _dev(mask)
-            iwpp.sweep(tm, tk, d, 8)
-            got = tm.cpu().numpy().view(NP[dt])
-            assert np.array_equal(got, oracle.sweep(marker, mask, d, 8)), (w, d)
+            for conn in (4, 8):
+                tm, tk = _dev(marker), _dev(mask)
+                iwpp.sweep(tm, tk, d, conn)
+                got = tm.cpu().numpy().view(NP[dt])
+                assert np.array_equal(got, oracle.sweep(marker, mask, d, conn)), (w, d, conn)
