@@ -648,7 +648,8 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     a.nimg = (int)job.descs.size();
     if (a.nimg == 1) {
         a.one = job.descs[0];
-        a.one.tmaps = job.has_tma[0] ? base + l.off_tmaps : nullptr;
+        a.one_tma = job.has_tma[0];
+        std::memcpy(a.one_maps, job.tmaps.data(), sizeof(a.one_maps));
     }
     a.G = (unsigned)job.G;
     a.state = reinterpret_cast<unsigned*>(base + l.off_state);
@@ -683,7 +684,7 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     }
 
     cudaError_t e = cudaSuccess;
-    if (upload_descs && !job.descs.empty()) {
+    if (upload_descs && job.descs.size() > 1) {
         std::vector<ImgDesc> descs = job.descs;
         for (size_t i = 0; i < descs.size(); ++i)
             descs[i].tmaps = job.has_tma[i] ? base + l.off_tmaps + i * 2u * sizeof(CUtensorMap) : nullptr;
@@ -790,8 +791,10 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     return IWPP_OK;
 }
 
+// Waits for a job and its counters with one synchronisation; ev0 / ev1
+// (nullable) were recorded around it.
 int read_stats(Ctrl* host_ctrl, const Workspace& ws, cudaStream_t s, long long tiles, int variant,
-               iwpp_stats* out, float ms, int launches = 0) {
+               iwpp_stats* out, cudaEvent_t ev0 = nullptr, cudaEvent_t ev1 = nullptr, int launches = 0) {
     cudaError_t e = cudaMemcpyAsync(host_ctrl, ws.base, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e);
@@ -808,6 +811,8 @@ int read_stats(Ctrl* host_ctrl, const Workspace& ws, cudaStream_t s, long long t
         out->restarts = (int)host_ctrl->restarts;
         out->status = st;
         out->variant = variant;
+        float ms = 0.f;
+        if (ev0 && cudaEventElapsedTime(&ms, ev0, ev1) != cudaSuccess) cudaGetLastError();
         out->device_ms = ms;
         out->row_steps = (long long)host_ctrl->row_steps;
         for (int i = 0; i < 5; ++i) out->phase_cycles[i] = (long long)host_ctrl->phase[i];
@@ -872,14 +877,7 @@ int run_job_sync(iwpp_handle h, const iwpp_image* imgs, int n, int variant, cons
     if (rc == IWPP_OK) rc = enqueue_job(job, h->ws, s, h->device, true, h->ev0, h->ev1, true, &h->staging, &nl);
     const int rc_stage = finish_staging(job, s);
     if (rc == IWPP_OK) {
-        float ms = 0.f;
-        cudaError_t e = cudaStreamSynchronize(s);
-        if (e != cudaSuccess)
-            rc = cuda_status(e);
-        else {
-            cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-            rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, stats, ms, nl + job.stage_launches);
-        }
+        rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, stats, h->ev0, h->ev1, nl + job.stage_launches);
     } else {
         cudaStreamSynchronize(s);
     }
@@ -1092,7 +1090,7 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
         // Workspace and descriptors first (outside the graph, once).
         const Layout l = job_layout(job);
         rc = ensure_workspace(p->ws, l.total);
-        if (rc == IWPP_OK && !job.descs.empty()) {
+        if (rc == IWPP_OK && job.descs.size() > 1) {
             char* wbase = static_cast<char*>(p->ws.base);
             std::vector<ImgDesc> descs = job.descs;
             for (size_t i = 0; i < descs.size(); ++i)
@@ -1306,7 +1304,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
                 return -1.0;
             }
             if (cudaStreamSynchronize(s) != cudaSuccess) return -1.0;
-            if (read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, nullptr, 0.f) != IWPP_OK) return -1.0;
+            if (read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, nullptr) != IWPP_OK) return -1.0;
             float ms = 0.f;
             if (job.G > 0) cudaEventElapsedTime(&ms, h->ev0, h->ev1);
             ts.push_back(ms);
@@ -1423,7 +1421,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
             const int src = finish_staging(job, s);
             if (rc == IWPP_OK) rc = src;
             if (cudaStreamSynchronize(s) != cudaSuccess && rc == IWPP_OK) rc = IWPP_ERR_CUDA;
-            if (rc == IWPP_OK) rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, nullptr, 0.f);
+            if (rc == IWPP_OK) rc = read_stats(h->host_ctrl, h->ws, s, job.G, job.variant, nullptr);
         }
     } else {
         restore();  // leave the markers as they came
@@ -1504,21 +1502,35 @@ int iwpp_sweep(void* marker, const void* mask, size_t pitch_marker, size_t pitch
     int rc = check_image(marker, mask, pitch_marker, pitch_mask, width, height, dtype, connectivity);
     if (rc != IWPP_OK) return set_last(rc);
     if (direction < 0 || direction > 3) return set_last(IWPP_ERR_INVALID);
-    iwpp_image im{marker, mask, pitch_marker, pitch_mask, width, height, dtype, connectivity};
-    Job job;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    iwpp_config c{};
-    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC, nullptr);
-    if (rc == IWPP_OK && !job.descs.empty()) {
+    auto sweep = [&](const ImgDesc& d) {
         void* scratch = nullptr;
-        const size_t sb = sweep_scratch_bytes(job.descs[0]);
+        const size_t sb = sweep_scratch_bytes(d);
         if (sb > 0 && cudaMallocAsync(&scratch, sb, s) != cudaSuccess) {
             cudaGetLastError();
             scratch = nullptr;  // one warp per whole column instead
         }
-        rc = cuda_status(launch_sweep(job.descs[0], direction, s, scratch));
+        const int r = cuda_status(launch_sweep(d, direction, s, scratch));
         if (scratch) cudaFreeAsync(scratch, s);
+        return r;
+    };
+    if (aligned_for_engine(marker, pitch_marker) && aligned_for_engine(mask, pitch_mask)) {
+        ImgDesc d{};
+        d.marker = static_cast<unsigned char*>(marker);
+        d.mask = static_cast<const unsigned char*>(mask);
+        d.pitch_m = (long long)pitch_marker;
+        d.pitch_k = (long long)pitch_mask;
+        d.W = width;
+        d.H = height;
+        d.dtype = dtype;
+        d.conn = connectivity;
+        return set_last(width > 0 && height > 0 ? sweep(d) : IWPP_OK);
     }
+    iwpp_image im{marker, mask, pitch_marker, pitch_mask, width, height, dtype, connectivity};
+    Job job;
+    iwpp_config c{};
+    rc = build_job(job, &im, 1, IWPP_QUEUE_UNIQUE, &c, s, STAGE_ASYNC, nullptr);
+    if (rc == IWPP_OK && !job.descs.empty()) rc = sweep(job.descs[0]);
     const int rc2 = finish_staging(job, s);
     return set_last(rc == IWPP_OK ? rc2 : rc);
 }

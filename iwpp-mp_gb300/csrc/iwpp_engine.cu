@@ -699,7 +699,7 @@ struct QueueOf<VAR_ASYNC> {
 // over a warp's blocks needs them; 16 and 32 warps measured the same or
 // slower (32: a fifth slower, spills).
 template <int VAR, int TH, int W, bool ALT>
-__global__ void __launch_bounds__(32 * W, ALT ? 8 : W == 2 ? 10 : 24 / W) engine_kernel(EngineArgs a) {
+__global__ void __launch_bounds__(32 * W, ALT ? 8 : W == 2 ? 10 : 24 / W) engine_kernel(const __grid_constant__ EngineArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     // 128-byte align the tile (the launch adds 128 bytes of slack)
@@ -711,8 +711,12 @@ __global__ void __launch_bounds__(32 * W, ALT ? 8 : W == 2 ? 10 : 24 / W) engine
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         sm.nb = 0u;
         sm.count = VisitCount{};
-        if (a.nimg == 1) sm.d = a.one;
-        else sm.d = a.imgs[0];
+        if (a.nimg == 1) {
+            sm.d = a.one;
+            sm.d.tmaps = a.one_tma ? a.one_maps : nullptr;
+        } else {
+            sm.d = a.imgs[0];
+        }
     }
     if (lane == 0) sm.mark[0][warp][0] = sm.mark[0][warp][1] = sm.mark[1][warp][0] = sm.mark[1][warp][1] = 0u;
     cta_sync<W>();
@@ -1066,11 +1070,14 @@ cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li
     cfg.blockDim = dim3((unsigned)k.threads);
     cfg.dynamicSmemBytes = k.smem;
     cfg.stream = s;
+    // The round queues' grid barrier and the mutex queue's initial slices need
+    // every CTA resident.  With the async queue any CTA can do any entry, so
+    // its launch may start with part of its CTAs beside another job's.
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeCooperative;
     attr[0].val.cooperative = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = variant == VAR_ASYNC ? 0 : 1;
     EngineArgs args = a;
     void* params[] = {&args};
     return cudaLaunchKernelExC(&cfg, k.fn, params);

@@ -29,6 +29,8 @@
 // raise a neighbour is followed by DIRTY on that neighbour after a fence.
 #pragma once
 
+#include <cuda.h>
+
 #include <vector>
 
 #include "iwpp_device.cuh"
@@ -88,7 +90,11 @@ struct Ctrl {
 
 struct EngineArgs {
     const ImgDesc* imgs;
-    ImgDesc one;        // the image of a one-image job (nimg 1): read from the launch's parameters
+    // A one-image job (nimg 1) has its image and its tensor maps (`one_tma`) in
+    // the launch's parameters: nothing to upload before it.
+    ImgDesc one;
+    CUtensorMap one_maps[2];
+    int one_tma;
     int nimg;
     unsigned G;         // tiles in the job
     unsigned* state;    // G tile state words

@@ -812,7 +812,7 @@ __device__ __forceinline__ void seed_unit(const ImgDesc& d, int ty, int gx, unsi
 }
 
 template <int DT, int WPL>
-__global__ void __launch_bounds__(kSeedThreads, 8)
+__global__ void __launch_bounds__(kSeedThreads, 6)
     seed_wide_kernel(const ImgDesc d, unsigned* state, unsigned* list, unsigned* nlist) {
     static_assert(WPL == 2, "8-byte lanes");
     if (gated_off(d)) return;
@@ -1014,8 +1014,8 @@ cudaError_t launch_seed_batch(const ImgDesc* dev_descs, const std::vector<ImgDes
     const int nimg = (int)host_descs.size();
     long long units = 0;
     for (const auto& d : host_descs) units += (long long)((d.tiles_x + kSeedWords - 1) / kSeedWords) * d.tiles_y;
-    if (nimg == 0 || nimg > kSeedMaxImages) {
-        // one launch per image
+    if (nimg <= 1 || nimg > kSeedMaxImages) {
+        // one launch per image (one image: its descriptor is not on the device)
         for (auto d : host_descs) {
             d.gate = gate;
             const cudaError_t e = launch_seed(d, state, list, nlist, s, launches);

@@ -32,8 +32,8 @@ cudaError_t launch_seed(const ImgDesc& d, unsigned* state, unsigned* list, unsig
                         int* launches);
 // The same check over every image of a job in one launch (one launch per
 // image when the job has more than 1024).  `dev_descs`: the job's descriptors in device
-// memory (`host_descs` the same on the host); `gate` (nullable) as
-// ImgDesc::gate.
+// memory (`host_descs` the same on the host; a single image is passed by
+// value); `gate` (nullable) as ImgDesc::gate.
 cudaError_t launch_seed_batch(const ImgDesc* dev_descs, const std::vector<ImgDesc>& host_descs, const unsigned* gate,
                               unsigned* state, unsigned* list, unsigned* nlist, cudaStream_t s, int* launches);
 // After a seed check over a job's G tiles (its count in *count): *gate = 1
