@@ -22,10 +22,12 @@
 #include <cuda_runtime.h>
 
 #include "iwpp.h"
+#include "iwpp_engine.cuh"
 
 namespace iwpp {
 int handle_reserve(iwpp_handle h, size_t bytes);  // iwpp_api.cu
 }
+using iwpp::StageCopy;
 
 namespace {
 
@@ -36,6 +38,35 @@ size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 double us_between(Clock::time_point a, Clock::time_point b) {
     return std::chrono::duration<double, std::micro>(b - a).count();
+}
+
+// The device's address of a host image of `h` rows if all of it is pinned (one
+// pinned allocation or registration), else nullptr.
+const void* pinned_address(const void* p, size_t pitch, size_t row, int h) {
+    using Get = CUresult (*)(unsigned, CUpointer_attribute*, void**, CUdeviceptr);
+    static const Get get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 7000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<Get>(f);
+    }();
+    if (!get) return nullptr;
+    unsigned type = 0;
+    CUdeviceptr dev = 0, start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[4] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+                                   CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void* out[4] = {&type, &dev, &start, &size};
+    const CUdeviceptr a = reinterpret_cast<CUdeviceptr>(p);
+    if (get(4, what, out, a) != CUDA_SUCCESS || type != CU_MEMORYTYPE_HOST || dev == 0 || start == 0) return nullptr;
+    const size_t bytes = pitch * (size_t)(h - 1) + row;
+    if (a < start || a + bytes > start + size) return nullptr;
+    return reinterpret_cast<const void*>(dev);
 }
 
 struct Request {
@@ -133,19 +164,30 @@ int iwpp_server_s::run_batch(Lane& lane, std::vector<Request*>& batch) {
     imgs.reserve(batch.size());
     cudaError_t e = cudaSuccess;
     long long taken = 0;
+    // Pinned planes are read by one kernel for all of the batch, straight from
+    // host memory into the aligned device planes, and results written back the
+    // same way; others go through the copy engine, whose 2-D copies of rows of
+    // a few hundred bytes to a few kilobytes took most of a batch's time.
+    std::vector<StageCopy> in, back;
     for (Request* r : batch) {
         if (r->w == 0 || r->h == 0) continue;
         const size_t row = (size_t)r->w * bpp_of(r->dtype);
+        auto bring = [&](void* dst, const void* src, size_t pitch) {
+            if (const void* p = pinned_address(src, pitch, row, r->h)) {
+                in.push_back({p, dst, (long long)pitch, (long long)r->pitch, (long long)row, r->h});
+                return cudaSuccess;
+            }
+            return cudaMemcpy2DAsync(dst, r->pitch, src, pitch, row, r->h, cudaMemcpyHostToDevice, s);
+        };
         const size_t plane = r->pitch * (size_t)r->h;
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&r->d_marker, plane, pool, s);
         if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&r->d_mask, plane, pool, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(r->d_marker, r->pitch, r->marker, r->pm, row, r->h, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess)
-            e = cudaMemcpy2DAsync(r->d_mask, r->pitch, r->mask, r->pk, row, r->h, cudaMemcpyHostToDevice, s);
+        if (e == cudaSuccess) e = bring(r->d_marker, r->marker, r->pm);
+        if (e == cudaSuccess) e = bring(r->d_mask, r->mask, r->pk);
         imgs.push_back(iwpp_image{r->d_marker, r->d_mask, r->pitch, r->pitch, r->w, r->h, r->dtype, r->conn});
         taken += (long long)r->bytes;
     }
+    if (e == cudaSuccess) e = iwpp::launch_stage_copies(in, s, nullptr);
     if (headroom >= 0) {
         // the batch's planes are now the pool's (used) memory
         std::lock_guard<std::mutex> lk(mu);
@@ -159,10 +201,18 @@ int iwpp_server_s::run_batch(Lane& lane, std::vector<Request*>& batch) {
         if (r->w == 0 || r->h == 0) continue;
         if (rc == IWPP_OK && r->d_marker) {
             const size_t row = (size_t)r->w * bpp_of(r->dtype);
+            if (const void* p = pinned_address(r->out, r->po, row, r->h)) {
+                back.push_back({r->d_marker, const_cast<void*>(p), (long long)r->pitch, (long long)r->po,
+                                (long long)row, r->h});
+                continue;
+            }
             cudaError_t e2 =
                 cudaMemcpy2DAsync(r->out, r->po, r->d_marker, r->pitch, row, r->h, cudaMemcpyDeviceToHost, s);
             if (e2 != cudaSuccess) rc = IWPP_ERR_CUDA;
         }
+    }
+    if (rc == IWPP_OK && iwpp::launch_stage_copies(back, s, nullptr) != cudaSuccess) rc = IWPP_ERR_CUDA;
+    for (Request* r : batch) {
         if (r->d_marker) cudaFreeAsync(r->d_marker, s);
         if (r->d_mask) cudaFreeAsync(r->d_mask, s);
         r->d_marker = r->d_mask = nullptr;
