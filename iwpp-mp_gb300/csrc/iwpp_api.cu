@@ -314,6 +314,16 @@ struct Job {
     Config cfg;
 };
 
+// The connectivity of a job's images, 0 where they mix them.
+int job_conn(const Job& job) {
+    int conn = 0;
+    for (const ImgDesc& d : job.descs) {
+        if (conn != 0 && d.conn != conn) return 0;
+        conn = d.conn;
+    }
+    return conn;
+}
+
 // Queue entries of a job: the variant's rule applied to the requested
 // capacity (negative: that multiple of the job's tiles).
 long long job_queue_capacity(const Job& job) {
@@ -771,7 +781,7 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     long long grid = 1;
     LaunchInfo li{};
     if (job.G > 0) {
-        e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job.G, device, &li);
+        e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, device, &li);
         if (e != cudaSuccess) return cuda_status(e);
         grid = li.grid;
         if (grid > job.G) grid = job.G;
@@ -1104,7 +1114,9 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
         }
         // Warm the kernel attributes before capture.
         LaunchInfo li;
-        if (rc == IWPP_OK && job.G > 0) rc = cuda_status(engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job.G, h->device, &li));
+        if (rc == IWPP_OK && job.G > 0)
+            rc = cuda_status(
+                engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, h->device, &li));
     }
     if (rc == IWPP_OK) {
         e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);

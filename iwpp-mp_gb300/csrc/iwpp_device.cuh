@@ -540,11 +540,17 @@ __device__ __forceinline__ void vstep(VRow<DT>& m, const VRow<DT>& k, const VRow
     for (int j = 0; j < VRow<DT>::N; ++j) m.v[j] = vmx<DT>(m.v[j], vmn<DT>(p.v[j], k.v[j]));
 }
 
+// 8-connectivity, known to the kernel (CONN) or, with CONN 0, looked up.
+template <int CONN>
+__device__ __forceinline__ bool eight(bool conn8) {
+    return CONN == 0 ? conn8 : CONN == 8;
+}
+
 // What a row offers the row above or below it.
 template <int DT, int CONN>
-__device__ __forceinline__ VRow<DT> offers(const VRow<DT>& p, const EdgeSel& sel) {
+__device__ __forceinline__ VRow<DT> offers(const VRow<DT>& p, const EdgeSel& sel, bool conn8 = false) {
     VRow<DT> q = p;
-    if (CONN == 8) {
+    if (eight<CONN>(conn8)) {
         const VRow<DT> h = beside<DT>(p, sel);
 #pragma unroll
         for (int j = 0; j < VRow<DT>::N; ++j) q.v[j] = vmx<DT>(p.v[j], h.v[j]);
@@ -567,7 +573,7 @@ __device__ __forceinline__ VRow<DT> offers(const VRow<DT>& p, const EdgeSel& sel
 enum : unsigned { VD_DOWN = 1u, VD_UP = 2u, VD_ABOVE = 4u, VD_BELOW = 8u };
 template <int DT, int CONN>
 __device__ __forceinline__ unsigned vblock(uint32_t* tm, const uint32_t* tk, int lane, int b, uint32_t edge_mask,
-                                           const EdgeSel& sel, unsigned due) {
+                                           const EdgeSel& sel, bool conn8, unsigned due) {
     constexpr int N = VRow<DT>::N;
     uint32_t* rows = tm + (8 * b + 1) * 32 + lane;
     const uint32_t* krows = tk + (8 * b + 1) * 32 + lane;
@@ -582,12 +588,12 @@ __device__ __forceinline__ unsigned vblock(uint32_t* tm, const uint32_t* tk, int
     }
     if (due & (VD_DOWN | VD_ABOVE)) {
         const VRow<DT> was = m[0];
-        vstep<DT>(m[0], k[0], offers<DT, CONN>(above, sel));
+        vstep<DT>(m[0], k[0], offers<DT, CONN>(above, sel, conn8));
         if (!(due & VD_DOWN) && __any_sync(FULL, m[0].differs(was))) due |= VD_DOWN;
     }
     if (due & (VD_UP | VD_BELOW)) {
         const VRow<DT> was = m[7];
-        vstep<DT>(m[7], k[7], offers<DT, CONN>(below, sel));
+        vstep<DT>(m[7], k[7], offers<DT, CONN>(below, sel, conn8));
         if (!(due & VD_UP) && __any_sync(FULL, m[7].differs(was))) due |= VD_UP;
     }
     if (!(due & (VD_DOWN | VD_UP))) return 0u;
@@ -602,7 +608,7 @@ __device__ __forceinline__ unsigned vblock(uint32_t* tm, const uint32_t* tk, int
         for (int i = 6; i >= 0; --i) vstep<DT>(m[i], k[i], m[i + 1]);
     }
     uint32_t diag = 0u;
-    if (CONN == 8) {
+    if (eight<CONN>(conn8)) {
         VRow<DT> before, here = beside<DT>(m[0], sel);
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -632,7 +638,7 @@ __device__ __forceinline__ unsigned vblock(uint32_t* tm, const uint32_t* tk, int
     if (__any_sync(FULL, inner != 0u)) f |= RF_INNER;
     if (__any_sync(FULL, last != 0u)) f |= RF_LAST;
     if (__any_sync(FULL, (all & edge_mask) != 0u)) f |= RF_COL;
-    if (CONN == 8 && __any_sync(FULL, diag != 0u)) f |= RF_AGAIN;
+    if (eight<CONN>(conn8) && __any_sync(FULL, diag != 0u)) f |= RF_AGAIN;
     return f;
 }
 
@@ -882,13 +888,13 @@ __device__ __forceinline__ unsigned hblock(uint32_t* tm, const uint32_t* tk, int
 // (for 8-connectivity their three neighbours there, corners included); lanes
 // 0-7 the rows of the first column, lanes 8-15 of the last.  Returns RF_*.
 template <int DT, int CONN, int TH>
-__device__ __forceinline__ unsigned halo_columns(TileSmem<TH>& sm, int lane, int b) {
+__device__ __forceinline__ unsigned halo_columns(TileSmem<TH>& sm, int lane, int b, bool conn8) {
     using P = Px<DT>;
     const int r = 8 * b + 1 + (lane & 7);
     const bool right = (lane & 8) != 0;
     const uint32_t* h = right ? sm.hRm : sm.hLm;
     uint32_t v = h[r];
-    if (CONN == 8) v = P::mx3(v, h[r - 1], h[r + 1]);
+    if (eight<CONN>(conn8)) v = P::mx3(v, h[r - 1], h[r + 1]);
     const int off = right ? 128 - P::BPP : 0;
     unsigned char* px = reinterpret_cast<unsigned char*>(&sm.tm[r * 32]) + off;
     v = P::mn(v, P::ld_px(reinterpret_cast<const unsigned char*>(&sm.tk[r * 32]) + off));
@@ -960,7 +966,8 @@ __device__ __forceinline__ void write_back_block(const ImgDesc& d, const TileSme
 // pixels as fetched; they can only have risen since, so a stale halo gives at
 // most an extra notification, never a missed one.
 template <int DT, int CONN, int TH>
-__device__ __forceinline__ unsigned detect_neighbours(const TileSmem<TH>& sm, int lane, int b, unsigned f) {
+__device__ __forceinline__ unsigned detect_neighbours(const TileSmem<TH>& sm, int lane, int b, unsigned f,
+                                                      bool conn8) {
     const EdgeSel sel(lane);
     using P = Px<DT>;
     constexpr int NB = TH / 8;
@@ -975,7 +982,7 @@ __device__ __forceinline__ unsigned detect_neighbours(const TileSmem<TH>& sm, in
         const uint32_t w = sm.tm[halo * 32 + lane];
         m.set(w);
         k.set(sm.tk[halo * 32 + lane]);
-        vstep<DT>(m, k, offers<DT, CONN>(p, sel));
+        vstep<DT>(m, k, offers<DT, CONN>(p, sel, conn8));
         if (__any_sync(FULL, m.word() != w)) nb |= n ? NB_N : NB_S;
     }
     if (f & RF_COL) {
@@ -984,10 +991,10 @@ __device__ __forceinline__ unsigned detect_neighbours(const TileSmem<TH>& sm, in
         const int i = lane & 15, r = 8 * b + i;
         const bool right = (lane & 16) != 0;
         bool up = false;
-        if (CONN == 8 ? i < 10 : i >= 1 && i < 9) {
+        if (eight<CONN>(conn8) ? i < 10 : i >= 1 && i < 9) {
             const unsigned char* col = reinterpret_cast<const unsigned char*>(sm.tm) + (right ? 128 - P::BPP : 0);
             uint32_t v = P::MINPX;
-            if (CONN == 8) {
+            if (eight<CONN>(conn8)) {
                 if (r > 1) v = P::mx(v, P::ld_px(col + (r - 1) * 128));
                 if (r < TH) v = P::mx(v, P::ld_px(col + (r + 1) * 128));
             }
@@ -1305,6 +1312,7 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
     unsigned dd = 0u, du = 0u, da = 0u, db = 0u, dh = 0u;
     unsigned marks = 0u;  // 1 the warp above, 2 the warp below is to look again
     const unsigned sides = sm.sides;
+    const bool conn8 = sm.d.conn == 8;
     // takes over what a pass raised (f, RF_*) in the warp's block i
     auto took = [&](unsigned f, int i) {
         if (!(f & RF_ROWS)) return;
@@ -1336,7 +1344,7 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
     if (sides & ~(NB_N | NB_S)) {
 #pragma unroll 1
         for (int i = 0; i < BPW; ++i) {
-            const unsigned f = halo_columns<DT, CONN, TH>(sm, lane, b0 + i);
+            const unsigned f = halo_columns<DT, CONN, TH>(sm, lane, b0 + i, conn8);
             if (f & RF_ROWS) {
                 dd |= 1u << i;
                 du |= 1u << i;
@@ -1369,7 +1377,7 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
                 du &= ~bit;
                 da &= ~bit;
                 db &= ~bit;
-                const unsigned f = vblock<DT, CONN>(sm.tm, sm.tk, lane, b0 + i, edge_mask, sel, due);
+                const unsigned f = vblock<DT, CONN>(sm.tm, sm.tk, lane, b0 + i, edge_mask, sel, conn8, due);
                 __syncwarp();
                 row_steps += 8u;
                 took(f, i);
@@ -1413,6 +1421,11 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
 // Called by all warps; after it the stores are visible to the GPU and the
 // first warp may go on to the next tile.  Returns false when a bounded wait
 // ran out.
+// CONN 0, for batches that mix connectivities: it is looked up.  Such a batch
+// runs all the code there is at once, a copy per pixel type and connectivity of
+// 40 KB each, and with four of them (64 mixed images, uint8 and uint16) an issue
+// waited 8.7 cycles for instructions; with one per type the batch takes 2.84 ms
+// instead of 3.59, where a single image would lose 2 % to the looking up.
 template <int DT, int CONN, int TH, int W>
 __device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane, unsigned& phase, long long timeout_ns,
                                            unsigned& row_steps) {
@@ -1450,7 +1463,7 @@ __device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane,
             unsigned f = (rose.col >> i) & 1u ? RF_COL : 0u;
             if (i == 0 && rose.top) f |= RF_FIRST;
             if (i == BPW - 1 && rose.bottom) f |= RF_LAST;
-            if (f != 0u) nb |= detect_neighbours<DT, CONN, TH>(sm, lane, BPW * warp + i, f);
+            if (f != 0u) nb |= detect_neighbours<DT, CONN, TH>(sm, lane, BPW * warp + i, f, sm.d.conn == 8);
         }
         if (nb != 0u && lane == 0) atomicOr(&sm.nb, nb);
         // release: the stores before the neighbours' DIRTY and before the
@@ -1537,7 +1550,8 @@ __device__ __forceinline__ bool visit_tile_alt(TileSmemAlt<TH>& sm, int lane, un
         if (rb != 0u) write_back_block<DT, TH>(sm.d, sm, lane, b, sm.tx * 32 * P::PPW, sm.ty * TH);
         if (rose != 0ull)
             nb |= detect_neighbours<DT, CONN, TH>(sm, lane, b,
-                                                  ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col);
+                                                  ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col,
+                                                  CONN == 8);
     }
     if (lane == 0) sm.nb = nb;
     if (rose != 0ull) fence_gpu();

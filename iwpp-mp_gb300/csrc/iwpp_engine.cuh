@@ -126,10 +126,13 @@ namespace iwpp {
 struct LaunchInfo {
     int grid;   // CTAs that the device keeps resident
     int shape;  // the kernel's shape (iwpp_engine.cu)
+    int conn;   // the connectivity it is for, 0: both
 };
 int engine_sm_count(int device);
-// The kernel for a job of `tiles` tiles and its resident grid.
-cudaError_t engine_prepare(int variant, int tile_rows, int solver, long long tiles, int device, LaunchInfo* li);
+// The kernel for a job of `tiles` tiles and its resident grid.  conn: the
+// images' connectivity, 0 where they mix them.
+cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int device,
+                           LaunchInfo* li);
 cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s);
 cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li, int grid, cudaStream_t s);
 cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s);

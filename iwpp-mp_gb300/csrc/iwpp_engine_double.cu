@@ -1,0 +1,6 @@
+// iwpp_engine_double.cu -- the engine's kernels of the double queue.
+#include "iwpp_engine_kernel.cuh"
+
+namespace iwpp {
+template void* kernel_for<VAR_DOUBLE>(int, int, bool, int);
+}

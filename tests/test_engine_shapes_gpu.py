@@ -95,3 +95,19 @@ def test_rows_off_the_word_boundary(dt, conn, off_m, off_k):
                 around = torch.ones_like(bm, dtype=torch.bool)
                 torch.as_strided(around, (h, w), (w + pad_m, 1), off_m).fill_(False)
                 assert torch.equal(bm[around], before[around]), (w, h, variant, solver)
+
+
+@pytest.mark.parametrize("tile_rows,height", [(32, 300), (64, 700), (64, 15000), (64, 26000)])
+@pytest.mark.parametrize("variant", ["mutex", "double", "unique", "async"])
+def test_batch_of_both_connectivities(variant, tile_rows, height):
+    # the kernels that look the connectivity up, at every warp count of a tile
+    import torch
+    pairs, refs = [], []
+    for i, (dt, conn, w) in enumerate([(0, 4, 129), (1, 8, 63), (2, 4, 33), (0, 8, 127), (1, 4, 1), (2, 8, 31)]):
+        mask = synth.noise_mask(w, height - 97 * i if i < 4 else 65, dt, 90 + i, 2.0, 40)
+        marker = synth.hdome_marker(mask, 15 + 9 * i)
+        refs.append(oracle.reconstruct(marker, mask, conn))
+        pairs.append([torch.from_numpy(a.view(np.int16) if dt == 1 else a).cuda() for a in (marker, mask)] + [conn])
+    iwpp.reconstruct_batch(pairs, variant=variant, config=iwpp.Config.make(tile_rows=tile_rows))
+    for (m, _, _), ref in zip(pairs, refs):
+        assert np.array_equal(m.cpu().numpy().view(ref.dtype), ref)
