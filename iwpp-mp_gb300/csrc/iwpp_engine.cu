@@ -1,5 +1,6 @@
 // iwpp_engine.cu -- job initialisation, queue self-test and the host side of
 // the persistent tile engine.
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 
@@ -250,6 +251,17 @@ cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, lon
         if (e != cudaSuccess) return e;
         cached.store(per_sm, std::memory_order_relaxed);
     }
+    // CTAs of the mutex queue take turns at its lock: past two per SM the longer
+    // line costs more than the visits beside one another gain.  1 / 2 / 3 / all
+    // that fit (10, 5 or 3) per SM, us: 4096^2 u8 h-domes, 4-connected, h = 10
+    // 757 / 843 / 905 / 2062, h = 100 1726 / 1260 / 1288 / 3054, 8-connected, h = 40
+    // 2600 / 2259 / 1540 / 3137; 6000 x 5000 u8 2530 / 1550 / 2388 / 2450; 2048 x 1500
+    // u16 600 / 757 / 1856 / 1855; sparse seeds 4096^2 u8 4120 / 3680 / 3266 / 3180,
+    // 5000^2 i32 19900 / 21100 / 21400 / 30300.
+    // The one-warp CTAs of the other solvers: 2 / 3 / 4 / 8, row sweeps, 4096^2
+    // u8 h = 10 1120 / 1450 / 1533 / 1491, 8-connected, h = 40 2813 / 2488 / 1984 / 1634,
+    // sparse seeds 5641 / 4083 / 3848 / 4868, 1024^2 490 / 498 / 431 / 472.
+    if (variant == VAR_MUTEX) per_sm = std::min(per_sm, shape == T32_ALT || shape == T64_ALT ? 4 : 2);
     li->grid = per_sm * sms;
     li->shape = shape;
     li->conn = conn;
