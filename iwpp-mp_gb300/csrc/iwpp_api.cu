@@ -160,14 +160,18 @@ long long tiles_of(int w, int h, int dtype, int th) {
 // uint8 77 / 66, 1024^2 uint16 124 / 106, 4096^2 uint8 191 / 144 (64 rows by
 // two warps).  The mutex queue is bound by its one lock (every take and insert
 // is a critical section), so its cost grows with the tile count: 64 rows always.
-int default_tile_rows(int variant, long long tiles64) {
+// The other solvers have one warp per tile: 32 rows below 2.5 64-row tiles per
+// warp that the grid keeps resident, 12 per SM.
+int default_tile_rows(int variant, int solver, long long tiles64) {
     if (variant == IWPP_QUEUE_MUTEX) return 64;
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess) {
         cudaGetLastError();
         return 64;
     }
-    return tiles64 <= engine_sm_count(device) ? 32 : 64;
+    const int sms = engine_sm_count(device);
+    if (solver == 1 || solver == 3) return tiles64 < 30ll * sms ? 32 : 64;
+    return tiles64 <= sms ? 32 : 64;
 }
 
 long long job_tiles64(const iwpp_image* imgs, int n) {
@@ -392,7 +396,7 @@ int build_job(Job& job, const iwpp_image* imgs, int n, int variant, const iwpp_c
         job.cfg.front_passes = largest >= kFrontDefaultPixels ? 3 : 2;
     }
     int th = job.cfg.tile_rows;
-    if (th == 0) th = n > 0 ? default_tile_rows(job.variant, job_tiles64(imgs, n)) : 64;
+    if (th == 0) th = n > 0 ? default_tile_rows(job.variant, job.cfg.solver, job_tiles64(imgs, n)) : 64;
     job.tile_rows = th;
     long long G = 0;
     for (int i = 0; i < n; ++i) {
@@ -985,7 +989,7 @@ long long iwpp_tile_count(int width, int height, int dtype, int tile_rows) {
     if (dtype != IWPP_U8 && dtype != IWPP_U16 && dtype != IWPP_I32) return -1;
     const int th = tile_rows == 32 || tile_rows == 64
                        ? tile_rows
-                       : default_tile_rows(resolve_variant(IWPP_QUEUE_DEFAULT), tiles_of(width, height, dtype, 64));
+                       : default_tile_rows(resolve_variant(IWPP_QUEUE_DEFAULT), 0, tiles_of(width, height, dtype, 64));
     return tiles_of(width, height, dtype, th);
 }
 
@@ -1342,7 +1346,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
     if (rc == IWPP_OK) {
         // the untuned default first when it is the front stage (large
         // images), then stage 1: tile height x in-tile solver, no passes
-        const int dflt_th = default_tile_rows(v, job_tiles64(images, n));
+        const int dflt_th = default_tile_rows(v, 0, job_tiles64(images, n));
         long long largest = 0;
         for (int i = 0; i < n; ++i)
             if (images[i].width > 0 && images[i].height > 0)

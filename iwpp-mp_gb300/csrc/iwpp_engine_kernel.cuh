@@ -705,7 +705,7 @@ struct QueueOf<VAR_ASYNC> {
 // over a warp's blocks needs them; 16 and 32 warps measured the same or
 // slower (32: a fifth slower, spills).
 template <int VAR, int TH, int W, bool ALT, int CONN>
-__global__ void __launch_bounds__(32 * W, ALT ? 8 : W == 2 ? 10 : 24 / W)
+__global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
     engine_kernel(const __grid_constant__ EngineArgs a) {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
