@@ -19,9 +19,10 @@ configuration fields, which the tuning table fills.
           inside the timed region, copies on their own streams and
           double-buffered so that one step's copies overlap its neighbours'
           reconstructions.
-  roofline : one reconstruction (front stage: top-level labelling, four
-          whole-image passes, seed check; then the tile engine -- all of
-          this library's kernels of the call) as the unit: algorithmic bytes
+  roofline : one reconstruction (front stage: seed check, top-level
+          labelling, whole-image passes where the configuration has them;
+          then the tile engine -- all of this library's kernels of the
+          call) as the unit: algorithmic bytes
           = 3 * W * H * bytes/pixel (read mask, read marker, write result)
           over its CUDA-event duration, against the measured HBM copy
           bandwidth.
@@ -952,8 +953,8 @@ def main():
                     help="with --config1-solver: the tile height as well (0: the default)")
     ap.add_argument("--profile-headline", type=int, default=0, metavar="N",
                     help="only N reconstructions of the headline image with the front stage (for profilers)")
-    ap.add_argument("--profile-passes", type=int, default=2,
-                    help="whole-image passes of the front stage in --profile-headline")
+    ap.add_argument("--profile-passes", type=int, default=None,
+                    help="whole-image passes of the front stage in --profile-headline (default: the untuned call)")
     args = ap.parse_args()
     if args.impl == "reference":
         return run_reference(args)
@@ -968,11 +969,11 @@ def main():
 
 
 def run_profile_headline(args):
-    """N reconstructions of the headline image with the front stage and
-    --profile-passes whole-image passes (the configuration the autotuner
-    picks for this image class in a plain run; under a profiler, which
-    serialises and replays every launch, its timings would pick another)
-    and --variant, each from the pristine marker, nothing else."""
+    """N reconstructions of the headline image in the untuned configuration
+    (which the autotuner picks for this image class in a plain run; under a
+    profiler, which serialises and replays every launch, its timings could
+    pick another), or with the front stage and --profile-passes whole-image
+    passes, and --variant, each from the pristine marker, nothing else."""
     import torch
 
     import iwpp
@@ -983,7 +984,9 @@ def run_profile_headline(args):
     mask = torch.from_numpy(mask_np).to(dev)
     pristine = torch.from_numpy(marker_np).to(dev)
     work = pristine.clone()
-    cfg = iwpp.Config.make(front_passes=1, init_passes=args.profile_passes)
+    cfg = iwpp.Config.make()
+    if args.profile_passes is not None:
+        cfg = iwpp.Config.make(front_passes=1, init_passes=args.profile_passes)
     for i in range(args.profile_headline):
         work.copy_(pristine)
         torch.cuda.synchronize()

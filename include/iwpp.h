@@ -213,8 +213,8 @@ IWPP_API int iwpp_queue_selftest(int device, int variant, int grid_side, int cop
 typedef struct iwpp_tune_result {
     iwpp_config best;  /* fastest configuration */
     double best_ms;    /* its median device time */
-    double default_ms; /* median device time of the untuned default (default tile height, automatic
-                          solver; front_passes 3 for images of 2^26 pixels or more) */
+    double default_ms; /* median device time of the untuned default (default tile height, the
+                          passes; front_passes 3 for images of 2^26 pixels or more) */
     int candidates;    /* configurations timed */
     int reserved;
 } iwpp_tune_result;
