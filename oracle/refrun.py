@@ -57,8 +57,9 @@ def _run(cmd, cwd=None):
 
 
 def build_cubins() -> bool:
-    """Compiles the reference kernels (needs the reference sources)."""
-    if not os.path.isdir(REFERENCE):
+    """Compiles the reference kernels; False where their sources are not."""
+    if not all(os.path.isfile(os.path.join(REFERENCE, d, "src", f)) for d in VARIANT_DIRS.values()
+               for f in ("globalQueue.cu", "MorphologicalReconstruction.cu")):
         return False
     os.makedirs(REF_OUT, exist_ok=True)
     for variant, d in VARIANT_DIRS.items():
