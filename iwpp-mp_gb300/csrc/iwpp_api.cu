@@ -812,10 +812,7 @@ int read_stats(Ctrl* host_ctrl, const Workspace& ws, cudaStream_t s, long long t
     cudaError_t e = cudaMemcpyAsync(host_ctrl, ws.base, sizeof(Ctrl), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) return cuda_status(e);
-    int st = IWPP_OK;
-    if (host_ctrl->error == DEV_ERR_TIMEOUT) st = IWPP_ERR_TIMEOUT;
-    if (host_ctrl->error == DEV_ERR_OVERFLOW) st = IWPP_ERR_OVERFLOW;
-    if (host_ctrl->error == DEV_ERR_INTERNAL) st = IWPP_ERR_INTERNAL;
+    const int st = status_of_job(host_ctrl->error);
     if (out) {
         out->tiles = tiles;
         out->visits = (long long)host_ctrl->visits;
@@ -1053,10 +1050,7 @@ int iwpp_handle_sync(iwpp_handle h, iwpp_stats* stats) {
     float ms = 0.f;
     if (h->timed) cudaEventElapsedTime(&ms, h->ev0, h->ev1);
     const Ctrl& c = *h->host_ctrl;
-    int st = IWPP_OK;
-    if (c.error == DEV_ERR_TIMEOUT) st = IWPP_ERR_TIMEOUT;
-    if (c.error == DEV_ERR_OVERFLOW) st = IWPP_ERR_OVERFLOW;
-    if (c.error == DEV_ERR_INTERNAL) st = IWPP_ERR_INTERNAL;
+    const int st = status_of_job(c.error);
     if (stats) {
         stats->tiles = h->last_tiles;
         stats->visits = (long long)c.visits;
@@ -1170,10 +1164,7 @@ int iwpp_plan_sync(iwpp_plan p, iwpp_stats* stats) {
     cudaError_t e = cudaStreamSynchronize(p->last_stream);
     if (e != cudaSuccess) return set_last(cuda_status(e));
     const Ctrl& c = *p->host_ctrl;
-    int st = IWPP_OK;
-    if (c.error == DEV_ERR_TIMEOUT) st = IWPP_ERR_TIMEOUT;
-    if (c.error == DEV_ERR_OVERFLOW) st = IWPP_ERR_OVERFLOW;
-    if (c.error == DEV_ERR_INTERNAL) st = IWPP_ERR_INTERNAL;
+    const int st = status_of_job(c.error);
     if (stats) {
         stats->tiles = p->tiles;
         stats->visits = (long long)c.visits;
@@ -1247,7 +1238,7 @@ int iwpp_queue_selftest(int device, int variant, int grid_side, int copies, iwpp
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     }
     rc = cuda_status(e);
-    if (rc == IWPP_OK && ctrl.error == DEV_ERR_TIMEOUT) rc = IWPP_ERR_TIMEOUT;
+    if (rc == IWPP_OK) rc = status_of_job(ctrl.error);
     if (rc == IWPP_OK && ctrl.overflow != 0u) rc = IWPP_ERR_OVERFLOW;
     if (out) {
         out->entries = (long long)res[0];

@@ -33,6 +33,7 @@
 
 #include <vector>
 
+#include "iwpp.h"
 #include "iwpp_device.cuh"
 
 namespace iwpp {
@@ -123,6 +124,15 @@ struct EngineArgs {
 
 // Host-side entry points implemented in iwpp_engine.cu.
 namespace iwpp {
+// The caller's status of a job whose counters hold this error word (DEV_*).
+inline int status_of_job(unsigned error) {
+    switch (error) {
+        case DEV_OK: return IWPP_OK;
+        case DEV_ERR_TIMEOUT: return IWPP_ERR_TIMEOUT;
+        case DEV_ERR_OVERFLOW: return IWPP_ERR_OVERFLOW;
+        default: return IWPP_ERR_INTERNAL;
+    }
+}
 struct LaunchInfo {
     int grid;   // CTAs that the device keeps resident
     int shape;  // the kernel's shape (iwpp_engine.cu)

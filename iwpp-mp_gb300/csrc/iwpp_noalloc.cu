@@ -149,7 +149,5 @@ extern "C" int iwpp_reconstruct_noalloc(void* marker, const void* mask, size_t p
         cudaGetLastError();
         return e == cudaErrorMemoryAllocation ? IWPP_ERR_OOM : IWPP_ERR_CUDA;
     }
-    if (c.error == DEV_ERR_TIMEOUT) return IWPP_ERR_TIMEOUT;
-    if (c.error == DEV_ERR_OVERFLOW) return IWPP_ERR_OVERFLOW;
-    return IWPP_OK;
+    return status_of_job(c.error);
 }
