@@ -14,7 +14,10 @@ namespace iwpp {
 // initFillGlobalQueue).  After the front stage (or a seed check alone) the
 // check has set the tile states and listed the tiles to start from: the
 // mutex stack and the first round's read queue are that list, the async
-// ring starts from it; the stage's error word and top-pixel count stand.
+// ring starts from it; the stage's error word and top-pixel count stand.  A
+// list that is longer than the double queue holds is left for the virtual
+// list of all tiles, as after an overflow: tiles that are not DIRTY are
+// released unvisited.
 __global__ void engine_init_kernel(EngineArgs a, int variant) {
     const unsigned stride = gridDim.x * blockDim.x;
     const bool seeded = a.init_list != nullptr;
@@ -29,11 +32,12 @@ __global__ void engine_init_kernel(EngineArgs a, int variant) {
         for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < a.cap; i += stride) a.q0[i] = 0u;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         Ctrl* c = a.ctrl;
-        c->rn = n0;
+        const bool listed = seeded && !(variant == VAR_DOUBLE && n0 > a.cap);
+        c->rn = listed ? n0 : a.G;
         c->wn = 0u;
         c->rcur = 0u;
         c->qsel = 0u;
-        c->vfull = seeded ? 0u : 1u;
+        c->vfull = listed ? 0u : 1u;
         c->done = n0 == 0u && !a.phantom ? 1u : 0u;
         c->overflow = n0 > a.cap && variant == VAR_MUTEX ? 1u : 0u;
         c->restarts = 0u;
