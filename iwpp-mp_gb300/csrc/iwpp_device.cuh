@@ -137,7 +137,8 @@ __device__ __forceinline__ bool gated_off(const ImgDesc& d) {
 // neighbour direction bits returned by a tile visit
 enum : unsigned {
     NB_N = 1u << 0, NB_S = 1u << 1, NB_W = 1u << 2, NB_E = 1u << 3,
-    NB_NW = 1u << 4, NB_NE = 1u << 5, NB_SW = 1u << 6, NB_SE = 1u << 7
+    NB_NW = 1u << 4, NB_NE = 1u << 5, NB_SW = 1u << 6, NB_SE = 1u << 7,
+    NB_STORED = 1u << 8  // the visit stored pixels
 };
 __device__ __constant__ static const int kNbDx[8] = {0, 0, -1, 1, -1, 1, -1, 1};
 __device__ __constant__ static const int kNbDy[8] = {-1, 1, 0, 0, -1, -1, 1, 1};
@@ -1418,8 +1419,8 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
 
 // One visit of tile (tx, ty) by a CTA of W warps: fetch, local convergence,
 // store of the blocks that rose, and the neighbour tiles to notify in sm.nb.
-// Called by all warps; after it the stores are visible to the GPU and the
-// first warp may go on to the next tile.  Returns false when a bounded wait
+// Called by all warps; after it the stores are the first warp's to publish,
+// which may then go on to the next tile.  Returns false when a bounded wait
 // ran out.
 // CONN 0, for batches that mix connectivities: it is looked up.  Such a batch
 // runs all the code there is at once, a copy per pixel type and connectivity of
@@ -1452,7 +1453,7 @@ __device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane,
         sm.count.cycles[3] -= t;
     }
     if (rose.rows != 0u) {
-        unsigned nb = 0u;
+        unsigned nb = NB_STORED;
 #pragma unroll 1
         for (int i = 0; i < BPW; ++i) {
             if (!((rose.rows >> i) & 1u)) continue;
@@ -1465,10 +1466,7 @@ __device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane,
             if (i == BPW - 1 && rose.bottom) f |= RF_LAST;
             if (f != 0u) nb |= detect_neighbours<DT, CONN, TH>(sm, lane, BPW * warp + i, f, sm.d.conn == 8);
         }
-        if (nb != 0u && lane == 0) atomicOr(&sm.nb, nb);
-        // release: the stores before the neighbours' DIRTY and before the
-        // tile's ACTIVE bit clears (its next owner reads them)
-        fence_gpu();
+        if (lane == 0) atomicOr(&sm.nb, nb);
     }
     fence_proxy_async_smem();
     cta_sync<W>();
@@ -1553,8 +1551,7 @@ __device__ __forceinline__ bool visit_tile_alt(TileSmemAlt<TH>& sm, int lane, un
                                                   ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col,
                                                   CONN == 8);
     }
-    if (lane == 0) sm.nb = nb;
-    if (rose != 0ull) fence_gpu();
+    if (lane == 0) sm.nb = nb | (rose != 0ull ? (unsigned)NB_STORED : 0u);
     fence_proxy_async_smem();
     __syncwarp();
     if (lane == 0) {

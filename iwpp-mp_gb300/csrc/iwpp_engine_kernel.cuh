@@ -741,6 +741,11 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
                 const unsigned nb = sm.nb;
                 __syncwarp();
                 if (lane == 0) sm.nb = 0u;
+                // Release: all warps' stores before the neighbours' DIRTY and
+                // before the tile's ACTIVE bit clears (its next owner reads
+                // them).  By the lanes whose atomics follow, after the barrier
+                // that ended the visit.
+                if (nb & NB_STORED) fence_gpu();
                 int pushed = 0;
                 const unsigned cont = leave_tile<VAR>(a, sm.d, sm.tx, sm.ty, g, nb, lane, queue.wq, &pushed);
                 if (lane == 0) {
