@@ -265,15 +265,17 @@ IWPP_API int iwpp_sweep_timing(void *marker, const void *mask, size_t pitch_mark
  * the device memory budget, or a latency-critical loop that cannot afford
  * the device-wide synchronisation of cudaMalloc / cudaFree.  The caller
  * passes device marker / mask buffers (rows 4-byte aligned, any pitch,
- * uint8 / uint16 / int32, 4- or 8-connectivity); the queues, tile states and
- * counters live in a static device array of IWPP_NOALLOC_SCRATCH_BYTES that
- * every GPU loading the library keeps until the process exits.  It holds
+ * uint8 / uint16 / int32, 4- or 8-connectivity); the queues and tile states
+ * live in a static device array of IWPP_NOALLOC_SCRATCH_BYTES (and the
+ * counters in a few KB behind it) that every GPU loading the library keeps
+ * until the process exits.  It holds
  * images up to about 340 000 tiles (e.g. 32768 x 32768 uint8, 16384 x 16384
  * int32); larger images return IWPP_ERR_TOO_LARGE.  Uses the async queue,
  * 64-row tiles, plain loads; synchronous on `stream` (NULL = legacy default
  * stream).  The first call on a device looks up the array's device address
- * (cudaGetSymbolAddress) and the engine's launch shape with that device
- * current.  Both are kept until the process exits, so a cudaDeviceReset
+ * (cudaGetSymbolAddress) and loads every kernel that a later call can launch,
+ * with that device current; later calls load and allocate nothing.  The
+ * address is kept until the process exits, so a cudaDeviceReset
  * between calls is not supported (the kept address would be stale).  All calls share the one
  * array: calls whose work overlaps on the GPU (concurrent host threads or
  * streams) race and must be serialised by the caller.  Each call clears the

@@ -241,20 +241,29 @@ int engine_sm_count(int device) {
     return n;
 }
 
+// CTAs of a kernel that a multiprocessor keeps resident, asked (and the kernel
+// loaded) once.
+static cudaError_t resident_ctas(int variant, Shape shape, int conn, int device, int* per_sm) {
+    static std::atomic<int> cache[64][4][SHAPES][3];
+    std::atomic<int>& cached = cache[device][variant][shape][conn / 4];
+    *per_sm = cached.load(std::memory_order_relaxed);
+    if (*per_sm != 0) return cudaSuccess;
+    const Kernel k = kernel_of(variant, shape, conn);
+    cudaFuncAttributes attr;
+    cudaError_t e = cudaFuncGetAttributes(&attr, k.fn);  // (loads it where kernels are loaded on demand)
+    if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k.fn, k.threads, k.smem);
+    if (e == cudaSuccess) cached.store(*per_sm, std::memory_order_relaxed);
+    return e;
+}
+
 cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int device,
                            LaunchInfo* li) {
-    static std::atomic<int> per_sm_cache[64][4][SHAPES][3];  // resident CTAs, asked once
     const int sms = engine_sm_count(device);
     if (sms <= 0 || variant < 0 || variant > 3 || conn < 0 || conn > 8) return cudaErrorInvalidValue;
     const Shape shape = select_shape(tile_rows, solver, tiles, sms);
-    std::atomic<int>& cached = per_sm_cache[device][variant][shape][conn / 4];
-    int per_sm = cached.load(std::memory_order_relaxed);
-    if (per_sm == 0) {
-        const Kernel k = kernel_of(variant, shape, conn);
-        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k.fn, k.threads, k.smem);
-        if (e != cudaSuccess) return e;
-        cached.store(per_sm, std::memory_order_relaxed);
-    }
+    int per_sm = 0;
+    const cudaError_t e = resident_ctas(variant, shape, conn, device, &per_sm);
+    if (e != cudaSuccess) return e;
     // CTAs of the mutex queue take turns at its lock: past two per SM the longer
     // line costs more than the visits beside one another gain.  1 / 2 / 3 / all
     // that fit (10, 5 or 3) per SM, us: 4096^2 u8 h-domes, 4-connected, h = 10
@@ -270,6 +279,18 @@ cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, lon
     li->shape = shape;
     li->conn = conn;
     return li->grid > 0 ? cudaSuccess : cudaErrorInvalidConfiguration;
+}
+
+cudaError_t engine_load(int variant, int tile_rows, int device) {
+    if (engine_sm_count(device) <= 0 || variant < 0 || variant > 3) return cudaErrorInvalidValue;
+    cudaError_t e = cudaSuccess;
+    for (int conn : {4, 8})
+        for (Shape shape : {T32_W4, T64_W8, T64_W4, T64_W2}) {
+            int per_sm = 0;
+            if ((shape == T32_W4) == (tile_rows == 32) && e == cudaSuccess)
+                e = resident_ctas(variant, shape, conn, device, &per_sm);
+        }
+    return e;
 }
 
 cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s) {

@@ -143,6 +143,9 @@ int engine_sm_count(int device);
 // images' connectivity, 0 where they mix them.
 cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int device,
                            LaunchInfo* li);
+// Loads every kernel that engine_prepare can choose for one-image jobs with
+// tiles of this height and the default solver.
+cudaError_t engine_load(int variant, int tile_rows, int device);
 cudaError_t engine_launch_init(const EngineArgs& a, int variant, cudaStream_t s);
 cudaError_t engine_launch(const EngineArgs& a, int variant, const LaunchInfo& li, int grid, cudaStream_t s);
 cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s);

@@ -38,16 +38,22 @@ constexpr int kNoallocTileRows = 64;
 std::mutex g_setup_mu;
 unsigned char* g_scratch_ptr[kMaxDevices] = {};
 
-// The scratch array's device address, looked up by the first call on a device
-// with that device current and kept for the life of the process so that later
-// calls do no host-side queries.  A cudaDeviceReset between calls would leave
-// it stale; it is not supported.
+// Per-device set-up, done by the first call on a device with that device
+// current: the scratch array's device address, and the engine's kernels (by
+// tile count and connectivity) loaded, so that no later call is the first to
+// launch one, which may take device memory and wait for the device.  Kept for
+// the life of the process; a cudaDeviceReset between calls would leave it
+// stale and is not supported.
 int device_setup(int device, unsigned char** out) {
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_scratch_ptr[device]) {
         void* p = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
         if (e != cudaSuccess || p == nullptr) {
+            cudaGetLastError();
+            return IWPP_ERR_CUDA;
+        }
+        if (engine_load(VAR_ASYNC, kNoallocTileRows, device) != cudaSuccess) {
             cudaGetLastError();
             return IWPP_ERR_CUDA;
         }

@@ -45,3 +45,20 @@ def _call(lib, w, h, conn, error=DEV_OK):
                                                   (DEV_ERR_OVERFLOW, ERR_OVERFLOW), (DEV_ERR_INTERNAL, ERR_INTERNAL)])
 def test_a_failed_job_is_no_success(lib, device_error, status):
     assert _call(lib, 300, 200, 8, device_error) == status
+
+
+def test_the_first_call_loads_every_kernel(lib):
+    # A kernel that a later call is the first to launch is loaded then, which
+    # may take device memory and wait for the device.
+    assert _call(lib, 300, 200, 8) == OK
+    loads = ctypes.c_int.in_dll(lib, "fake_launches_that_load")
+    loaded = lib.fake_loaded()
+    kernels = 0
+    for conn in (4, 8):
+        for w, h in ((300, 200), (4096, 2112), (4224, 4037), (32768, 20000)):
+            before = loads.value
+            assert _call(lib, w, h, conn) == OK
+            assert lib.fake_launches() == 1
+            assert (loads.value, lib.fake_loaded()) == (before, loaded), (conn, w, h)
+            kernels += 1
+    assert kernels == 8
