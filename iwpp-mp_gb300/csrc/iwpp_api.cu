@@ -1028,7 +1028,7 @@ int iwpp_reconstruct_batch_async(iwpp_handle h, const iwpp_image* images, int n,
     h->last_tiles = job.G;
     h->last_variant = job.variant;
     h->last_launch_status = rc;
-    h->last_launches = nl;
+    h->last_launches = nl + job.stage_launches;
     h->timed = job.G > 0;
     if (prev_dev != h->device) cudaSetDevice(prev_dev);
     return set_last(rc);
