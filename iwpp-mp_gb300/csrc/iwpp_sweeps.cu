@@ -456,7 +456,13 @@ constexpr int kRing = 64, kGroup = 8;
 // Same bytes as the walk.  Measured on 4096^2 uint8 h-domes (+Y / -Y, us): the
 // walk 496 / 516; segments of 64 rows with 1 / 2 / 4 / 8 enter steps 144 / 81 /
 // 70 / 87, of 128 rows 70 / 60 / 66 / 83, of 32 rows 304 / 203 / 111 / 105.
-// Bound by the chain: a row is about 100 cycles of one warp.
+// Bound by the chain, about 70 cycles a row of one warp, where a front runs down
+// many segments (the settle step's walk: rows far ahead in shared memory, the
+// last strip's partial words masked and not loaded pixel by pixel).  With a
+// group of rows ahead in registers and the last strip's pixels one by one, and
+// now, us: 16384^2 uint8 spiral 8-connected 1931 / 838, 8191 x 8190 uint16
+// spiral 4-connected (staged) 4734 / 1392, 8190 x 8192 int32 spiral 8-connected
+// 1008 / 428, 1028 x 8192 uint8, one front down the whole height, 1346 / 567.
 constexpr int kStripRows = 128;
 constexpr int kStripEnter = 2;
 // images up to this height: one walk, whose launch is all it costs (1024 x 182
@@ -472,9 +478,11 @@ struct Strip {
     const unsigned char* k;
     long long pitch_m, pitch_k;
     int npx, H;
+    uint32_t keep;  // the bits of the lane's word that are the image's
     __device__ __forceinline__ Strip(const ImgDesc& d, int strip, int lane) : H(d.H) {
         const int px0 = strip * 32 * P::PPW + lane * P::PPW;
         npx = d.W - px0;
+        keep = npx >= P::PPW ? FULL : npx > 0 ? (1u << (8 * P::BPP * npx)) - 1u : 0u;
         const size_t off = (size_t)(npx > 0 ? px0 : 0) * P::BPP;
         const int first = DOWN ? 0 : d.H - 1;
         pitch_m = DOWN ? d.pitch_m : -d.pitch_m;
@@ -491,11 +499,80 @@ struct Strip {
     __device__ __forceinline__ void store(int i, uint32_t w) const {
         if (npx > 0) store_word_plain<DT>(m + i * pitch_m, npx, w);
     }
-    // Walks rows from `i` below row i - 1 (in `prev`), the next eight rows'
-    // loads ahead of the chain; with STOP until a group of eight ends with a
-    // row that does not rise, else to row `end`.  Strips inside the image's
-    // width (all but the last) run on bare words: with the checks for a
-    // partial word in every row a row took 300 cycles.
+    // The word of a row, in every row but the image's last where the strip is
+    // not inside the image's width (INSIDE): there a lane has a word, a part of
+    // one or nothing, and loads a whole word all the same (with what lies
+    // between the row's end and the next row, or its row's first word).
+    __device__ __forceinline__ uint32_t word_at(const unsigned char* row) const {
+        return __ldcg(reinterpret_cast<const unsigned int*>(row));
+    }
+    // What of it is the image's.
+    template <bool INSIDE>
+    __device__ __forceinline__ uint32_t own(uint32_t w) const {
+        if (INSIDE) return w;
+        return DT == DT_I32 ? (npx > 0 ? w : P::MINW) : w & keep;
+    }
+    // Row i below row i - 1 (in `prev`); true when it rises.
+    __device__ __forceinline__ bool step(VRow<DT>& prev, int i, const EdgeSel& sel) const {
+        const uint32_t was = marker(i);
+        VRow<DT> v, kv;
+        v.set(was);
+        kv.set(mask(i));
+        vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
+        const uint32_t w = v.word();
+        if (w != was) store(i, w);
+        prev = v;
+        return __any_sync(FULL, w != was);
+    }
+    // Eight rows from row i (marker words `old`, at `at`, mask words `kw`);
+    // whether the lane's word of the last one rises.  Stores after the chain: a
+    // branch for them in every row of the last strip cost as much as the row.
+    template <bool INSIDE>
+    __device__ __forceinline__ bool group(VRow<DT>& prev, const uint32_t (&old)[8], const uint32_t (&kw)[8], int i,
+                                          unsigned char* at, const EdgeSel& sel) const {
+        uint32_t out[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            VRow<DT> v, kv;
+            v.set(own<INSIDE>(old[q]));
+            kv.set(own<INSIDE>(kw[q]));
+            vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
+            out[q] = v.word();
+            prev = v;
+        }
+        uint32_t rose = 0u;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const bool r = out[q] != own<INSIDE>(old[q]);
+            rose |= r ? 1u << q : 0u;
+            if ((INSIDE || npx >= P::PPW) && r) *reinterpret_cast<unsigned int*>(at + q * pitch_m) = out[q];
+        }
+        if (!INSIDE && DT != DT_I32 && npx < P::PPW && rose != 0u) {
+#pragma unroll
+            for (int q = 0; q < 8; ++q)
+                if ((rose >> q) & 1u) store(i + q, out[q]);
+        }
+        return (rose & 128u) != 0u;
+    }
+    // The first row of a walk's groups of eight and the end of them: the image's
+    // last row is stepped by itself in the last strip.  False: the walk is over.
+    template <bool STOP, bool INSIDE>
+    __device__ __forceinline__ bool groups(VRow<DT>& prev, int& i, int end, int& groups_end, const EdgeSel& sel) const {
+        groups_end = end;
+        if (!INSIDE) {
+            if (DOWN)
+                groups_end = min(end, H - 1);
+            else if (i == 0)
+                return step(prev, i++, sel) || !STOP;
+        }
+        return true;
+    }
+    // Walks rows from `i` below row i - 1 (in `prev`); with STOP until a group
+    // of eight ends with a row that does not rise, else to row `end`.  Strips
+    // inside the image's width (all but the last) run on bare words.
+    //   walk: the next group's words in registers.
+    //   walk_ahead: kRing rows ahead in shared memory, for one warp's long way
+    //     down: 70 cycles a row, where a group ahead waits for memory (150).
     template <bool STOP>
     __device__ __forceinline__ void walk(const VRow<DT>& prev, int i, int end, const EdgeSel& sel) const {
         if (__all_sync(FULL, npx >= P::PPW))
@@ -503,67 +580,93 @@ struct Strip {
         else
             walk_rows<STOP, false>(prev, i, end, sel);
     }
-    template <bool STOP, bool WORDS>
+    template <bool STOP, bool INSIDE>
     __device__ __forceinline__ void walk_rows(VRow<DT> prev, int i, int end, const EdgeSel& sel) const {
-        const unsigned char *pm = m + i * pitch_m, *pk = k + i * pitch_k;
-        auto load = [&](const unsigned char* p, long long pitch, uint32_t (&w)[8]) {
+        int groups_end;
+        if (!groups<STOP, INSIDE>(prev, i, end, groups_end, sel)) return;
+        uint32_t gm[2][8], gk[2][8];
+        const unsigned char *pm = m + i * pitch_m, *pk = k + i * pitch_k;  // the next group to load
+        unsigned char* at = m + i * pitch_m;                               // the group in hand
+        int next = i;
+        auto refill = [&](int g) {
+            if (next + 8 <= groups_end) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q)
-                w[q] = WORDS     ? __ldcg(reinterpret_cast<const unsigned int*>(p + q * pitch))
-                       : npx > 0 ? load_word_plain<DT>(p + q * pitch, npx, true)
-                                 : P::MINW;
+                for (int q = 0; q < 8; ++q) gm[g][q] = word_at(pm + q * pitch_m);
+#pragma unroll
+                for (int q = 0; q < 8; ++q) gk[g][q] = word_at(pk + q * pitch_k);
+            }
+            next += 8;
+            pm += 8 * pitch_m;
+            pk += 8 * pitch_k;
         };
-        uint32_t old[8], kw[8];
-        if (i + 8 <= end) {
-            load(pm, pitch_m, old);
-            load(pk, pitch_k, kw);
-        }
+        refill(0);
+        refill(1);
 #pragma unroll 1
-        for (; i + 8 <= end; i += 8) {
-            uint32_t nm[8], nk[8];
-            const unsigned char *qm = pm + 8 * pitch_m, *qk = pk + 8 * pitch_k;
-            if (i + 16 <= end) {
-                load(qm, pitch_m, nm);
-                load(qk, pitch_k, nk);
-            }
-            uint32_t x = 0u;
+        while (i + 8 <= groups_end) {
 #pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                VRow<DT> v, kv;
-                v.set(old[q]);
-                kv.set(kw[q]);
-                vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
-                const uint32_t w = v.word();
-                x = w ^ old[q];
-                if (WORDS) {
-                    if (x != 0u)
-                        *reinterpret_cast<unsigned int*>(const_cast<unsigned char*>(pm) + q * pitch_m) = w;
-                } else if (x != 0u) {
-                    store(i + q, w);
+            for (int g = 0; g < 2; ++g) {
+                if (i + 8 <= groups_end) {
+                    const bool x = group<INSIDE>(prev, gm[g], gk[g], i, at, sel);
+                    if (STOP && !__any_sync(FULL, x)) return;
+                    refill(g);
+                    i += 8;
+                    at += 8 * pitch_m;
                 }
-                prev = v;
             }
-            if (STOP && !__any_sync(FULL, x != 0u)) return;
-#pragma unroll
-            for (int q = 0; q < 8; ++q) {
-                old[q] = nm[q];
-                kw[q] = nk[q];
-            }
-            pm = qm;
-            pk = qk;
         }
 #pragma unroll 1
-        for (; i < end; ++i) {
-            const uint32_t was = marker(i);
-            VRow<DT> v, kv;
-            v.set(was);
-            kv.set(mask(i));
-            vstep<DT>(v, kv, offers<DT, CONN>(prev, sel));
-            const uint32_t w = v.word();
-            if (w != was) store(i, w);
-            if (STOP && !__any_sync(FULL, w != was)) return;
-            prev = v;
+        for (; i < end; ++i)
+            if (!step(prev, i, sel) && STOP) return;
+    }
+    using Ring = uint32_t[kRing][32];
+    // Returns the row that it stopped at.
+    __device__ __forceinline__ int walk_ahead(const VRow<DT>& prev, int i, int end, const EdgeSel& sel, Ring& rm,
+                                              Ring& rk, int lane) const {
+        return __all_sync(FULL, npx >= P::PPW) ? walk_ring<true>(prev, i, end, sel, rm, rk, lane)
+                                               : walk_ring<false>(prev, i, end, sel, rm, rk, lane);
+    }
+    template <bool INSIDE>
+    __device__ __forceinline__ int walk_ring(VRow<DT> prev, int i, int end, const EdgeSel& sel, Ring& rm, Ring& rk,
+                                             int lane) const {
+        int groups_end;
+        if (!groups<true, INSIDE>(prev, i, end, groups_end, sel)) return i;
+        const unsigned char *pm = m + i * pitch_m, *pk = k + i * pitch_k;
+        unsigned char* at = m + i * pitch_m;
+        int next = i, slot = 0;
+        auto refill = [&](int s) {  // a lane reads only words that it copied
+            if (next + 8 <= groups_end) {
+#pragma unroll
+                for (int q = 0; q < 8; ++q) {
+                    cp_async_4(&rm[s + q][lane], pm + q * pitch_m);
+                    cp_async_4(&rk[s + q][lane], pk + q * pitch_k);
+                }
+            }
+            cp_async_commit();
+            next += 8;
+            pm += 8 * pitch_m;
+            pk += 8 * pitch_k;
+        };
+        for (int s = 0; s < kRing; s += 8) refill(s);
+        bool rises = true;
+#pragma unroll 1
+        while (rises && i + 8 <= groups_end) {
+            cp_async_wait<kRing / 8 - 1>();
+            uint32_t old[8], kw[8];
+#pragma unroll
+            for (int q = 0; q < 8; ++q) {
+                old[q] = rm[slot + q][lane];
+                kw[q] = rk[slot + q][lane];
+            }
+            rises = __any_sync(FULL, group<INSIDE>(prev, old, kw, i, at, sel));
+            refill(slot);
+            slot = (slot + 8) % kRing;
+            i += 8;
+            at += 8 * pitch_m;
         }
+        cp_async_wait<0>();
+#pragma unroll 1
+        while (rises && i < end) rises = step(prev, i++, sel);
+        return i;
     }
 };
 
@@ -600,14 +703,17 @@ __global__ void __launch_bounds__(kStripThreads) sweep_strip_enter_kernel(ImgDes
 template <int DT, int CONN, bool DOWN>
 __global__ void __launch_bounds__(32) sweep_strip_settle_kernel(ImgDesc d, int segs) {
     if (gated_off(d)) return;
+    __shared__ uint32_t ring_m[kRing][32], ring_k[kRing][32];
     const int lane = threadIdx.x;
     const Strip<DT, CONN, DOWN> st(d, (int)blockIdx.x, lane);
     const EdgeSel sel(lane);
+    int reached = 0;
 #pragma unroll 1
     for (int s0 = 1; s0 < segs; s0 += 8) {
         // eight entries' rows in flight together; a walk that goes past an
         // entry below has satisfied it, and one that does not reach it leaves
-        // the row above it as read
+        // the row above it as read.  So no row is copied to shared memory
+        // after this thread wrote it.
         uint32_t above[8], first[8], kw[8];
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
@@ -629,9 +735,10 @@ __global__ void __launch_bounds__(32) sweep_strip_settle_kernel(ImgDesc d, int s
         while (due != 0u) {
             const int i = (s0 + __ffs((int)due) - 1) * kStripRows;
             due &= due - 1u;
+            if (i < reached) continue;
             VRow<DT> prev;
             prev.set(st.marker(i - 1));
-            st.template walk<true>(prev, i, d.H, sel);
+            reached = st.walk_ahead(prev, i, d.H, sel, ring_m, ring_k, lane);
         }
     }
 }
