@@ -74,9 +74,10 @@ typedef struct iwpp_config {
     int plain_loads;           /* 1: never use TMA box loads (else TMA whenever base and
                                   pitch are 16-byte aligned) */
     int solver;                /* in-tile solver: 0 = default, the vertical / horizontal
-                                  passes (2, several warps per tile), 1 = row sweeps (one
-                                  warp per tile), 3 = revisits by a per-tile pixel queue in
-                                  shared memory (first visits by row sweeps) */
+                                  passes (2, several warps per tile); with one warp per
+                                  tile and four tiles per CTA: 1 = row sweeps, 3 = revisits
+                                  by a per-tile pixel queue in shared memory (first visits
+                                  by passes) */
     int front_passes;          /* the front stage: the pixels at the mask's largest value
                                   raised by connected-component labelling, init_passes
                                   whole-image passes, and the tile engine started

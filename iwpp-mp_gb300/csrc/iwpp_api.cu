@@ -788,7 +788,7 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
         e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, device, &li);
         if (e != cudaSuccess) return cuda_status(e);
         grid = li.grid;
-        if (grid > job.G) grid = job.G;
+        grid = std::min(grid, (job.G + li.workers - 1) / li.workers);
         if (job.cfg.grid_ctas > 0 && job.cfg.grid_ctas < grid) grid = job.cfg.grid_ctas;
         if (grid < 1) grid = 1;
     }

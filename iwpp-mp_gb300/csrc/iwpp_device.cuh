@@ -143,8 +143,8 @@ enum : unsigned {
 __device__ __constant__ static const int kNbDx[8] = {0, 0, -1, 1, -1, 1, -1, 1};
 __device__ __constant__ static const int kNbDy[8] = {-1, 1, 0, 0, -1, -1, 1, 1};
 
-// In-tile solvers of a visit (iwpp_config.solver): passes, row sweeps, or
-// revisits by the pixel queue.
+// In-tile solvers of a kernel (iwpp_config.solver): passes by several warps; by
+// one warp per tile, row sweeps, or revisits by the pixel queue.
 enum : int { SOLVE_PASSES = 0, SOLVE_SWEEPS = 1, SOLVE_PQ = 2 };
 
 // A CTA's counters.
@@ -177,13 +177,17 @@ struct __align__(128) TileSmem {
     unsigned nb;      // NB_* bits found by the warps
     unsigned go;      // 1 a tile, 0 the job is over
     VisitCount count;  // the first warp's counters
+};
+// with what the W warps of a visit by passes tell one another
+template <int TH, int W>
+struct __align__(128) TileSmemPasses : TileSmem<TH> {
     // a row beside a warp's first / last block rose: by the parity of the
     // round, the warp, from above / below
-    unsigned mark[2][TH / 8][2];
+    unsigned mark[2][W][2];
 };
 // with the pixel-queue solver's FIFO: tile pixel indices r * TW + c
 template <int TH>
-struct __align__(128) TileSmemAlt : TileSmem<TH> {
+struct __align__(128) TileSmemPq : TileSmem<TH> {
     unsigned short pq[kPqCap];
 };
 
@@ -1071,7 +1075,7 @@ __device__ __forceinline__ bool pq_raise(uint32_t* words, int r, int c, uint32_t
 }
 
 template <int DT, int CONN, int TH>
-__device__ bool pq_solve(TileSmemAlt<TH>& sm, int lane, unsigned long long& rows_chg, bool& col_now, unsigned& rounds) {
+__device__ bool pq_solve(TileSmemPq<TH>& sm, int lane, unsigned long long& rows_chg, bool& col_now, unsigned& rounds) {
     using P = Px<DT>;
     constexpr int TW = 32 * P::PPW;
     int head = 0, tail = 0;  // warp-uniform
@@ -1300,8 +1304,8 @@ struct Rose {
 // `sides` (NB_* bits) names the halo sides whose pixels are new since the
 // tile last converged (all sides on a first visit).  Returns false when the
 // rounds do not end (a defect, reported instead of a hang).
-template <int DT, int CONN, int TH, int W>
-__device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane, unsigned& row_steps, Rose& rose) {
+template <int DT, int CONN, int TH, int W, class SM>
+__device__ __forceinline__ bool solve_tile(SM& sm, int warp, int lane, unsigned& row_steps, Rose& rose) {
     using P = Px<DT>;
     constexpr int BPW = TH / 8 / W;
     constexpr unsigned LASTB = 1u << (BPW - 1);
@@ -1358,14 +1362,16 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
     bool up = false;
 #pragma unroll 1
     for (unsigned round = 0;; ++round, up = !up) {
-        if (W > 1 && round != 0u) {
-            volatile unsigned* mine = sm.mark[round & 1u][warp];
-            const unsigned above = mine[0], below = mine[1];
-            __syncwarp();
-            if (above) da |= 1u;
-            if (below) db |= LASTB;
-            if (lane == 0 && above) mine[0] = 0u;
-            if (lane == 0 && below) mine[1] = 0u;
+        if constexpr (W > 1) {
+            if (round != 0u) {
+                volatile unsigned* mine = sm.mark[round & 1u][warp];
+                const unsigned above = mine[0], below = mine[1];
+                __syncwarp();
+                if (above) da |= 1u;
+                if (below) db |= LASTB;
+                if (lane == 0 && above) mine[0] = 0u;
+                if (lane == 0 && below) mine[1] = 0u;
+            }
         }
 #pragma unroll 1
         for (int n = 0; n < BPW; ++n) {
@@ -1401,7 +1407,7 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
             }
         }
         bool more = (dd | du | da | db) != 0u;
-        if (W > 1) {
+        if constexpr (W > 1) {
             if (lane == 0 && marks != 0u) {
                 __threadfence_block();  // the rows before the marks
                 if (marks & 1u) *(volatile unsigned*)&sm.mark[(round & 1u) ^ 1u][warp - 1][1] = 1u;
@@ -1428,8 +1434,8 @@ __device__ __forceinline__ bool solve_tile(TileSmem<TH>& sm, int warp, int lane,
 // waited 8.7 cycles for instructions; with one per type the batch takes 2.84 ms
 // instead of 3.59, where a single image would lose 2 % to the looking up.
 template <int DT, int CONN, int TH, int W>
-__device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane, unsigned& phase, long long timeout_ns,
-                                           unsigned& row_steps) {
+__device__ __forceinline__ bool visit_tile(TileSmemPasses<TH, W>& sm, int warp, int lane, unsigned& phase,
+                                           long long timeout_ns, unsigned& row_steps) {
     constexpr int BPW = TH / 8 / W;
     const bool clerk = warp == 0 && lane == 0;  // keeps the visit's clock
     if (clerk) sm.count.cycles[1] -= clock64();
@@ -1474,93 +1480,148 @@ __device__ __forceinline__ bool visit_tile(TileSmem<TH>& sm, int warp, int lane,
     return ok;
 }
 
-// The visit with the alternative solvers, for callers that ask for them
-// (iwpp_config.solver 1 and 3), by a CTA of one warp.  All solvers are
-// sequences of valid monotone updates that stop at the tile's fixed point, so
-// they give the same bytes.
+// The visits with the alternative solvers, for callers that ask for them
+// (iwpp_config.solver 1 and 3), by one warp.  All solvers are sequences of valid
+// monotone updates that stop at the tile's fixed point, so they give the same
+// bytes.
+
+// What rose in a visit by one warp, or since it last published: rows (bit r - 1
+// for SMEM row r), and a side column (per lane).
+struct RoseAlt {
+    unsigned long long rows = 0ull;
+    bool col = false;
+    bool published = false;  // some of it was published before
+};
+
+// Stores what rose and returns the NB_* bits of the neighbours that it raises.
+// (A pixel is next to halo pixels that its own block's detection looks at.)
 template <int DT, int CONN, int TH>
-__device__ __forceinline__ bool visit_tile_alt(TileSmemAlt<TH>& sm, int lane, unsigned& phase, long long timeout_ns,
-                                               int solver, unsigned& row_steps) {
+__device__ __forceinline__ unsigned publish_alt(const TileSmem<TH>& sm, int lane, const RoseAlt& rose) {
+    const unsigned f_col = __any_sync(FULL, rose.col) ? RF_COL : 0u;
+    unsigned nb = 0u;
+#pragma unroll 1
+    for (int b = 0; b < TH / 8; ++b) {
+        const unsigned rb = (unsigned)(rose.rows >> (8 * b)) & 0xffu;
+        if (rb == 0u) continue;
+        write_back_block<DT, TH>(sm.d, sm, lane, b, sm.tx * 32 * Px<DT>::PPW, sm.ty * TH);
+        nb |= detect_neighbours<DT, CONN, TH>(sm, lane, b,
+                                              ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col,
+                                              CONN == 8);
+    }
+    return nb;
+}
+
+// Row sweeps, raster and anti-raster, until one after the first two changes
+// nothing.  `early` can publish intermediate results: after a sweep that raised
+// a boundary row or column, if early.want() says so (the async queue, while many
+// warps wait for work), the rows risen so far are stored and the neighbours that
+// they raise handed to early.flush() while the sweeps go on, which one warp
+// takes long over; `rose` then holds what rose after the last flush.
+template <int DT, int CONN, int TH, class Early>
+__device__ __forceinline__ void solve_sweeps(TileSmem<TH>& sm, int lane, unsigned& row_steps, RoseAlt& rose,
+                                             Early& early) {
     using P = Px<DT>;
-    constexpr int NB = TH / 8;
     constexpr unsigned long long ALL = TH == 64 ? ~0ull : ((1ull << TH) - 1ull);
     constexpr unsigned long long TOP = 1ull, BOT = 1ull << (TH - 1);
-    const long long c0 = clock64();
-    unsigned sides = sm.sides, sweeps = 0u;
-    const bool ok = fetch_tile<DT, TH, 1>(sm.d, sm.tx, sm.ty, sm, 0, lane, phase, timeout_ns);
-    __syncwarp();
-    if (!ok) return false;
-    const long long c1 = clock64();
     const uint32_t edge_mask = lane == 0 ? P::FIRST_MASK : lane == 31 ? P::LAST_MASK : 0u;
-    unsigned long long rose = 0ull;  // rows that rose
-    bool col = false;                // a side column rose (per lane)
-    bool solved = false;
-    if (solver == SOLVE_PQ && sides != 0xffu) {
-        // a revisit by the pixel queue; if it cannot finish, the sweeps take
-        // the tile with every row dirty
-        unsigned rounds = 0u;
-        unsigned long long mine = 0ull;
-        solved = pq_solve<DT, CONN, TH>(sm, lane, mine, col, rounds);
-        __syncwarp();
-        rose = warp_or64(mine);
-        row_steps += rounds;
-        sweeps += 1u;
-        if (!solved) sides = 0xffu;
-    }
-    if (!solved) {
-        // Row sweeps, raster and anti-raster, until one after the first two
-        // changes nothing.  Rows whose halo inputs are new are processed by
-        // the first two sweeps: the top row by the raster sweep (N, NW, NE),
-        // the bottom row by the anti-raster sweep (S, SW, SE), every row when
-        // a side column that feeds the sweep changed (W, and E through the
-        // up-right / down-right diagonals for 8-connectivity; the reverse for
-        // the anti-raster sweep).  Other rows are skipped while nothing they
-        // depend on has changed.
-        const unsigned side_down = CONN == 8 ? (NB_W | NB_E) : NB_W;
-        const unsigned side_up = CONN == 8 ? (NB_W | NB_E) : NB_E;
-        const unsigned long long force_down =
-            (sides & side_down) ? ALL : (sides & (NB_N | NB_NW | NB_NE)) ? TOP : 0ull;
-        const unsigned long long force_up = (sides & side_up) ? ALL : (sides & (NB_S | NB_SW | NB_SE)) ? BOT : 0ull;
-        unsigned long long chg_prev = 0ull;
-        for (unsigned n = 0;; ++n) {
-            unsigned long long dil = chg_prev | (chg_prev << 1) | (chg_prev >> 1);
-            if (n == 0) dil |= force_down;
-            if (n == 1) dil |= force_up;
-            dil &= ALL;
-            unsigned long long chg = 0ull;
-            if (dil != 0ull) {
-                if ((n & 1u) == 0u)
-                    sweep<DT, CONN, TH, true>(sm, lane, dil, chg, col, edge_mask, row_steps);
-                else
-                    sweep<DT, CONN, TH, false>(sm, lane, dil, chg, col, edge_mask, row_steps);
+    const unsigned sides = sm.sides;
+    // Rows whose halo inputs are new are processed by the first two sweeps:
+    // the top row by the raster sweep (N, NW, NE), the bottom row by the
+    // anti-raster sweep (S, SW, SE), every row when a side column that feeds
+    // the sweep changed (W, and E through the up-right / down-right diagonals
+    // for 8-connectivity; the reverse for the anti-raster sweep).  Other rows
+    // are skipped while nothing they depend on has changed.
+    const unsigned side_down = CONN == 8 ? (NB_W | NB_E) : NB_W;
+    const unsigned side_up = CONN == 8 ? (NB_W | NB_E) : NB_E;
+    const unsigned long long force_down = (sides & side_down) ? ALL : (sides & (NB_N | NB_NW | NB_NE)) ? TOP : 0ull;
+    const unsigned long long force_up = (sides & side_up) ? ALL : (sides & (NB_S | NB_SW | NB_SE)) ? BOT : 0ull;
+    unsigned long long chg_prev = 0ull;
+    unsigned n = 0u;
+    for (;; ++n) {
+        unsigned long long dil = chg_prev | (chg_prev << 1) | (chg_prev >> 1);
+        if (n == 0) dil |= force_down;
+        if (n == 1) dil |= force_up;
+        dil &= ALL;
+        unsigned long long chg = 0ull;
+        bool col_now = false;
+        if (dil != 0ull) {
+            if ((n & 1u) == 0u)
+                sweep<DT, CONN, TH, true>(sm, lane, dil, chg, col_now, edge_mask, row_steps);
+            else
+                sweep<DT, CONN, TH, false>(sm, lane, dil, chg, col_now, edge_mask, row_steps);
+        }
+        rose.rows |= chg;
+        rose.col |= col_now;
+        chg_prev = chg;
+        if (chg == 0ull && n >= 1u) break;
+        if constexpr (Early::kEnabled) {
+            if (((chg & (TOP | BOT)) != 0ull || __any_sync(FULL, col_now)) && early.want(lane)) {
+                early.flush(publish_alt<DT, CONN, TH>(sm, lane, rose), lane);
+                rose.rows = 0ull;
+                rose.col = false;
+                rose.published = true;
             }
-            sweeps += 1u;
-            rose |= chg;
-            chg_prev = chg;
-            if (chg == 0ull && n >= 1u) break;
         }
     }
-    const long long c2 = clock64();
-    const unsigned f_col = __any_sync(FULL, col) ? RF_COL : 0u;
-    unsigned nb = 0u;
-    for (int b = 0; b < NB; ++b) {
-        const unsigned rb = (unsigned)(rose >> (8 * b)) & 0xffu;
-        if (rb != 0u) write_back_block<DT, TH>(sm.d, sm, lane, b, sm.tx * 32 * P::PPW, sm.ty * TH);
-        if (rose != 0ull)
-            nb |= detect_neighbours<DT, CONN, TH>(sm, lane, b,
-                                                  ((rb & 1u) ? RF_FIRST : 0u) | ((rb & 0x80u) ? RF_LAST : 0u) | f_col,
-                                                  CONN == 8);
+    if (lane == 0) sm.count.sweeps += n + 1u;
+}
+
+// A revisit by the pixel queue; a first visit, or one that the queue cannot
+// finish, by the passes.
+template <int DT, int CONN, int TH>
+__device__ __forceinline__ bool solve_pq(TileSmemPq<TH>& sm, int lane, unsigned& row_steps, RoseAlt& rose) {
+    constexpr unsigned long long TOP = 1ull, BOT = 1ull << (TH - 1);
+    if (sm.sides != 0xffu) {
+        unsigned rounds = 0u;
+        unsigned long long mine = 0ull;
+        const bool solved = pq_solve<DT, CONN, TH>(sm, lane, mine, rose.col, rounds);
+        __syncwarp();
+        rose.rows = warp_or64(mine);
+        row_steps += rounds;
+        if (lane == 0) sm.count.sweeps += 1u;
+        if (solved) return true;
+        if (lane == 0) sm.sides = 0xffu;
+        __syncwarp();
     }
-    if (lane == 0) sm.nb = nb | (rose != 0ull ? (unsigned)NB_STORED : 0u);
+    Rose r;
+    const bool ok = solve_tile<DT, CONN, TH, 1>(sm, 0, lane, row_steps, r);
+    for (int b = 0; b < TH / 8; ++b)
+        if ((r.rows >> b) & 1u) rose.rows |= 0x7eull << (8 * b);  // (which of a block's inner rows does not matter)
+    if (r.top) rose.rows |= TOP;
+    if (r.bottom) rose.rows |= BOT;
+    rose.col |= r.col != 0u;
+    return ok;
+}
+
+// PQ: by the pixel queue, else by row sweeps.
+template <int DT, int CONN, int TH, bool PQ, class SM, class Early>
+__device__ __forceinline__ bool visit_tile_alt(SM& sm, int lane, unsigned& phase, long long timeout_ns,
+                                               unsigned& row_steps, Early& early) {
+    if (lane == 0) sm.count.cycles[1] -= clock64();
+    bool ok = fetch_tile<DT, TH, 1>(sm.d, sm.tx, sm.ty, sm, 0, lane, phase, timeout_ns);
+    __syncwarp();
+    if (!ok) return false;
+    if (lane == 0) {
+        const long long t = clock64();
+        sm.count.cycles[1] += t;
+        sm.count.cycles[2] -= t;
+    }
+    RoseAlt rose;
+    if constexpr (PQ)
+        ok = solve_pq<DT, CONN, TH>(sm, lane, row_steps, rose);
+    else
+        solve_sweeps<DT, CONN, TH>(sm, lane, row_steps, rose, early);
+    if (lane == 0) {
+        const long long t = clock64();
+        sm.count.cycles[2] += t;
+        sm.count.cycles[3] -= t;
+    }
+    const unsigned nb = publish_alt<DT, CONN, TH>(sm, lane, rose);
+    if (lane == 0) sm.nb = nb | (rose.rows != 0ull || rose.published ? (unsigned)NB_STORED : 0u);
     fence_proxy_async_smem();
     __syncwarp();
-    if (lane == 0) {
-        sm.count.sweeps += sweeps;
-        sm.count.cycles[1] += c1 - c0;
-        sm.count.cycles[2] += c2 - c1;
-        sm.count.cycles[3] += clock64() - c2;
-    }
-    return true;
+    if (lane == 0) sm.count.cycles[3] += clock64();
+    return ok;
 }
 
 }  // namespace iwpp

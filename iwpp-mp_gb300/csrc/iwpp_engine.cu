@@ -176,12 +176,12 @@ cudaError_t queue_selftest(const EngineArgs& a, int variant, int copies, unsigne
 }
 
 // ------------------------------------------------------------ host side
-// The engine's kernel shapes: tile height, warps per tile, and whether it has
-// the alternative in-tile solvers.
-enum Shape : int { T32_W4, T64_W8, T64_W4, T64_W2, T32_ALT, T64_ALT, SHAPES };
+// The engine's kernel shapes: tile height, and warps per tile for the passes or
+// one of the alternative in-tile solvers.
+enum Shape : int { T32_W4, T64_W8, T64_W4, T64_W2, T32_SWEEPS, T64_SWEEPS, T32_PQ, T64_PQ, SHAPES };
 
 // Shape of a job's kernel.  solver: iwpp_config.solver (0 and 2 are the
-// passes, 1 and 3 the kernels with the alternative solvers).  Warps per tile:
+// passes, 1 the row sweeps, 3 the pixel queue).  Warps per tile:
 // the fewer tiles an SM has, the more warps work on one, since only a part
 // of a job's tiles can be visited at any time and a visit's length then sets
 // the pace; with many tiles the warps that wait for others of their tile cost
@@ -193,9 +193,9 @@ enum Shape : int { T32_W4, T64_W8, T64_W4, T64_W2, T32_ALT, T64_ALT, SHAPES };
 //                 30   (6144^2 u8)  400 / 298 / 256
 //                 54   (8192^2 u8)  791 / 561 / 453
 static Shape select_shape(int tile_rows, int solver, long long tiles, int sms) {
-    const bool alt = solver == 1 || solver == 3;
-    if (tile_rows == 32) return alt ? T32_ALT : T32_W4;
-    if (alt) return T64_ALT;
+    if (solver == 1) return tile_rows == 32 ? T32_SWEEPS : T64_SWEEPS;
+    if (solver == 3) return tile_rows == 32 ? T32_PQ : T64_PQ;
+    if (tile_rows == 32) return T32_W4;
     return 4 * tiles <= 27ll * sms ? T64_W8 : 2 * tiles <= 25ll * sms ? T64_W4 : T64_W2;
 }
 
@@ -203,28 +203,35 @@ struct Kernel {
     void* fn;
     int threads;
     size_t smem;
+    int workers;  // tiles that a CTA works on at a time
 };
 static Kernel kernel_of(int variant, Shape shape, int conn) {
     constexpr size_t slack = 128;
-    auto fn = [&](int tile_rows, int warps, bool alt) {
+    auto fn = [&](int tile_rows, int warps, int solve) {
         switch (variant) {
-            case VAR_MUTEX: return kernel_for<VAR_MUTEX>(tile_rows, warps, alt, conn);
-            case VAR_DOUBLE: return kernel_for<VAR_DOUBLE>(tile_rows, warps, alt, conn);
-            case VAR_ASYNC: return kernel_for<VAR_ASYNC>(tile_rows, warps, alt, conn);
-            default: return kernel_for<VAR_UNIQUE>(tile_rows, warps, alt, conn);
+            case VAR_MUTEX: return kernel_for<VAR_MUTEX>(tile_rows, warps, solve, conn);
+            case VAR_DOUBLE: return kernel_for<VAR_DOUBLE>(tile_rows, warps, solve, conn);
+            case VAR_ASYNC: return kernel_for<VAR_ASYNC>(tile_rows, warps, solve, conn);
+            default: return kernel_for<VAR_UNIQUE>(tile_rows, warps, solve, conn);
         }
     };
+    auto passes = [&](int tile_rows, int warps, size_t tile) {
+        return Kernel{fn(tile_rows, warps, SOLVE_PASSES), 32 * warps, slack + tile, 1};
+    };
+    auto alt = [&](int tile_rows, int solve, size_t tile) {
+        return Kernel{fn(tile_rows, 1, solve), 32 * kAltWorkers, slack + kAltWorkers * tile, kAltWorkers};
+    };
     switch (shape) {
-        case T32_W4: return {fn(32, 4, false), 128, slack + sizeof(TileSmem<32>)};
-        case T64_W8: return {fn(64, 8, false), 256, slack + sizeof(TileSmem<64>)};
-        case T64_W4: return {fn(64, 4, false), 128, slack + sizeof(TileSmem<64>)};
-        case T64_W2: return {fn(64, 2, false), 64, slack + sizeof(TileSmem<64>)};
-        case T32_ALT: return {fn(32, 1, true), 32, slack + sizeof(TileSmemAlt<32>)};
-        default: return {fn(64, 1, true), 32, slack + sizeof(TileSmemAlt<64>)};
+        case T32_W4: return passes(32, 4, sizeof(TileSmemPasses<32, 4>));
+        case T64_W8: return passes(64, 8, sizeof(TileSmemPasses<64, 8>));
+        case T64_W4: return passes(64, 4, sizeof(TileSmemPasses<64, 4>));
+        case T64_W2: return passes(64, 2, sizeof(TileSmemPasses<64, 2>));
+        case T32_SWEEPS: return alt(32, SOLVE_SWEEPS, sizeof(TileSmem<32>));
+        case T64_SWEEPS: return alt(64, SOLVE_SWEEPS, sizeof(TileSmem<64>));
+        case T32_PQ: return alt(32, SOLVE_PQ, sizeof(TileSmemPq<32>));
+        default: return alt(64, SOLVE_PQ, sizeof(TileSmemPq<64>));
     }
 }
-// below the size from which a kernel has to ask for its shared memory
-static_assert(128 + sizeof(TileSmemAlt<64>) <= 48 * 1024, "dynamic shared memory");
 
 // Multiprocessors of a device (asked once), 0 when it cannot be asked.
 int engine_sm_count(int device) {
@@ -251,6 +258,8 @@ static cudaError_t resident_ctas(int variant, Shape shape, int conn, int device,
     const Kernel k = kernel_of(variant, shape, conn);
     cudaFuncAttributes attr;
     cudaError_t e = cudaFuncGetAttributes(&attr, k.fn);  // (loads it where kernels are loaded on demand)
+    if (e == cudaSuccess && k.smem > 48 * 1024)
+        e = cudaFuncSetAttribute(k.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(per_sm, k.fn, k.threads, k.smem);
     if (e == cudaSuccess) cached.store(*per_sm, std::memory_order_relaxed);
     return e;
@@ -264,18 +273,22 @@ cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, lon
     int per_sm = 0;
     const cudaError_t e = resident_ctas(variant, shape, conn, device, &per_sm);
     if (e != cudaSuccess) return e;
-    // CTAs of the mutex queue take turns at its lock: past two per SM the longer
-    // line costs more than the visits beside one another gain.  1 / 2 / 3 / all
+    // CTAs of the mutex queue take turns at its lock, and past a few per SM the
+    // longer line costs more than the visits beside one another gain.  Where that
+    // is depends on the image; two is a compromise that is seldom far off, not
+    // the best for each (8-connected, h = 40, likes three).  1 / 2 / 3 / all
     // that fit (10, 5 or 3) per SM, us: 4096^2 u8 h-domes, 4-connected, h = 10
     // 757 / 843 / 905 / 2062, h = 100 1726 / 1260 / 1288 / 3054, 8-connected, h = 40
     // 2600 / 2259 / 1540 / 3137; 6000 x 5000 u8 2530 / 1550 / 2388 / 2450; 2048 x 1500
     // u16 600 / 757 / 1856 / 1855; sparse seeds 4096^2 u8 4120 / 3680 / 3266 / 3180,
-    // 5000^2 i32 19900 / 21100 / 21400 / 30300.
-    // The one-warp CTAs of the other solvers: 2 / 3 / 4 / 8, row sweeps, 4096^2
-    // u8 h = 10 1120 / 1450 / 1533 / 1491, 8-connected, h = 40 2813 / 2488 / 1984 / 1634,
-    // sparse seeds 5641 / 4083 / 3848 / 4868, 1024^2 490 / 498 / 431 / 472.
-    if (variant == VAR_MUTEX) per_sm = std::min(per_sm, shape == T32_ALT || shape == T64_ALT ? 4 : 2);
+    // 5000^2 i32 19900 / 21100 / 21400 / 30300.  CTAs of four workers, row sweeps,
+    // 1 / 2 / 3: 4096^2 u8 4-connected 1181 / 1705 / 1574, 8-connected 3403 / 3090 /
+    // 3031, sparse 3911 / 4514 / 6403, 8192^2 sparse 13132 / 13672 / 14395; pixel
+    // queue 1100 / 1682 / 2245, 3348 / 2357 / 2866, 5459 / 4930 / 5348, 20713 / 15843 /
+    // 15093.
+    if (variant == VAR_MUTEX) per_sm = std::min(per_sm, 2);
     li->grid = per_sm * sms;
+    li->workers = kernel_of(variant, shape, conn).workers;
     li->shape = shape;
     li->conn = conn;
     return li->grid > 0 ? cudaSuccess : cudaErrorInvalidConfiguration;

@@ -135,6 +135,7 @@ inline int status_of_job(unsigned error) {
 }
 struct LaunchInfo {
     int grid;   // CTAs that the device keeps resident
+    int workers;  // tiles that a CTA works on at a time
     int shape;  // the kernel's shape (iwpp_engine.cu)
     int conn;   // the connectivity it is for, 0: both
 };

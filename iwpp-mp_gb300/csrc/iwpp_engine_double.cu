@@ -2,5 +2,5 @@
 #include "iwpp_engine_kernel.cuh"
 
 namespace iwpp {
-template void* kernel_for<VAR_DOUBLE>(int, int, bool, int);
+template void* kernel_for<VAR_DOUBLE>(int, int, int, int);
 }

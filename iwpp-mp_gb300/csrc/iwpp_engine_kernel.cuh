@@ -33,36 +33,39 @@ __device__ __forceinline__ int find_image(const EngineArgs& a, unsigned g) {
     return lo;
 }
 
-// A tile's shared memory in a kernel, and its visit for the image's pixel type.
-template <int TH, bool ALT>
+// A tile's shared memory in a kernel (SOLVE_*), and its visit for the image's
+// pixel type.
+template <int TH, int W, int SOLVE>
 struct SmemOf {
+    using T = TileSmemPasses<TH, W>;
+};
+template <int TH, int W>
+struct SmemOf<TH, W, SOLVE_SWEEPS> {
     using T = TileSmem<TH>;
 };
-template <int TH>
-struct SmemOf<TH, true> {
-    using T = TileSmemAlt<TH>;
+template <int TH, int W>
+struct SmemOf<TH, W, SOLVE_PQ> {
+    using T = TileSmemPq<TH>;
 };
 
-template <int DT, int CONN, int TH, int W, bool ALT, class SM>
+template <int DT, int CONN, int TH, int W, int SOLVE, class SM, class Early>
 __device__ __forceinline__ bool visit_as(const EngineArgs& a, SM& sm, int warp, int lane, unsigned& phase,
-                                         unsigned& row_steps) {
-    if constexpr (!ALT)
+                                         unsigned& row_steps, Early& early) {
+    if constexpr (SOLVE == SOLVE_PASSES)
         return visit_tile<DT, CONN, TH, W>(sm, warp, lane, phase, a.timeout_ns, row_steps);
     else if (sm.d.conn == 8)
-        return visit_tile_alt<DT, 8, TH>(sm, lane, phase, a.timeout_ns, a.solver == 3 ? SOLVE_PQ : SOLVE_SWEEPS,
-                                         row_steps);
+        return visit_tile_alt<DT, 8, TH, SOLVE == SOLVE_PQ>(sm, lane, phase, a.timeout_ns, row_steps, early);
     else
-        return visit_tile_alt<DT, 4, TH>(sm, lane, phase, a.timeout_ns, a.solver == 3 ? SOLVE_PQ : SOLVE_SWEEPS,
-                                         row_steps);
+        return visit_tile_alt<DT, 4, TH, SOLVE == SOLVE_PQ>(sm, lane, phase, a.timeout_ns, row_steps, early);
 }
 
-template <int CONN, int TH, int W, bool ALT, class SM>
+template <int CONN, int TH, int W, int SOLVE, class SM, class Early>
 __device__ __forceinline__ bool dispatch_visit(const EngineArgs& a, SM& sm, int warp, int lane, unsigned& phase,
-                                               unsigned& row_steps) {
+                                               unsigned& row_steps, Early& early) {
     switch (sm.d.dtype) {
-        case DT_U8: return visit_as<DT_U8, CONN, TH, W, ALT>(a, sm, warp, lane, phase, row_steps);
-        case DT_U16: return visit_as<DT_U16, CONN, TH, W, ALT>(a, sm, warp, lane, phase, row_steps);
-        default: return visit_as<DT_I32, CONN, TH, W, ALT>(a, sm, warp, lane, phase, row_steps);
+        case DT_U8: return visit_as<DT_U8, CONN, TH, W, SOLVE>(a, sm, warp, lane, phase, row_steps, early);
+        case DT_U16: return visit_as<DT_U16, CONN, TH, W, SOLVE>(a, sm, warp, lane, phase, row_steps, early);
+        default: return visit_as<DT_I32, CONN, TH, W, SOLVE>(a, sm, warp, lane, phase, row_steps, early);
     }
 }
 
@@ -217,8 +220,10 @@ __device__ int push_entries(const EngineArgs& a, bool want, unsigned gn, int lan
 // from it first; the global stack sees a batch take when the buffer runs dry,
 // a spill when it fills, and a share when the global stack is empty while
 // CTAs elsewhere wait.  Buffered entries count in `pending`, so the
-// termination rule (nothing pending, nothing stacked) is unchanged.  The
-// CTA's first warp alone works the queue, so the buffer needs no lock.
+// termination rule (nothing pending, nothing stacked) is unchanged.  Where the
+// CTA's first warp alone works the queue the buffer needs no lock; where its
+// warps each work it (SHARED, the solvers of one warp per tile) they take
+// turns at it, and one of them at a time goes to the global stack for all.
 constexpr int kCtaBuf = 64;    // entries a CTA buffers
 constexpr int kCtaSpill = 48;  // above this a push spills the buffer down to kCtaKeep
 constexpr int kCtaKeep = 16;
@@ -226,53 +231,106 @@ constexpr int kCtaKeep = 16;
 struct MutexCtaBuf {
     int n;
     unsigned e[kCtaBuf];
+    int lock;
+    int taker;    // 1 while one of this CTA's warps works the global stack
+    int waiting;  // this CTA's warps waiting for work
 };
 __shared__ MutexCtaBuf s_cq;
 
 __device__ __forceinline__ int cq_count() { return *(volatile int*)&s_cq.n; }
 
+// The buffer's lock, held by one of this CTA's warps (lane 0) for a few
+// shared-memory accesses at a time; the bound is never reached in a working job.
+template <bool SHARED>
+__device__ __forceinline__ bool cq_lock(const EngineArgs& a) {
+    if (SHARED) {
+        unsigned spins = 0;
+        while (atomicCAS(&s_cq.lock, 0, 1) != 0) {
+            __nanosleep(32);
+            if (++spins > (1u << 22)) {
+                set_error(a.ctrl, DEV_ERR_TIMEOUT);
+                return false;
+            }
+        }
+        __threadfence_block();
+    }
+    return true;
+}
+template <bool SHARED>
+__device__ __forceinline__ void cq_unlock() {
+    if (SHARED) {
+        __threadfence_block();
+        atomicExch(&s_cq.lock, 0);
+    }
+}
+
 // Moves up to 32 of the buffer's newest entries beyond `keep` to the global
 // stack (one acquisition).
+template <bool SHARED>
 __device__ inline void cta_spill(const EngineArgs& a, int lane, int keep) {
-    const int n = cq_count();
-    const int m = min(max(n - keep, 0), 32);
+    int m = 0, base = 0;
+    if (lane == 0 && cq_lock<SHARED>(a)) {
+        const int n = cq_count();
+        m = min(max(n - keep, 0), 32);
+        base = n - m;
+        *(volatile int*)&s_cq.n = base;
+        if (m == 0) cq_unlock<SHARED>();
+    }
+    m = __shfl_sync(FULL, m, 0);
+    base = __shfl_sync(FULL, base, 0);
     if (m == 0) return;
-    const unsigned mine = lane < m ? *(volatile unsigned*)&s_cq.e[n - m + lane] : 0u;
+    const unsigned mine = lane < m ? *(volatile unsigned*)&s_cq.e[base + lane] : 0u;
     __syncwarp();
-    if (lane == 0) s_cq.n = n - m;
-    __syncwarp();
+    if (lane == 0) cq_unlock<SHARED>();
     mutex_push_global(a, lane < m, mine, lane, true);
 }
 
 // Inserts the entries of the lanes with `want` set into this CTA's buffer
 // (what does not fit goes to the global stack), spilling a full buffer.
 // `counted`: `pending` already holds them.  Returns their number.
+template <bool SHARED>
 __device__ inline int cta_push(const EngineArgs& a, bool want, unsigned gn, int lane, bool counted = false) {
     const unsigned ballot = __ballot_sync(FULL, want);
     if (ballot == 0u) return 0;
     const int n = __popc(ballot);
     const int rank = __popc(ballot & ((1u << lane) - 1u));
-    if (lane == 0 && !counted) atomicAdd(&a.ctrl->pending, n);  // before any of them can be taken
-    const int base = cq_count();
-    const int k = min(n, kCtaBuf - base);
+    int base = 0, k = 0;
+    bool mine = false;  // lane 0: the lock is held
+    if (lane == 0) {
+        if (!counted) atomicAdd(&a.ctrl->pending, n);  // before any of them can be taken
+        mine = cq_lock<SHARED>(a);
+        if (mine) {
+            base = cq_count();
+            k = min(n, kCtaBuf - base);
+        }
+    }
+    base = __shfl_sync(FULL, base, 0);
+    k = __shfl_sync(FULL, k, 0);
     if (want && rank < k) *(volatile unsigned*)&s_cq.e[base + rank] = gn;
     __syncwarp();
-    if (lane == 0) s_cq.n = base + k;
+    if (mine) {
+        *(volatile int*)&s_cq.n = base + k;
+        cq_unlock<SHARED>();
+    }
     __syncwarp();
     if (n > k) mutex_push_global(a, want && rank >= k, gn, lane, true);
-    if (cq_count() > kCtaSpill) cta_spill(a, lane, kCtaKeep);
+    if (__shfl_sync(FULL, cq_count(), 0) > kCtaSpill) cta_spill<SHARED>(a, lane, kCtaKeep);
     return n;
 }
 
 // The buffer's newest entry, or ~0u.
-__device__ inline unsigned cta_take(int lane) {
-    const int n = cq_count();
-    if (n == 0) return ~0u;
-    const unsigned g = *(volatile unsigned*)&s_cq.e[n - 1];
-    __syncwarp();
-    if (lane == 0) s_cq.n = n - 1;
-    __syncwarp();
-    return g;
+template <bool SHARED>
+__device__ inline unsigned cta_take(const EngineArgs& a, int lane) {
+    unsigned g = ~0u;
+    if (lane == 0 && cq_count() > 0 && cq_lock<SHARED>(a)) {
+        const int n = cq_count();
+        if (n > 0) {
+            g = *(volatile unsigned*)&s_cq.e[n - 1];
+            *(volatile int*)&s_cq.n = n - 1;
+        }
+        cq_unlock<SHARED>();
+    }
+    return __shfl_sync(FULL, g, 0);
 }
 
 // ------------------------------------------------------------ one entry
@@ -299,6 +357,56 @@ __device__ __forceinline__ bool take_tile(const EngineArgs& a, unsigned g, int l
     return true;
 }
 
+// Lane < 8: marks the neighbour tile in direction `lane` DIRTY if it is in
+// `nb`; true where it is to be inserted (*gn).  *fresh: it was neither DIRTY nor
+// being visited.
+template <int VAR>
+__device__ __forceinline__ bool mark_neighbour(const EngineArgs& a, const ImgDesc& d, int tx, int ty, unsigned nb,
+                                               int lane, unsigned* gn, bool* fresh) {
+    if (!((nb >> lane) & 1u)) return false;
+    const int nx = tx + kNbDx[lane], ny = ty + kNbDy[lane];
+    if (nx < 0 || nx >= d.tiles_x || ny < 0 || ny >= d.tiles_y) return false;
+    *gn = (unsigned)d.tile_base + (unsigned)(ny * d.tiles_x + nx);
+    const unsigned old = atomicOr(&a.state[*gn], ST_DIRTY | (1u << (ST_SIDE_SHIFT + (unsigned)kNbOpposite[lane])));
+    *fresh = (old & (ST_DIRTY | ST_ACTIVE)) == 0u;
+    return VAR == VAR_UNIQUE || VAR == VAR_ASYNC ? *fresh : true;
+}
+
+// Publication before a tile has converged, for the solvers of one warp per
+// tile with the async queue: while more than half of the warps wait for work (a
+// quarter or an eighth switches too early on h-dome images, three quarters too
+// late on long corridors) a visit that raised a boundary of its tile stores
+// what it has and inserts those neighbours at once, so that they can start.
+// Several warps per tile are done too soon for it to pay (every workload
+// slower).  Row sweeps, us with / without it: sparse seeds 4096^2 u8 710 / 822,
+// h-domes 2048 x 1500 u16 338 / 378, 300 x 200 u8 211 / 225, 4096^2 u8 446 / 434.
+template <int VAR>
+struct EarlyFlush {
+    static constexpr bool kEnabled = VAR == VAR_ASYNC;
+    const EngineArgs& a;
+    const ImgDesc& d;
+    const int &tx, &ty;
+    unsigned& pushes;
+    int half;  // of the warps that take entries
+    __device__ __forceinline__ bool want(int lane) const {
+        unsigned v = 0u;
+        if (lane == 0) {
+            const unsigned head = ld_volatile(&a.ctrl->ahead), tail = ld_volatile(&a.ctrl->atail);
+            v = (int)(head - tail) > half ? 1u : 0u;
+        }
+        return __shfl_sync(FULL, v, 0) != 0u;
+    }
+    __device__ __forceinline__ void flush(unsigned nb, int lane) const {
+        __syncwarp();
+        fence_gpu();  // release: the rows just stored before the neighbours' DIRTY
+        bool fresh = false;
+        unsigned gn = 0u;
+        const bool want = lane < 8 && mark_neighbour<VAR>(a, d, tx, ty, nb, lane, &gn, &fresh);
+        const int pushed = push_entries<VAR>(a, want, gn, lane, nullptr);
+        if (lane == 0) pushes += (unsigned)pushed;
+    }
+};
+
 // After a visit of tile (tx, ty) = g: marks the neighbour tiles in `nb`
 // DIRTY and inserts them (VAR_UNIQUE / VAR_ASYNC: only those that were
 // neither pending nor being visited), and releases g, inserting it again if
@@ -308,20 +416,13 @@ __device__ __forceinline__ bool take_tile(const EngineArgs& a, unsigned g, int l
 // of the newly dirty neighbours is not inserted but returned: the CTA visits
 // it next itself, following the propagation front without a trip through the
 // queue.  Returns ~0u when there is none.
-template <int VAR>
+template <int VAR, bool SHARED>
 __device__ __forceinline__ unsigned leave_tile(const EngineArgs& a, const ImgDesc& d, int tx, int ty, unsigned g,
                                                unsigned nb, int lane, unsigned* wq, int* pushed) {
-    bool want = false, fresh = false;
+    bool fresh = false, want = false;
     unsigned gn = 0u;
-    if (lane < 8 && ((nb >> lane) & 1u)) {
-        const int nx = tx + kNbDx[lane], ny = ty + kNbDy[lane];
-        if (nx >= 0 && nx < d.tiles_x && ny >= 0 && ny < d.tiles_y) {
-            gn = (unsigned)d.tile_base + (unsigned)(ny * d.tiles_x + nx);
-            const unsigned old =
-                atomicOr(&a.state[gn], ST_DIRTY | (1u << (ST_SIDE_SHIFT + (unsigned)kNbOpposite[lane])));
-            fresh = (old & (ST_DIRTY | ST_ACTIVE)) == 0u;
-            want = (VAR == VAR_UNIQUE || VAR == VAR_ASYNC) ? fresh : true;
-        }
+    if (lane < 8) {
+        want = mark_neighbour<VAR>(a, d, tx, ty, nb, lane, &gn, &fresh);
     } else if (lane == 8) {
         gn = g;
         want = (atomicAnd(&a.state[g], ~ST_ACTIVE) & ST_DIRTY) != 0u;
@@ -335,7 +436,7 @@ __device__ __forceinline__ unsigned leave_tile(const EngineArgs& a, const ImgDes
             if (lane == leader) want = false;
         }
     }
-    *pushed = VAR == VAR_MUTEX ? cta_push(a, want, gn, lane) : push_entries<VAR>(a, want, gn, lane, wq);
+    *pushed = VAR == VAR_MUTEX ? cta_push<SHARED>(a, want, gn, lane) : push_entries<VAR>(a, want, gn, lane, wq);
     return cont;
 }
 
@@ -348,6 +449,7 @@ __device__ __forceinline__ unsigned leave_tile(const EngineArgs& a, const ImgDes
 // entry, 1 when the job is over for this warp (finished or an error), 2 when
 // there is nothing to take now.  On overflow the quiescent stack is refilled
 // with every tile (MR.cu:785-806).
+template <bool SHARED>
 __device__ inline int mutex_global_take(const EngineArgs& a, int lane, unsigned* g) {
     // Look before queueing for the lock: a ticket only while the stack holds
     // more entries than there are warps in line (a ticket lock serves in
@@ -376,7 +478,7 @@ __device__ inline int mutex_global_take(const EngineArgs& a, int lane, unsigned*
             outcome = 1;
         } else {
             if (top > 0) {
-                n = max(top / (int)gridDim.x, 1);
+                n = max(top / (int)gridDim.x, 1 + (SHARED ? *(volatile int*)&s_cq.waiting : 0));
                 n = n > kMutexBatch ? kMutexBatch : n;
                 n = n > top ? top : n;
                 base = top - n;
@@ -422,7 +524,7 @@ __device__ inline int mutex_global_take(const EngineArgs& a, int lane, unsigned*
     __ballot_sync(FULL, mine == ~0u);
     if (lane == 0) mutex_unlock(a, ticket, base);
     *g = __shfl_sync(FULL, mine, 0);
-    cta_push(a, lane >= 1 && lane < n, mine, lane, true);
+    cta_push<SHARED>(a, lane >= 1 && lane < n, mine, lane, true);
     return 0;
 }
 
@@ -433,17 +535,20 @@ __device__ __forceinline__ bool names_a_tile(const EngineArgs& a, int lane, unsi
     return false;
 }
 
-// The queues, as the CTA's first warp works them: get() finds the next entry
-// (false when the job is over or failed), done() counts it finished after its
-// visit and those of the neighbours that the CTA went on to.
+// The queues, as a CTA's first warp works them, or each of the WORKERS warps of
+// one where a warp visits a tile alone: get() finds the next entry (false when
+// the job is over or failed), done() counts it finished after its visit and
+// those of the neighbours that the worker went on to.
 
 // One persistent launch.  The next entry comes from the CTA's buffer; when
 // that is empty, a batch is taken from the global LIFO stack
 // (mutex_global_take).  Termination: nothing is stacked and no inserted entry
 // is unfinished (`pending` == 0, buffered entries included), which replaces
 // activeBlocksCount (IWPP MP/src/globalQueue.cu:134-145).
+template <int WORKERS>
 struct MutexQueue {
     static constexpr int VAR = VAR_MUTEX;
+    static constexpr bool SHARED = WORKERS > 1;
     unsigned* wq = nullptr;
     unsigned ns = 64;
 
@@ -451,11 +556,19 @@ struct MutexQueue {
     // the stack's top, and `pending` counts it already); the lowest position
     // ends on the buffer's top, so it is taken first, as from the stack
     __device__ void start(const EngineArgs& a, int lane) {
-        const unsigned pf = ld_volatile(&a.ctrl->prefill);
-        const unsigned base = ld_volatile(&a.ctrl->prefill_base) + blockIdx.x * pf;
-        for (unsigned j = (unsigned)lane; j < pf; j += 32u) s_cq.e[j] = __ldcg(&a.q0[base + pf - 1u - j]);
-        if (lane == 0) s_cq.n = (int)pf;
-        __syncwarp();
+        if (!SHARED || threadIdx.x < 32) {
+            const unsigned pf = ld_volatile(&a.ctrl->prefill);
+            const unsigned base = ld_volatile(&a.ctrl->prefill_base) + blockIdx.x * pf;
+            for (unsigned j = (unsigned)lane; j < pf; j += 32u) s_cq.e[j] = __ldcg(&a.q0[base + pf - 1u - j]);
+            if (lane == 0) {
+                s_cq.n = (int)pf;
+                s_cq.lock = s_cq.taker = s_cq.waiting = 0;
+            }
+        }
+        if (SHARED)
+            __syncthreads();
+        else
+            __syncwarp();
     }
     __device__ bool get(const EngineArgs& a, int lane, unsigned* out) {
         long long idle_since = 0;
@@ -464,8 +577,23 @@ struct MutexQueue {
         ns = 64;
         for (;;) {
             if (ld_volatile(&a.ctrl->error) != 0u) break;
-            unsigned g = cta_take(lane);
-            const int outcome = g != ~0u ? 0 : mutex_global_take(a, lane, &g);
+            unsigned g = cta_take<SHARED>(a, lane);
+            int outcome = 0;
+            if (g == ~0u) {
+                int taker = 1;
+                if (SHARED) taker = __shfl_sync(FULL, lane == 0 ? atomicCAS(&s_cq.taker, 0, 1) == 0 : 0, 0);
+                if (taker) {
+                    outcome = mutex_global_take<SHARED>(a, lane, &g);
+                    __syncwarp();
+                    if (SHARED && lane == 0) atomicExch(&s_cq.taker, 0);
+                } else {
+                    // another warp of this CTA is at the global stack: wait for
+                    // its batch, leaving when the job is over
+                    const bool over = ld_volatile(&a.ctrl->pending) == 0 && stack_top(a.ctrl) == 0 &&
+                                      ld_volatile(&a.ctrl->overflow) == 0u;
+                    outcome = __shfl_sync(FULL, over ? 1 : 2, 0);
+                }
+            }
             if (outcome == 1) break;
             if (outcome == 0) {
                 got = names_a_tile(a, lane, g);
@@ -473,7 +601,10 @@ struct MutexQueue {
                 break;
             }
             // nothing to take but work in flight: back off, bounded by progress
-            if (!idle && lane == 0) atomicAdd(&a.ctrl->idle, 1u);
+            if (!idle && lane == 0) {
+                atomicAdd(&a.ctrl->idle, 1u);
+                if (SHARED) atomicAdd(&s_cq.waiting, 1);
+            }
             idle = true;
             const unsigned prog = ld_volatile(&a.ctrl->progress);
             const long long now = globaltimer_ns();
@@ -487,7 +618,10 @@ struct MutexQueue {
             __nanosleep(ns);
             if (ns < 2048) ns <<= 1;
         }
-        if (idle && lane == 0) atomicSub(&a.ctrl->idle, 1u);
+        if (idle && lane == 0) {
+            atomicSub(&a.ctrl->idle, 1u);
+            if (SHARED) atomicSub(&s_cq.waiting, 1);
+        }
         return __shfl_sync(FULL, got ? 1 : 0, 0) != 0;
     }
     __device__ void done(const EngineArgs& a, int lane) {
@@ -497,8 +631,10 @@ struct MutexQueue {
         }
         // share: the global stack is empty while CTAs elsewhere wait
         int share = 0;
-        if (lane == 0 && cq_count() >= 2 && stack_top(a.ctrl) == 0 && ld_volatile(&a.ctrl->idle) > 0u) share = 1;
-        if (__shfl_sync(FULL, share, 0)) cta_spill(a, lane, cq_count() / 2);
+        if (lane == 0 && cq_count() >= 2 && stack_top(a.ctrl) == 0 &&
+            ld_volatile(&a.ctrl->idle) > (SHARED ? (unsigned)*(volatile int*)&s_cq.waiting : 0u))
+            share = 1;
+        if (__shfl_sync(FULL, share, 0)) cta_spill<SHARED>(a, lane, __shfl_sync(FULL, cq_count(), 0) / 2);
     }
 };
 
@@ -583,26 +719,27 @@ struct AsyncQueue {
         if (!__shfl_sync(FULL, last, 0)) return;
         from = __shfl_sync(FULL, from, 0);
         to = __shfl_sync(FULL, to, 0);
-        // at most one claimed position per CTA of the grid, fewer than `cap`
+        // at most one claimed position per worker of the grid, fewer than `cap`
         for (unsigned p = from + (unsigned)lane; (int)(to - p) > 0; p += 32u)
             *(volatile unsigned*)&a.q0[(p - n0) % a.cap] = kRingEnd;
     }
 };
 
 // --------------------------------------------------------- grid barrier
-// All CTAs of the (cooperative) launch.  The last CTA to arrive performs the
+// All workers of the (cooperative) launch.  The last one to arrive performs the
 // round transition.  Waits are bounded; returns false when the job failed.
+template <int WORKERS>
 __device__ inline bool grid_barrier_round(const EngineArgs& a) {
     int ok = 1;
     __syncwarp();
-    if (threadIdx.x == 0) {
+    if ((threadIdx.x & 31) == 0) {
         Ctrl* c = a.ctrl;
         const unsigned gen = ld_volatile(&c->bar_gen);
         __threadfence();
         const unsigned arrived = atomicAdd(&c->bar_count, 1u);
-        // (with the phantom-work test hook the barrier waits for one CTA
+        // (with the phantom-work test hook the barrier waits for one worker
         // more than the grid has, so every waiter runs out of time)
-        if (arrived == gridDim.x - 1u + (a.phantom ? 1u : 0u)) {
+        if (arrived == gridDim.x * WORKERS - 1u + (a.phantom ? 1u : 0u)) {
             // Round transition (IWPP MP DQ/src/globalQueue.cu:139-157 swapQueues,
             // UQ/src/globalQueue.cu:159-168 resetReadQueue, and the overflow
             // restart of DQ/MR.cu:1242-1323, all on the device).
@@ -655,7 +792,7 @@ __device__ inline bool grid_barrier_round(const EngineArgs& a) {
 }
 
 // ------------------------------------------------------- round queues
-template <int V>
+template <int V, int WORKERS>
 struct RoundQueue {
     static constexpr int VAR = V;
     unsigned* wq = nullptr;
@@ -675,7 +812,7 @@ struct RoundQueue {
                 *out = vfull ? idx : __ldcg(&(wq == a.q0 ? a.q1 : a.q0)[idx]);
                 return names_a_tile(a, lane, *out);
             }
-            if (!grid_barrier_round(a)) return false;
+            if (!grid_barrier_round<WORKERS>(a)) return false;
             if (ld_volatile(&a.ctrl->done) != 0u) return false;
             start(a, lane);
         }
@@ -683,37 +820,44 @@ struct RoundQueue {
     __device__ void done(const EngineArgs&, int) {}
 };
 
-template <int VAR>
+template <int VAR, int WORKERS>
 struct QueueOf {
-    using T = RoundQueue<VAR>;
+    using T = RoundQueue<VAR, WORKERS>;
 };
-template <>
-struct QueueOf<VAR_MUTEX> {
-    using T = MutexQueue;
+template <int WORKERS>
+struct QueueOf<VAR_MUTEX, WORKERS> {
+    using T = MutexQueue<WORKERS>;
 };
-template <>
-struct QueueOf<VAR_ASYNC> {
+template <int WORKERS>
+struct QueueOf<VAR_ASYNC, WORKERS> {
     using T = AsyncQueue;
 };
 
 // --------------------------------------------------------------- kernels
 // A CTA of W warps works on one tile at a time.  Its first warp runs the
-// queue and hands the tile to the CTA's warps through shared memory.  ALT:
-// the kernels with the alternative in-tile solvers, apart so that their
-// registers and code cost the passes nothing.  Registers: 24 warps per SM (80
-// registers) with four and eight warps per tile, 20 (96) with two, whose loop
-// over a warp's blocks needs them; 16 and 32 warps measured the same or
-// slower (32: a fifth slower, spills).
-template <int VAR, int TH, int W, bool ALT, int CONN>
-__global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
+// queue and hands the tile to the CTA's warps through shared memory.  The
+// kernels with the alternative in-tile solvers, apart so that their registers
+// and code cost the passes nothing, have WORKERS warps that each work on a
+// tile of their own (W 1).  Registers: 24 warps per SM (80 registers) with four
+// and eight warps per tile, 20 (96) with two, whose loop over a warp's blocks
+// needs them; 16 and 32 warps measured the same or slower (32: a fifth slower,
+// spills); 12 (168) with one.
+constexpr int kAltWorkers = 4;
+
+template <int VAR, int TH, int W, int SOLVE, int CONN>
+__global__ void __launch_bounds__(SOLVE == SOLVE_PASSES ? 32 * W : 32 * kAltWorkers,
+                                  SOLVE != SOLVE_PASSES ? 12 / kAltWorkers : W == 2 ? 10 : 24 / W)
     engine_kernel(const __grid_constant__ EngineArgs a) {
+    constexpr int WORKERS = SOLVE == SOLVE_PASSES ? 1 : kAltWorkers;
+    static_assert(WORKERS == 1 || W == 1, "several workers: a warp each");
     extern __shared__ __align__(128) unsigned char smem_raw[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // 128-byte align the tile (the launch adds 128 bytes of slack)
+    const int lane = threadIdx.x & 31;
+    const int worker = WORKERS > 1 ? threadIdx.x >> 5 : 0, warp = WORKERS > 1 ? 0 : threadIdx.x >> 5;
+    // 128-byte align the tiles (the launch adds 128 bytes of slack)
     const uint32_t base = smem_u32(smem_raw);
-    using Smem = typename SmemOf<TH, ALT>::T;
-    Smem& sm = *reinterpret_cast<Smem*>(smem_raw + ((128u - (base & 127u)) & 127u));
-    if (threadIdx.x == 0) {
+    using Smem = typename SmemOf<TH, W, SOLVE>::T;
+    Smem& sm = reinterpret_cast<Smem*>(smem_raw + ((128u - (base & 127u)) & 127u))[worker];
+    if (warp == 0 && lane == 0) {
         mbar_init(&sm.mbar, 1u);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         sm.nb = 0u;
@@ -725,10 +869,12 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
             sm.d = a.imgs[0];
         }
     }
-    if (lane == 0) sm.mark[0][warp][0] = sm.mark[0][warp][1] = sm.mark[1][warp][0] = sm.mark[1][warp][1] = 0u;
+    if constexpr (SOLVE == SOLVE_PASSES) {
+        if (lane == 0) sm.mark[0][warp][0] = sm.mark[0][warp][1] = sm.mark[1][warp][0] = sm.mark[1][warp][1] = 0u;
+    }
     cta_sync<W>();
     unsigned phase = 0u, row_steps = 0u;
-    typename QueueOf<VAR>::T queue;
+    typename QueueOf<VAR, WORKERS>::T queue;
     if (warp == 0) queue.start(a, lane);
     bool visited = false;  // first warp: tile g was visited
     unsigned g = 0u;
@@ -747,7 +893,8 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
                 // that ended the visit.
                 if (nb & NB_STORED) fence_gpu();
                 int pushed = 0;
-                const unsigned cont = leave_tile<VAR>(a, sm.d, sm.tx, sm.ty, g, nb, lane, queue.wq, &pushed);
+                const unsigned cont =
+                    leave_tile<VAR, (WORKERS > 1)>(a, sm.d, sm.tx, sm.ty, g, nb, lane, queue.wq, &pushed);
                 if (lane == 0) {
                     sm.count.cycles[4] += clock64() - q0;
                     sm.count.visits += 1u;
@@ -772,7 +919,8 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
                     bool again = false;
                     if (lane == 0) again = (atomicAnd(&a.state[g], ~ST_ACTIVE) & ST_DIRTY) != 0u;
                     const int pushed =
-                        VAR == VAR_MUTEX ? cta_push(a, again, g, lane) : push_entries<VAR>(a, again, g, lane, queue.wq);
+                        VAR == VAR_MUTEX ? cta_push<(WORKERS > 1)>(a, again, g, lane)
+                                         : push_entries<VAR>(a, again, g, lane, queue.wq);
                     if (lane == 0) sm.count.pushes += (unsigned)pushed;
                 }
                 queue.done(a, lane);
@@ -802,8 +950,9 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
         }
         cta_sync<W>();
         if (sm.go == 0u) break;
-        if (!dispatch_visit<CONN, TH, W, ALT>(a, sm, warp, lane, phase, row_steps)) {
-            if (threadIdx.x == 0) set_error(a.ctrl, DEV_ERR_TIMEOUT);
+        EarlyFlush<VAR> early{a, sm.d, sm.tx, sm.ty, sm.count.pushes, (int)(gridDim.x * WORKERS / 2u)};
+        if (!dispatch_visit<CONN, TH, W, SOLVE>(a, sm, warp, lane, phase, row_steps, early)) {
+            if (warp == 0 && lane == 0) set_error(a.ctrl, DEV_ERR_TIMEOUT);
             break;
         }
     }
@@ -822,29 +971,34 @@ __global__ void __launch_bounds__(32 * W, ALT ? 12 : W == 2 ? 10 : 24 / W)
 
 template <int VAR, int CONN>
 void* kernel_for(int tile_rows, int warps) {
-    if (tile_rows == 32) return reinterpret_cast<void*>(&engine_kernel<VAR, 32, 4, false, CONN>);
-    if (warps == 8) return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 8, false, CONN>);
-    if (warps == 4) return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 4, false, CONN>);
-    return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 2, false, CONN>);
+    if (tile_rows == 32) return reinterpret_cast<void*>(&engine_kernel<VAR, 32, 4, SOLVE_PASSES, CONN>);
+    if (warps == 8) return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 8, SOLVE_PASSES, CONN>);
+    if (warps == 4) return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 4, SOLVE_PASSES, CONN>);
+    return reinterpret_cast<void*>(&engine_kernel<VAR, 64, 2, SOLVE_PASSES, CONN>);
 }
 
-// The kernel of a queue for tiles of a shape and images of one connectivity
-// (4, 8) or of both (0).
+template <int VAR, int SOLVE>
+void* kernel_for(int tile_rows) {
+    return tile_rows == 32 ? reinterpret_cast<void*>(&engine_kernel<VAR, 32, 1, SOLVE, 0>)
+                           : reinterpret_cast<void*>(&engine_kernel<VAR, 64, 1, SOLVE, 0>);
+}
+
+// The kernel of a queue and an in-tile solver (SOLVE_*) for tiles of a shape and
+// images of one connectivity (4, 8) or of both (0).
 template <int VAR>
-void* kernel_for(int tile_rows, int warps, bool alt, int conn) {
-    if (alt)
-        return tile_rows == 32 ? reinterpret_cast<void*>(&engine_kernel<VAR, 32, 1, true, 0>)
-                               : reinterpret_cast<void*>(&engine_kernel<VAR, 64, 1, true, 0>);
-    return conn == 4   ? kernel_for<VAR, 4>(tile_rows, warps)
-           : conn == 8 ? kernel_for<VAR, 8>(tile_rows, warps)
-                       : kernel_for<VAR, 0>(tile_rows, warps);
+void* kernel_for(int tile_rows, int warps, int solve, int conn) {
+    return solve == SOLVE_SWEEPS ? kernel_for<VAR, SOLVE_SWEEPS>(tile_rows)
+           : solve == SOLVE_PQ   ? kernel_for<VAR, SOLVE_PQ>(tile_rows)
+           : conn == 4           ? kernel_for<VAR, 4>(tile_rows, warps)
+           : conn == 8           ? kernel_for<VAR, 8>(tile_rows, warps)
+                                 : kernel_for<VAR, 0>(tile_rows, warps);
 }
 
 // Each queue's kernels are a translation unit of their own
 // (iwpp_engine_{mutex,double,unique,async}.cu): they take long to compile.
-extern template void* kernel_for<VAR_MUTEX>(int, int, bool, int);
-extern template void* kernel_for<VAR_DOUBLE>(int, int, bool, int);
-extern template void* kernel_for<VAR_UNIQUE>(int, int, bool, int);
-extern template void* kernel_for<VAR_ASYNC>(int, int, bool, int);
+extern template void* kernel_for<VAR_MUTEX>(int, int, int, int);
+extern template void* kernel_for<VAR_DOUBLE>(int, int, int, int);
+extern template void* kernel_for<VAR_UNIQUE>(int, int, int, int);
+extern template void* kernel_for<VAR_ASYNC>(int, int, int, int);
 
 }  // namespace iwpp

@@ -49,6 +49,7 @@ cudaError_t cudaFuncGetAttributes(cudaFuncAttributes* a, const void* fn) {
     g_loaded.insert(fn);
     return cudaSuccess;
 }
+cudaError_t cudaFuncSetAttribute(const void*, cudaFuncAttribute, int) { return cudaSuccess; }
 cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags(int* n, const void* fn, int, size_t, unsigned) {
     *n = 3;
     g_loaded.insert(fn);
