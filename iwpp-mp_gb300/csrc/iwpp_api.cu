@@ -161,8 +161,9 @@ long long tiles_of(int w, int h, int dtype, int th) {
 // two warps).  The mutex queue is bound by its one lock (every take and insert
 // is a critical section), so its cost grows with the tile count: 64 rows always.
 // The other solvers have one warp per tile: 32 rows below 2.5 64-row tiles per
-// warp that the grid keeps resident, 12 per SM.
-int default_tile_rows(int variant, int solver, long long tiles64) {
+// warp that the grid keeps resident, 12 per SM.  A grid that the caller limits
+// to fewer CTAs than there are 64-row tiles leaves no SM that it uses without one.
+int default_tile_rows(int variant, int solver, long long tiles64, int grid_ctas = 0) {
     if (variant == IWPP_QUEUE_MUTEX) return 64;
     int device = -1;
     if (cudaGetDevice(&device) != cudaSuccess) {
@@ -171,7 +172,7 @@ int default_tile_rows(int variant, int solver, long long tiles64) {
     }
     const int sms = engine_sm_count(device);
     if (solver == 1 || solver == 3) return tiles64 < 30ll * sms ? 32 : 64;
-    return tiles64 <= sms ? 32 : 64;
+    return tiles64 <= (grid_ctas > 0 ? std::min(grid_ctas, sms) : sms) ? 32 : 64;
 }
 
 long long job_tiles64(const iwpp_image* imgs, int n) {
@@ -396,7 +397,10 @@ int build_job(Job& job, const iwpp_image* imgs, int n, int variant, const iwpp_c
         job.cfg.front_passes = largest >= kFrontDefaultPixels ? 3 : 2;
     }
     int th = job.cfg.tile_rows;
-    if (th == 0) th = n > 0 ? default_tile_rows(job.variant, job.cfg.solver, job_tiles64(imgs, n)) : 64;
+    if (th == 0 && n > 0)
+        th = default_tile_rows(job.variant, job.cfg.solver, job_tiles64(imgs, n), job.cfg.grid_ctas);
+    else if (th == 0)
+        th = 64;
     job.tile_rows = th;
     long long G = 0;
     for (int i = 0; i < n; ++i) {
@@ -785,7 +789,8 @@ int enqueue_job(const Job& job, Workspace& ws, cudaStream_t s, int device, bool 
     long long grid = 1;
     LaunchInfo li{};
     if (job.G > 0) {
-        e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, device, &li);
+        e = engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, job.cfg.grid_ctas, device,
+                           &li);
         if (e != cudaSuccess) return cuda_status(e);
         grid = li.grid;
         grid = std::min(grid, (job.G + li.workers - 1) / li.workers);
@@ -1114,7 +1119,8 @@ int iwpp_plan_create(iwpp_plan* out, iwpp_handle h, const iwpp_image* images, in
         LaunchInfo li;
         if (rc == IWPP_OK && job.G > 0)
             rc = cuda_status(
-                engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, h->device, &li));
+                engine_prepare(job.variant, job.tile_rows, job.cfg.solver, job_conn(job), job.G, job.cfg.grid_ctas,
+                               h->device, &li));
     }
     if (rc == IWPP_OK) {
         e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);

@@ -192,11 +192,16 @@ enum Shape : int { T32_W4, T64_W8, T64_W4, T64_W2, T32_SWEEPS, T64_SWEEPS, T32_P
 //                 13.5 (4096^2 u8)  195 / 152 / 144, 8-connected 366 / 331 / 322
 //                 30   (6144^2 u8)  400 / 298 / 256
 //                 54   (8192^2 u8)  791 / 561 / 453
-static Shape select_shape(int tile_rows, int solver, long long tiles, int sms) {
+// A grid that the caller limits (grid_ctas > 0) works on that many tiles at
+// most, with as many warps per tile as leave that many CTAs resident.  4096^2 u8
+// 8-connected h-domes, us, by the rule for the tiles alone / so: 8 CTAs 13132 /
+// 9158, 38 2990 / 2082, 304 488 / 394.
+static Shape select_shape(int tile_rows, int solver, long long tiles, int grid_ctas, int sms) {
     if (solver == 1) return tile_rows == 32 ? T32_SWEEPS : T64_SWEEPS;
     if (solver == 3) return tile_rows == 32 ? T32_PQ : T64_PQ;
     if (tile_rows == 32) return T32_W4;
-    return 4 * tiles <= 27ll * sms ? T64_W8 : 2 * tiles <= 25ll * sms ? T64_W4 : T64_W2;
+    if (4 * tiles <= 27ll * sms || (grid_ctas > 0 && grid_ctas <= 3ll * sms)) return T64_W8;
+    return 2 * tiles <= 25ll * sms || (grid_ctas > 0 && grid_ctas <= 6ll * sms) ? T64_W4 : T64_W2;
 }
 
 struct Kernel {
@@ -265,11 +270,11 @@ static cudaError_t resident_ctas(int variant, Shape shape, int conn, int device,
     return e;
 }
 
-cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int device,
-                           LaunchInfo* li) {
+cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int grid_ctas,
+                           int device, LaunchInfo* li) {
     const int sms = engine_sm_count(device);
     if (sms <= 0 || variant < 0 || variant > 3 || conn < 0 || conn > 8) return cudaErrorInvalidValue;
-    const Shape shape = select_shape(tile_rows, solver, tiles, sms);
+    const Shape shape = select_shape(tile_rows, solver, tiles, grid_ctas, sms);
     int per_sm = 0;
     const cudaError_t e = resident_ctas(variant, shape, conn, device, &per_sm);
     if (e != cudaSuccess) return e;

@@ -141,9 +141,10 @@ struct LaunchInfo {
 };
 int engine_sm_count(int device);
 // The kernel for a job of `tiles` tiles and its resident grid.  conn: the
-// images' connectivity, 0 where they mix them.
-cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int device,
-                           LaunchInfo* li);
+// images' connectivity, 0 where they mix them; grid_ctas: the caller's limit on
+// the grid, 0 for none.
+cudaError_t engine_prepare(int variant, int tile_rows, int solver, int conn, long long tiles, int grid_ctas,
+                           int device, LaunchInfo* li);
 // Loads every kernel that engine_prepare can choose for one-image jobs with
 // tiles of this height and the default solver.
 cudaError_t engine_load(int variant, int tile_rows, int device);

@@ -105,7 +105,7 @@ extern "C" int iwpp_reconstruct_noalloc(void* marker, const void* mask, size_t p
     int rc = device_setup(device, &base);
     if (rc != IWPP_OK) return rc;
     LaunchInfo li;
-    if (engine_prepare(VAR_ASYNC, kNoallocTileRows, 0, connectivity, G, device, &li) != cudaSuccess) {
+    if (engine_prepare(VAR_ASYNC, kNoallocTileRows, 0, connectivity, G, 0, device, &li) != cudaSuccess) {
         cudaGetLastError();
         return IWPP_ERR_CUDA;
     }
