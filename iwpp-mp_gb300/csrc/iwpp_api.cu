@@ -1518,7 +1518,7 @@ int iwpp_sweep(void* marker, const void* mask, size_t pitch_marker, size_t pitch
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto sweep = [&](const ImgDesc& d) {
         void* scratch = nullptr;
-        const size_t sb = sweep_scratch_bytes(d);
+        const size_t sb = direction == 1 || direction == 3 ? sweep_scratch_bytes(d) : 0;
         if (sb > 0 && cudaMallocAsync(&scratch, sb, s) != cudaSuccess) {
             cudaGetLastError();
             scratch = nullptr;  // one warp per whole column instead

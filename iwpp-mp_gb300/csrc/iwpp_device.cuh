@@ -238,18 +238,9 @@ __device__ __forceinline__ void cp_async_4(void* smem_dst, const void* src) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Global-memory flag accesses with acquire / release ordering at GPU scope.
-__device__ __forceinline__ unsigned ld_acquire(const unsigned* p) {
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
 // acquire / release fence at GPU scope (cheaper than __threadfence, which is
 // sequentially consistent)
 __device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ void st_release(unsigned* p, unsigned v) {
-    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
 
 __device__ __forceinline__ long long globaltimer_ns() {
     long long t;
@@ -257,27 +248,14 @@ __device__ __forceinline__ long long globaltimer_ns() {
     return t;
 }
 
-// ------------------------------------------------ packed-word min / max
-// Per-pixel max / min of two packed words (uint8: four bytes, uint16: two
-// halves, int32: one signed value), and whether some pixel of a is above
-// the same pixel of b.
+// ------------------------------------------------------ packed-word max
+// Per-pixel max of two packed words (uint8: four bytes, uint16: two halves,
+// int32: one signed value).
 template <int DT>
 __device__ __forceinline__ uint32_t word_max(uint32_t a, uint32_t b) {
     if (DT == DT_U8) return __vmaxu4(a, b);
     if (DT == DT_U16) return __vmaxu2(a, b);
     return (uint32_t)max((int)a, (int)b);
-}
-template <int DT>
-__device__ __forceinline__ uint32_t word_min(uint32_t a, uint32_t b) {
-    if (DT == DT_U8) return __vminu4(a, b);
-    if (DT == DT_U16) return __vminu2(a, b);
-    return (uint32_t)min((int)a, (int)b);
-}
-template <int DT>
-__device__ __forceinline__ bool word_any_gt(uint32_t a, uint32_t b) {
-    if (DT == DT_U8) return __vcmpgtu4(a, b) != 0u;
-    if (DT == DT_U16) return __vcmpgtu2(a, b) != 0u;
-    return (int)a > (int)b;
 }
 
 // ------------------------------------------------ clamp-map scan steps
@@ -1246,17 +1224,10 @@ __device__ __forceinline__ bool fetch_tile(const ImgDesc& d, int tx, int ty, Til
 #pragma unroll
         for (int i = 0; i < BPW; ++i) v[i] = halo(8 * (BPW * warp + i) + 1 + j);
         const int corner = warp == 0 && j == 0 ? 0 : warp == W - 1 && j == 7 ? TH + 1 : -1;
-        int corner2 = -1;
-        uint32_t vc2 = 0u;
         if (corner >= 0) vc = halo(corner);
-        if (W == 1 && j == 7) {
-            corner2 = TH + 1;
-            vc2 = halo(corner2);
-        }
 #pragma unroll
         for (int i = 0; i < BPW; ++i) h[8 * (BPW * warp + i) + 1 + j] = v[i];
         if (corner >= 0) h[corner] = vc;
-        if (corner2 >= 0) h[corner2] = vc2;
     }
     if (tma) {
         // bounded wait for the box loads

@@ -743,18 +743,13 @@ __global__ void __launch_bounds__(32) sweep_strip_settle_kernel(ImgDesc d, int s
     }
 }
 
-// Vertical sweep for 4-connectivity, int32 (the whole-image init passes use
-// the 4-connected vertical sweeps for either connectivity: the pixel above /
-// below alone is a valid update).  One pixel per lane, 128-byte strips,
-// segments and modes as in sweep_y4n_kernel below.
-template <bool DOWN, int MODE>
-__global__ void __launch_bounds__(32) sweep_y4i_kernel(ImgDesc d, uint32_t* seg_a, uint32_t* seg_b,
-                                                       const uint32_t* seg_in);
-
 constexpr int kRingN = 64;  // rows in flight per plane in the narrow variant
 
-// Narrow variant for uint8 / uint16: a warp covers a 64-byte strip, two
-// bytes per lane (uint8: two pixels as one u16x2 register; uint16: one
+// Vertical sweeps for 4-connectivity (the whole-image init passes use them for
+// either connectivity: the pixel above / below alone is a valid update), rows
+// of whole strips on 16-byte boundaries (by_strips takes the others).
+//
+// uint8 / uint16: a warp covers a 64-byte strip, two bytes per lane (uint8: two pixels as one u16x2 register; uint16: one
 // pixel), so the chain per row is one min and one max, and twice as many
 // warps share the image.
 //
@@ -773,15 +768,12 @@ __global__ void __launch_bounds__(32) sweep_y4n_kernel(ImgDesc d, uint32_t* seg_
                                                        const uint32_t* seg_in) {
     if (gated_off(d)) return;
     static_assert(DT == DT_U8 || DT == DT_U16, "two-byte lanes");
-    using P = Px<DT>;
     constexpr int NR = kRingN, NG = kRingN / kGroup;
     __shared__ __align__(16) uint16_t ring_m[kRingN][32];
     __shared__ __align__(16) uint16_t ring_k[kRingN][32];
     const int lane = threadIdx.x & 31;
     const int strip = (int)blockIdx.x;
-    const long long row_bytes = (long long)d.W * P::BPP;
-    const long long b0 = (long long)strip * 64 + lane * 2;  // this lane's first byte in a row
-    const long long nbytes = row_bytes - b0;                 // >= 2: whole element, 1: half, <= 0: none
+    const long long b0 = (long long)strip * 64 + lane * 2;  // this lane's bytes in a row
     // rows (in sweep order) of this block's segment
     const int i0 = MODE == 0 ? 0 : (int)blockIdx.y * kSegRows;
     const int H = MODE == 0 ? d.H : min(kSegRows, d.H - i0);
@@ -789,38 +781,14 @@ __global__ void __launch_bounds__(32) sweep_y4n_kernel(ImgDesc d, uint32_t* seg_
     const long long step_m = DOWN ? d.pitch_m : -d.pitch_m, step_k = DOWN ? d.pitch_k : -d.pitch_k;
     const unsigned char* m0 = d.marker + (size_t)(DOWN ? 0 : d.H - 1) * d.pitch_m + (long long)i0 * step_m;
     const unsigned char* k0 = d.mask + (size_t)(DOWN ? 0 : d.H - 1) * d.pitch_k + (long long)i0 * step_k;
-    const bool wide = (long long)(strip + 1) * 64 <= row_bytes &&
-                      ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
-                      ((d.pitch_m | d.pitch_k) & 15) == 0;
+    // 4 pieces of 16 bytes per row and plane, 8 rows per instruction
     auto issue_group = [&](int g0) {
-        if (wide) {  // 4 pieces of 16 bytes per row and plane, 8 rows per instruction
-            const int piece = lane & 3;
-            const int rr = lane >> 2;
-            const int i = g0 + rr;
-            if (i < H) {
-                const int slot = i % NR;
-                const long long o = (long long)strip * 64 + piece * 16;
-                cp_async16(&ring_m[slot][piece * 8], m0 + (long long)i * step_m + o);
-                cp_async16(&ring_k[slot][piece * 8], k0 + (long long)i * step_k + o);
-            }
-        } else {
-            for (int q = 0; q < kGroup; ++q) {
-                const int i = g0 + q;
-                if (i >= H) break;
-                const int slot = i % NR;
-                const unsigned char* mrow = m0 + (long long)i * step_m + (nbytes > 0 ? b0 : 0);
-                const unsigned char* krow = k0 + (long long)i * step_k + (nbytes > 0 ? b0 : 0);
-                uint16_t mv = 0, kv = 0;
-                if (nbytes >= 2) {
-                    mv = *reinterpret_cast<const uint16_t*>(mrow);
-                    kv = *reinterpret_cast<const uint16_t*>(krow);
-                } else if (nbytes == 1) {  // uint8 only: the last pixel of the row
-                    mv = *mrow;
-                    kv = *krow;
-                }
-                ring_m[slot][lane] = mv;
-                ring_k[slot][lane] = kv;
-            }
+        const int piece = lane & 3, i = g0 + (lane >> 2);
+        if (i < H) {
+            const int slot = i % NR;
+            const long long o = (long long)strip * 64 + piece * 16;
+            cp_async16(&ring_m[slot][piece * 8], m0 + (long long)i * step_m + o);
+            cp_async16(&ring_k[slot][piece * 8], k0 + (long long)i * step_k + o);
         }
     };
     for (int g = 0; g < NG; ++g) {
@@ -829,7 +797,7 @@ __global__ void __launch_bounds__(32) sweep_y4n_kernel(ImgDesc d, uint32_t* seg_
     }
     uint32_t prev = MODE == 2 ? seg_in[seg_idx] : 0u;
     uint32_t kmin = DT == DT_U8 ? 0x00ff00ffu : 0xffffu;
-    unsigned char* mo = const_cast<unsigned char*>(m0) + (nbytes > 0 ? b0 : 0);
+    unsigned char* mo = const_cast<unsigned char*>(m0) + b0;
     for (int base = 0; base < H; base += kGroup) {
         cp_async_wait<NG - 1>();
         __syncwarp();
@@ -869,16 +837,10 @@ __global__ void __launch_bounds__(32) sweep_y4n_kernel(ImgDesc d, uint32_t* seg_
         if (MODE != 1) {
             // only the elements that rose are stored: an unchanged store
             // would still dirty its L2 sector and cost a DRAM write-back
-            if (nbytes >= 2) {
 #pragma unroll
-                for (int q = 0; q < kGroup; ++q)
-                    if (base + q < H && out[q] != orig[q])
-                        *reinterpret_cast<uint16_t*>(mo + (long long)(base + q) * step_m) = (uint16_t)out[q];
-            } else if (nbytes == 1) {
-                for (int q = 0; q < kGroup; ++q)
-                    if (base + q < H && (out[q] & 0xffu) != (orig[q] & 0xffu))
-                        *(mo + (long long)(base + q) * step_m) = (unsigned char)out[q];
-            }
+            for (int q = 0; q < kGroup; ++q)
+                if (base + q < H && out[q] != orig[q])
+                    *reinterpret_cast<uint16_t*>(mo + (long long)(base + q) * step_m) = (uint16_t)out[q];
         }
         __syncwarp();
         issue_group(base + NR);
@@ -891,51 +853,32 @@ __global__ void __launch_bounds__(32) sweep_y4n_kernel(ImgDesc d, uint32_t* seg_
     }
 }
 
-template <bool DOWN, int MODE>
-__global__ void __launch_bounds__(32) sweep_y4i_kernel(ImgDesc d, uint32_t* seg_a, uint32_t* seg_b,
-                                                       const uint32_t* seg_in) {
+// int32: one pixel per lane, 128-byte strips, a warp each over the whole
+// height.  Not in segments: at four bytes a pixel the two extra plane reads cost
+// more than the parallelism gains (its strips already give 512 warps on a
+// 16384-wide image).
+template <bool DOWN>
+__global__ void __launch_bounds__(32) sweep_y4i_kernel(ImgDesc d) {
     if (gated_off(d)) return;
     constexpr int NG = kRing / kGroup;
     __shared__ __align__(16) uint32_t ring_m[kRing][32];
     __shared__ __align__(16) uint32_t ring_k[kRing][32];
     const int lane = threadIdx.x & 31;
-    const int strip = (int)blockIdx.x;
-    const int x = strip * 32 + lane;
-    const bool inside = x < d.W;
-    const int i0 = MODE == 0 ? 0 : (int)blockIdx.y * kSegRows;
-    const int H = MODE == 0 ? d.H : min(kSegRows, d.H - i0);
-    const size_t seg_idx = ((size_t)blockIdx.y * gridDim.x + strip) * 32 + lane;
+    const long long sbase = (long long)blockIdx.x * 128;
+    const int H = d.H;
     const long long step_m = DOWN ? d.pitch_m : -d.pitch_m, step_k = DOWN ? d.pitch_k : -d.pitch_k;
-    const unsigned char* m0 = d.marker + (size_t)(DOWN ? 0 : d.H - 1) * d.pitch_m + (long long)i0 * step_m;
-    const unsigned char* k0 = d.mask + (size_t)(DOWN ? 0 : d.H - 1) * d.pitch_k + (long long)i0 * step_k;
-    const long long sbase = (long long)strip * 128;
-    const bool wide = (long long)(strip + 1) * 32 <= (long long)d.W &&
-                      ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
-                      ((d.pitch_m | d.pitch_k) & 15) == 0;
+    unsigned char* m0 = d.marker + (size_t)(DOWN ? 0 : H - 1) * d.pitch_m + sbase;
+    const unsigned char* k0 = d.mask + (size_t)(DOWN ? 0 : H - 1) * d.pitch_k + sbase;
+    // 8 pieces of 16 bytes per row and plane, 4 rows per instruction
     auto issue_group = [&](int g0) {
-        if (wide) {  // 8 pieces of 16 bytes per row and plane, 4 rows per instruction
-            const int piece = lane & 7;
+        const int piece = lane & 7;
 #pragma unroll
-            for (int rr = 0; rr < kGroup; rr += 4) {
-                const int i = g0 + rr + (lane >> 3);
-                if (i < H) {
-                    const int slot = i % kRing;
-                    cp_async16(&ring_m[slot][piece * 4], m0 + (long long)i * step_m + sbase + piece * 16);
-                    cp_async16(&ring_k[slot][piece * 4], k0 + (long long)i * step_k + sbase + piece * 16);
-                }
-            }
-        } else {
-            for (int q = 0; q < kGroup; ++q) {
-                const int i = g0 + q;
-                if (i >= H) break;
+        for (int rr = 0; rr < kGroup; rr += 4) {
+            const int i = g0 + rr + (lane >> 3);
+            if (i < H) {
                 const int slot = i % kRing;
-                uint32_t mv = 0x80000000u, kv = 0x80000000u;
-                if (inside) {
-                    mv = *reinterpret_cast<const uint32_t*>(m0 + (long long)i * step_m + (long long)x * 4);
-                    kv = *reinterpret_cast<const uint32_t*>(k0 + (long long)i * step_k + (long long)x * 4);
-                }
-                ring_m[slot][lane] = mv;
-                ring_k[slot][lane] = kv;
+                cp_async16(&ring_m[slot][piece * 4], m0 + (long long)i * step_m + piece * 16);
+                cp_async16(&ring_k[slot][piece * 4], k0 + (long long)i * step_k + piece * 16);
             }
         }
     };
@@ -943,9 +886,8 @@ __global__ void __launch_bounds__(32) sweep_y4i_kernel(ImgDesc d, uint32_t* seg_
         issue_group(g * kGroup);
         cp_async_commit();
     }
-    int prev = MODE == 2 ? (int)seg_in[seg_idx] : INT_MIN;
-    int kmin = INT_MAX;
-    unsigned char* mo = const_cast<unsigned char*>(m0) + (long long)(inside ? x : 0) * 4;
+    int prev = INT_MIN;
+    unsigned char* mo = m0 + lane * 4;
     for (int base = 0; base < H; base += kGroup) {
         cp_async_wait<NG - 1>();
         __syncwarp();  // pieces copied by other lanes are visible to this one
@@ -954,31 +896,16 @@ __global__ void __launch_bounds__(32) sweep_y4i_kernel(ImgDesc d, uint32_t* seg_
 #pragma unroll
         for (int q = 0; q < kGroup; ++q) {
             const int m = (int)ring_m[sb + q][lane], k = (int)ring_k[sb + q][lane];
-            const int v = max(m, min(prev, k));
-            if (MODE == 1) {
-                if (base + q < H) {  // rows past the segment: stale slots
-                    prev = v;
-                    kmin = min(kmin, k);
-                }
-            } else {
-                prev = v;
-            }
-            out[q] = v;
+            out[q] = prev = max(m, min(prev, k));
         }
-        if (MODE != 1 && inside) {
 #pragma unroll
-            for (int q = 0; q < kGroup; ++q)
-                if (base + q < H) *reinterpret_cast<int*>(mo + (long long)(base + q) * step_m) = out[q];
-        }
+        for (int q = 0; q < kGroup; ++q)
+            if (base + q < H) *reinterpret_cast<int*>(mo + (long long)(base + q) * step_m) = out[q];
         __syncwarp();  // the slots just read are refilled next
         issue_group(base + kRing);
         cp_async_commit();
     }
     cp_async_wait<0>();
-    if (MODE == 1) {
-        seg_a[seg_idx] = (uint32_t)prev;
-        seg_b[seg_idx] = (uint32_t)kmin;
-    }
 }
 
 // The value entering every segment of every column: x_0 = nothing (0),
@@ -988,26 +915,38 @@ __global__ void sweep_y_carry_kernel(int nseg, int slots, const uint32_t* seg_a,
                                      uint32_t* seg_in) {
     const int t = (int)(blockIdx.x * blockDim.x + threadIdx.x);
     if (t >= slots) return;
-    uint32_t x = DT == DT_I32 ? 0x80000000u : 0u;
+    uint32_t x = 0u;
     for (int j = 0; j < nseg; ++j) {
         const size_t idx = (size_t)j * slots + t;
         seg_in[idx] = x;
         if (DT == DT_U8)
             x = __vmaxu2(__vminu2(x, seg_b[idx]), seg_a[idx]);
-        else if (DT == DT_U16)
-            x = max(min(x, seg_b[idx]), seg_a[idx]);
         else
-            x = (uint32_t)max(min((int)x, (int)seg_b[idx]), (int)seg_a[idx]);
+            x = max(min(x, seg_b[idx]), seg_a[idx]);
     }
 }
 
-// int32 is not segmented: at four bytes a pixel the two extra plane reads
-// cost more than the parallelism gains (its strips already give 512 warps
-// on a 16384-wide image).
+static bool aligned16(const ImgDesc& d) {
+    return ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
+           ((d.pitch_m | d.pitch_k) & 15) == 0;
+}
+
+// Vertical sweeps by 128-byte strips in place: 8-connected ones, and
+// 4-connected ones of rows off the 16-byte boundary or not a whole number of
+// the ring kernels' strips wide, which those would have to load element by
+// element (2000 x 768 uint8 240 us, by strips 42; 1416 x 5514 uint8 574 and
+// 54, uint16 487 and 54; 708 x 5514 int32 1640 and 33).  The others stay with
+// the ring kernels: their segments' maps compose, so a long vertical path costs
+// nothing (whole calls: 16384^2 spiral 409 us, by strips 594; 128 x 100000 sparse
+// seeds 263 and 2730).
+static bool by_strips(const ImgDesc& d) {
+    const long long row = (long long)d.W * (d.dtype == DT_U8 ? 1 : d.dtype == DT_U16 ? 2 : 4);
+    return d.conn == 8 || !aligned16(d) || row % (d.dtype == DT_I32 ? 128 : 64) != 0;
+}
+
 size_t sweep_scratch_bytes(const ImgDesc& d) {
-    if (d.conn != 4 || d.dtype == DT_I32 || d.H <= 2 * kSegRows) return 0;
-    const long long strips = d.dtype == DT_I32 ? ((long long)d.W + 31) / 32
-                                               : ((long long)d.W * (d.dtype == DT_U8 ? 1 : 2) + 63) / 64;
+    if (by_strips(d) || d.dtype == DT_I32 || d.H <= 2 * kSegRows) return 0;
+    const long long strips = (long long)d.W * (d.dtype == DT_U8 ? 1 : 2) / 64;
     const long long nseg = (d.H + kSegRows - 1) / kSegRows;
     return (size_t)(3 * nseg * strips * 32 * 4);
 }
@@ -1066,12 +1005,9 @@ template <int DT>
 static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void* scratch) {
     using P = Px<DT>;
     constexpr int TW = 32 * P::PPW;
-    const bool aligned16 =
-        ((reinterpret_cast<uintptr_t>(d.marker) | reinterpret_cast<uintptr_t>(d.mask)) & 15u) == 0u &&
-        ((d.pitch_m | d.pitch_k) & 15) == 0;
     if (direction == 0 || direction == 2) {
         const unsigned blocks = blocks_for((long long)d.H * 32, 128);
-        if (aligned16 && DT == DT_U8) {
+        if (aligned16(d) && DT == DT_U8) {
             // two rows per warp (uint16 measured no faster: its lanes hold
             // half as many pixels, so the scan is a smaller share)
             const unsigned pblocks = blocks_for((long long)((d.H + 1) / 2) * 32, 128);
@@ -1079,7 +1015,7 @@ static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void*
                 sweep_x16p_kernel<DT_U8, true><<<pblocks, 128, 0, s>>>(d);
             else
                 sweep_x16p_kernel<DT_U8, false><<<pblocks, 128, 0, s>>>(d);
-        } else if (aligned16) {
+        } else if (aligned16(d)) {
             if (direction == 0)
                 sweep_x16_kernel<DT, true><<<blocks, 128, 0, s>>>(d);
             else
@@ -1095,42 +1031,15 @@ static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void*
         const bool down = direction == 1;
         if (d.conn == 8)
             return down ? launch_strips<DT, 8, true>(d, strips, s) : launch_strips<DT, 8, false>(d, strips, s);
-        // 4-connected rows off the 16-byte boundary, or not a whole number of
-        // the ring kernels' strips wide: those kernels load what is not 16
-        // bytes element by element (2000 x 768 uint8 240 us, by strips 42;
-        // 1416 x 5514 uint8 574 and 54, uint16 487 and 54; 708 x 5514 int32
-        // 1640 and 33).  The others stay with them: their segments' maps
-        // compose, so a long vertical path costs nothing (16384^2 spiral 250
-        // us, by strips 1614; without one 250 and 222).
-        if (!aligned16 || (long long)d.W * P::BPP % (DT == DT_I32 ? 128 : 64) != 0)
+        if (by_strips(d))
             return down ? launch_strips<DT, 4, true>(d, strips, s) : launch_strips<DT, 4, false>(d, strips, s);
-        if (DT == DT_I32) {
-            const unsigned nblocks = (unsigned)((d.W + 31) / 32);
-            if (scratch && sweep_scratch_bytes(d) > 0) {
-                const int nseg = (d.H + kSegRows - 1) / kSegRows;
-                const int slots = (int)nblocks * 32;
-                uint32_t* a = static_cast<uint32_t*>(scratch);
-                uint32_t* b = a + (size_t)nseg * slots;
-                uint32_t* in = b + (size_t)nseg * slots;
-                const dim3 grid(nblocks, (unsigned)nseg);
-                if (down)
-                    sweep_y4i_kernel<true, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
-                else
-                    sweep_y4i_kernel<false, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
-                sweep_y_carry_kernel<DT_I32><<<(unsigned)((slots + 127) / 128), 128, 0, s>>>(nseg, slots, a, b, in);
-                if (down)
-                    sweep_y4i_kernel<true, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
-                else
-                    sweep_y4i_kernel<false, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
-                return 3;
-            } else if (down) {
-                sweep_y4i_kernel<true, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
-            } else {
-                sweep_y4i_kernel<false, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
-            }
+        if constexpr (DT == DT_I32) {
+            if (down)
+                sweep_y4i_kernel<true><<<(unsigned)strips, 32, 0, s>>>(d);
+            else
+                sweep_y4i_kernel<false><<<(unsigned)strips, 32, 0, s>>>(d);
         } else {
-            constexpr int NDT = DT == DT_I32 ? DT_U8 : DT;  // (never i32 here)
-            const unsigned nblocks = (unsigned)(((long long)d.W * P::BPP + 63) / 64);
+            const unsigned nblocks = (unsigned)((long long)d.W * P::BPP / 64);
             if (scratch && sweep_scratch_bytes(d) > 0) {
                 // segments: aggregate, chain, sweep
                 const int nseg = (d.H + kSegRows - 1) / kSegRows;
@@ -1140,19 +1049,19 @@ static int launch_sweep_t(const ImgDesc& d, int direction, cudaStream_t s, void*
                 uint32_t* in = b + (size_t)nseg * slots;
                 const dim3 grid(nblocks, (unsigned)nseg);
                 if (down)
-                    sweep_y4n_kernel<NDT, true, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
+                    sweep_y4n_kernel<DT, true, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
                 else
-                    sweep_y4n_kernel<NDT, false, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
-                sweep_y_carry_kernel<NDT><<<(unsigned)((slots + 127) / 128), 128, 0, s>>>(nseg, slots, a, b, in);
+                    sweep_y4n_kernel<DT, false, 1><<<grid, 32, 0, s>>>(d, a, b, nullptr);
+                sweep_y_carry_kernel<DT><<<(unsigned)((slots + 127) / 128), 128, 0, s>>>(nseg, slots, a, b, in);
                 if (down)
-                    sweep_y4n_kernel<NDT, true, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
+                    sweep_y4n_kernel<DT, true, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
                 else
-                    sweep_y4n_kernel<NDT, false, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
+                    sweep_y4n_kernel<DT, false, 2><<<grid, 32, 0, s>>>(d, nullptr, nullptr, in);
                 return 3;
             } else if (down) {
-                sweep_y4n_kernel<NDT, true, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
+                sweep_y4n_kernel<DT, true, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
             } else {
-                sweep_y4n_kernel<NDT, false, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
+                sweep_y4n_kernel<DT, false, 0><<<nblocks, 32, 0, s>>>(d, nullptr, nullptr, nullptr);
             }
         }
         return 1;
