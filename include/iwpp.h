@@ -201,7 +201,7 @@ IWPP_API int iwpp_queue_selftest(int device, int variant, int grid_side, int cop
  * initial passes are compile-time constants, IWPP MP/include/
  * MorphologicalReconstruction.cuh:6-7, and commented-out sweeps, MR.cu:792-795).
  * Times candidate configurations on the caller's own batch -- the untuned
- * default for large images, tile rows 64 / 32 x in-tile solver, the best of
+ * default for large images, tile rows 64 / 32 x passes / row sweeps, the best of
  * those started from a seed check, the front stage with 0 / 1 / 2 / 3 / 4 / 8
  * whole-image passes, then (if it lost) 1, 2, 4, ... 64 initial raster +
  * anti-raster passes while each doubling is faster, then (mutex / double

@@ -1358,7 +1358,7 @@ int iwpp_autotune(iwpp_handle h, const iwpp_image* images, int n, int variant, i
             consider(c, true);
         }
         for (int th : {64, 32})
-            for (int solver : {0, 1, 2}) {
+            for (int solver : {0, 1}) {  // (2 is the kernel of 0)
                 iwpp_config c{};
                 c.tile_rows = th;
                 c.solver = solver;
