@@ -14,6 +14,8 @@
 //            previous row inside a 128-byte strip, segments of rows first on
 //            their own, then their entries.  The result is the walk's, row
 //            by row, whatever the order.
+#include <algorithm>
+
 #include "iwpp_engine.cuh"
 
 namespace iwpp {
@@ -64,37 +66,49 @@ __global__ void clip_kernel(ImgDesc d) {
 }
 
 // ---------------------------------------------------------------- staging
-// Copies the rows of up to 64 images at once (grid.y), a warp per row in
-// turn.  The row is written as the aligned words inside it, each put together
-// from the two aligned source words around it, and single bytes at the ends
-// (at most three each), so that a row of any alignment costs what an aligned
-// one does.  Bound by DRAM / L2 traffic: read and write each byte once.
+// Copies the rows of up to 64 images at once (grid.y), a warp per piece of a
+// row in turn.  The row is written as the aligned words inside it, each put
+// together from the two aligned source words around it, and single bytes at
+// the ends (at most three each), so that a row of any alignment costs what an
+// aligned one does.  Bound by DRAM / L2 / link traffic: read and write each byte
+// once.  Pieces, since a warp per row left a short wide image to a few warps,
+// each with a few hundred bytes in flight (a clip of one row of 20
+// million bytes 81 ms, 0.35 so).
 struct StageList {
     StageCopy c[64];
 };
+constexpr int kStageWords = 256;  // words of a piece
 
-__global__ void __launch_bounds__(256) stage_copy_kernel(const __grid_constant__ StageList list) {
-    const StageCopy& c = list.c[blockIdx.y];
-    const int lane = threadIdx.x & 31;
+// Pieces of a row of `bytes` bytes, whatever its alignment.
+__host__ __device__ static long long stage_pieces(long long bytes) {
+    return bytes <= 4ll * kStageWords ? 1 : (bytes / 4 + kStageWords - 1) / kStageWords;
+}
+
+// PIECES: rows of more than one.
+template <bool PIECES>
+__device__ __forceinline__ void stage_copy(const StageCopy& c, int lane, long long pieces) {
     const long long nwarps = (long long)gridDim.x * (blockDim.x >> 5);
-    for (long long y = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); y < c.rows; y += nwarps) {
+    for (long long u = blockIdx.x * (long long)(blockDim.x >> 5) + (threadIdx.x >> 5); u < c.rows * pieces;
+         u += nwarps) {
+        const long long y = PIECES ? u / pieces : u, piece = PIECES ? u - y * pieces : 0;
         const unsigned char* src = static_cast<const unsigned char*>(c.src) + y * c.src_pitch;
         unsigned char* dst = static_cast<unsigned char*>(c.dst) + y * c.dst_pitch;
         const long long n = c.row_bytes;
         const long long lead = min((long long)((0u - (unsigned)reinterpret_cast<size_t>(dst)) & 3u), n);
         const long long words = (n - lead) >> 2, tail = lead + 4 * words;
+        const long long end = PIECES ? min(words, (piece + 1) * kStageWords) : words;
         const unsigned char* from = src + lead;  // source of the first aligned word of dst
         const unsigned sh = (unsigned)reinterpret_cast<size_t>(from) & 3u;
         const unsigned* ws = reinterpret_cast<const unsigned*>(from - sh);
         unsigned* wd = reinterpret_cast<unsigned*>(dst + lead);
         if (sh == 0u) {
 #pragma unroll 4
-            for (long long i = lane; i < words; i += 32) wd[i] = ws[i];
+            for (long long i = piece * kStageWords + lane; i < end; i += 32) wd[i] = ws[i];
         } else {
             // the source words around the row's first and last bytes hold
             // bytes of other rows or of nothing: those words byte by byte
 #pragma unroll 4
-            for (long long i = lane; i < words; i += 32) {
+            for (long long i = piece * kStageWords + lane; i < end; i += 32) {
                 unsigned w;
                 if (i > 0 && i + 1 < words) {
                     w = __funnelshift_r(ws[i], ws[i + 1], 8 * sh);
@@ -105,23 +119,34 @@ __global__ void __launch_bounds__(256) stage_copy_kernel(const __grid_constant__
                 wd[i] = w;
             }
         }
+        if (PIECES && piece != 0) continue;
         if (lane < 3 && lane < lead) dst[lane] = src[lane];
         if (lane >= 4 && tail + lane - 4 < n) dst[tail + lane - 4] = src[tail + lane - 4];
     }
+}
+
+__global__ void __launch_bounds__(256) stage_copy_kernel(const __grid_constant__ StageList list) {
+    const StageCopy& c = list.c[blockIdx.y];
+    const int lane = threadIdx.x & 31;
+    const long long pieces = stage_pieces(c.row_bytes);
+    if (pieces == 1)
+        stage_copy<false>(c, lane, 1);
+    else
+        stage_copy<true>(c, lane, pieces);
 }
 
 cudaError_t launch_stage_copies(const std::vector<StageCopy>& copies, cudaStream_t s, int* launches) {
     for (size_t i = 0; i < copies.size(); i += 64) {
         StageList list{};
         const size_t n = copies.size() - i < 64 ? copies.size() - i : 64;
-        long long rows = 1;
+        long long units = 1;
         for (size_t j = 0; j < n; ++j) {
             list.c[j] = copies[i + j];
-            rows = rows < copies[i + j].rows ? copies[i + j].rows : rows;
+            units = std::max(units, copies[i + j].rows * stage_pieces(copies[i + j].row_bytes));
         }
-        // eight rows per block at most in flight; four waves of blocks share
-        // the longest image
-        const long long want = (rows + 7) / 8, most = 152 * 32 / (long long)n + 1;
+        // eight pieces per block; at most four waves of blocks, which share the
+        // largest image
+        const long long want = (units + 7) / 8, most = 152 * 32 / (long long)n + 1;
         stage_copy_kernel<<<dim3((unsigned)(want < most ? want : most), (unsigned)n), 256, 0, s>>>(list);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
