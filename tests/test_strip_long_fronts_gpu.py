@@ -13,7 +13,7 @@ NP = {0: np.uint8, 1: np.uint16, 2: np.int32}
 
 
 @pytest.mark.parametrize("dt", [0, 1, 2])
-@pytest.mark.parametrize("h", [385, 512, 777, 1289])
+@pytest.mark.parametrize("h", [385, 512, 777, 1289, 4224, 4225, 8321])
 @pytest.mark.parametrize("extra", [0, 1, 2, 3])
 def test_one_front_down_the_whole_height(dt, h, extra):
     import torch
