@@ -124,6 +124,7 @@ struct EngineArgs {
 
 // Host-side entry points implemented in iwpp_engine.cu.
 namespace iwpp {
+constexpr int kSms = 152;  // a GB300's multiprocessors, for grids that only need to be about right
 // The caller's status of a job whose counters hold this error word (DEV_*).
 inline int status_of_job(unsigned error) {
     switch (error) {

@@ -146,7 +146,7 @@ cudaError_t launch_stage_copies(const std::vector<StageCopy>& copies, cudaStream
         }
         // eight pieces per block; at most four waves of blocks, which share the
         // largest image
-        const long long want = (units + 7) / 8, most = 152 * 32 / (long long)n + 1;
+        const long long want = (units + 7) / 8, most = kSms * 32 / (long long)n + 1;
         stage_copy_kernel<<<dim3((unsigned)(want < most ? want : most), (unsigned)n), 256, 0, s>>>(list);
         const cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
@@ -800,8 +800,8 @@ constexpr int kRingN = 64;  // rows in flight per plane in the narrow variant
 // either connectivity: the pixel above / below alone is a valid update), rows
 // of whole strips on 16-byte boundaries (by_strips takes the others).
 //
-// uint8 / uint16: a warp covers a 64-byte strip, two bytes per lane (uint8: two pixels as one u16x2 register; uint16: one
-// pixel), so the chain per row is one min and one max, and twice as many
+// uint8 / uint16: a warp covers a 64-byte strip, two bytes per lane (uint8: two
+// pixels as one u16x2 register; uint16: one pixel), so the chain per row is one min and one max, and twice as many
 // warps share the image.
 //
 // Tall images are cut into segments of kSegRows rows so that more warps
@@ -1013,7 +1013,7 @@ static unsigned blocks_for(long long threads, int block) {
 cudaError_t launch_fixed_point_check(const ImgDesc& d, unsigned long long* count, cudaStream_t s) {
     if (d.W == 0 || d.H == 0) return cudaSuccess;
     unsigned blocks = blocks_for((long long)d.W * d.H, 256);
-    if (blocks > 152u * 16u) blocks = 152u * 16u;
+    if (blocks > kSms * 16u) blocks = kSms * 16u;
     if (d.dtype == DT_U8)
         fixed_point_kernel<DT_U8><<<blocks, 256, 0, s>>>(d, count);
     else if (d.dtype == DT_U16)
@@ -1028,7 +1028,7 @@ cudaError_t launch_clip(const ImgDesc& d, cudaStream_t s) {
     const int ppw = d.dtype == DT_U8 ? 4 : d.dtype == DT_U16 ? 2 : 1;
     const long long words = (long long)((d.W + ppw - 1) / ppw) * d.H;
     unsigned blocks = blocks_for(words, 256);
-    if (blocks > 152u * 16u) blocks = 152u * 16u;
+    if (blocks > kSms * 16u) blocks = kSms * 16u;
     if (d.dtype == DT_U8)
         clip_kernel<DT_U8><<<blocks, 256, 0, s>>>(d);
     else if (d.dtype == DT_U16)

@@ -1037,7 +1037,7 @@ cudaError_t launch_seed_batch(const ImgDesc* dev_descs, const std::vector<ImgDes
     }
     if (units == 0) return cudaSuccess;
     long long blocks = (units * 32 + kSeedThreads - 1) / kSeedThreads;
-    if (blocks > 152ll * 64) blocks = 152ll * 64;
+    if (blocks > kSms * 64ll) blocks = kSms * 64ll;
     seed_batch_kernel<kSeedWords><<<(unsigned)blocks, kSeedThreads, 0, s>>>(dev_descs, nimg, gate, state, list, nlist);
     if (launches) ++*launches;
     return cudaGetLastError();
@@ -1056,7 +1056,7 @@ cudaError_t launch_seed(const ImgDesc& d, unsigned* state, unsigned* list, unsig
     constexpr int WPL = kSeedWords;
     const long long units = (long long)((d.tiles_x + WPL - 1) / WPL) * d.tiles_y;
     long long blocks = (units * 32 + kSeedThreads - 1) / kSeedThreads;
-    if (blocks > 152ll * 64) blocks = 152ll * 64;
+    if (blocks > kSms * 64ll) blocks = kSms * 64ll;
     if (blocks < 1) blocks = 1;
     if (d.dtype == DT_U8)
         seed_wide_kernel<DT_U8, WPL><<<(unsigned)blocks, kSeedThreads, 0, s>>>(d, state, list, nlist);
