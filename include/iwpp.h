@@ -141,7 +141,9 @@ typedef struct iwpp_plan_s *iwpp_plan;
 IWPP_API const char *iwpp_status_string(int status);
 IWPP_API int iwpp_version(void);
 /* Workspace owner (queues, tile states, counters) bound to one device.
- * Calls that share a handle must be ordered on one stream. */
+ * Calls that share a handle must be ordered on one stream.  It keeps what its
+ * calls needed until it is destroyed: the workspace, and up to 256 MB of the
+ * staging buffers of images whose rows do not start on 4-byte boundaries. */
 IWPP_API int iwpp_handle_create(iwpp_handle *out, int device);
 IWPP_API int iwpp_handle_destroy(iwpp_handle h);
 /* Bytes of device workspace a job of `tiles` tiles needs. */

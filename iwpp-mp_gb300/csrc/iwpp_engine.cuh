@@ -1,4 +1,4 @@
-// iwpp_engine.cuh -- the persistent tile engine and its three work queues.
+// iwpp_engine.cuh -- the persistent tile engine and its four work queues.
 //
 // Reference counterparts:
 //   MUTEX  IWPP MP/src/globalQueue.cu:25-81 (insert under a spin mutex),
@@ -18,7 +18,8 @@
 // of a host round trip, the unique queue de-duplicates when a tile is
 // inserted, and all insertions are warp-aggregated (one atomic per warp).
 //
-// A CTA works on one tile at a time; its first warp runs the queue.
+// A CTA works on one tile at a time; its first warp runs the queue.  (With the
+// in-tile solvers of one warp per tile, four workers each do both.)
 //
 // Tile ownership.  Each tile has a state word: DIRTY (needs a visit) and
 // ACTIVE (a CTA is visiting it).  A CTA takes a tile by one exchange that sets
